@@ -773,7 +773,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                      cu_seqlens.data_ptr<int>(),
                                      state_idx.has_value() ? state_idx->data_ptr<int>() : nullptr,
                                      has_init.has_value() ? has_init->data_ptr<int>() : nullptr,
-                                     cu_seqlens.numel() - 1, x.size(1), w.size(1), x.stride(0), y.stride(0),
+                                     cu_seqlens.numel() - 1, x.size(0), x.size(1), w.size(1), x.stride(0), y.stride(0),
                                      silu ? 1 : 0, cur_stream()),
              "causal_conv1d_varlen");
   });
@@ -784,11 +784,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                     const c10::optional<Tensor>& state_idx, const c10::optional<Tensor>& has_init,
                                     bool dt_softplus) {
     need_cuda(u, "u");
-    TORCH_CHECK(u.is_contiguous() && delta.is_contiguous() && y.is_contiguous() && B.is_contiguous() &&
-                    C.is_contiguous() && A.is_contiguous() && A.scalar_type() == at::kFloat &&
+    TORCH_CHECK(u.is_contiguous() && delta.is_contiguous() && y.is_contiguous() && B.dim() == 2 && B.stride(1) == 1 &&
+                    C.dim() == 2 && C.stride(1) == 1 && A.is_contiguous() && A.scalar_type() == at::kFloat &&
                     u.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16,
-                "selective_scan: contiguous bf16 u/delta/B/C, fp32 A");
-    TORCH_CHECK(!z.has_value() || z->is_contiguous(), "selective_scan: z contiguous");
+                "selective_scan: contiguous bf16 u/delta, bf16 B/C of contiguous rows, fp32 A");
+    TORCH_CHECK(!z.has_value() || (z->dim() == 2 && z->stride(1) == 1), "selective_scan: rows of z contiguous");
     check_rc(mb_selective_scan_varlen(u.data_ptr(), delta.data_ptr(), A.data_ptr<float>(), B.data_ptr(),
                                       C.data_ptr(), D.has_value() ? D->data_ptr<float>() : nullptr, optptr(z),
                                       dt_bias.has_value() ? dt_bias->data_ptr<float>() : nullptr, y.data_ptr(),
@@ -796,8 +796,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                       cu_seqlens.data_ptr<int>(),
                                       state_idx.has_value() ? state_idx->data_ptr<int>() : nullptr,
                                       has_init.has_value() ? has_init->data_ptr<int>() : nullptr,
-                                      cu_seqlens.numel() - 1, u.size(1), A.size(1), u.size(1), B.size(1),
-                                      dt_softplus ? 1 : 0, cur_stream()),
+                                      cu_seqlens.numel() - 1, u.size(1), A.size(1), u.size(1),
+                                      z.has_value() ? z->stride(0) : 0, B.stride(0), C.stride(0), dt_softplus ? 1 : 0, cur_stream()),
              "selective_scan_varlen");
   });
   m.def("ssd_scan_varlen", [](const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C,
@@ -806,10 +806,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                               const c10::optional<Tensor>& state_idx, const c10::optional<Tensor>& has_init,
                               bool dt_softplus) {
     need_cuda(x, "x");
-    TORCH_CHECK(x.dim() == 3 && x.is_contiguous() && dt.is_contiguous() && B.dim() == 3 && B.is_contiguous() &&
-                    C.is_contiguous() && y.is_contiguous() && A.scalar_type() == at::kFloat &&
-                    x.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16,
-                "ssd_scan: x [T, H, P], dt [T, H], B/C [T, G, N] contiguous bf16, A fp32 [H]");
+    auto rows = [](const Tensor& t) { return t.dim() == 3 && t.stride(2) == 1 && t.stride(1) == t.size(2); };
+    TORCH_CHECK(rows(x) && dt.dim() == 2 && dt.stride(1) == 1 && rows(B) && rows(C) && y.is_contiguous() &&
+                    A.scalar_type() == at::kFloat && x.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16,
+                "ssd_scan: x [T, H, P], dt [T, H], B/C [T, G, N] bf16 of contiguous rows, A fp32 [H]");
     check_rc(mb_ssd_scan_varlen(x.data_ptr(), dt.data_ptr(), A.data_ptr<float>(), B.data_ptr(), C.data_ptr(),
                                 D.has_value() ? D->data_ptr<float>() : nullptr,
                                 dt_bias.has_value() ? dt_bias->data_ptr<float>() : nullptr, y.data_ptr(),
@@ -817,9 +817,20 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                 cu_seqlens.data_ptr<int>(),
                                 state_idx.has_value() ? state_idx->data_ptr<int>() : nullptr,
                                 has_init.has_value() ? has_init->data_ptr<int>() : nullptr,
-                                cu_seqlens.numel() - 1, x.size(1), x.size(2), B.size(2), B.size(1),
-                                dt_softplus ? 1 : 0, cur_stream()),
+                                cu_seqlens.numel() - 1, x.size(0), x.size(1), x.size(2), B.size(2), B.size(1),
+                                x.stride(0), dt.stride(0), B.stride(0), C.stride(0), dt_softplus ? 1 : 0, cur_stream()),
              "ssd_scan_varlen");
+  });
+  m.def("gated_rms_norm", [](const Tensor& y, const Tensor& z, const Tensor& w, Tensor& out, double eps) {
+    need_cuda(y, "y");
+    TORCH_CHECK(y.dim() == 2 && y.is_contiguous() && out.is_contiguous() && z.dim() == 2 && z.stride(1) == 1 && w.is_contiguous() &&
+                    y.scalar_type() == at::kBFloat16 && z.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
+                    out.scalar_type() == at::kBFloat16 && z.size(0) == y.size(0) && z.size(1) == y.size(1) && w.numel() == y.size(1) &&
+                    out.sizes() == y.sizes(),
+                "gated_rms_norm: y, out [T, D] contiguous, z [T, D] of contiguous rows, w [D], all bf16");
+    check_rc(mb_gated_rms_norm(y.data_ptr(), z.data_ptr(), w.data_ptr(), out.data_ptr(), y.size(0), y.size(1), z.stride(0),
+                               static_cast<float>(eps), cur_stream()),
+             "gated_rms_norm");
   });
   // grouped block-scaled fp8 GEMM: xq [rows, K] e4m3 (tokens in expert order), xs fp32 [ceil(K/128), rows],
   // wq [E, N, K] e4m3, ws fp32 [E, N/128, ceil(K/128)], offsets int32 [E + 1]

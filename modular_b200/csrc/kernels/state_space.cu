@@ -1,14 +1,15 @@
 // State-space layer kernels for ragged (variable-length) batches: causal depthwise conv1d,
 // the Mamba-1 selective scan and the Mamba-2 SSD recurrence, each carrying per-sequence state so the
-// same kernel serves prefill chunks and single-token decode.
+// same entry serves prefill chunks and single-token decode, and the gated norm of a Mamba-2 block.
 //
 // Sequences are rows [cu_seqlens[s], cu_seqlens[s+1]) of the token-major inputs. State tensors are
 // indexed by `state_idx[s]` (a slot per live request; -1 = no state: start from zero, write nothing),
 // are read when `has_init[s]` is non-zero and always written back.
 //
-// These are the time-sequential forms: one thread (or one thread per state column) walks a sequence
-// and keeps the recurrent state in registers. They are bandwidth-bound for decode and for short
-// chunks; a chunked (matmul-form) SSD prefill is not built.
+//   causal_conv1d_kernel    all tokens at once, 4 channels per thread
+//   selective_scan_kernel   walks the tokens; a tile of them is staged in shared memory ahead of its use
+//   ssd_scan_kernel         walks the tokens, fp32 state in registers: decode steps, short prompts, odd sizes
+//   ssd_chunk_kernel        prompts, 64 tokens at a time on the tensor cores
 //
 // Reference counterparts: max/kernels/src/state_space/causal_conv1d.mojo (varlen fwd + update),
 // selective_scan.mojo (selective_scan_fwd / _update) and the Mamba-2 SSD kernels of the same package,
@@ -18,6 +19,7 @@
 #include <stdint.h>
 
 #include "../common/api.h"
+#include "../common/launch.h"
 
 namespace mb {
 namespace ssm {
@@ -25,97 +27,285 @@ namespace ssm {
 __device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
 __device__ __forceinline__ float softplus(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
 
-// y[t, d] = act(bias[d] + sum_k w[d, k] * x[t - (W-1) + k, d]); tokens before the sequence start come
-// from conv_state[slot, d, :] (the last W-1 inputs of the previous chunk). One thread per channel walks
-// the sequence with a sliding window in registers. W <= 8.
-template <int W>
-__global__ void causal_conv1d_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                                     const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ y,
-                                     float* __restrict__ conv_state, const int* __restrict__ cu_seqlens,
-                                     const int* __restrict__ state_idx, const int* __restrict__ has_init,
-                                     int D, int ldx, int ldy, int act) {
-  const int s = blockIdx.y;
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= D) return;
-  const int t0 = cu_seqlens[s], t1 = cu_seqlens[s + 1];
-  const int slot = state_idx ? state_idx[s] : -1;
-  float win[W];
-  float wk[W];
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+constexpr float kLog2e = 1.4426950408889634f;
+
+template <int VEC>
+__device__ __forceinline__ void load_bf16(float (&v)[VEC], const __nv_bfloat16* p) {
+  if constexpr (VEC == 8) {
+    const uint4 r = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
-  for (int k = 0; k < W; ++k) wk[k] = __bfloat162float(w[d * W + k]);
-#pragma unroll
-  for (int k = 0; k < W - 1; ++k)
-    win[k + 1] = (slot >= 0 && has_init && has_init[s]) ? conv_state[(static_cast<size_t>(slot) * D + d) * (W - 1) + k]
-                                                        : 0.f;
-  const float b = bias ? __bfloat162float(bias[d]) : 0.f;
-  for (int t = t0; t < t1; ++t) {
-#pragma unroll
-    for (int k = 0; k < W - 1; ++k) win[k] = win[k + 1];
-    win[W - 1] = __bfloat162float(x[static_cast<size_t>(t) * ldx + d]);
-    float acc = b;
-#pragma unroll
-    for (int k = 0; k < W; ++k) acc = fmaf(wk[k], win[k], acc);
-    if (act) acc = silu(acc);
-    y[static_cast<size_t>(t) * ldy + d] = __float2bfloat16(acc);
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = __uint_as_float(w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+  } else if constexpr (VEC == 4) {
+    const uint2 r = *reinterpret_cast<const uint2*>(p);
+    v[0] = __uint_as_float(r.x << 16); v[1] = __uint_as_float(r.x & 0xffff0000u);
+    v[2] = __uint_as_float(r.y << 16); v[3] = __uint_as_float(r.y & 0xffff0000u);
+  } else {
+    v[0] = __bfloat162float(*p);
   }
-  if (slot >= 0) {
+}
+template <int VEC>
+__device__ __forceinline__ void store_bf16(__nv_bfloat16* p, const float (&v)[VEC]) {
+  if constexpr (VEC >= 4) {
+    uint32_t w[VEC / 2];
+#pragma unroll
+    for (int i = 0; i < VEC / 2; ++i) {
+      const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    if constexpr (VEC == 8) *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+    else *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
+  } else {
+    *p = __float2bfloat16(v[0]);
+  }
+}
+
+// y[t, d] = act(bias[d] + sum_k w[d, k] * x[t - (W-1) + k, d]); tokens before the sequence start come
+// from conv_state[slot, d, :] (the last W-1 inputs of the previous chunk). W <= 8.
+// Bound by memory: x is read and y written once (and W - 1 rows per tile again, from L2). A thread owns VEC
+// channels and the tokens of one tile, so all tiles run at once; blocks whose row is below n_seqs take the
+// sequences' first W - 1 tokens instead, the only ones that need the state, and the same thread that reads
+// the state writes the new one (one reader, one writer, in order).
+// 4099 tokens x 4096 channels, width 4: 1104 us with one thread per channel walking a sequence, 30 us so.
+constexpr int kConvTile = 16;
+template <int W, int VEC>
+__global__ void __launch_bounds__(128) causal_conv1d_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                     const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ y,
+                                     float* conv_state, const int* __restrict__ cu_seqlens,
+                                     const int* __restrict__ state_idx, const int* __restrict__ has_init,
+                                     int n_seqs, int D, int ldx, int ldy, int act) {
+  const int d = (blockIdx.y * blockDim.x + threadIdx.x) * VEC, row = blockIdx.x;
+  if (d >= D) return;
+  float wk[W][VEC], b[VEC], win[W][VEC];
+#pragma unroll
+  for (int c = 0; c < VEC; ++c) b[c] = 0.f;
+  if (bias) load_bf16<VEC>(b, bias + d);
+#pragma unroll
+  for (int i = 0; i < W; ++i) {                    // the weights of VEC channels are one run of VEC * W values
+    float v[VEC];
+    load_bf16<VEC>(v, w + static_cast<size_t>(d) * W + i * VEC);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) wk[(i * VEC + e) % W][(i * VEC + e) / W] = v[e];
+  }
+  // one token: win[W - 1] holds its input, win[0 ..] those before it
+  auto emit = [&](int t) {
+    float acc[VEC];
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) {
+      acc[c] = b[c];
+#pragma unroll
+      for (int k = 0; k < W; ++k) acc[c] = fmaf(wk[k][c], win[k][c], acc[c]);
+      if (act) acc[c] = silu(acc[c]);
+    }
+    store_bf16<VEC>(y + static_cast<size_t>(t) * ldy + d, acc);
+  };
+  auto shift = [&]() {
 #pragma unroll
     for (int k = 0; k < W - 1; ++k)
-      conv_state[(static_cast<size_t>(slot) * D + d) * (W - 1) + k] = win[k + 1];
+#pragma unroll
+      for (int c = 0; c < VEC; ++c) win[k][c] = win[k + 1][c];
+  };
+  if (row < n_seqs) {
+    const int s = row, t0 = cu_seqlens[s], t1 = cu_seqlens[s + 1];
+    const int slot = state_idx && conv_state ? state_idx[s] : -1;
+    float* st = conv_state + static_cast<size_t>(slot >= 0 ? slot : 0) * D * (W - 1) + static_cast<size_t>(d) * (W - 1);
+    const bool resume = slot >= 0 && has_init && has_init[s];
+#pragma unroll
+    for (int k = 0; k < W - 1; ++k)
+#pragma unroll
+      for (int c = 0; c < VEC; ++c) win[k + 1][c] = resume ? st[c * (W - 1) + k] : 0.f;
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) win[0][c] = 0.f;
+    const int head = min(t1, t0 + W - 1);
+    for (int t = t0; t < head; ++t) {
+      shift();
+      load_bf16<VEC>(win[W - 1], x + static_cast<size_t>(t) * ldx + d);
+      emit(t);
+    }
+    if (slot < 0) return;
+    if (t1 > head) {                               // the last W - 1 inputs, all of this step
+#pragma unroll
+      for (int k = 1; k < W; ++k) load_bf16<VEC>(win[k], x + static_cast<size_t>(t1 - W + k) * ldx + d);
+    }
+#pragma unroll
+    for (int k = 0; k < W - 1; ++k)
+#pragma unroll
+      for (int c = 0; c < VEC; ++c) st[c * (W - 1) + k] = win[k + 1][c];
+    return;
+  }
+  const int lo = (row - n_seqs) * kConvTile, hi = lo + kConvTile;
+  int a = 0, z = n_seqs;                           // the first sequence that ends beyond lo
+  while (a < z) {
+    const int m = (a + z) >> 1;
+    if (cu_seqlens[m + 1] > lo) z = m; else a = m + 1;
+  }
+  for (int s = a; s < n_seqs; ++s) {
+    const int t0 = cu_seqlens[s];
+    if (t0 >= hi) break;
+    const int first = max(lo, t0 + W - 1), last = min(hi, cu_seqlens[s + 1]);
+    if (first >= last) continue;
+#pragma unroll
+    for (int k = 1; k < W; ++k) load_bf16<VEC>(win[k], x + static_cast<size_t>(first - W + k) * ldx + d);
+#pragma unroll 4
+    for (int t = first; t < last; ++t) {
+      shift();
+      load_bf16<VEC>(win[W - 1], x + static_cast<size_t>(t) * ldx + d);
+      emit(t);
+    }
   }
 }
 
 // Mamba-1 selective scan. Per channel d and state n:
 //   dt = softplus(delta[t, d] + dt_bias[d]);  h = exp(dt * A[d, n]) * h + dt * B[t, n] * u[t, d]
 //   y[t, d] = sum_n C[t, n] * h + Dskip[d] * u[t, d];   y *= silu(z[t, d]) when z is given
-// One thread per channel, N (<= 32, compile-time) states in registers; B_t / C_t rows are staged in
-// shared memory once per time step for the whole block.
+// The recurrence needs one exponential per state and token (all fp32): 268 M of them for 4099 tokens x 4096
+// channels x 16 states are 60 us of the special-function units, which is the floor for prompts that fill the chip.
+// Eight lanes share a channel (N / 8 states each, in registers), so that a few long sequences still give every SM
+// several warps (with four lanes the longest of three sequences had 1.8 per scheduler and took 285 us); a CTA walks one sequence for 32 channels. Inputs arrive kScanTile tokens at a time through cp.async,
+// one tile ahead; step sizes (softplus) are made once per token and channel by all threads before the walk, and
+// the lanes' partial outputs of eight tokens meet in seven shuffles. Rows that are not 16-byte aligned are fetched
+// with plain loads, into the same tiles.
+// That prompt (three sequences): 3475 us with one thread per channel and two barriers per token, 233 us so.
+constexpr int kScanTile = 32, kScanCh = 32, kScanThreads = 256;
 template <int N>
-__global__ void selective_scan_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16* __restrict__ delta,
+__global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16* __restrict__ delta,
                                       const float* __restrict__ A, const __nv_bfloat16* __restrict__ B,
                                       const __nv_bfloat16* __restrict__ C, const float* __restrict__ Dskip,
                                       const __nv_bfloat16* __restrict__ z, const float* __restrict__ dt_bias,
                                       __nv_bfloat16* __restrict__ y, float* __restrict__ ssm_state,
                                       const int* __restrict__ cu_seqlens, const int* __restrict__ state_idx,
-                                      const int* __restrict__ has_init, int D, int ld_u, int ld_bc,
-                                      int dt_softplus) {
-  __shared__ float sB[N], sC[N];
-  const int s = blockIdx.y;
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = d < D;
-  const int t0 = cu_seqlens[s], t1 = cu_seqlens[s + 1];
-  const int slot = state_idx ? state_idx[s] : -1;
-  float h[N], a[N];
+                                      const int* __restrict__ has_init, int D, int ld_u, int ld_z, int ld_b, int ld_c,
+                                      int dt_softplus, int vec) {
+  constexpr int NS = N / 8, TT = kScanTile, CH = kScanCh;
+  struct Stage { __nv_bfloat16 u[TT][CH], dl[TT][CH], z[TT][CH], B[TT][N], C[TT][N]; };
+  __shared__ __align__(16) Stage stages[2];
+  __shared__ __align__(16) float sB[TT][N], sC[TT][N];
+  __shared__ float2 sdt[TT][CH];                     // step size, step size * input
+  __shared__ __align__(16) __nv_bfloat16 sy[TT][CH];
+  const int s = blockIdx.y, tid = threadIdx.x, lane = tid & 31, q = lane & 7, c = (tid >> 5) * 4 + (lane >> 3);
+  const int d0 = blockIdx.x * CH, d = d0 + c;
+  const int t0 = cu_seqlens[s], n = cu_seqlens[s + 1] - t0;
+  const int slot = state_idx && ssm_state ? state_idx[s] : -1;
+  const bool live = d < D, resume = live && slot >= 0 && has_init && has_init[s];
+  float h[NS], a2[NS];
+  float* st = ssm_state + (static_cast<size_t>(slot >= 0 ? slot : 0) * D + (live ? d : 0)) * N + q * NS;
 #pragma unroll
-  for (int n = 0; n < N; ++n) {
-    a[n] = live ? A[static_cast<size_t>(d) * N + n] : 0.f;
-    h[n] = (live && slot >= 0 && has_init && has_init[s]) ? ssm_state[(static_cast<size_t>(slot) * D + d) * N + n] : 0.f;
+  for (int i = 0; i < NS; ++i) {
+    a2[i] = live ? A[static_cast<size_t>(d) * N + q * NS + i] * kLog2e : 0.f;
+    h[i] = resume ? st[i] : 0.f;
   }
   const float dsk = (live && Dskip) ? Dskip[d] : 0.f;
-  const float dtb = (live && dt_bias) ? dt_bias[d] : 0.f;
-  for (int t = t0; t < t1; ++t) {
-    __syncthreads();
-    if (threadIdx.x < N) {
-      sB[threadIdx.x] = __bfloat162float(B[static_cast<size_t>(t) * ld_bc + threadIdx.x]);
-      sC[threadIdx.x] = __bfloat162float(C[static_cast<size_t>(t) * ld_bc + threadIdx.x]);
+  auto fetch = [&](int c0, Stage& g) {
+    if (vec) {
+      const int j = (tid >> 2) & 31, k = (tid & 3) * 8;      // the first half of the threads fetches u and z, the other delta
+      const bool ok = c0 + j < n && d0 + k < D;
+      const size_t row = static_cast<size_t>(t0 + (c0 + j < n ? c0 + j : 0)), col = d0 + k < D ? d0 + k : 0;
+      if (tid < 128) {
+        cp_async16(&g.u[j][k], u + row * ld_u + col, ok);
+        if (z) cp_async16(&g.z[j][k], z + row * ld_z + col, ok);
+      } else {
+        cp_async16(&g.dl[j][k], delta + row * ld_u + col, ok);
+      }
+      for (int i = kScanThreads - 1 - tid; i < TT * (N / 8); i += kScanThreads) {
+        const int jj = i / (N / 8), kk = (i % (N / 8)) * 8;
+        const bool in = c0 + jj < n;
+        const size_t r = static_cast<size_t>(t0 + (in ? c0 + jj : 0));
+        cp_async16(&g.B[jj][kk], B + r * ld_b + kk, in);
+        cp_async16(&g.C[jj][kk], C + r * ld_c + kk, in);
+      }
+    } else {
+      const __nv_bfloat16 zero = __float2bfloat16(0.f);
+      for (int i = tid; i < TT * CH; i += kScanThreads) {
+        const int j = i / CH, k = i % CH;
+        const bool ok = c0 + j < n && d0 + k < D;
+        const size_t row = static_cast<size_t>(t0 + c0 + j);
+        g.u[j][k] = ok ? u[row * ld_u + d0 + k] : zero;
+        g.dl[j][k] = ok ? delta[row * ld_u + d0 + k] : zero;
+        if (z) g.z[j][k] = ok ? z[row * ld_z + d0 + k] : zero;
+      }
+      for (int i = tid; i < TT * N; i += kScanThreads) {
+        const int j = i / N, k = i % N;
+        const bool ok = c0 + j < n;
+        const size_t row = static_cast<size_t>(t0 + c0 + j);
+        g.B[j][k] = ok ? B[row * ld_b + k] : zero;
+        g.C[j][k] = ok ? C[row * ld_c + k] : zero;
+      }
     }
-    __syncthreads();
-    if (!live) continue;
-    const float ut = __bfloat162float(u[static_cast<size_t>(t) * ld_u + d]);
-    float dt = __bfloat162float(delta[static_cast<size_t>(t) * ld_u + d]) + dtb;
-    if (dt_softplus) dt = softplus(dt);
-    float acc = dsk * ut;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int pc = tid & 31;                           // the channel whose step sizes this thread makes
+  const float pb = (d0 + pc < D && dt_bias) ? dt_bias[d0 + pc] : 0.f;
+  if (n > 0) fetch(0, stages[0]);
+  for (int c0 = 0, it = 0; c0 < n; c0 += TT, ++it) {
+    Stage& g = stages[it & 1];
+    const int m = min(TT, n - c0);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                 // this tile is in; everyone is done with the one before
+    if (c0 + TT < n) fetch(c0 + TT, stages[(it + 1) & 1]);
 #pragma unroll
-    for (int n = 0; n < N; ++n) {
-      h[n] = __expf(dt * a[n]) * h[n] + dt * sB[n] * ut;
-      acc = fmaf(sC[n], h[n], acc);
+    for (int j = tid >> 5; j < TT; j += kScanThreads / 32) {
+      float dt = __bfloat162float(g.dl[j][pc]) + pb;
+      if (dt_softplus) dt = softplus(dt);
+      if (j >= m) dt = 0.f;                          // tokens beyond the sequence leave the state alone
+      sdt[j][pc] = make_float2(dt, dt * __bfloat162float(g.u[j][pc]));
     }
-    if (z) acc *= silu(__bfloat162float(z[static_cast<size_t>(t) * ld_u + d]));
-    y[static_cast<size_t>(t) * ld_u + d] = __float2bfloat16(acc);
+    for (int i = tid; i < TT * N; i += kScanThreads) {
+      (&sB[0][0])[i] = __bfloat162float((&g.B[0][0])[i]);
+      (&sC[0][0])[i] = __bfloat162float((&g.C[0][0])[i]);
+    }
+    __syncthreads();
+    for (int j0 = 0; j0 < m; j0 += 8) {
+      float part[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const float2 e = sdt[j0 + r][c];
+        float acc = 0.f;
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+          h[i] = fmaf(ex2(e.x * a2[i]), h[i], e.y * sB[j0 + r][q * NS + i]);
+          acc = fmaf(sC[j0 + r][q * NS + i], h[i], acc);
+        }
+        part[r] = acc;
+      }
+      // lane q of the channel ends up with token j0 + q
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < o; ++r) {
+          const float send = (q & o) ? part[r] : part[r + o], keep = (q & o) ? part[r + o] : part[r];
+          part[r] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      float v = part[0];
+      const int j = j0 + q;
+      v = fmaf(dsk, __bfloat162float(g.u[j][c]), v);
+      if (z) v *= silu(__bfloat162float(g.z[j][c]));
+      sy[j][c] = __float2bfloat16(v);
+    }
+    __syncthreads();
+    if (vec) {
+      const int j = tid >> 2, k = (tid & 3) * 8;
+      if (tid < 128 && j < m && d0 + k < D)
+        *reinterpret_cast<uint4*>(y + static_cast<size_t>(t0 + c0 + j) * ld_u + d0 + k) = *reinterpret_cast<const uint4*>(&sy[j][k]);
+    } else {
+      for (int i = tid; i < m * CH; i += kScanThreads)
+        if (d0 + i % CH < D) y[static_cast<size_t>(t0 + c0 + i / CH) * ld_u + d0 + i % CH] = sy[i / CH][i % CH];
+    }
   }
   if (live && slot >= 0) {
 #pragma unroll
-    for (int n = 0; n < N; ++n) ssm_state[(static_cast<size_t>(slot) * D + d) * N + n] = h[n];
+    for (int i = 0; i < NS; ++i) st[i] = h[i];
   }
 }
 
@@ -131,7 +321,7 @@ __global__ void ssd_scan_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
                                 const float* __restrict__ dt_bias, __nv_bfloat16* __restrict__ y,
                                 float* __restrict__ ssm_state, const int* __restrict__ cu_seqlens,
                                 const int* __restrict__ state_idx, const int* __restrict__ has_init,
-                                int H, int P, int N, int G, int J, int dt_softplus) {
+                                int H, int P, int N, int G, int J, int ldx, int ld_dt, int ldb, int ldc, int dt_softplus) {
   extern __shared__ float sbc[];   // B_t[N] | C_t[N]
   const int s = blockIdx.y, hd = blockIdx.x;
   const int g = hd / (H / G);
@@ -151,14 +341,14 @@ __global__ void ssd_scan_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
   for (int t = t0; t < t1; ++t) {
     __syncthreads();
     for (int n = threadIdx.x; n < N; n += blockDim.x) {
-      sbc[n] = __bfloat162float(B[(static_cast<size_t>(t) * G + g) * N + n]);
-      sbc[N + n] = __bfloat162float(C[(static_cast<size_t>(t) * G + g) * N + n]);
+      sbc[n] = __bfloat162float(B[static_cast<size_t>(t) * ldb + g * N + n]);
+      sbc[N + n] = __bfloat162float(C[static_cast<size_t>(t) * ldc + g * N + n]);
     }
     __syncthreads();
-    float dt = __bfloat162float(dt_in[static_cast<size_t>(t) * H + hd]) + dtb;
+    float dt = __bfloat162float(dt_in[static_cast<size_t>(t) * ld_dt + hd]) + dtb;
     if (dt_softplus) dt = softplus(dt);
     const float decay = __expf(dt * a);
-    const float xt = __bfloat162float(x[(static_cast<size_t>(t) * H + hd) * P + p]);
+    const float xt = __bfloat162float(x[static_cast<size_t>(t) * ldx + hd * P + p]);
     const float dx = dt * xt;
     float acc = 0.f;
 #pragma unroll
@@ -181,29 +371,392 @@ __global__ void ssd_scan_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
   }
 }
 
+// The SSD recurrence 64 tokens at a time. With l_i = log2 of the decay of token i of a chunk, c_i = l_0 + .. + l_i and
+// the state S before the chunk:
+//   y_i = 2^c_i S C_i + sum_{j <= i} 2^(c_i - c_j) dt_j (C_i . B_j) x_j + D x_i
+//   S'  = 2^c_m S + sum_j 2^(l_(j+1) + .. + l_m) dt_j x_j B_j^T
+// All powers are at most 1. x, B and C are 16-bit activations and enter the products as they are; what is made from them
+// is fp32 and enters as a sum of bf16 numbers: two for S and the weighted products C . B (they end in a 16-bit y), three
+// for the weighted inputs of the state, so that the fp32 state keeps 24 bits. The powers of the state's sum run from the
+// chunk's end backwards, where the large ones are the short sums.
+// S^T stays in the accumulator fragments of the warp that owns its 16 rows p, which are also the B fragments of S C.
+// The chain from chunk to chunk is the bound (one CTA per sequence, head and 64 rows walks the chunks in order, about
+// 7 us each), so it is kept short: two barriers a chunk, tiles and step sizes fetched one chunk ahead.
+// Two sequences, 4096 tokens, 80 heads x 64 x 128: 12742 us token by token (two barriers and a load from global memory on
+// every token's chain), 239 us so.
+constexpr int kChunk = 64, kNV = 64, kChunkThreads = 128, kLdV = kNV + 8, kLdP = kChunk + 8;
+
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)) : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)) : "memory");
+}
+__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// the bf16 pair nearest to (x, y); x and y become what is left
+__device__ __forceinline__ uint32_t take_bf16(float& x, float& y) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+  const float2 f = __bfloat1622float2(h);
+  x -= f.x;
+  y -= f.y;
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+struct SsdChunk {
+  const __nv_bfloat16 *x, *dt, *B, *C;
+  const float *A, *Dskip, *dt_bias;
+  __nv_bfloat16* y;
+  float* state;
+  const int *cu_seqlens, *state_idx, *has_init;
+  int H, P, N, G, ldx, ld_dt, ldb, ldc, dt_softplus, col_blocks;
+};
+// per chunk: c_i, 2^(sum beyond j) dt_j, dt_j, 2^c_i
+struct SsdTimes { float cum[kChunk], tail[kChunk], dt[kChunk], grow[kChunk], total; };
+
+// 16 queries (rows 16 W ..) with the keys at or before them, weighted, into sP as hi and lo parts
+template <int W, int DK>
+__device__ __forceinline__ void ssd_products(const __nv_bfloat16* sC, const __nv_bfloat16* sB, __nv_bfloat16* sP, const SsdTimes& tm, int lane) {
+  constexpr int LDK = DK + 8;
+  const int mi = lane >> 3, r8 = lane & 7, row4 = lane >> 2, col2 = 2 * (lane & 3);
+  float sc[2 * (W + 1)][4];
+#pragma unroll
+  for (int i = 0; i < 2 * (W + 1); ++i) sc[i][0] = sc[i][1] = sc[i][2] = sc[i][3] = 0.f;
+#pragma unroll
+  for (int kb = 0; kb < DK / 16; ++kb) {
+    uint32_t a[4];
+    ldsm4(a, sC + (W * 16 + (lane & 15)) * LDK + kb * 16 + (lane >> 4) * 8);
+#pragma unroll
+    for (int np = 0; np <= W; ++np) {
+      uint32_t b[4];
+      ldsm4(b, sB + (np * 16 + (mi >> 1) * 8 + r8) * LDK + kb * 16 + (mi & 1) * 8);
+      mma(sc[2 * np], a, b[0], b[1]);
+      mma(sc[2 * np + 1], a, b[2], b[3]);
+    }
+  }
+#pragma unroll
+  for (int nt = 0; nt < 2 * (W + 1); ++nt) {
+    const int j = nt * 8 + col2;
+    const float c0 = tm.cum[j], c1 = tm.cum[j + 1], d0 = tm.dt[j], d1 = tm.dt[j + 1];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int i = W * 16 + row4 + 8 * e;
+      const float ci = tm.cum[i];
+      float a0 = i >= j ? sc[nt][2 * e] * (ex2(ci - c0) * d0) : 0.f, a1 = i > j ? sc[nt][2 * e + 1] * (ex2(ci - c1) * d1) : 0.f;
+      *reinterpret_cast<uint32_t*>(sP + i * kLdP + j) = take_bf16(a0, a1);
+      *reinterpret_cast<uint32_t*>(sP + (kChunk + i) * kLdP + j) = take_bf16(a0, a1);
+    }
+  }
+}
+
+template <int DK>
+__global__ void __launch_bounds__(kChunkThreads, 2) ssd_chunk_kernel(const SsdChunk p) {
+  typedef __nv_bfloat16 bf16;
+  constexpr int LDK = DK + 8, KB = DK / 16, kStage = kChunk * (2 * LDK + kLdV);
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  bf16* stages = reinterpret_cast<bf16*>(smem_raw);
+  bf16* sP = stages + 2 * kStage;                    // [hi | lo][chunk][kLdP]
+  __shared__ SsdTimes times[2];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, mi = lane >> 3, r8 = lane & 7, row4 = lane >> 2, col2 = 2 * (lane & 3);
+  const int h = blockIdx.x / p.col_blocks, v0 = (blockIdx.x % p.col_blocks) * kNV, s = blockIdx.y, P = p.P, N = p.N;
+  const int t0 = p.cu_seqlens[s], n = p.cu_seqlens[s + 1] - t0, slot = p.state_idx && p.state ? p.state_idx[s] : -1;
+  const bool resume = slot >= 0 && p.has_init && p.has_init[s];
+  const int group = h / (p.H / p.G);
+  const bf16 *xh = p.x + static_cast<size_t>(t0) * p.ldx + h * P, *Bh = p.B + static_cast<size_t>(t0) * p.ldb + group * N,
+             *Ch = p.C + static_cast<size_t>(t0) * p.ldc + group * N, *dth = p.dt + static_cast<size_t>(t0) * p.ld_dt + h;
+  auto fetch = [&](int c0, bf16* dst) {              // rows beyond the sequence and columns beyond the head become zero
+    constexpr int CH = DK / 8;
+    for (int i = tid; i < kChunk * CH; i += kChunkThreads) {
+      const int j = i / CH, c = (i % CH) * 8;
+      const bool ok = c0 + j < n && c < N;
+      const size_t row = ok ? c0 + j : 0;
+      cp_async16(dst + j * LDK + c, Ch + row * p.ldc + (ok ? c : 0), ok);
+      cp_async16(dst + (kChunk + j) * LDK + c, Bh + row * p.ldb + (ok ? c : 0), ok);
+    }
+    bf16* dv = dst + 2 * kChunk * LDK;
+    for (int i = tid; i < kChunk * (kNV / 8); i += kChunkThreads) {
+      const int j = i / (kNV / 8), c = (i % (kNV / 8)) * 8;
+      const bool ok = c0 + j < n && v0 + c < P;
+      cp_async16(dv + j * kLdV + c, xh + (ok ? static_cast<size_t>(c0 + j) * p.ldx + v0 + c : 0), ok);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // warp 0 makes the step sizes and their sums, two tokens per lane; the raw values are read one chunk earlier
+  const float a2 = p.A[h] * kLog2e, dtb = p.dt_bias ? p.dt_bias[h] : 0.f;
+  float raw[2];
+  auto read_dt = [&](int c0) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) raw[e] = c0 + 2 * lane + e < n ? __bfloat162float(dth[static_cast<size_t>(c0 + 2 * lane + e) * p.ld_dt]) : 0.f;
+  };
+  auto make_times = [&](int c0, SsdTimes& tm) {
+    float dt[2], l[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      dt[e] = raw[e] + dtb;
+      if (p.dt_softplus) dt[e] = softplus(dt[e]);
+      if (c0 + 2 * lane + e >= n) dt[e] = 0.f;
+      l[e] = dt[e] * a2;
+    }
+    const float pair = l[0] + l[1];
+    float up = pair, down = pair;                    // sums up to and from this pair
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float u = __shfl_up_sync(0xffffffffu, up, o), w = __shfl_down_sync(0xffffffffu, down, o);
+      if (lane >= o) up += u;
+      if (lane + o < 32) down += w;
+    }
+    float before = __shfl_up_sync(0xffffffffu, up, 1), after = __shfl_down_sync(0xffffffffu, down, 1);
+    if (lane == 0) before = 0.f;
+    if (lane == 31) after = 0.f;
+    const float c0_ = before + l[0], c1_ = before + pair;
+    tm.cum[2 * lane] = c0_; tm.cum[2 * lane + 1] = c1_;
+    tm.grow[2 * lane] = ex2(c0_); tm.grow[2 * lane + 1] = ex2(c1_);
+    tm.tail[2 * lane] = ex2(after + l[1]) * dt[0]; tm.tail[2 * lane + 1] = ex2(after) * dt[1];
+    tm.dt[2 * lane] = dt[0]; tm.dt[2 * lane + 1] = dt[1];
+    if (lane == 31) tm.total = ex2(c1_);
+  };
+  if (n > 0) {
+    fetch(0, stages);
+    if (warp == 0) {
+      read_dt(0);
+      make_times(0, times[0]);
+      read_dt(kChunk);
+    }
+  }
+  const float dsk = p.Dskip ? p.Dskip[h] : 0.f;
+  // S^T: 16 rows p of this warp as accumulator tiles of 8 columns n: [0], [1] row row4, [2], [3] row row4 + 8
+  float S[2 * KB][4];
+  float* st = p.state + (static_cast<size_t>(slot >= 0 ? slot : 0) * p.H + h) * P * N;
+  const int vr = v0 + warp * 16 + row4;
+#pragma unroll
+  for (int t = 0; t < 2 * KB; ++t)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      float2 f = make_float2(0.f, 0.f);
+      if (resume && vr + 8 * e < P && 8 * t < N) f = *reinterpret_cast<const float2*>(st + static_cast<size_t>(vr + 8 * e) * N + 8 * t + col2);
+      S[t][2 * e] = f.x; S[t][2 * e + 1] = f.y;
+    }
+  bool have_state = resume;
+  for (int c0 = 0, it = 0; c0 < n; c0 += kChunk, ++it) {
+    const int m = min(kChunk, n - c0);
+    const bf16 *sC = stages + (it & 1) * kStage, *sB = sC + kChunk * LDK, *sV = sB + kChunk * LDK;
+    const SsdTimes& tm = times[it & 1];
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                 // this chunk is in; everyone is done with the last one's stage, times and sP
+    if (c0 + kChunk < n) fetch(c0 + kChunk, stages + ((it + 1) & 1) * kStage);
+    switch (warp) {
+      case 0:                                        // the fewest products: this warp also prepares the next chunk's times
+        ssd_products<0, DK>(sC, sB, sP, tm, lane);
+        if (c0 + kChunk < n) {
+          make_times(c0 + kChunk, times[(it + 1) & 1]);
+          read_dt(c0 + 2 * kChunk);
+        }
+        break;
+      case 1: ssd_products<1, DK>(sC, sB, sP, tm, lane); break;
+      case 2: ssd_products<2, DK>(sC, sB, sP, tm, lane); break;
+      default: ssd_products<3, DK>(sC, sB, sP, tm, lane); break;
+    }
+    // what the state before the chunk contributes, for all tokens and this warp's 16 rows
+    float o[4][2][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) o[i][j][0] = o[i][j][1] = o[i][j][2] = o[i][j][3] = 0.f;
+    if (have_state) {
+#pragma unroll
+      for (int kb = 0; kb < KB; ++kb) {
+        uint32_t hi[2][2], lo[2][2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float u = S[2 * kb + e][2 * j], w = S[2 * kb + e][2 * j + 1];
+            hi[j][e] = take_bf16(u, w);
+            lo[j][e] = take_bf16(u, w);
+          }
+        uint32_t a[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ldsm4(a[i], sC + (i * 16 + (lane & 15)) * LDK + kb * 16 + (lane >> 4) * 8);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { mma(o[i][0], a[i], hi[0][0], hi[0][1]); mma(o[i][1], a[i], hi[1][0], hi[1][1]); }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { mma(o[i][0], a[i], lo[0][0], lo[0][1]); mma(o[i][1], a[i], lo[1][0], lo[1][1]); }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float f0 = tm.grow[i * 16 + row4], f1 = tm.grow[i * 16 + row4 + 8];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) { o[i][j][0] *= f0; o[i][j][1] *= f0; o[i][j][2] *= f1; o[i][j][3] *= f1; }
+      }
+    }
+    __syncthreads();                                 // the products of every warp are in sP
+#pragma unroll
+    for (int kb = 0; kb < 4; ++kb) {
+      uint32_t b[4];
+      ldsm4_t(b, sV + (kb * 16 + (mi & 1) * 8 + r8) * kLdV + warp * 16 + (mi >> 1) * 8);
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int i = kb; i < 4; ++i) {
+          uint32_t a[4];
+          ldsm4(a, sP + (half * kChunk + i * 16 + (lane & 15)) * kLdP + kb * 16 + (lane >> 4) * 8);
+          mma(o[i][0], a, b[0], b[1]);
+          mma(o[i][1], a, b[2], b[3]);
+        }
+    }
+    bf16* out = p.y + (static_cast<size_t>(t0 + c0) * p.H + h) * P;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = i * 16 + row4 + 8 * e;
+        if (r >= m) continue;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int cl = warp * 16 + j * 8 + col2, c = v0 + cl;
+          if (c >= P) continue;
+          const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sV + r * kLdV + cl));
+          *reinterpret_cast<__nv_bfloat162*>(out + static_cast<size_t>(r) * p.H * P + c) =
+              __floats2bfloat162_rn(fmaf(dsk, xv.x, o[i][j][2 * e]), fmaf(dsk, xv.y, o[i][j][2 * e + 1]));
+        }
+      }
+    // the state after the chunk
+    if (have_state) {
+      const float f = tm.total;
+#pragma unroll
+      for (int t = 0; t < 2 * KB; ++t) { S[t][0] *= f; S[t][1] *= f; S[t][2] *= f; S[t][3] *= f; }
+    }
+    have_state = true;
+#pragma unroll
+    for (int kb = 0; kb < 4; ++kb) {
+      uint32_t a[4], w3[3][4];                       // rows p: transposed fragments of x, weighted, in three parts
+      ldsm4_t(a, sV + (kb * 16 + (mi >> 1) * 8 + r8) * kLdV + warp * 16 + (mi & 1) * 8);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = kb * 16 + (q >> 1) * 8 + col2;
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[q]));
+        float u = f.x * tm.tail[j], w = f.y * tm.tail[j + 1];
+#pragma unroll
+        for (int part = 0; part < 3; ++part) w3[part][q] = take_bf16(u, w);
+      }
+#pragma unroll
+      for (int t = 0; t < KB; t += 2) {
+        uint32_t b[4], c[4];
+        ldsm4_t(b, sB + (kb * 16 + (mi & 1) * 8 + r8) * LDK + t * 16 + (mi >> 1) * 8);
+        ldsm4_t(c, sB + (kb * 16 + (mi & 1) * 8 + r8) * LDK + t * 16 + 16 + (mi >> 1) * 8);
+#pragma unroll
+        for (int part = 0; part < 3; ++part) {
+          mma(S[2 * t], w3[part], b[0], b[1]);
+          mma(S[2 * t + 1], w3[part], b[2], b[3]);
+          mma(S[2 * t + 2], w3[part], c[0], c[1]);
+          mma(S[2 * t + 3], w3[part], c[2], c[3]);
+        }
+      }
+    }
+  }
+  if (slot >= 0) {
+#pragma unroll
+    for (int t = 0; t < 2 * KB; ++t)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (vr + 8 * e < P && 8 * t < N)
+          *reinterpret_cast<float2*>(st + static_cast<size_t>(vr + 8 * e) * N + 8 * t + col2) = make_float2(S[t][2 * e], S[t][2 * e + 1]);
+  }
+}
+
+template <int DK>
+static int launch_ssd_chunk(const SsdChunk& p, int n_seqs, cudaStream_t stream) {
+  constexpr int smem = (2 * kChunk * (2 * (DK + 8) + kLdV) + 2 * kChunk * kLdP) * 2;
+  static PerDeviceOnce configured;
+  if (configured.needed()) {
+    if (cudaFuncSetAttribute(ssd_chunk_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+      return MB_ERR_LAUNCH;
+    configured.done();
+  }
+  ssd_chunk_kernel<DK><<<dim3(p.H * p.col_blocks, n_seqs), kChunkThreads, smem, stream>>>(p);
+  return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ERR_LAUNCH;
+}
+
+// out = rmsnorm(y * silu(z)) * w, rows of up to 256 x 8 x NV values held in registers by one CTA (one pass over memory,
+// bound by it; the same steps as separate operators read and wrote seven fp32 copies of the row).
+template <int NV>
+__global__ void __launch_bounds__(256) gated_rms_norm_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ z,
+                                                             const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
+                                                             int D, int ldz, float eps) {
+  __shared__ float part[8];
+  const size_t t = blockIdx.x;
+  const int tid = threadIdx.x;
+  float g[NV][8], sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = (i * 256 + tid) * 8;
+    if (c >= D) break;
+    float gate[8];
+    load_bf16<8>(g[i], y + t * D + c);
+    load_bf16<8>(gate, z + t * ldz + c);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      g[i][e] *= silu(gate[e]);
+      sum = fmaf(g[i][e], g[i][e], sum);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((tid & 31) == 0) part[tid >> 5] = sum;
+  __syncthreads();
+  sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) sum += part[i];
+  const float r = rsqrtf(sum / D + eps);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = (i * 256 + tid) * 8;
+    if (c >= D) break;
+    float wv[8];
+    load_bf16<8>(wv, w + c);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) wv[e] *= g[i][e] * r;
+    store_bf16<8>(out + t * D + c, wv);
+  }
+}
+
 }  // namespace ssm
 }  // namespace mb
 
 using namespace mb::ssm;
 
+static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// `tokens`: rows of x, an upper bound of cu_seqlens[n_seqs]
 extern "C" int mb_causal_conv1d_varlen(const void* x, const void* w, const void* bias, void* y, float* conv_state,
                                        const int* cu_seqlens, const int* state_idx, const int* has_init,
-                                       int n_seqs, int D, int width, int ldx, int ldy, int act,
+                                       int n_seqs, int tokens, int D, int width, int ldx, int ldy, int act,
                                        cudaStream_t stream) {
   if (n_seqs <= 0 || D <= 0) return MB_OK;
-  dim3 grid((D + 127) / 128, n_seqs);
-#define MB_CONV(Wv)                                                                                              \
-  causal_conv1d_kernel<Wv><<<grid, 128, 0, stream>>>(                                                            \
+  // 8-byte accesses where every row starts on such a boundary (of 16-byte ones a thread's eight channels take 120 registers)
+  const bool vec = D % 8 == 0 && ldx % 8 == 0 && ldy % 8 == 0 && aligned16(x) && aligned16(y) && aligned16(w) &&
+                   (bias == nullptr || aligned16(bias));
+  const int per = 128 * (vec ? 4 : 1);
+  dim3 grid(n_seqs + (tokens + kConvTile - 1) / kConvTile, (D + per - 1) / per);
+#define MB_CONV(Wv, Vv)                                                                                          \
+  causal_conv1d_kernel<Wv, Vv><<<grid, 128, 0, stream>>>(                                                        \
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w),                                \
       static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(y), conv_state, cu_seqlens, state_idx, \
-      has_init, D, ldx, ldy, act)
+      has_init, n_seqs, D, ldx, ldy, act)
+#define MB_CONV2(Wv) do { if (vec) MB_CONV(Wv, 4); else MB_CONV(Wv, 1); } while (0)
   switch (width) {
-    case 2: MB_CONV(2); break;
-    case 3: MB_CONV(3); break;
-    case 4: MB_CONV(4); break;
-    case 8: MB_CONV(8); break;
+    case 2: MB_CONV2(2); break;
+    case 3: MB_CONV2(3); break;
+    case 4: MB_CONV2(4); break;
+    case 8: MB_CONV2(8); break;
     default: return MB_ERR_SHAPE;
   }
+#undef MB_CONV2
 #undef MB_CONV
   return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ERR_LAUNCH;
 }
@@ -211,16 +764,18 @@ extern "C" int mb_causal_conv1d_varlen(const void* x, const void* w, const void*
 extern "C" int mb_selective_scan_varlen(const void* u, const void* delta, const float* A, const void* B,
                                         const void* C, const float* Dskip, const void* z, const float* dt_bias,
                                         void* y, float* ssm_state, const int* cu_seqlens, const int* state_idx,
-                                        const int* has_init, int n_seqs, int D, int N, int ld_u, int ld_bc,
-                                        int dt_softplus, cudaStream_t stream) {
+                                        const int* has_init, int n_seqs, int D, int N, int ld_u, int ld_z, int ld_b,
+                                        int ld_c, int dt_softplus, cudaStream_t stream) {
   if (n_seqs <= 0 || D <= 0) return MB_OK;
-  dim3 grid((D + 127) / 128, n_seqs);
+  const int vec = D % 8 == 0 && ld_u % 8 == 0 && ld_b % 8 == 0 && ld_c % 8 == 0 && aligned16(u) && aligned16(delta) &&
+                  aligned16(B) && aligned16(C) && aligned16(y) && (z == nullptr || (ld_z % 8 == 0 && aligned16(z)));
+  dim3 grid((D + kScanCh - 1) / kScanCh, n_seqs);
 #define MB_SCAN(Nv)                                                                                             \
-  selective_scan_kernel<Nv><<<grid, 128, 0, stream>>>(                                                          \
+  selective_scan_kernel<Nv><<<grid, kScanThreads, 0, stream>>>(                                                          \
       static_cast<const __nv_bfloat16*>(u), static_cast<const __nv_bfloat16*>(delta), A,                        \
       static_cast<const __nv_bfloat16*>(B), static_cast<const __nv_bfloat16*>(C), Dskip,                        \
       static_cast<const __nv_bfloat16*>(z), dt_bias, static_cast<__nv_bfloat16*>(y), ssm_state, cu_seqlens,     \
-      state_idx, has_init, D, ld_u, ld_bc, dt_softplus)
+      state_idx, has_init, D, ld_u, ld_z, ld_b, ld_c, dt_softplus, vec)
   switch (N) {
     case 8: MB_SCAN(8); break;
     case 16: MB_SCAN(16); break;
@@ -234,9 +789,21 @@ extern "C" int mb_selective_scan_varlen(const void* u, const void* delta, const 
 extern "C" int mb_ssd_scan_varlen(const void* x, const void* dt, const float* A, const void* B, const void* C,
                                   const float* Dskip, const float* dt_bias, void* y, float* ssm_state,
                                   const int* cu_seqlens, const int* state_idx, const int* has_init, int n_seqs,
-                                  int H, int P, int N, int G, int dt_softplus, cudaStream_t stream) {
+                                  int tokens, int H, int P, int N, int G, int ldx, int ld_dt, int ldb, int ldc,
+                                  int dt_softplus, cudaStream_t stream) {
   if (n_seqs <= 0 || H <= 0) return MB_OK;
   if (P <= 0 || P > 256 || (P & (P - 1)) || G <= 0 || H % G || N <= 0 || N > 256) return MB_ERR_SHAPE;
+  // A chunk takes 7 us, full or not, a token of the walk 1.5 to 5 us: from four tokens per sequence on, the chunks win (and
+  // earlier where one sequence is much longer than the others). They take 16-byte copies of whole 8-value groups, so sizes and addresses that do not fit stay with the walk.
+  if (tokens >= 4LL * n_seqs && N <= 128 && N % 8 == 0 && P % 8 == 0 && ldx % 8 == 0 && ldb % 8 == 0 && ldc % 8 == 0 &&
+      aligned16(x) && aligned16(B) && aligned16(C) && (reinterpret_cast<uintptr_t>(ssm_state) & 7) == 0) {
+    SsdChunk p{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dt), static_cast<const __nv_bfloat16*>(B),
+               static_cast<const __nv_bfloat16*>(C), A, Dskip, dt_bias, static_cast<__nv_bfloat16*>(y), ssm_state, cu_seqlens,
+               state_idx, has_init, H, P, N, G, ldx, ld_dt, ldb, ldc, dt_softplus, (P + kNV - 1) / kNV};
+    if (N <= 32) return launch_ssd_chunk<32>(p, n_seqs, stream);
+    if (N <= 64) return launch_ssd_chunk<64>(p, n_seqs, stream);
+    return launch_ssd_chunk<128>(p, n_seqs, stream);
+  }
   int J = 256 / P;            // threads per state row
   if (J > 32) J = 32;
   if (J < 1) J = 1;
@@ -248,7 +815,8 @@ extern "C" int mb_ssd_scan_varlen(const void* x, const void* dt, const float* A,
   ssd_scan_kernel<NPTv><<<grid, threads, smem, stream>>>(                                                       \
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dt), A,                           \
       static_cast<const __nv_bfloat16*>(B), static_cast<const __nv_bfloat16*>(C), Dskip, dt_bias,               \
-      static_cast<__nv_bfloat16*>(y), ssm_state, cu_seqlens, state_idx, has_init, H, P, N, G, J, dt_softplus)
+      static_cast<__nv_bfloat16*>(y), ssm_state, cu_seqlens, state_idx, has_init, H, P, N, G, J, ldx, ld_dt,    \
+      ldb, ldc, dt_softplus)
   if (npt <= 4) MB_SSD(4);
   else if (npt <= 8) MB_SSD(8);
   else if (npt <= 16) MB_SSD(16);
@@ -256,5 +824,22 @@ extern "C" int mb_ssd_scan_varlen(const void* x, const void* dt, const float* A,
   else if (npt <= 64) MB_SSD(64);
   else return MB_ERR_SHAPE;
 #undef MB_SSD
+  return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ERR_LAUNCH;
+}
+
+extern "C" int mb_gated_rms_norm(const void* y, const void* z, const void* w, void* out, int T, int D, int ldz, float eps,
+                                 cudaStream_t stream) {
+  if (T <= 0) return MB_OK;
+  if (D <= 0 || D % 8 || D > 16384 || ldz % 8 || !aligned16(y) || !aligned16(z) || !aligned16(w) || !aligned16(out))
+    return MB_ERR_SHAPE;
+#define MB_NORM(NV)                                                                                                      \
+  gated_rms_norm_kernel<NV><<<T, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(y), static_cast<const __nv_bfloat16*>(z), \
+                                                   static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(out), D, ldz, eps)
+  if (D <= 2048) MB_NORM(1);
+  else if (D <= 4096) MB_NORM(2);
+  else if (D <= 6144) MB_NORM(3);
+  else if (D <= 8192) MB_NORM(4);
+  else MB_NORM(8);
+#undef MB_NORM
   return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ERR_LAUNCH;
 }

@@ -116,6 +116,12 @@ def _native_ok(t):
     return t.is_cuda and t.dtype == torch.bfloat16
 
 
+def _rows(t):
+    """``t`` as the kernels take it: any distance between rows (tokens), each row contiguous."""
+    inner = t.stride(-1) == 1 and (t.dim() == 2 or t.stride(1) == t.shape[2])
+    return t if inner else t.contiguous()
+
+
 def causal_conv1d_varlen(x, w, bias, cu_seqlens, conv_state=None, state_idx=None, has_init=None, silu=True):
     """x [T, D]; w [D, W]; conv_state fp32 [slots, D, W-1] holds the last W-1 inputs of each live sequence."""
     if not _native_ok(x) or w.shape[1] not in (2, 3, 4, 8):
@@ -133,9 +139,9 @@ def selective_scan_varlen(u, delta, A, B, C, D=None, z=None, dt_bias=None, cu_se
         return selective_scan_reference(u, delta, A, B, C, D, z, dt_bias, cu_seqlens, ssm_state, state_idx,
                                         has_init, dt_softplus)
     y = torch.empty_like(u)
-    _lib().selective_scan_varlen(u.contiguous(), delta.contiguous(), A.float().contiguous(), B.contiguous(),
-                                 C.contiguous(), None if D is None else D.float().contiguous(),
-                                 None if z is None else z.contiguous(),
+    _lib().selective_scan_varlen(u.contiguous(), delta.contiguous(), A.float().contiguous(), _rows(B),
+                                 _rows(C), None if D is None else D.float().contiguous(),
+                                 None if z is None else _rows(z),
                                  None if dt_bias is None else dt_bias.float().contiguous(), y, ssm_state,
                                  _opt_i32(cu_seqlens, u.device), _opt_i32(state_idx, u.device),
                                  _opt_i32(has_init, u.device), dt_softplus)
@@ -150,12 +156,25 @@ def ssd_scan_varlen(x, dt, A, B, C, D=None, dt_bias=None, cu_seqlens=None, ssm_s
         return ssd_scan_reference(x, dt, A, B, C, D, dt_bias, cu_seqlens, ssm_state, state_idx, has_init,
                                   dt_softplus)
     y = torch.empty_like(x)
-    _lib().ssd_scan_varlen(x.contiguous(), dt.contiguous(), A.float().contiguous(), B.contiguous(), C.contiguous(),
+    _lib().ssd_scan_varlen(_rows(x), _rows(dt), A.float().contiguous(), _rows(B), _rows(C),
                            None if D is None else D.float().contiguous(),
                            None if dt_bias is None else dt_bias.float().contiguous(), y, ssm_state,
                            _opt_i32(cu_seqlens, x.device), _opt_i32(state_idx, x.device),
                            _opt_i32(has_init, x.device), dt_softplus)
     return y
+
+
+def gated_rms_norm(y, z, w, eps):
+    """``rms_norm(y * silu(z)) * w`` in fp32, rounded once; y [T, D], z [T, D] (rows at any distance), w [D]."""
+    D = y.shape[1]
+    if (_native_ok(y) and z.dtype == w.dtype == y.dtype and D % 8 == 0 and D <= 16384 and z.stride(0) % 8 == 0 and z.stride(1) == 1
+            and not any(t.data_ptr() & 15 for t in (y, z, w)) and y.is_contiguous() and w.is_contiguous()):
+        out = torch.empty_like(y)
+        _lib().gated_rms_norm(y, z, w, out, eps)
+        return out
+    g = y.float() * F.silu(z.float())
+    g = g * torch.rsqrt(g.pow(2).mean(-1, keepdim=True) + eps) * w.float()
+    return g.to(y.dtype)
 
 
 # ------------------------------------------------------------------------------------ blocks
@@ -188,13 +207,12 @@ class MambaMixer(torch.nn.Module):
     def forward(self, h, cu_seqlens, state=None, state_idx=None, has_init=None):
         conv_state, ssm_state = state if state is not None else (None, None)
         xz = self.in_proj(h)
-        x, z = xz[:, : self.d_inner].contiguous(), xz[:, self.d_inner:].contiguous()
+        x, z = xz[:, : self.d_inner], xz[:, self.d_inner:]        # the kernels take rows at any distance
         x = causal_conv1d_varlen(x, self.conv_w, self.conv_b, cu_seqlens, conv_state, state_idx, has_init, True)
         dbc = self.x_proj(x)
-        dt = self.dt_proj.weight @ dbc[:, : self.dt_rank].t()
-        dt = dt.t().contiguous()
-        B = dbc[:, self.dt_rank : self.dt_rank + self.d_state].contiguous()
-        C = dbc[:, self.dt_rank + self.d_state:].contiguous()
+        dt = F.linear(dbc[:, : self.dt_rank], self.dt_proj.weight)
+        B = dbc[:, self.dt_rank : self.dt_rank + self.d_state]
+        C = dbc[:, self.dt_rank + self.d_state:]
         y = selective_scan_varlen(x, dt, -torch.exp(self.A_log.float()), B, C, self.D, z,
                                   self.dt_proj.bias.float(), cu_seqlens, ssm_state, state_idx, has_init, True)
         return self.out_proj(y)
@@ -231,16 +249,14 @@ class Mamba2Mixer(torch.nn.Module):
         conv_state, ssm_state = state if state is not None else (None, None)
         proj = self.in_proj(h)
         z = proj[:, : self.d_inner]
-        xbc = proj[:, self.d_inner : self.d_inner + self.conv_dim].contiguous()
-        dt = proj[:, self.d_inner + self.conv_dim:].contiguous()
+        xbc = proj[:, self.d_inner : self.d_inner + self.conv_dim]
+        dt = proj[:, self.d_inner + self.conv_dim:]
         xbc = causal_conv1d_varlen(xbc, self.conv_w, self.conv_b, cu_seqlens, conv_state, state_idx, has_init, True)
         T = h.shape[0]
-        x = xbc[:, : self.d_inner].reshape(T, self.H, self.P).contiguous()
+        x = xbc[:, : self.d_inner].unflatten(1, (self.H, self.P))
         gn = self.G * self.N
-        B = xbc[:, self.d_inner : self.d_inner + gn].reshape(T, self.G, self.N).contiguous()
-        C = xbc[:, self.d_inner + gn:].reshape(T, self.G, self.N).contiguous()
+        B = xbc[:, self.d_inner : self.d_inner + gn].unflatten(1, (self.G, self.N))
+        C = xbc[:, self.d_inner + gn:].unflatten(1, (self.G, self.N))
         y = ssd_scan_varlen(x, dt, -torch.exp(self.A_log.float()), B, C, self.D, self.dt_bias, cu_seqlens,
                             ssm_state, state_idx, has_init, True).reshape(T, self.d_inner)
-        g = (y.float() * F.silu(z.float()))
-        g = g * torch.rsqrt(g.pow(2).mean(-1, keepdim=True) + self.eps) * self.norm_w.float()
-        return self.out_proj(g.to(h.dtype))
+        return self.out_proj(gated_rms_norm(y, z, self.norm_w, self.eps))

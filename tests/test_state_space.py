@@ -123,3 +123,83 @@ def test_ssd_scan_kernel(H, P, N, G):
     y_ref = ss.ssd_scan_reference(x, dt, A, B, C, Dk, bias, _cu(lens), st_ref, idx.cpu(), init.cpu(), True)
     assert _rel(y, y_ref) < 1e-2
     assert _rel(st, st_ref) < 1e-3
+
+
+def _strided(t, lead=8):
+    """The same values as rows of a wider tensor (another distance between rows, another first column)."""
+    wide = torch.zeros(t.shape[0], lead + t[0].numel() + 8, device=t.device, dtype=t.dtype)
+    wide[:, lead: lead + t[0].numel()] = t.flatten(1)
+    return wide[:, lead: lead + t[0].numel()].view(t.shape)
+
+
+EDGES = [1, 63, 0, 64, 65, 2, 130, 31, 33]        # around tiles of 16, 32 and 64 tokens, an empty sequence among them
+
+
+def _state_args(dev):
+    idx = torch.tensor([3, -1, 0, 1, 2, 4, 8, 5, 6], dtype=torch.int32, device=dev)
+    init = torch.tensor([1, 0, 0, 1, 0, 1, 1, 1, 0], dtype=torch.int32, device=dev)
+    return idx, init
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,D,lead", [(4, 1032, 8), (2, 64, 16), (8, 8, 8), (3, 24, 1), (4, 13, 3)])
+def test_conv_tiles(W, D, lead):
+    """Aligned rows (8 channels a thread) and rows that are not (1)."""
+    torch.manual_seed(5)
+    dev = "cuda"
+    idx, init = _state_args(dev)
+    x = _strided(torch.randn(sum(EDGES), D, device=dev).to(torch.bfloat16), lead)
+    w, b = (torch.randn(D, W, device=dev) * 0.5).to(torch.bfloat16), torch.randn(D, device=dev).to(torch.bfloat16)
+    st = torch.randn(9, D, W - 1, device=dev)
+    ref = st.clone()
+    y = ss.causal_conv1d_varlen(x, w, b, _cu(EDGES, dev), st, idx, init, True)
+    want = ss.causal_conv1d_reference(x, w, b, _cu(EDGES), ref, idx.cpu(), init.cpu(), True)
+    assert _rel(y, want) < 2 ** -8                 # one rounding to bf16 on either side
+    assert torch.equal(st, ref)                    # the state is a copy of inputs
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,D,lead", [(16, 40, 8), (8, 32, 8), (32, 72, 8), (16, 37, 8), (16, 64, 1)])
+def test_selective_scan_tiles(N, D, lead):
+    torch.manual_seed(6)
+    dev, T = "cuda", sum(EDGES)
+    idx, init = _state_args(dev)
+    bf = lambda *s, k=1.0: (torch.randn(*s, device=dev) * k).to(torch.bfloat16)
+    u, delta, z, B, C = bf(T, D), bf(T, D, k=0.5), _strided(bf(T, D), lead), _strided(bf(T, N), lead), _strided(bf(T, N), lead)
+    A, Dk, bias = -torch.rand(D, N, device=dev) * 4 - 0.1, torch.randn(D, device=dev), torch.randn(D, device=dev) * 0.1
+    st = torch.randn(9, D, N, device=dev)
+    ref = st.clone()
+    y = ss.selective_scan_varlen(u, delta, A, B, C, Dk, z, bias, _cu(EDGES, dev), st, idx, init, True)
+    want = ss.selective_scan_reference(u, delta, A, B, C, Dk, z, bias, _cu(EDGES), ref, idx.cpu(), init.cpu(), True)
+    assert _rel(y, want) < 2 ** -8
+    assert _rel(st, ref) < 1e-5                    # fp32: 2 ulp of ex2.approx per step over the state's memory of a few steps
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,P,N,G,A0", [(4, 64, 128, 1, 1.0), (6, 32, 64, 2, 16.0), (2, 128, 16, 2, 0.1), (3, 8, 24, 1, 1.0), (2, 16, 40, 2, 4.0),
+                                        (2, 4, 16, 1, 1.0), (2, 64, 136, 1, 1.0)])
+def test_ssd_chunks(H, P, N, G, A0):
+    """Chunks of 64 on the tensor cores; the last two sizes stay with the token walk."""
+    torch.manual_seed(7)
+    dev, T = "cuda", sum(EDGES)
+    idx, init = _state_args(dev)
+    bf = lambda *s, k=1.0: (torch.randn(*s, device=dev) * k).to(torch.bfloat16)
+    x, dt, B, C = _strided(bf(T, H, P)), _strided(bf(T, H, k=0.5), 1), _strided(bf(T, G, N, k=0.3)), _strided(bf(T, G, N, k=0.3))
+    A, Dk, bias = -A0 * (torch.rand(H, device=dev) + 0.1), torch.randn(H, device=dev), torch.randn(H, device=dev) * 0.1
+    st = torch.randn(9, H, P, N, device=dev)
+    ref = st.clone()
+    y = ss.ssd_scan_varlen(x, dt, A, B, C, Dk, bias, _cu(EDGES, dev), st, idx, init, True)
+    want = ss.ssd_scan_reference(x, dt, A, B, C, Dk, bias, _cu(EDGES), ref, idx.cpu(), init.cpu(), True)
+    assert _rel(y, want) < 2 ** -8
+    assert _rel(st, ref) < 1e-5                    # three-part operands keep 24 bits; a sum of up to 130 fp32 terms and powers
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [8, 2048, 2056, 5120, 16384, 100])
+def test_gated_rms_norm(D):
+    torch.manual_seed(8)
+    y, z = (torch.randn(5, D, device="cuda").to(torch.bfloat16) for _ in range(2))
+    w, z = torch.randn(D, device="cuda").to(torch.bfloat16), _strided(z)
+    g = y.double() * z.double() / (1 + torch.exp(-z.double()))
+    want = g * torch.rsqrt(g.pow(2).mean(-1, keepdim=True) + 1e-5) * w.double()
+    assert _rel(ss.gated_rms_norm(y, z, w, 1e-5), want) < 2 ** -8
