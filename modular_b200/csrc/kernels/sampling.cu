@@ -4,8 +4,8 @@
 // sample_kernel: one CTA of 1024 threads owns one batch row. Top-k and top-p cut-offs are found by
 // bisection on the order-preserving integer image of the fp32 logits, so no sort and
 // no scratch memory is needed; pure temperature sampling takes the one-pass Gumbel-max
-// route. sample_cluster_kernel, launched before it for rows with a filter, spreads a row over a thread-block
-// cluster and leaves only the rows it cannot take. Behavioural counterparts in the reference: max/kernels/src/nn/topk.mojo
+// route. sample_cluster_kernel spreads a row over a thread-block cluster and is the one that runs; sample_kernel is for
+// devices that cannot place such clusters. Behavioural counterparts in the reference: max/kernels/src/nn/topk.mojo
 // (fused token sampling :2037, Gumbel argmax :2369), nn/sampling/topk_fi.mojo,
 // nn/sampling/sampling.mojo:31 (penalties).
 #include <cuda_runtime.h>
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(kSampThreads, 1)
 sample_kernel(const float* __restrict__ logits, int64_t* __restrict__ out, int vocab, int ld,
               const float* __restrict__ temperature, const int32_t* __restrict__ top_k,
               const float* __restrict__ top_p, const float* __restrict__ min_p,
-              const uint64_t* __restrict__ seeds, uint64_t step, int only_pending) {
+              const uint64_t* __restrict__ seeds, uint64_t step) {
   __shared__ ArgMax sh_am[32];
   __shared__ float sh_f[32];
   __shared__ float sh_scan[kSampThreads / 32];
@@ -321,7 +321,6 @@ sample_kernel(const float* __restrict__ logits, int64_t* __restrict__ out, int v
   pdl_wait();
   pdl_trigger();
   const int rowi = blockIdx.x;
-  if (only_pending && out[rowi] >= 0) return;   // sample_cluster_kernel already drew this row
   const float* row = logits + static_cast<size_t>(rowi) * ld;
   const float T = temperature ? temperature[rowi] : 1.f;
   const int k = top_k ? top_k[rowi] : 0;
@@ -447,39 +446,44 @@ sample_kernel(const float* __restrict__ logits, int64_t* __restrict__ out, int v
   }
 }
 
-// ---- truncated sampling with a row spread over a cluster of eight CTAs
-// sample_kernel walks a row with one CTA, so a batch of 64 rows keeps 64 SMs busy with eight or more
-// latency-bound passes each. Here the 256 warps of a cluster each own a contiguous share of the row and
-// read it three times (L2 hits after the first): maximum; candidate counts and softmax mass inside three
-// windows below the maximum; then the candidates of the smallest window that provably holds the whole kept
-// set are written, in index order, into the list of the cluster's first CTA through distributed shared
-// memory. That CTA finds the top-k / top-p cut-offs and draws the token on the list alone. A row whose kept
-// set does not fit a window (flat distributions, huge k) gets out[row] = -1 and is left to sample_kernel,
-// as are greedy and plain-temperature rows.
-constexpr int kClu = 8;   // largest cluster; the launcher picks 8, 4, 2 or 1 CTAs per row from the batch size
-constexpr int kCluList = (kSampThreads / 32) * kListPerWarp;
-// Histogram under the maximum: bin b holds the elements with b <= mx - x / T < b + 1. "Window w" is bins 0..w.
-constexpr int kCntBins = 32;    // counts reach 32 units down (a top-k of a few hundred on a peaked row)
-static_assert(kListPerWarp * (kSampThreads / 32) >= 4 * kSampThreads, "room for the rank-ordered copies");
-static_assert(kCntBins == kSampThreads / 32, "one warp adds up one count bin");
-constexpr int kMassBins = 16;   // masses only 16: what lies lower weighs less than e^-16 of the maximum each
+// ---- a row spread over a cluster of CTAs
+// The 16 c warps of a cluster each own a contiguous share of the row and read it two or three times (L2 hits after the
+// first). Greedy and plain-temperature rows are one pass. Rows with a filter take the maximum, then a histogram of
+// mx - x / T in shared memory (bins of 1/32, counts and, for a nucleus over the whole row, softmax mass; bins that
+// narrow spread the bulk of the row over hundreds of counters, so the atomics hardly meet). If the bins that provably
+// hold the kept set have at most kList elements, those go to the first CTA, which ranks them by counting and reads both
+// cut-offs off the sorted values. Otherwise the cut-off is found exactly by refining the bin it lies in, 2048 buckets
+// of keys at a time (a few more passes), and the draw is a prefix sum over the warps' shares.
+// Masses are integers, so sums do not depend on their order: 42 fractional bits where few weights meet in registers, and
+// per bin the weights relative to the bin's upper edge as 26-bit numbers in two halves, because 32-bit atomics on shared
+// memory are native and 64-bit ones are not (with those 64 nucleus rows took 122 us, with these 101).
+// 64 rows of 128256 logits, a quarter of the rows with a nucleus of thousands of tokens: 364 us when such rows (and
+// confident ones, whose k-th token lies far below the first) were left to sample_kernel, which walks a row with one
+// CTA, 58 to 66 us so (127 us before where all kept sets were short); one row 28 us, 64 greedy rows 11 us.
+constexpr int kClu = 8;          // largest cluster; the launcher picks 8, 4, 2 or 1 CTAs per row from the batch size
+constexpr int kCluThreads = 512, kCluWarps = kCluThreads / 32;
+constexpr int kBins = 2048, kOwn = kBins / kCluThreads;
+static_assert(kOwn == 4, "a thread reads its bins as one vector");
+constexpr int kList = kCluThreads;
+constexpr float kBinsPerUnit = 32.f;
+constexpr int kMaxShare = 1 << 18;   // elements per CTA: the halves of 2^18 weights of one bin still add up below 2^32
+typedef unsigned long long u64;
 
 struct ClusterSmem {
-  SearchSmem search;            // search.list: x / T of the candidates (filled in the first CTA only)
-  int idx[kCluList];            // their vocabulary indices
+  uint32_t cnt[kBins], hi[kBins], lo[kBins];
+  float lx[kList];              // x / T of the candidates and their indices, as they arrive (first CTA only)
+  int li[kList];
+  float sx[kList];              // by rank
+  u64 sp[kList];                // by rank: inclusive prefix of the masses
+  float ox[kList];              // by index
+  int oi[kList];
   ArgMax cmax;                  // maximum of this CTA's share
-  int cnt[kCntBins][32];        // per warp: elements with floor(mx - x / T) == bin
-  float mass[kMassBins][32];    // per warp: their softmax mass
-  float zall[32];               // per warp: softmax mass of the whole share
-  int cta_cnt[kCntBins];        // the same over this CTA's warps (what the peers read)
-  float cta_mass[kMassBins];
-  float cta_z;
-  int peer_cnt[kClu][kCntBins]; // every CTA's figures, gathered
-  int tot_cnt[kCntBins];        // over the cluster
-  float tot_mass[kMassBins];
-  float tot_z;
-  float red[32];
-  int pick, last, cut;
+  u64 wsum[kCluWarps];          // kept mass of every warp's share
+  u64 all[kClu * kCluWarps];
+  u64 red[kCluWarps];
+  u64 above;
+  int bin, n, cut;
+  uint32_t fill;
 };
 
 __device__ __forceinline__ void load4(const float* __restrict__ row, int i, int end, bool vec, float (&xv)[4]) {
@@ -491,28 +495,45 @@ __device__ __forceinline__ void load4(const float* __restrict__ row, int i, int 
     for (int e = 0; e < 4; ++e) xv[e] = i + e < end ? row[i + e] : -FLT_MAX;
   }
 }
-
-// softmax mass of the list entries with key >= thr; every thread gets the same value
-__device__ float list_mass_ge(SearchSmem* sm, float mx, uint32_t thr) {
+__device__ __forceinline__ u64 weight_of(float below) { return __float2ull_rn(__expf(-below) * 4398046511104.f); }
+__device__ __forceinline__ int bin_of(float below) {       // NaN goes to the last bin
+  const float b = below * kBinsPerUnit;
+  return b < static_cast<float>(kBins - 1) ? static_cast<int>(b) : kBins - 1;
+}
+__device__ __forceinline__ uint4 ld_cluster_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared::cluster.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ u64 ld_cluster_u64(uint32_t addr) {
+  u64 v;
+  asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
+  return v;
+}
+// sum of `mine` over the threads before this one, and over all of them
+__device__ __forceinline__ u64 block_before(u64 mine, u64* red, u64& total) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float v = 0.f;
-  const int n = sm->wcnt[warp];
-  for (int q = lane; q < n; q += 32) {
-    const float x = sm->list[warp * kListPerWarp + q];
-    v += fkey(x) >= thr ? __expf(x - mx) : 0.f;
-  }
+  u64 incl = mine;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = 1; o < 32; o <<= 1) {
+    const u64 t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) red[warp] = incl;
   __syncthreads();
-  if (lane == 0) sm->acc[warp] = v;
+  u64 before = 0;
+  total = 0;
+#pragma unroll
+  for (int q = 0; q < kCluWarps; ++q) {
+    const u64 t = red[q];
+    if (q < warp) before += t;
+    total += t;
+  }
   __syncthreads();
-  float tot = 0.f;
-  for (int q = 0; q < kSampThreads / 32; ++q) tot += sm->acc[q];
-  __syncthreads();
-  return tot;
+  return before + incl - mine;
 }
 
-__global__ void __launch_bounds__(kSampThreads, 1)
+__global__ void __launch_bounds__(kCluThreads, 2)
 sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ out, int vocab, int ld,
                       const float* __restrict__ temperature, const int32_t* __restrict__ top_k,
                       const float* __restrict__ top_p, const float* __restrict__ min_p,
@@ -520,45 +541,54 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
   extern __shared__ __align__(16) unsigned char sm_raw[];
   ClusterSmem* sm = reinterpret_cast<ClusterSmem*>(sm_raw);
   __shared__ ArgMax sh_am[32];
-  const int rowi = blockIdx.y;
+  pdl_wait();
+  pdl_trigger();
+  const int rowi = blockIdx.y, tid = threadIdx.x;
   const uint32_t rank = cluster_ctarank(), nclu = cluster_nctarank();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tid >> 5, lane = tid & 31;
   const float* row = logits + static_cast<size_t>(rowi) * ld;
   const float T = temperature ? temperature[rowi] : 1.f;
   const int k = top_k ? top_k[rowi] : 0;
   const float tp = top_p ? top_p[rowi] : 1.f;
   const float mp = min_p ? min_p[rowi] : 0.f;
+  const uint64_t seed = seeds ? seeds[rowi] : 0x1234ull + rowi;
+  const bool greedy = T <= 0.f || k == 1;
   const bool use_k = k > 0 && k < vocab, use_p = tp < 1.f, use_m = mp > 0.f;
-  // the same decision in all eight CTAs, so a row is left by the whole cluster at once
-  if (T <= 0.f || k == 1 || !(use_k || use_p || use_m)) {
-    if (rank == 0 && threadIdx.x == 0) out[rowi] = -1;
-    return;
-  }
-  const float invT = 1.f / T;
+  const bool plain = !greedy && !(use_k || use_p || use_m);
+  const float invT = greedy ? 1.f : 1.f / T;
   const bool vec = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
   // warp g of the cluster owns [g * seg, (g + 1) * seg): a multiple of 128 elements (aligned float4 loads)
-  const int nwarps = static_cast<int>(nclu) * 32;
+  const int nwarps = static_cast<int>(nclu) * kCluWarps;
   const int seg = (((vocab + nwarps - 1) / nwarps) + 127) & ~127;
-  const int gw = static_cast<int>(rank) * 32 + warp;
-  const int beg = gw * seg < vocab ? gw * seg : vocab;
-  const int end = beg + seg < vocab ? beg + seg : vocab;
+  const int gw = static_cast<int>(rank) * kCluWarps + warp;
+  const int beg = static_cast<long long>(gw) * seg < vocab ? gw * seg : vocab;
+  const int end = vocab - beg < seg ? vocab : beg + seg;
+  // f(x / T, index) for every element of this warp's share, sixteen loads in flight per lane (-0 as 0: equal values are
+  // one tie, whatever their sign bit)
+  auto visit = [&](auto&& f) {
+    for (int i0 = beg; i0 < end; i0 += 512) {
+      float xv[4][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) load4(row, i0 + u * 128 + 4 * lane, end, vec, xv[u]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = i0 + u * 128 + 4 * lane + e;
+          if (i < end) f(__fadd_rn(__fmul_rn(xv[u][e], invT), 0.f), i);
+        }
+    }
+  };
 
-  // 1. maximum of x / T
+  // 1. maximum of x / T (greedy: of x; no filter: of x / T + Gumbel noise, which is the draw)
   ArgMax a{-FLT_MAX, 0x7fffffff};
-  for (int i0 = beg; i0 < end; i0 += 512) {
-    float xv[4][4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) load4(row, i0 + u * 128 + 4 * lane, end, vec, xv[u]);
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int i = i0 + u * 128 + 4 * lane + e;
-        if (i < end) a = amax2(a, ArgMax{__fmul_rn(xv[u][e], invT), i});
-      }
+  if (plain) {
+    visit([&](float x, int i) { a = amax2(a, ArgMax{x - __logf(-__logf(uniform01(seed, step, i))), i}); });
+  } else {
+    visit([&](float x, int i) { a = amax2(a, ArgMax{x, i}); });
   }
   a = block_argmax(a, sh_am);
-  if (threadIdx.x == 0) sm->cmax = a;
+  if (tid == 0) sm->cmax = a;
   cluster_sync_all();
   {
     ArgMax g{-FLT_MAX, 0x7fffffff};
@@ -570,291 +600,268 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
     }
     a = g;
   }
-  const float mx = a.v;
-  const uint32_t hi_key = fkey(mx);
-
-  // 2. histogram of mx - x / T in unit bins: counts (two 16-bit counters per register) and softmax mass
-  {
-    uint32_t c[kCntBins / 2];
-    float m[kMassBins];
-#pragma unroll
-    for (int j = 0; j < kCntBins / 2; ++j) c[j] = 0u;
-#pragma unroll
-    for (int j = 0; j < kMassBins; ++j) m[j] = 0.f;
-    float z = 0.f;
-    for (int i0 = beg; i0 < end; i0 += 512) {
-      float xv[4][4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) load4(row, i0 + u * 128 + 4 * lane, end, vec, xv[u]);
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = i0 + u * 128 + 4 * lane + e;
-          if (i >= end) continue;
-          const float d = __fsub_rn(mx, __fmul_rn(xv[u][e], invT));   // no contraction: step 3 must agree
-          const float w = __expf(-d);
-          z += w;
-          if (d < static_cast<float>(kCntBins)) {
-            const int b = static_cast<int>(d);
-            const uint32_t inc = (b & 1) ? 0x10000u : 1u;
-#pragma unroll
-            for (int j = 0; j < kCntBins / 2; ++j) c[j] += ((b >> 1) == j) ? inc : 0u;
-#pragma unroll
-            for (int j = 0; j < kMassBins; ++j) m[j] += (b == j) ? w : 0.f;
-          }
-        }
-    }
-    // a warp's share is below 65536 elements for any vocabulary under 16 M, so the packed sums cannot carry
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      z += __shfl_xor_sync(0xffffffffu, z, o);
-#pragma unroll
-      for (int j = 0; j < kCntBins / 2; ++j) c[j] += __shfl_xor_sync(0xffffffffu, c[j], o);
-#pragma unroll
-      for (int j = 0; j < kMassBins; ++j) m[j] += __shfl_xor_sync(0xffffffffu, m[j], o);
-    }
-    if (lane == 0) {
-      sm->zall[warp] = z;
-#pragma unroll
-      for (int j = 0; j < kCntBins / 2; ++j) {
-        sm->cnt[2 * j][warp] = static_cast<int>(c[j] & 0xffffu);
-        sm->cnt[2 * j + 1][warp] = static_cast<int>(c[j] >> 16);
-      }
-#pragma unroll
-      for (int j = 0; j < kMassBins; ++j) sm->mass[j][warp] = m[j];
-    }
-  }
-  __syncthreads();
-  // this CTA's sums: warp b adds bin b over the warps (lane q holds warp q's figure)
-  {
-    int cb = sm->cnt[warp][lane];
-    float mb_ = warp < kMassBins ? sm->mass[warp][lane] : (warp == kMassBins ? sm->zall[lane] : 0.f);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      cb += __shfl_xor_sync(0xffffffffu, cb, o);
-      mb_ += __shfl_xor_sync(0xffffffffu, mb_, o);
-    }
-    if (lane == 0) {
-      sm->cta_cnt[warp] = cb;
-      if (warp < kMassBins) sm->cta_mass[warp] = mb_;
-      if (warp == kMassBins) sm->cta_z = mb_;
-    }
-  }
-  cluster_sync_all();
-  // the cluster's sums, added in CTA order by one thread per figure: all eight CTAs get the same numbers
-  if (threadIdx.x < kCntBins) {
-    int t = 0;
-    for (uint32_t r = 0; r < nclu; ++r) {
-      const int v = static_cast<int>(ld_cluster_u32(mapa_shared(&sm->cta_cnt[threadIdx.x], r)));
-      sm->peer_cnt[r][threadIdx.x] = v;
-      t += v;
-    }
-    sm->tot_cnt[threadIdx.x] = t;
-  } else if (threadIdx.x < kCntBins + kMassBins + 1) {
-    const int j = threadIdx.x - kCntBins;
-    const float* src = j < kMassBins ? &sm->cta_mass[j] : &sm->cta_z;
-    float t = 0.f;
-    for (uint32_t r = 0; r < nclu; ++r) t += __uint_as_float(ld_cluster_u32(mapa_shared(src, r)));
-    if (j < kMassBins) sm->tot_mass[j] = t; else sm->tot_z = t;
-  }
-  __syncthreads();
-  const float z_all = sm->tot_z;
-  // smallest window that holds the whole kept set: the k-th largest lies in it, the min-p bound does, and
-  // without either of those the nucleus does (its mass is at most tp times the total, which the window has)
-  const float d_m = use_m ? -__logf(mp) : 0.f;
-  int wsel = -1, n = 0;
-  {
-    int cum = 0;
-    float cum_m = 0.f;
-    for (int w = 0; w < kCntBins; ++w) {
-      cum += sm->tot_cnt[w];
-      if (w < kMassBins) cum_m += sm->tot_mass[w];
-      if (cum > kCluList) break;
-      const bool ok = (!use_k || cum >= k) && (!use_m || d_m + 0.01f < static_cast<float>(w + 1)) &&
-                      (use_k || use_m || (w < kMassBins && cum_m >= tp * z_all));
-      if (ok) { wsel = w; n = cum; break; }
-    }
-  }
-  if (wsel < 0) {
-    if (rank == 0 && threadIdx.x == 0) out[rowi] = -1;
-    cluster_sync_all();   // nobody leaves while a peer may still read its counters
+  if (greedy || plain) {           // the same decision in all CTAs of the cluster
+    if (rank == 0 && tid == 0) out[rowi] = a.i;
+    cluster_sync_all();            // nobody leaves while a peer may still read its maximum
     return;
   }
-  const float d_max = static_cast<float>(wsel + 1);       // candidates: mx - x / T < d_max
-  const uint32_t wlo = fkey(mx - d_max - 1.f);            // a key below every candidate's
+  const float mx = a.v;
+  const uint32_t hi_key = fkey(mx);
   const uint32_t km = use_m ? fkey(mx + __logf(mp)) : 0u;
-  int off = 0;   // candidates of the warps before this one, in index order
-  {
-    int mine = 0;   // lane l: candidates of this CTA's warp l
-    for (int b = 0; b <= wsel; ++b) mine += sm->cnt[b][lane];
-    int before = lane < warp ? mine : 0;
-    for (int r = lane; r < static_cast<int>(rank); r += 32)
-      for (int b = 0; b <= wsel; ++b) before += sm->peer_cnt[r][b];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
-    off = before;
-  }
 
-  // 3. candidates of the chosen window into the first CTA's list, in index order
-  {
-    const uint32_t list0 = mapa_shared(&sm->search.list[0], 0);
-    const uint32_t idx0 = mapa_shared(&sm->idx[0], 0);
-    for (int i0 = beg; i0 < end; i0 += 128) {
-      float xv[4];
-      load4(row, i0 + 4 * lane, end, vec, xv);
-      bool in[4];
-      int c = 0;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        xv[e] = __fmul_rn(xv[e], invT);
-        in[e] = i0 + 4 * lane + e < end && __fsub_rn(mx, xv[e]) < d_max;
-        c += in[e] ? 1 : 0;
+  // Histogram over the cluster: place(x, below, key) gives an element's bin or -1. This thread's kOwn bins come back as
+  // counts (want & 1) and masses (want & 2).
+  // `all_in`: the unit bin that holds every element placed, or -1 when the bins are the unit bins themselves.
+  auto histogram = [&](int want, int all_in, auto&& place, u64 (&c)[kOwn], u64 (&m)[kOwn]) {
+    cluster_sync_all();            // peers are done reading the bins of the pass before
+    for (int i = tid; i < kBins; i += kCluThreads) { sm->cnt[i] = 0; sm->hi[i] = 0; sm->lo[i] = 0; }
+    __syncthreads();
+    visit([&](float x, int) {
+      const float below = __fsub_rn(mx, x);
+      const int b = place(below, fkey(x));
+      if (b < 0) return;
+      if (want & 1) atomicAdd(&sm->cnt[b], 1u);
+      if (want & 2) {
+        const uint32_t q = __float2uint_rn(__expf((all_in < 0 ? b : all_in) / kBinsPerUnit - below) * 67108864.f);
+        atomicAdd(&sm->hi[b], q >> 13);
+        atomicAdd(&sm->lo[b], q & 0x1fffu);
       }
-      int incl = c;
+    });
+    cluster_sync_all();
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
+    for (int j = 0; j < kOwn; ++j) c[j] = m[j] = 0;
+    for (uint32_t r = 0; r < nclu; ++r) {
+      if (want & 1) {
+        const uint4 v = ld_cluster_v4(mapa_shared(&sm->cnt[tid * kOwn], r));
+        c[0] += v.x; c[1] += v.y; c[2] += v.z; c[3] += v.w;
       }
-      int pos = off + incl - c;
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (in[e]) {
-          if (pos < kCluList) {
-            st_cluster_u32(list0 + 4u * pos, __float_as_uint(xv[e]));
-            st_cluster_u32(idx0 + 4u * pos, static_cast<uint32_t>(i0 + 4 * lane + e));
-          }
-          ++pos;
-        }
-      off += __shfl_sync(0xffffffffu, incl, 31);
+      if (want & 2) {
+        const uint4 h = ld_cluster_v4(mapa_shared(&sm->hi[tid * kOwn], r)), l = ld_cluster_v4(mapa_shared(&sm->lo[tid * kOwn], r));
+        m[0] += (static_cast<u64>(h.x) << 13) + l.x; m[1] += (static_cast<u64>(h.y) << 13) + l.y;
+        m[2] += (static_cast<u64>(h.z) << 13) + l.z; m[3] += (static_cast<u64>(h.w) << 13) + l.w;
+      }
     }
-  }
-  cluster_sync_all();
-  if (rank != 0) return;
+    if (want & 2) {                // from 26 bits under the bin's edge to 42 under the maximum
+#pragma unroll
+      for (int j = 0; j < kOwn; ++j)
+        if (m[j]) m[j] = static_cast<u64>(static_cast<double>(m[j]) * (65536.0 * exp(-(all_in < 0 ? tid * kOwn + j : all_in) / static_cast<double>(kBinsPerUnit))));
+    }
+  };
+  // the first bin where the running sum of v reaches `target` (-1: none) and the sum before it
+  auto cross = [&](const u64 (&v)[kOwn], u64 target, int& bin, u64& above) {
+    if (tid == 0) sm->bin = -1;
+    u64 sum = 0, total;
+#pragma unroll
+    for (int j = 0; j < kOwn; ++j) sum += v[j];
+    u64 run = block_before(sum, sm->red, total);
+#pragma unroll
+    for (int j = 0; j < kOwn; ++j) {
+      if (run < target && run + v[j] >= target) { sm->bin = tid * kOwn + j; sm->above = run; }
+      run += v[j];
+    }
+    __syncthreads();
+    bin = sm->bin;
+    above = sm->above;
+    __syncthreads();
+  };
+  // the part of `whole` that a fraction in (0, 1) covers, at least 1
+  auto portion = [](float f, u64 whole) {
+    const double t = ceil(static_cast<double>(f) * static_cast<double>(whole));
+    const u64 r = t < 1.0 ? 1 : static_cast<u64>(t);
+    return r > whole ? whole : r;
+  };
 
-  // 4. cut-offs and the draw, on the list alone
-  SearchSmem* ss = &sm->search;
-  if (threadIdx.x < kSampThreads / 32) {
-    const int left = n - static_cast<int>(threadIdx.x) * kListPerWarp;
-    ss->wcnt[threadIdx.x] = left < 0 ? 0 : (left > kListPerWarp ? kListPerWarp : left);
+  // 2. bins under the maximum
+  u64 c[kOwn], m[kOwn], z_all = 0;
+  const bool nucleus = use_p && !use_k && !use_m;
+  histogram(nucleus ? 3 : 1, -1, [](float below, uint32_t) { return bin_of(below); }, c, m);
+  int last = -1, kbin = -1;
+  u64 kabove = 0, pabove = 0, ptarget = 0;
+  if (use_k) { cross(c, static_cast<u64>(k), kbin, kabove); last = kbin; }
+  if (use_m) last = max(last, bin_of(-__logf(mp) + 0.01f));
+  if (nucleus) {
+    block_before(m[0] + m[1] + m[2] + m[3], sm->red, z_all);
+    ptarget = portion(tp, z_all);
+    cross(m, ptarget, last, pabove);
   }
-  if (threadIdx.x == 0) { sm->pick = -1; sm->last = -1; sm->cut = -1; }
-  __syncthreads();
-  uint32_t thr_key = wlo;
-  float Z;
-  if (n <= kSampThreads) {
-    // Short list (the usual case): one candidate per thread. Its rank in descending order is the number of
-    // candidates ahead of it, counted directly; masses are then prefix-summed in rank order, and both
-    // cut-offs are read off the sorted values - a few microseconds instead of a dozen bisection passes.
-    float* sx = ss->list + kSampThreads;        // x / T by rank
-    float* sw = ss->list + 2 * kSampThreads;    // softmax mass by rank
-    float* sp = ss->list + 3 * kSampThreads;    // inclusive prefix of sw
-    const int t = threadIdx.x;
+  int n = 0x7fffffff;
+  {
+    u64 sum = c[0] + c[1] + c[2] + c[3], total, run = block_before(sum, sm->red, total);
+#pragma unroll
+    for (int j = 0; j < kOwn; ++j) {
+      run += c[j];
+      if (tid * kOwn + j == last) sm->n = run > 0x7fffffffu ? 0x7fffffff : static_cast<int>(run);
+    }
+    __syncthreads();
+    if (last >= 0) n = sm->n;
+  }
+
+  if (n <= kList) {
+    // 3a. candidates into the first CTA's list, in any order within a CTA's part of it. The positions come from a local
+    // counter: one shared by the cluster is a queue of remote atomics (512 of them took 25 us).
+    u64 part = 0, here;
+#pragma unroll
+    for (int j = 0; j < kOwn; ++j)
+      if (tid * kOwn + j <= last) part += sm->cnt[tid * kOwn + j];
+    block_before(part, sm->red, here);
+    if (tid == 0) { sm->wsum[0] = here; sm->fill = 0; }
+    cluster_sync_all();
+    uint32_t first = 0;
+    for (uint32_t r = 0; r < rank; ++r) first += static_cast<uint32_t>(ld_cluster_u64(mapa_shared(&sm->wsum[0], r)));
+    const uint32_t lx = mapa_shared(&sm->lx[0], 0), li = mapa_shared(&sm->li[0], 0);
+    visit([&](float x, int i) {
+      if (bin_of(__fsub_rn(mx, x)) > last) return;
+      const uint32_t pos = first + atomicAdd(&sm->fill, 1u);
+      if (pos >= kList) return;    // cannot happen: the same elements were counted
+      st_cluster_u32(lx + 4u * pos, __float_as_uint(x));
+      st_cluster_u32(li + 4u * pos, static_cast<uint32_t>(i));
+    });
+    cluster_sync_all();
+    if (rank != 0) return;
+    // one candidate per thread: its rank by value and by index, counted directly
     const int n4 = (n + 3) & ~3;
-    if (t >= n && t < n4) ss->list[t] = -FLT_MAX;
+    if (tid >= n && tid < n4) { sm->lx[tid] = -FLT_MAX; sm->li[tid] = 0x7fffffff; }
+    if (tid == 0) sm->cut = -1;
     __syncthreads();
-    if (t < n) {
-      const float x = ss->list[t];
-      const float4* l4 = reinterpret_cast<const float4*>(ss->list);
-      int rk = 0;
+    float x = 0.f;
+    int rk = 0;
+    if (tid < n) {
+      x = sm->lx[tid];
+      const int id = sm->li[tid];
+      int ri = 0;
       for (int j = 0; j < n4; j += 4) {
-        const float4 q = l4[j >> 2];
-        rk += (q.x > x || (q.x == x && j < t)) ? 1 : 0;
-        rk += (q.y > x || (q.y == x && j + 1 < t)) ? 1 : 0;
-        rk += (q.z > x || (q.z == x && j + 2 < t)) ? 1 : 0;
-        rk += (q.w > x || (q.w == x && j + 3 < t)) ? 1 : 0;
+        const float4 q = *reinterpret_cast<const float4*>(&sm->lx[j]);
+        const int4 o = *reinterpret_cast<const int4*>(&sm->li[j]);
+        rk += (q.x > x || (q.x == x && o.x < id)) + (q.y > x || (q.y == x && o.y < id)) + (q.z > x || (q.z == x && o.z < id)) +
+              (q.w > x || (q.w == x && o.w < id));
+        ri += (o.x < id) + (o.y < id) + (o.z < id) + (o.w < id);
       }
-      sx[rk] = x;
-      sw[rk] = __expf(x - mx);
+      sm->sx[rk] = x;
+      sm->ox[ri] = x;
+      sm->oi[ri] = id;
     }
     __syncthreads();
-    {
-      const float mine = t < n ? sw[t] : 0.f;
-      float incl = mine;
+    u64 total;
+    const u64 mine = tid < n ? weight_of(__fsub_rn(mx, sm->sx[tid])) : 0;
+    const u64 incl = block_before(mine, sm->red, total) + mine;
+    sm->sp[tid] = incl;
+    __syncthreads();
+    const float mx_rank = tid < n ? sm->sx[tid] : 0.f;
+    const uint32_t mykey = fkey(mx_rank);
+    uint32_t thr = 0;
+    if (use_k) thr = fkey(sm->sx[k - 1]);                  // k <= n by the choice of the bins
+    if (use_m) thr = max(thr, km);
+    if (thr > hi_key) thr = hi_key;                        // a min_p above one keeps the maximum alone
+    int kept = __syncthreads_count(tid < n && mykey >= thr);
+    u64 Z = kept > 0 ? sm->sp[kept - 1] : 0;
+    if (use_p && kept > 0) {
+      const u64 target = nucleus ? ptarget : portion(tp, Z);
+      if (tid < kept && incl >= target && incl - mine < target) sm->cut = tid;
+      __syncthreads();
+      const int r = sm->cut >= 0 ? sm->cut : kept - 1;
+      thr = max(thr, fkey(sm->sx[r]));
+      kept = __syncthreads_count(tid < n && mykey >= thr);
+      Z = sm->sp[kept - 1];
+    }
+    // inverse-CDF draw over the kept entries in index order
+    const u64 target = portion(uniform01(seed, step, 0xffffffffull), Z);
+    const float xo = tid < n ? sm->ox[tid] : 0.f;
+    const u64 w = (tid < n && fkey(xo) >= thr) ? weight_of(__fsub_rn(mx, xo)) : 0;
+    const u64 cum = block_before(w, sm->red, total);
+    if (w > 0 && cum < target && cum + w >= target) out[rowi] = sm->oi[tid];
+    if (total == 0 && tid == 0) out[rowi] = a.i;           // nothing has a weight (infinite or NaN logits)
+    return;
+  }
+
+  // 3b. exact cut-offs by refining the bin they lie in
+  auto refine = [&](int want, uint32_t least, int bin, u64 above, u64 target) -> uint32_t {
+    const float slack = fmaxf(fabsf(mx), 64.f) * 2e-6f;    // rounding of mx - x
+    uint32_t khi = min(hi_key, fkey(mx - bin / kBinsPerUnit + slack));
+    uint32_t klo = bin == kBins - 1 ? 0u : fkey(mx - (bin + 1) / kBinsPerUnit - slack);
+    klo = min(max(klo, least), khi);
+    uint32_t from = 0u, to = 0xffffffffu;
+    for (;;) {
+      const uint32_t range = khi - klo;
+      const int sh = range < static_cast<uint32_t>(kBins) ? 0 : 21 - __clz(range);
+      histogram(want, bin, [&](float below, uint32_t key) {
+        if (key < from || key > to || key < least || bin_of(below) != bin) return -1;
+        return static_cast<int>((khi - min(max(key, klo), khi)) >> sh);
+      }, c, m);
+      int b;
+      u64 before;
+      cross(want & 1 ? c : m, target - above, b, before);
+      if (b < 0) return klo;
+      above += before;
+      const uint32_t top = khi - (static_cast<uint32_t>(b) << sh);
+      if (sh == 0) return top;
+      const uint32_t width = (1u << sh) - 1;
+      klo = top - klo < width ? klo : top - width;
+      khi = top;
+      from = klo;
+      to = khi;
+    }
+  };
+  uint32_t thr = 0;
+  if (use_k) thr = kbin >= 0 ? refine(1, 0u, kbin, kabove, static_cast<u64>(k)) : 0u;
+  if (use_m) thr = max(thr, km);
+  if (thr > hi_key) thr = hi_key;
+  if (use_p) {
+    int bin = last;
+    if (!nucleus) {                                        // the mass of what the other filters keep
+      const uint32_t least = thr;
+      histogram(2, -1, [&](float below, uint32_t key) { return key >= least ? bin_of(below) : -1; }, c, m);
+      block_before(m[0] + m[1] + m[2] + m[3], sm->red, z_all);
+      ptarget = portion(tp, z_all);
+      cross(m, ptarget, bin, pabove);
+    }
+    if (bin >= 0) thr = max(thr, refine(2, thr, bin, pabove, ptarget));
+  }
+  // inverse-CDF draw in index order: the shares' masses, then the share that holds the target
+  u64 mass = 0;
+  visit([&](float x, int) { if (fkey(x) >= thr) mass += weight_of(__fsub_rn(mx, x)); });
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const float u = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += u;
-      }
-      if (lane == 31) sm->red[warp] = incl;
-      __syncthreads();
-      float woff = 0.f;
-      for (int q = 0; q < warp; ++q) woff += sm->red[q];
-      if (t < n) sp[t] = woff + incl;
-    }
-    __syncthreads();
-    if (use_k) thr_key = max(thr_key, fkey(sx[k - 1]));   // k <= n by the choice of the window
-    if (use_m) thr_key = max(thr_key, km);
-    if (thr_key > hi_key) thr_key = hi_key;               // a min_p above one keeps the maximum alone
-    int m = __syncthreads_count(t < n && fkey(sx[t]) >= thr_key);
-    Z = (use_k || use_m) ? sp[m - 1] : z_all;
-    if (use_p) {
-      const float target = tp * Z;
-      if (t < m && sp[t] >= target && (t == 0 || sp[t - 1] < target)) sm->cut = t;
-      __syncthreads();
-      const int r = sm->cut >= 0 ? sm->cut : m - 1;
-      thr_key = max(thr_key, fkey(sx[r]));
-      m = __syncthreads_count(t < n && fkey(sx[t]) >= thr_key);
-      Z = sp[m - 1];
-    }
+  for (int o = 16; o > 0; o >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, o);
+  if (lane == 0) sm->wsum[warp] = mass;
+  cluster_sync_all();
+  if (tid < nwarps) sm->all[tid] = ld_cluster_u64(mapa_shared(&sm->wsum[tid % kCluWarps], tid / kCluWarps));
+  __syncthreads();
+  u64 Z = 0, base = 0;
+  for (int q = 0; q < nwarps; ++q) {
+    if (q == gw) base = Z;
+    Z += sm->all[q];
+  }
+  if (Z == 0) {
+    if (rank == 0 && tid == 0) out[rowi] = a.i;
   } else {
-    if (use_k) {
-      uint32_t lo = wlo, hi = hi_key;
-      float above = 0.f;
-      while (lo < hi) multiway_pass<false, true>(row, vocab, invT, mx, ss, lo, hi, static_cast<float>(k), above);
-      thr_key = lo;
+    const u64 target = portion(uniform01(seed, step, 0xffffffffull), Z);
+    if (base < target && base + mass >= target) {
+      for (int i0 = beg; i0 < end && base < target; i0 += 128) {
+        float xv[4];
+        load4(row, i0 + 4 * lane, end, vec, xv);
+        u64 w[4], mine = 0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float x = __fadd_rn(__fmul_rn(xv[e], invT), 0.f);
+          w[e] = (i0 + 4 * lane + e < end && fkey(x) >= thr) ? weight_of(__fsub_rn(mx, x)) : 0;
+          mine += w[e];
+        }
+        u64 incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const u64 t = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += t;
+        }
+        u64 cum = base + incl - mine;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (w[e] > 0 && cum < target && cum + w[e] >= target) out[rowi] = i0 + 4 * lane + e;
+          cum += w[e];
+        }
+        base += __shfl_sync(0xffffffffu, incl, 31);
+      }
     }
-    if (use_m) thr_key = max(thr_key, km);
-    if (thr_key > hi_key) thr_key = hi_key;
-    Z = (use_k || use_m) ? list_mass_ge(ss, mx, thr_key) : z_all;
-    if (use_p) {
-      uint32_t lo = thr_key, hi = hi_key;
-      float above = 0.f;
-      const float target = tp * Z;
-      while (lo < hi) multiway_pass<true, true>(row, vocab, invT, mx, ss, lo, hi, target, above);
-      thr_key = lo;
-      Z = list_mass_ge(ss, mx, thr_key);
-    }
   }
-  // inverse-CDF draw over the kept entries, which sit in index order: eight consecutive entries per thread
-  const uint64_t seed = seeds ? seeds[rowi] : 0x1234ull + rowi;
-  const float target = uniform01(seed, step, 0xffffffffull) * Z;
-  constexpr int kPer = kCluList / kSampThreads;
-  float w[kPer];
-  float mine = 0.f;
-  int last_kept = -1;
-#pragma unroll
-  for (int e = 0; e < kPer; ++e) {
-    const int p = threadIdx.x * kPer + e;
-    const float x = p < n ? ss->list[p] : 0.f;
-    w[e] = (p < n && fkey(x) >= thr_key) ? __expf(x - mx) : 0.f;
-    mine += w[e];
-    if (w[e] > 0.f) last_kept = p;
-  }
-  float incl = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  if (lane == 31) sm->red[warp] = incl;
-  __syncthreads();
-  float woff = 0.f;
-  for (int q = 0; q < warp; ++q) woff += sm->red[q];
-  float cum = woff + incl - mine;
-#pragma unroll
-  for (int e = 0; e < kPer; ++e) {
-    if (w[e] > 0.f && cum + w[e] >= target && cum < target) atomicMax(&sm->pick, static_cast<int>(threadIdx.x) * kPer + e);
-    cum += w[e];
-  }
-  if (last_kept >= 0) atomicMax(&sm->last, last_kept);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    // rounding can leave the target just above the total mass: the last kept entry then
-    const int p = sm->pick >= 0 ? sm->pick : sm->last;
-    out[rowi] = p >= 0 ? sm->idx[p] : a.i;
-  }
+  cluster_sync_all();              // nobody leaves while a peer may still read its sums
 }
 
 // One thread per (row, distinct history token). counts > 0 are output-token counts for
@@ -895,10 +902,7 @@ extern "C" int mb_sample_topk_topp(const float* logits, int64_t* out, int rows, 
                                    const float* top_p, const float* min_p, const uint64_t* seeds,
                                    uint64_t step, cudaStream_t stream) {
   if (rows <= 0) return MB_OK;
-  // rows with a top-k / top-p / min-p filter go to the cluster kernel first; what it leaves (out = -1: greedy
-  // and plain-temperature rows, kept sets too wide for its list) is drawn by the one-CTA kernel after it
-  bool clustered = g_sample_cluster && (top_k || top_p || min_p) && rows <= 65535;
-  if (clustered) {
+  if (g_sample_cluster && rows <= 65535 && vocab <= kClu * kMaxShare) {
     static PerDeviceOnce once;
     if (once.needed()) {
       if (cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -906,7 +910,7 @@ extern "C" int mb_sample_topk_topp(const float* logits, int64_t* out, int rows, 
         return MB_ERR_LAUNCH;
       once.done();
     }
-    // as many CTAs per row as still lets the whole batch run at once (one CTA of this size per SM)
+    // as many CTAs per row as still lets the whole batch run at once (two CTAs of this size per SM)
     static int sms = 0;
     if (sms == 0) {
       int dev = 0;
@@ -914,29 +918,30 @@ extern "C" int mb_sample_topk_topp(const float* logits, int64_t* out, int rows, 
       if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     }
     int c = kClu;
-    while (c > 1 && rows * c > sms) c >>= 1;
+    while (c > 1 && rows * c > 2 * sms && vocab <= (kMaxShare / 2) * c) c >>= 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(c, rows);
-    cfg.blockDim = dim3(kSampThreads);
+    cfg.blockDim = dim3(kCluThreads);
     cfg.dynamicSmemBytes = sizeof(ClusterSmem);
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = c;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
     if (cudaLaunchKernelEx(&cfg, sample_cluster_kernel, logits, out, vocab, ld, temperature, top_k, top_p, min_p,
-                           seeds, step) != cudaSuccess) {
-      // a device (or partition) that cannot place such clusters: every row goes to the one-CTA kernel from now on
-      cudaGetLastError();
-      g_sample_cluster = false;
-      clustered = false;
-    }
+                           seeds, step) == cudaSuccess)
+      return MB_OK;
+    // a device (or partition) that cannot place such clusters: every row goes to the one-CTA kernel from now on
+    cudaGetLastError();
+    g_sample_cluster = false;
   }
   return launch_k(sample_kernel, dim3(rows), dim3(kSampThreads), 0, stream, logits, out, vocab, ld, temperature,
-                  top_k, top_p, min_p, seeds, step, clustered ? 1 : 0) == cudaSuccess ? MB_OK : MB_ERR_LAUNCH;
+                  top_k, top_p, min_p, seeds, step) == cudaSuccess ? MB_OK : MB_ERR_LAUNCH;
 }
 
 // 0: every row is sampled by the one-CTA kernel (the cluster kernel is not launched)

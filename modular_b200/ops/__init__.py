@@ -423,8 +423,8 @@ def set_gemm_pair_token_major(mask: int) -> None:
 
 
 def set_sample_cluster(on: bool) -> None:
-    """Whether rows with a top-k / top-p / min-p filter are first sampled by the kernel that spreads a row
-    over a cluster of eight CTAs (default on); off leaves every row to the one-CTA-per-row kernel."""
+    """Whether rows are sampled by the kernel that spreads a row over a cluster of up to eight CTAs (default on); off
+    leaves every row to the one-CTA-per-row kernel."""
     _lib().set_sample_cluster(bool(on))
 
 

@@ -335,6 +335,34 @@ def test_cluster_sampler_matches_one_cta_sampler():
     ops.check_device_error()
 
 
+@pytest.mark.parametrize("V", [128256, 50001, 700, 1])
+def test_sampler_kept_sets_beyond_the_list(V):
+    """Cut-offs that need the refinement passes: a nucleus of thousands, a k-th token far below the first, ties, masked tokens."""
+    torch.manual_seed(82)
+    R = 40
+    flat = torch.randn(R, V, device=DEV) * 1.5
+    confident = torch.randn(R, V, device=DEV)
+    confident[:, V // 2] += 45.0
+    ties = torch.round(torch.randn(R, V, device=DEV) * 2) / 2 + 0.0      # no -0: the other kernel orders it below 0
+    masked = flat.clone()
+    masked[:, V // 3 + 1:] = float("-inf")
+    seeds = torch.arange(R, device=DEV, dtype=torch.int64) * 17 + 3
+    temp = torch.full((R,), 0.7, device=DEV)
+    i32 = lambda v: torch.full((R,), v, device=DEV, dtype=torch.int32)
+    f32 = lambda v: torch.full((R,), v, device=DEV)
+    for name, lg in (("flat", flat), ("confident", confident), ("ties", ties), ("masked", masked)):
+        for kw in (dict(top_p=f32(0.9)), dict(top_k=i32(40)), dict(top_k=i32(5000), top_p=f32(0.8)), dict(min_p=f32(1e-4)),
+                   dict(top_p=f32(0.999), min_p=f32(1e-5)), dict()):
+            a = ops.sample(lg, temperature=temp, seeds=seeds, step=5, **kw)
+            ops.set_sample_cluster(False)
+            b = ops.sample(lg, temperature=temp, seeds=seeds, step=5, **kw)
+            ops.set_sample_cluster(True)
+            # one row may meet a bucket edge within the rounding of the other kernel's fp32 sums
+            assert (a != b).sum().item() <= 1, (name, list(kw), a.tolist(), b.tolist())
+            again = ops.sample(lg, temperature=temp, seeds=seeds, step=5, **kw)
+            assert torch.equal(a, again)
+
+
 def test_penalties():
     torch.manual_seed(9)
     logits = torch.randn(3, 1000, device=DEV)
