@@ -310,6 +310,315 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   }
 }
 
+// ---------------------------------------------------------------- tokens on the M side
+// The same product for larger token counts, operands the other way round: 128 token rows per CTA on the MMA's M side, 256
+// weight rows (two scale blocks) on its N side, so a promotion thread owns one token and 128 features and one K group
+// has one factor per thread, in a register. With weights on M every column has a factor of its own, and reading those
+// from shared memory (512 wavefronts a K group, beside 512 for the operands) is what bounds that form: L1 pipe 80 % busy,
+// tensor pipe 20 %. Accumulators are 128 fp32 registers per thread, added two at a time; the K group after next is
+// multiplied into the other of two 256-column TMEM buffers meanwhile. The sums run over K in the same order as above.
+// CTAs are persistent, so one tile's stores run under the next one's first loads.
+//   PAIR    dense: two CTAs share the tile (256 tokens x 256 weight rows, each loads half of either operand), which halves
+//           the bytes per operation that come from L2: 2050 x 57344 x 8192 in 1140 us (2094 with weights on M).
+//   !PAIR   experts: the tiles of one expert's tokens after another; weights are read from memory once and are the bound:
+//           16800 rows, 256 experts of 4096 x 7168: 1400 us (2998 with weights on M).
+constexpr int kRowStages = 6, kRowTileN = 256, kMaxRowTiles = 1024;
+// warp 0 TMA, warp 1 MMA, warp 2 the experts' tiles, warps 4-11 promotion (setmaxnreg works on groups of four warps)
+constexpr int kRowThreads = 384;
+constexpr int kAhead = 4;             // K groups whose factors are on their way
+constexpr int kRowsFrom = 128;
+
+struct RowTail {
+  uint64_t full[8];
+  uint64_t empty[8];
+  uint64_t acc_full[2];
+  uint64_t acc_empty[2];
+  uint32_t tmem_base;
+  int abort_word;
+  int n_tiles;                        // grouped: token tiles
+  int2 tile[kMaxRowTiles];            // grouped: expert, first row
+  float factor[8][kAhead][64];        // per promotion warp and K group: sx of its 32 rows, then sw 32 times
+};
+
+__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ uint64_t fma2(uint32_t lo, uint32_t hi, uint64_t s, uint64_t acc) {
+  uint64_t v, r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(v), "l"(s), "l"(acc));
+  return r;
+}
+
+template <bool PAIR, bool RESID>
+__global__ void __launch_bounds__(kRowThreads, 1)
+gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  constexpr int kB = PAIR ? kATile : 2 * kATile, kStage = kATile + kB;
+  RowTail* tail = reinterpret_cast<RowTail*>(smem + p.stages * kStage);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+  const int worker = PAIR ? blockIdx.x >> 1 : blockIdx.x, workers = PAIR ? gridDim.x >> 1 : gridDim.x;
+  const int kb_total = (p.K + 127) / 128;
+  const int n_blocks = (p.N + kRowTileN - 1) / kRowTileN;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(&tail->full[s], 1);
+      mbar_init(&tail->empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&tail->acc_full[b], 1);
+      mbar_init(&tail->acc_empty[b], PAIR ? 16 : 8);
+    }
+    tail->abort_word = 0;
+    fence_mbar_init();
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
+  if (warp == 1) {
+    if (PAIR) { tmem_alloc_pair(&tail->tmem_base, 512); tmem_relinquish_pair(); }
+    else { tmem_alloc(&tail->tmem_base, 512); tmem_relinquish(); }
+  }
+  if (!PAIR && warp == 2) {
+    // the token tiles of all experts, in expert order
+    int base = 0;
+    for (int c = 0; c < p.n_experts; c += 32) {
+      const int j = c + lane;
+      const int b = j < p.n_experts ? p.expert_offsets[j] : 0;
+      const int en = j < p.n_experts ? p.expert_offsets[j + 1] : 0;
+      const int nt = (en - b + kBM - 1) / kBM;
+      int incl = nt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      for (int i = 0; i < nt && base + incl - nt + i < kMaxRowTiles; ++i) tail->tile[base + incl - nt + i] = make_int2(j, b + i * kBM);
+      base += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) tail->n_tiles = min(base, kMaxRowTiles);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (PAIR) cluster_sync_all();         // the peer's barriers exist before anything is sent to them
+  tc_fence_after();
+  const uint32_t tmem_base = tail->tmem_base;
+  volatile int* abort_word = &tail->abort_word;
+  const int m_tiles = PAIR ? (p.M + 2 * kBM - 1) / (2 * kBM) : tail->n_tiles;
+  const int total = m_tiles * n_blocks;
+  // tile t: first token row of this CTA, end of its rows, first weight row, first rows of the expert
+  auto place = [&](int t, int& row0, int& row_end, int& n0, int& expert) {
+    if (PAIR) {
+      row0 = (t % m_tiles) * (2 * kBM) + static_cast<int>(rank) * kBM;
+      row_end = p.M;
+      n0 = (t / m_tiles) * kRowTileN;
+      expert = 0;
+    } else {
+      const int2 at = tail->tile[t / n_blocks];
+      row0 = at.y;
+      row_end = p.expert_offsets[at.x + 1];
+      n0 = (t % n_blocks) * kRowTileN;
+      expert = at.x;
+    }
+  };
+
+  // 384 x 168 registers at launch: four warps give theirs up, eight take them (128 x 56 + 256 x 224 is the same sum)
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if (warp == 0 && lane == 0) {
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int t = worker; t < total && ok; t += workers) {
+        int row0, row_end, n0, expert;
+        place(t, row0, row_end, n0, expert);
+        const int w0 = expert * p.w_rows + n0;
+        for (int kb = 0; kb < kb_total; ++kb) {
+          if (!mbar_wait(&tail->empty[s], ph ^ 1, abort_word, p.err, 511)) { ok = false; break; }
+          uint8_t* sa = smem + s * kStage;
+          if (PAIR) {
+            if (rank == 0) mbar_arrive_expect_tx(&tail->full[s], 2 * kStage);
+            const uint32_t full_leader = mapa_shared(&tail->full[s], 0);
+            tma_load_2d_pair(sa, &tmX, full_leader, kb * 128, row0);
+            tma_load_2d_pair(sa + kATile, &tmW, full_leader, kb * 128, w0 + static_cast<int>(rank) * kBM);
+          } else {
+            mbar_arrive_expect_tx(&tail->full[s], kStage);
+            tma_load_2d(sa, &tmX, &tail->full[s], kb * 128, row0);
+            tma_load_2d(sa + kATile, &tmW, &tail->full[s], kb * 128, w0);
+            tma_load_2d(sa + 2 * kATile, &tmW, &tail->full[s], kb * 128, w0 + kBM);
+          }
+          if (++s == p.stages) { s = 0; ph ^= 1; }
+        }
+      }
+    } else if (warp == 1 && lane == 0 && rank == 0) {
+      const uint32_t idesc = umma_idesc(PAIR ? 2 * kBM : kBM, kRowTileN, 0, 0);
+      const uint32_t empty0 = mapa_shared(&tail->empty[0], 0), empty1 = PAIR ? mapa_shared(&tail->empty[0], 1) : 0u;
+      const uint32_t afull0 = mapa_shared(&tail->acc_full[0], 0), afull1 = PAIR ? mapa_shared(&tail->acc_full[0], 1) : 0u;
+      int s = 0;
+      uint32_t ph = 0, g = 0;            // g: K groups so far, over all tiles
+      bool ok = true;
+      for (int t = worker; t < total && ok; t += workers) {
+        for (int kb = 0; kb < kb_total; ++kb, ++g) {
+          const uint32_t buf = g & 1;
+          ok = mbar_wait(&tail->acc_empty[buf], ((g >> 1) & 1) ^ 1, abort_word, p.err, 512) &&
+               mbar_wait(&tail->full[s], ph, abort_word, p.err, 513);
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t da = umma_desc_sw128(smem + s * kStage), db = umma_desc_sw128(smem + s * kStage + kATile);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint64_t koff = static_cast<uint64_t>(k * 32 >> 4);
+            if (PAIR) umma_fp8_pair(tmem_base + buf * kRowTileN, da + koff, db + koff, idesc, k > 0 ? 1u : 0u);
+            else umma_fp8(tmem_base + buf * kRowTileN, da + koff, db + koff, idesc, k > 0 ? 1u : 0u);
+          }
+          if (PAIR) {
+            tc_commit_pair(empty0 + 8u * s);
+            tc_commit_pair(empty1 + 8u * s);
+            tc_commit_pair(afull0 + 8u * buf);
+            tc_commit_pair(afull1 + 8u * buf);
+          } else {
+            tc_commit(&tail->empty[s]);
+            tc_commit(&tail->acc_full[buf]);
+          }
+          if (++s == p.stages) { s = 0; ph ^= 1; }
+        }
+      }
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    const int quad = warp & 3, half = (warp - 4) >> 2;
+    const uint32_t addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + half * 128;
+    const uint32_t aempty = mapa_shared(&tail->acc_empty[0], 0);
+    uint32_t g = 0;
+    bool ok = true;
+    for (int t = worker; t < total && ok; t += workers) {
+      int row0, row_end, n0, expert;
+      place(t, row0, row_end, n0, expert);
+      const int row = row0 + quad * 32 + lane, col0 = n0 + half * 128;
+      const bool live = row < row_end;
+      const float* sx = p.sx + (live ? row : 0);
+      const float* sw = p.sw + static_cast<size_t>(expert * p.sw_rows + (col0 < p.N ? col0 : 0) / 128) * p.sw_ld;
+      uint64_t acc[64];
+#pragma unroll
+      for (int i = 0; i < 64; ++i) acc[i] = 0;
+      // a lane fetches its own factors, kAhead K groups ahead (one commit per K group, empty beyond the last one)
+      float* mine = &tail->factor[warp - 4][0][lane];
+      auto fetch = [&](int kb) {
+        if (kb < kb_total) {
+          cp_async4(mine + (kb % kAhead) * 64, sx + static_cast<size_t>(kb) * p.M);
+          cp_async4(mine + (kb % kAhead) * 64 + 32, sw + kb);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) fetch(j);
+      for (int kb = 0; kb < kb_total; ++kb) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
+          const float* at = mine + (kb % kAhead) * 64;
+          const float f = live ? at[0] * at[32] : 0.f;
+          fetch(kb + kAhead);
+          uint64_t f2;
+          asm("mov.b64 %0, {%1, %1};" : "=l"(f2) : "r"(__float_as_uint(f)));
+          const uint32_t buf = g & 1;
+          ok = mbar_wait(&tail->acc_full[buf], (g >> 1) & 1, abort_word, p.err, 514);
+          if (!ok) break;
+          ++g;
+          tc_fence_after();
+          // a load of the next columns is in flight while these are added
+          constexpr int W = 32;
+          uint32_t v[2][W];
+          tmem_ld_32x32(addr + buf * kRowTileN, v[0]);
+#pragma unroll
+          for (int c = 0; c < 128 / W; ++c) {
+            tc_wait_ld();
+            if (c < 128 / W - 1) {
+              tmem_ld_32x32(addr + buf * kRowTileN + (c + 1) * W, v[(c + 1) & 1]);
+            } else {                     // everything is read: the buffer may be overwritten
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_cluster_relaxed(aempty + 8u * buf);
+            }
+#pragma unroll
+            for (int i = 0; i < W / 2; ++i) acc[c * (W / 2) + i] = fma2(v[c & 1][2 * i], v[c & 1][2 * i + 1], f2, acc[c * (W / 2) + i]);
+          }
+      }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      if (!ok) break;
+      // 64 features (one 128-byte line) at a time; a residual line is read before the line before it is written
+      __nv_bfloat16* y = p.Y + static_cast<size_t>(live ? row : 0) * p.ldy + col0;
+      const __nv_bfloat16* r = RESID ? p.R + static_cast<size_t>(live ? row : 0) * p.ldr + col0 : nullptr;
+      uint4 res[2][8];
+      auto read_line = [&](int l, uint4 (&to)[8]) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          to[q] = live && col0 + l * 64 + q * 8 + 8 <= p.N ? *reinterpret_cast<const uint4*>(r + l * 64 + q * 8) : make_uint4(0, 0, 0, 0);
+      };
+      if (RESID) read_line(0, res[0]);
+#pragma unroll
+      for (int l = 0; l < 2; ++l) {
+        if (RESID && l == 0) read_line(1, res[1]);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          uint4 o;
+          uint32_t* w = &o.x;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint64_t a = acc[l * 32 + q * 4 + i];
+            __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(static_cast<uint32_t>(a)), __uint_as_float(static_cast<uint32_t>(a >> 32)));
+            if (RESID) {                 // the product is rounded before the residual is added, as with weights on M
+              const float2 fa = __bfloat1622float2(h);
+              const float2 fb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&(&res[l][q].x)[i]));
+              h = __floats2bfloat162_rn(fa.x + fb.x, fa.y + fb.y);
+            }
+            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+          }
+          if (live && col0 + l * 64 + q * 8 + 8 <= p.N) *reinterpret_cast<uint4*>(y + l * 64 + q * 8) = o;
+        }
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (PAIR) cluster_sync_all();         // neither CTA leaves while the other may still use its memory or barriers
+  if (warp == 1) {
+    tc_fence_after();
+    if (PAIR) tmem_dealloc_pair(tmem_base, 512);
+    else tmem_dealloc(tmem_base, 512);
+  }
+}
+
+template <bool PAIR, bool RESID>
+static int launch_rows(const Params& q, int num_sms, int tiles, const CUtensorMap& tw, const CUtensorMap& tx, cudaStream_t stream) {
+  Params p = q;
+  p.stages = PAIR ? kRowStages : 4;
+  const size_t smem = static_cast<size_t>(p.stages) * (PAIR ? 2 : 3) * kATile + sizeof(RowTail) + 1024;
+  auto kern = gemm_fp8_rows_kernel<PAIR, RESID>;
+  static PerDeviceOnce configured;
+  if (configured.needed()) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return MB_ERR_LAUNCH;
+    configured.done();
+  }
+  cudaLaunchConfig_t cfg = {};
+  const int workers = PAIR ? num_sms / 2 : num_sms;
+  cfg.gridDim = dim3(static_cast<unsigned>((tiles < workers ? tiles : workers) * (PAIR ? 2 : 1)));
+  cfg.blockDim = dim3(kRowThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = PAIR ? 2 : 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, tw, tx, p) == cudaSuccess ? MB_OK : MB_ERR_LAUNCH;
+}
+
 // Sum of the split-K partials [splits, M, N] (+ residual) -> bf16 Y; N % 4 == 0.
 __global__ void fp8_splitk_reduce_kernel(const float* __restrict__ part, const __nv_bfloat16* __restrict__ R,
                                          __nv_bfloat16* __restrict__ Y, int M, int N, int splits) {
@@ -494,16 +803,28 @@ extern "C" int mb_gemm_fp8_blockscaled(const void* Xq, const float* Xs, const vo
   if ((reinterpret_cast<uintptr_t>(Xq) | reinterpret_cast<uintptr_t>(Wq) | reinterpret_cast<uintptr_t>(Y) |
        reinterpret_cast<uintptr_t>(R)) & 15)
     return MB_ERR_ALIGN;
+  // Up to 128 tokens the other form streams the weights faster (64 tokens, 57344 x 8192: 157 against 177 us, one token 113
+  // against 178: its narrow token tiles leave room for more stages); at 300 tokens 28672 -> 8192 it takes 301 us, this one 153.
+  const bool rows_form = bn <= 0 && splits <= 0 && M > kRowsFrom && N >= kRowTileN && num_sms >= 2;
   if (bn <= 0) {
     const int mt = (M + 127) / 128;
     bn = ((M + mt - 1) / mt + 31) / 32 * 32;
   }
   if (bn % 32 || bn < 32 || bn > 128) return MB_ERR_SHAPE;
-  Params p;
+  Params p = {};
   p.Y = static_cast<__nv_bfloat16*>(Y);
   p.R = static_cast<const __nv_bfloat16*>(R);
   p.sw = Ws; p.sx = Xs; p.err = err;
   p.M = M; p.N = N; p.K = K; p.ldy = N; p.ldr = N; p.sw_ld = (K + 127) / 128; p.BN = bn;
+  if (rows_form) {
+    CUtensorMap tw, tx;
+    int rc = cached_tmap(&tw, Wq, N, K, K, kBM, 1);
+    if (rc != MB_OK) return rc;
+    rc = cached_tmap(&tx, Xq, M, K, K, kBM, 1);
+    if (rc != MB_OK) return rc;
+    const int tiles = ((M + 2 * kBM - 1) / (2 * kBM)) * ((N + kRowTileN - 1) / kRowTileN);
+    return (flags & 2) ? launch_rows<true, true>(p, num_sms, tiles, tw, tx, stream) : launch_rows<true, false>(p, num_sms, tiles, tw, tx, stream);
+  }
   const int stage_bytes = kATile + bn * kBKBytes;
   const int max_stages = (227 * 1024 - 1024 - 8 * kStgWarp - static_cast<int>(sizeof(Tail)) - 256) / stage_bytes;
   if (stages <= 0 || stages > max_stages) stages = max_stages;
@@ -565,17 +886,35 @@ extern "C" int mb_grouped_gemm_fp8_blockscaled(const void* Xq, const float* Xs, 
   if ((reinterpret_cast<uintptr_t>(Xq) | reinterpret_cast<uintptr_t>(Wq) | reinterpret_cast<uintptr_t>(Y)) & 15)
     return MB_ERR_ALIGN;
   if (max_rows <= 0 || max_rows > total_rows) max_rows = total_rows;
+  // tokens on the M side for any number of rows (256 experts of 4096 x 7168: 48 tokens with 8 experts each 1003 against 1384 us,
+  // 512 tokens 1340 against 2292): the weights' stream is the bound, and tiles of 256 weight rows keep it full
+  const bool rows_form = bn <= 0 && n_experts + total_rows / kBM <= kMaxRowTiles;
   if (bn <= 0) {
     // expected rows per expert decide the token tile: small tiles when experts see few tokens
     const int avg = (total_rows + n_experts - 1) / n_experts;
     bn = avg <= 32 ? 32 : (avg <= 64 ? 64 : 128);
   }
   if (bn % 32 || bn < 32 || bn > 128) return MB_ERR_SHAPE;
-  Params p;
+  Params p = {};
   p.Y = static_cast<__nv_bfloat16*>(Y);
   p.R = nullptr;
   p.sw = Ws; p.sx = Xs; p.err = err;
   p.M = total_rows; p.N = N; p.K = K; p.ldy = N; p.ldr = N; p.sw_ld = (K + 127) / 128; p.BN = bn;
+  if (rows_form) {
+    p.expert_offsets = expert_offsets;
+    p.n_experts = n_experts;
+    p.w_rows = N;
+    p.sw_rows = N / 128;
+    CUtensorMap tw, tx;
+    int rc = cached_tmap(&tw, Wq, static_cast<uint64_t>(n_experts) * N, K, K, kBM, 1);
+    if (rc != MB_OK) return rc;
+    rc = cached_tmap(&tx, Xq, total_rows, K, ldx, kBM, 1);
+    if (rc != MB_OK) return rc;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return launch_rows<false, false>(p, sms, 1 << 30, tw, tx, stream);
+  }
   const int stage_bytes = kATile + bn * kBKBytes;
   const int max_stages = (227 * 1024 - 1024 - 8 * kStgWarp - static_cast<int>(sizeof(Tail)) - 256) / stage_bytes;
   if (stages <= 0 || stages > max_stages) stages = max_stages;

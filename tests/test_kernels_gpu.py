@@ -422,6 +422,40 @@ def test_gemm_fp8_blockscaled_split_k_matches_single_pass():
     assert _rel_err(y1, ref.linear_fp8_blockscaled(xq, xs, wq, ws, r)) < 5e-3
 
 
+@pytest.mark.parametrize("M,N,K", [(129, 256, 128), (256, 264, 144), (257, 384, 640), (300, 1000, 1152), (513, 4096, 512), (1024, 256, 4096)])
+def test_gemm_fp8_tokens_on_m(M, N, K):
+    """Larger token counts put tokens on the MMA's M side: the same sums in the same order as with weights there."""
+    torch.manual_seed(M)
+    wq, ws = ref.quant_fp8_weight_block128(torch.randn(N, K, device=DEV) * 0.05)
+    xq, xs = ops.quant_fp8_group128((torch.randn(M, K, device=DEV) * 2).to(torch.bfloat16))
+    r = torch.randn(M, N, device=DEV).to(torch.bfloat16)
+    for res in (None, r):
+        y = ops.linear_fp8_blockscaled(xq, xs, wq, ws, residual=res)
+        assert torch.equal(y, ops.linear_fp8_blockscaled(xq, xs, wq, ws, residual=res, bn=128, splits=1))
+        assert _rel_err(y, ref.linear_fp8_blockscaled(xq, xs, wq, ws, res)) < 5e-3
+    h = r.clone()
+    ops.linear_fp8_blockscaled(xq, xs, wq, ws, residual=h, out=h)          # in place, as the step executor does
+    assert torch.equal(h, y)
+    ops.check_device_error()
+
+
+@pytest.mark.parametrize("counts,N,K", [([0, 1, 127, 128, 129, 300, 0, 2], 384, 256), ([40] * 33, 128, 144), ([700, 0, 0, 5], 512, 1152)])
+def test_grouped_gemm_fp8_tokens_on_m(counts, N, K):
+    from modular_b200._native import lib
+
+    torch.manual_seed(len(counts))
+    E, n = len(counts), sum(counts)
+    wq = torch.randn(E, N, K, device=DEV).mul_(60).clamp_(-448, 448).to(torch.float8_e4m3fn)
+    ws = torch.rand(E, N // 128, (K + 127) // 128, device=DEV) * 1e-3
+    xq, xs = ops.quant_fp8_group128(torch.randn(n + 3, K, device=DEV).to(torch.bfloat16))        # three rows of nobody
+    off = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device=DEV)
+    y, want = (torch.full((n + 3, N), 7.0, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    lib().grouped_gemm_fp8(xq, xs, wq, ws, y, off, 0, 0)
+    lib().grouped_gemm_fp8(xq, xs, wq, ws, want, off, 0, 128)                                     # weights on M
+    assert torch.equal(y, want)
+    ops.check_device_error()
+
+
 def test_grouped_gemm_fp8_and_fp8_experts():
     """Grouped block-scaled fp8 GEMM against per-expert references, and a MoE layer with fp8 expert weights
     against the same layer with those weights dequantised to bf16."""
