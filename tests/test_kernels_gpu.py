@@ -263,6 +263,30 @@ def test_paged_attention_mixed_batch(n_q, n_kv, hd, ps, tma):
     assert (o.float() - o_ref.float()).abs().max() < 3e-2
 
 
+@pytest.mark.parametrize("counts,N,K,swiglu", [([0, 257, 1, 900, 255, 256, 0, 3], 384, 128, False), ([700, 0, 513], 200, 72, True),
+                                              ([300] * 5, 1408, 256, True), ([128, 128], 256, 64, False)])
+def test_grouped_gemm_pairs(counts, N, K, swiglu):
+    """Experts with many rows take the token-major pairs: rows and features around tiles of 256 and 128, empty experts."""
+    from modular_b200._native import lib
+
+    torch.manual_seed(len(counts))
+    E, n = len(counts), sum(counts)
+    x = torch.randn(n, K, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(E, (2 if swiglu else 1) * N, K, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    off = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device=DEV)
+    y = torch.full((n, N), 7.0, device=DEV, dtype=torch.bfloat16)
+    lib().grouped_gemm_bf16(x, w, y, off, max(counts), swiglu, 0)
+    for e in range(E):
+        a, b = int(off[e]), int(off[e + 1])
+        if a == b:
+            continue
+        want = x[a:b].float() @ w[e].float().t()
+        if swiglu:
+            want = torch.nn.functional.silu(want[:, :N]) * want[:, N:]
+        assert _rel_err(y[a:b], want) < 5e-3, e
+    ops.check_device_error()
+
+
 def test_argmax_and_sampling():
     torch.manual_seed(8)
     logits = torch.randn(9, 128256, device=DEV)
