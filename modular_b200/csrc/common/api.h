@@ -190,6 +190,13 @@ size_t mb_attn_split_workspace_bytes(int num_sms);
 void mb_set_attn_split_workspace(void* ws, size_t ws_bytes, int* counters, int counter_ints);
 void mb_set_attn_split(int on);
 
+// latent attention of prompts with projected keys and values (attention_tc.cu), and the rows to project out of the pages
+int mb_latent_prefill_tc(const void* q, int ldq, int q_head, const void* q_rope, int ld_rope, int rope_head, void* out, int ldo, const void* kv,
+                         int ld_kv, const void* k_rope, long long rows, const int32_t* kv_start, const int32_t* q_start, const int32_t* q_len,
+                         const int32_t* kv_len, const int32_t* tile_seq, const int32_t* tile_q0, int n_tiles, int n_heads, float scale,
+                         const MbAttnOptions* opt, int* err, cudaStream_t stream);
+int mb_latent_gather(const void* cache, long long page_stride, int ld, int page, const int32_t* block_table, int bt_stride,
+                     const int32_t* kv_start, const int32_t* kv_len, int B, int R, void* c, void* rope, long long rows, cudaStream_t stream);
 // tcgen05 prefill attention (attention_tc.cu): same addressing as mb_paged_attention_tma, head_dim 128 only.
 int mb_paged_attention_prefill_tc(const void* q, int ldq, void* out, int ldo, const void* kv_base,
                                   long long total_rows, long long k_off_rows, long long v_off_rows,
