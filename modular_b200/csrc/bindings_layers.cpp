@@ -252,6 +252,39 @@ void latent_post_down(const Tensor& x, int q_rank, const Opt& gamma_q, const Opt
            "latent_post_down");
 }
 
+// q, q_rope [T, h, 128 / 64] (any strides, heads' columns contiguous), kv [rows, 2 h 128], k_rope [rows, 64]; the plan's
+// sequences start at rows kv_start. out [T, >= h 128]
+void latent_prefill(const Tensor& q, const Tensor& q_rope, const Tensor& kv, const Tensor& k_rope, const Tensor& kv_start, const Tensor& q_start,
+                    const Tensor& q_len, const Tensor& kv_len, const Tensor& tile_seq, const Tensor& tile_q0, Tensor& out, double scale,
+                    const Opt& sink, int window, const Opt& gate) {
+  const int T = q.size(0), h = q.size(1), B = q_len.numel(), n_tiles = tile_seq.numel();
+  auto bf = [](const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16; };
+  TORCH_CHECK(bf(q) && bf(q_rope) && bf(kv) && bf(k_rope) && bf(out) && q.dim() == 3 && q.size(2) == 128 && q.stride(2) == 1 && q_rope.dim() == 3 &&
+                  q_rope.size(0) == T && q_rope.size(1) == h && q_rope.size(2) == 64 && q_rope.stride(2) == 1 && kv.dim() == 2 &&
+                  kv.size(1) == 2 * h * 128 && kv.stride(1) == 1 && k_rope.is_contiguous() && k_rope.size(0) == kv.size(0) && k_rope.size(1) == 64 &&
+                  out.dim() == 2 && out.size(0) == T && out.size(1) >= h * 128 && out.stride(1) == 1,
+              "latent_prefill layout");
+  const AttnOptions opt(window, sink, gate, 1.0, T, h, q.scalar_type(), "latent_prefill");
+  check_rc(mb_latent_prefill_tc(q.data_ptr(), q.stride(0), q.stride(1), q_rope.data_ptr(), q_rope.stride(0), q_rope.stride(1), out.data_ptr(),
+                                out.stride(0), kv.data_ptr(), kv.stride(0), k_rope.data_ptr(), kv.size(0), i32(kv_start, B, "kv_start"),
+                                i32(q_start, B, "q_start"), i32(q_len, B, "q_len"), i32(kv_len, B, "kv_len"), i32(tile_seq, n_tiles, "tile_seq"),
+                                i32(tile_q0, n_tiles, "tile_q0"), n_tiles, h, static_cast<float>(scale), opt.use, error_flag(), cur_stream()),
+           "latent_prefill");
+}
+
+// cache [pages, page, >= R + 64] -> c [rows, R], rope [rows, 64]: the rows of all sequences, one after another
+void latent_gather(const Tensor& cache, const Tensor& block_table, const Tensor& kv_start, const Tensor& kv_len, Tensor& c, Tensor& rope) {
+  const int B = kv_len.numel(), R = c.size(1);
+  TORCH_CHECK(cache.is_cuda() && cache.scalar_type() == at::kBFloat16 && cache.dim() == 3 && cache.stride(2) == 1 && cache.size(2) >= R + 64 &&
+                  c.is_contiguous() && rope.is_contiguous() && c.scalar_type() == at::kBFloat16 && rope.scalar_type() == at::kBFloat16 &&
+                  rope.size(0) == c.size(0) && rope.size(1) == 64 && block_table.scalar_type() == at::kInt && block_table.stride(1) == 1 &&
+                  block_table.size(0) >= B,
+              "latent_gather layout");
+  check_rc(mb_latent_gather(cache.data_ptr(), cache.stride(0), cache.stride(1), cache.size(1), block_table.data_ptr<int32_t>(), block_table.stride(0),
+                            i32(kv_start, B, "kv_start"), i32(kv_len, B, "kv_len"), B, R, c.data_ptr(), rope.data_ptr(), c.size(0), cur_stream()),
+           "latent_gather");
+}
+
 // q_lat [T, h, Rp], q_rope [T, h, Dp] (any token stride, heads contiguous blocks), cache [pages, page, >= Rp + Dp]
 void latent_attention(const Tensor& q_lat, const Tensor& q_rope, const Tensor& cache, const Tensor& block_table,
                       const Tensor& q_start, const Tensor& q_len, const Tensor& kv_len, Tensor& out, double scale,
@@ -565,6 +598,10 @@ void mb::bind_layers(py::module_& m) {
                              i32(positions, x.size(0), "positions"), f32(cos_sin, 0, "cos_sin"), dtype_of(x, "x"), cur_stream()),
              "rotate_heads");
   });
+  m.def("latent_gather", &latent_gather);
+  m.def("latent_prefill", &latent_prefill, py::arg("q"), py::arg("q_rope"), py::arg("kv"), py::arg("k_rope"), py::arg("kv_start"), py::arg("q_start"),
+        py::arg("q_len"), py::arg("kv_len"), py::arg("tile_seq"), py::arg("tile_q0"), py::arg("out"), py::arg("scale"), py::arg("sink") = py::none(),
+        py::arg("window") = 0, py::arg("gate") = py::none());
   m.def("latent_attention", &latent_attention, py::arg("q_lat"), py::arg("q_rope"), py::arg("cache"), py::arg("block_table"),
         py::arg("q_start"), py::arg("q_len"), py::arg("kv_len"), py::arg("out"), py::arg("scale"), py::arg("sink") = none,
         py::arg("one_token") = false, py::arg("ws") = none, py::arg("allow_tc") = true, py::arg("window") = 0,

@@ -28,6 +28,7 @@ from typing import Optional
 import torch
 
 from .. import ops
+from ..nn.latent_attention import prompt_attention, prompt_plan, stacked_up
 from ..nn.moe import Fp8ExpertWeights, MoE, MoEConfig
 from ..nn.rotary_embedding import RopeScaling, cos_sin_table
 from .decode_graphs import no_gc_during_capture as _no_gc_during_capture
@@ -191,6 +192,7 @@ class DSLayer:
     w_uv: torch.Tensor               # [h, v_dim, kv_lora]  applied to the latent output  (N=v_dim, K=kv_lora)
     wo: object                       # [H, h * v_dim]
     mlp_norm: torch.Tensor
+    w_up: Optional[torch.Tensor] = None  # [2 * h * 128, kv_lora]: both halves of kv_b stacked, for prompts
     w_a: Optional[torch.Tensor] = None   # [q_lora + kv_lora + rope, H]: q_a and kv_a stacked (bf16 weights only)
     wgu: Optional[object] = None     # dense layers: [2 * inter, H]
     wd: Optional[object] = None      # dense layers: [H, inter]
@@ -427,6 +429,9 @@ class DeepseekV3Model:
                 if l.q_a is not None:
                     ql = l.q_a.shape[0]
                     l.q_a, l.kv_a = l.w_a[:ql], l.w_a[ql:]
+            if (l.w_up is None and self.device.type == "cuda" and self.dtype == torch.bfloat16 and cfg.qk_nope_head_dim == cfg.v_head_dim == 128
+                    and cfg.qk_rope_head_dim == 64):
+                l.w_up = stacked_up(l.w_uk, l.w_uv)
         self.ep = ep
         self._ep_layers = {}
         if ep is not None:
@@ -536,7 +541,7 @@ class DeepseekV3Model:
                              torch.zeros(1, 1, dtype=torch.int32, device=dev), i32(0), i32(1), i32(1), i32(0))
 
     # ------------------------------------------------------------ attention
-    def _attention_fused(self, li: int, l: DSLayer, x, positions, slots, block_table, q_start, q_len, kv_len):
+    def _attention_fused(self, li: int, l: DSLayer, x, positions, slots, block_table, q_start, q_len, kv_len, plan=None):
         """The CUDA path for bf16 attention weights: one down-projection GEMM, one kernel for both norms, the key
         rotation and the cache store, per-head absorption GEMMs that address the heads in place (no transposes)."""
         from .._native import lib
@@ -553,6 +558,12 @@ class DeepseekV3Model:
         q = lin(q_a if ql else x, l.q_b)                                      # [T, h * (nope + rope)]
         q_rope = torch.empty(T, h, c.qk_rope_head_dim, dtype=x.dtype, device=dev)
         L.mla_q_rope(q, h, c.qk_nope_head_dim, positions, self.cos_sin, q_rope)
+        if plan is not None and l.w_up is not None:
+            # long prompts: the cached latents projected up to keys and values per head
+            o = torch.empty(T, h * c.v_head_dim, dtype=x.dtype, device=dev)
+            prompt_attention(plan, q.view(T, h, c.qk_head_dim)[:, :, : c.qk_nope_head_dim], q_rope, l.w_up, cache, block_table, q_start, q_len,
+                             kv_len, o, self.scale)
+            return o
         q_lat = torch.empty(T, h * R, dtype=x.dtype, device=dev)
         ops.batched_linear_heads(q, l.w_uk, q_lat, c.qk_head_dim, R)          # absorb W_uk per head
         o_lat = ops.mla_paged_attention(q_lat.view(T, h, R), q_rope, cache, block_table, q_start, q_len, kv_len,
@@ -561,11 +572,11 @@ class DeepseekV3Model:
         ops.batched_linear_heads(o_lat.view(T, h * R), l.w_uv, o, R, c.v_head_dim)   # apply W_uv per head
         return o
 
-    def _attention(self, li: int, l: DSLayer, x, positions, slots, block_table, q_start, q_len, kv_len):
+    def _attention(self, li: int, l: DSLayer, x, positions, slots, block_table, q_start, q_len, kv_len, plan=None):
         c = self.cfg
         if (x.is_cuda and x.dtype == torch.bfloat16 and l.w_a is not None and torch.is_tensor(l.q_b)
                 and c.qk_rope_head_dim == 64 and positions.dtype == torch.int32):
-            return self._attention_fused(li, l, x, positions, slots, block_table, q_start, q_len, kv_len)
+            return self._attention_fused(li, l, x, positions, slots, block_table, q_start, q_len, kv_len, plan)
         T, h = x.shape[0], c.num_attention_heads
         if l.q_a is not None:
             q = _linear(ops.rms_norm(_linear(x, l.q_a), l.q_a_norm, c.rms_norm_eps), l.q_b)
@@ -606,8 +617,9 @@ class DeepseekV3Model:
         # decode-sized steps on the GPU use the GEMM that carries the residual add and the next norm in its tail
         small = h.is_cuda and h.dtype == torch.bfloat16 and h.shape[0] <= ops.DECODE_GEMM_MAX_TOKENS
         x = ops.rms_norm(h, layers[0].attn_norm, eps)
+        plan = prompt_plan(tokens.shape[0], q_len, kv_len) if layers[0].w_up is not None else None
         for li, l in enumerate(layers):
-            a = self._attention(li, l, x, positions, slots, block_table, q_start, q_len, kv_len)
+            a = self._attention(li, l, x, positions, slots, block_table, q_start, q_len, kv_len, plan)
             if small and torch.is_tensor(l.wo):
                 x, h = ops.linear_decode(a, l.wo, "add_norm", h=h, gamma=l.mlp_norm, eps=eps)
             else:

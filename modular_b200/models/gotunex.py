@@ -22,7 +22,7 @@ import torch
 
 from .. import ops
 from ..nn.delta_rule import DeltaRule, DeltaRuleConfig, gemm_k, pad_to, up8
-from ..nn.latent_attention import LatentAttention, LatentAttentionConfig
+from ..nn.latent_attention import LatentAttention, LatentAttentionConfig, prompt_plan
 from ..nn.moe import TableRouter, expert_mlp
 from ..nn.residual import residual_norm
 from ..nn.rotary_embedding import cos_sin_table
@@ -356,6 +356,7 @@ class GotunexModel:
         # the tiled GEMM for every step size: the decode-step GEMM measured 2 to 29 % slower per step at these widths
         lin = ops.linear
         one_token = T == q_len.shape[0]
+        plan = prompt_plan(T, q_len, kv_len) if any(getattr(l.mixer, "w_up", None) is not None for l in w.layers) else None
         routes = w.router.route(tokens)
         x = torch.empty(T, Wp, dtype=torch.float32, device=dev)
         # what the next seam adds to the stream: the embedding first, then both branches of a layer
@@ -369,7 +370,7 @@ class GotunexModel:
             residual_norm(x, w1=l.norm1, n1=n1, w2=l.norm2, n2=n2, scatter=inverse, cols=c.hidden_size, eps=eps, **pending)
             if c.is_attention(i):
                 y = l.mixer(n1, lin, self.kv[:, 0, self.plane[i], 0], self.cos_sin[i], positions, slots, block_table, q_start,
-                            q_len, kv_len, one_token)
+                            q_len, kv_len, one_token, plan)
             else:
                 y = l.mixer(n1, lin, self.state[f"l{i}.delta"], self.state[f"l{i}.conv"], state_slot, q_start, q_len, kv_len,
                             one_token)

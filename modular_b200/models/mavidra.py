@@ -26,7 +26,7 @@ from ..nn.bigram import STATE as BIGRAM_STATE
 from ..nn.bigram import BigramConfig, bigram_rows
 from ..nn.delta_rule import DeltaRule, DeltaRuleConfig, gemm_k, pad_to, up8
 from ..nn.gated_linear_attention import GatedLinearAttention, GatedLinearConfig
-from ..nn.latent_attention import LatentAttention, LatentAttentionConfig
+from ..nn.latent_attention import LatentAttention, LatentAttentionConfig, prompt_plan
 from ..nn.moe import ScoreRouter, ScoreRouterConfig, expert_mlp
 from ..nn.parallel_mixer import ParallelMixer
 from ..nn.residual import sandwich_norm
@@ -414,6 +414,7 @@ class MavidraModel:
         new = lambda rows: torch.empty(rows, Wp, dtype=self.dtype, device=dev)
         seam = lambda x, **kw: sandwich_norm(x, cols=c.hidden_size, eps=c.norm_eps, **kw)
         one_token = T == q_len.shape[0]
+        plan = prompt_plan(T, q_len, kv_len) if any(getattr(l.mixer, "w_up", None) is not None for l in w.layers) else None
         plans = {g: tensor_core_plan(g, self.kv.shape[5], self.dtype, self.page_size, q_start, q_len, T, one_token)
                  for g in self.groups}
         counts = torch.zeros(len(self.moe_layers), self.max_experts, dtype=torch.int32, device=dev)
@@ -431,7 +432,7 @@ class MavidraModel:
                 y = l.mixer(h, ops.linear, self.state[f"l{i}.gla"], state_slot, q_start, q_len, kv_len, one_token)
             elif kind == LATENT:
                 y = l.mixer(h, ops.linear, self.paged["latent"][:, self.plane[i]], self.cos_sin[i], positions, slots, block_table,
-                            q_start, q_len, kv_len, one_token)
+                            q_start, q_len, kv_len, one_token, plan)
             else:
                 y = l.mixer(h, ops.linear, self.kv, self.plane[i], self.state[f"l{i}.delta"], self.state[f"l{i}.conv"], self.cos_sin[i],
                             positions, slots, block_table, q_start, q_len, kv_len, state_slot, plans[l.mixer.left.cfg.group_pad],

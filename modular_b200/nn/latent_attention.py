@@ -1,15 +1,15 @@
 """Latent attention: queries and keys / values go through low-rank latents, and the cache keeps one row per token
 (the normed key/value latent and a rotated key part that all heads share).
 
-Runs in the absorbed form for prefill and decode alike: ``q_lat = W_uk^T q`` per head, attention over the cached rows,
-``o = W_uv o_lat`` per head. Options: rotate-half or interleaved rotary pairs, a sliding window, a learned sink per head (a
+Runs in the absorbed form (``q_lat = W_uk^T q`` per head, attention over the cached rows, ``o = W_uv o_lat`` per head); long
+prompts of the usual sizes project the rows up to keys and values per head instead (:func:`prompt_plan`). Options: rotate-half or interleaved rotary pairs, a sliding window, a learned sink per head (a
 score without key or value in the softmax denominator), a sigmoid output gate per value column or per head, and reading
 another layer's cache rows (a layer without a key/value projection of its own).
 
 Column layouts are padded for the kernels, with zeros: per head ``[dim -> multiple of 64 | rot_dim -> 64]`` for queries,
 ``[kv_rank -> a kernel size | rot_dim -> 64]`` for cache rows, vdim -> multiple of 8.
 
-Kernels: ``mla_tc.cu`` (tcgen05: 512-wide latents, multiples of 128 heads), ``mla.cu`` (other sizes in bf16),
+Kernels: ``attention_tc.cu`` (projected prompts), ``mla_tc.cu`` (tcgen05: 512-wide latents, multiples of 128 heads), ``mla.cu`` (other sizes in bf16),
 ``mla_ragged.cu`` (fp32 and anything wider); CPU tensors take the PyTorch form.
 """
 
@@ -121,11 +121,16 @@ class LatentAttention:
         uv = new(H, vp, Rp)
         uv[:, : c.vdim, : c.kv_rank] = t["uv"].view(H, c.vdim, c.kv_rank)
         self.w_uv = put(uv)                                          # [h, vdim, latent]: latent outputs to values
+        # prompts project latents up to keys and values where the sizes are those of the kernel
+        self.w_up = stacked_up(self.w_uk, self.w_uv) if (up64(d) == vp == 128 and rot_pad(r) == 64 and self.w_uk.is_cuda
+                                                         and dtype == torch.bfloat16) else None
         self.sink = put(t["sink"], torch.float32) if c.sink else None
         self.w_o = put(pad_to(pad_heads(t["o"].t().contiguous(), H, c.vdim, vp).t(), width_pad, gemm_k(H * vp)))
 
-    def __call__(self, x, lin, cache, cos_sin, positions, slots, block_table, q_start, q_len, kv_len, one_token: bool):
-        """x [T, width] -> [T, width]; ``cache`` [pages, page, >= cache_width] is this layer's (or the shared) plane."""
+    def __call__(self, x, lin, cache, cos_sin, positions, slots, block_table, q_start, q_len, kv_len, one_token: bool,
+                 plan: Optional["PromptPlan"] = None):
+        """x [T, width] -> [T, width]; ``cache`` [pages, page, >= cache_width] is this layer's (or the shared) plane.
+        ``plan``: :func:`prompt_plan` of the step."""
         c, T = self.cfg, x.shape[0]
         H, dp, Dp, Rp = c.heads, up64(c.dim), rot_pad(c.rot_dim), latent_pad(c.kv_rank)
         px = lin(x, self.w_in)
@@ -133,19 +138,78 @@ class LatentAttention:
         latent_post_down(self, px, c_q, positions, cos_sin, slots, cache)
         q = lin(c_q, self.w_uq)                                      # [T, h * (dim | rotated)]
         rotate_heads(q[:, dp:], H, c.head_width, c.rot_dims, c.interleaved, positions, cos_sin)
-        q_lat = torch.empty(T, H * Rp, dtype=x.dtype, device=x.device)
-        ops.batched_linear_heads(q, self.w_uk, q_lat, c.head_width, Rp)
         q_rope = q.view(T, H, c.head_width)[:, :, dp:]
-        o_lat = latent_attention(q_lat.view(T, H, Rp), q_rope, cache, block_table, q_start, q_len, kv_len, c.scale, self.sink,
-                                 one_token, c.window, px[:, self.g_off: self.g_off + H] if c.head_gate else None)
+        gate = px[:, self.g_off: self.g_off + H] if c.head_gate else None
         width = H * c.vdim_pad
         o = torch.empty(T, self.w_o.shape[1], dtype=x.dtype, device=x.device)
         if o.shape[1] != width:
             o[:, width:].zero_()
-        ops.batched_linear_heads(o_lat.view(T, H * Rp), self.w_uv, o, Rp, c.vdim_pad)
+        if plan is not None and self.w_up is not None and (c.window == 0 or c.window > 256):
+            prompt_attention(plan, q.view(T, H, c.head_width)[:, :, :dp], q_rope, self.w_up, cache, block_table, q_start, q_len, kv_len, o,
+                             c.scale, self.sink, c.window, gate)
+        else:
+            q_lat = torch.empty(T, H * Rp, dtype=x.dtype, device=x.device)
+            ops.batched_linear_heads(q, self.w_uk, q_lat, c.head_width, Rp)
+            o_lat = latent_attention(q_lat.view(T, H, Rp), q_rope, cache, block_table, q_start, q_len, kv_len, c.scale, self.sink,
+                                     one_token, c.window, gate)
+            ops.batched_linear_heads(o_lat.view(T, H * Rp), self.w_uv, o, Rp, c.vdim_pad)
         if not c.head_gate:
             ops.sigmoid_gate(o, px[:, self.g_off:], width)
         return lin(o, self.w_o)
+
+
+# ------------------------------------------------------------------ prompts: projected keys and values
+PROMPT_ROWS = 16384          # most cache rows of a step whose keys and values are projected (128 heads: 1 GiB of them)
+_PER_ROW, _PER_PAIR = 256 * 512, (512 + 64 + 512) - (128 + 64 + 128)
+
+
+@dataclass
+class PromptPlan:
+    """Work of a prompt step in the projected form: ``rows`` cache rows, those of sequence s from ``kv_start[s]`` on, and the
+    query tiles of 128 tokens."""
+    rows: int
+    kv_start: torch.Tensor
+    tile_seq: torch.Tensor
+    tile_q0: torch.Tensor
+
+
+def prompt_plan(T: int, q_len, kv_len) -> Optional[PromptPlan]:
+    """The plan of a step whose latents are better projected up to keys and values per head, or None. A query and a key then
+    meet in 320 products a head instead of 1088, but every cache row costs 256 x 512 a head first: it pays where a row is
+    seen by more than 171 queries. Steps below 256 tokens, captured steps and rows beyond the scratch limit stay absorbed.
+    Reads both lengths back (one synchronisation a step)."""
+    if not q_len.is_cuda or T < 256 or T == q_len.numel() or torch.cuda.is_current_stream_capturing():
+        return None
+    ql, kl = torch.stack((q_len.int(), kv_len.int())).tolist()
+    pairs = sum(n * (k - n) + n * (n + 1) // 2 for n, k in zip(ql, kl))
+    rows = sum(kl)
+    if rows > PROMPT_ROWS or pairs * _PER_PAIR <= rows * _PER_ROW:
+        return None
+    start, seq, q0 = [0], [], []
+    for s, (n, k) in enumerate(zip(ql, kl)):
+        start.append(start[-1] + k)
+        for t in range(0, n, 128):
+            seq.append(s)
+            q0.append(t)
+    B, n = len(ql), len(seq)
+    buf = torch.tensor(start[:B] + seq + q0, dtype=torch.int32).to(q_len.device)
+    return PromptPlan(rows, buf[:B], buf[B: B + n], buf[B + n:])
+
+
+def stacked_up(w_uk: torch.Tensor, w_uv: torch.Tensor) -> torch.Tensor:
+    """[heads * 128 | heads * 128, latent] from ``w_uk`` [heads, latent, 128] and ``w_uv`` [heads, 128, latent]."""
+    R = w_uk.shape[1]
+    return torch.cat((w_uk.transpose(1, 2).reshape(-1, R), w_uv.reshape(-1, R))).contiguous()
+
+
+def prompt_attention(plan: PromptPlan, q, q_rope, w_up, cache, block_table, q_start, q_len, kv_len, out, scale, sink=None, window=0, gate=None):
+    """q [T, h, 128], q_rope [T, h, 64] (rotated, any strides), cache [pages, page, latent + 64]; out [T, h * 128 ..]."""
+    R, L = w_up.shape[1], _lib()
+    c = torch.empty(plan.rows, R, dtype=q.dtype, device=q.device)
+    k_rope = torch.empty(plan.rows, 64, dtype=q.dtype, device=q.device)
+    L.latent_gather(cache, block_table, plan.kv_start, kv_len, c, k_rope)
+    L.latent_prefill(q, q_rope, ops.linear(c, w_up), k_rope, plan.kv_start, q_start, q_len, kv_len, plan.tile_seq, plan.tile_q0, out, scale,
+                     sink=sink, window=window, gate=gate)
 
 
 def latent_post_down(m: LatentAttention, px, c_q, positions, cos_sin, slots, cache):

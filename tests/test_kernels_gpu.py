@@ -263,6 +263,53 @@ def test_paged_attention_mixed_batch(n_q, n_kv, hd, ps, tma):
     assert (o.float() - o_ref.float()).abs().max() < 3e-2
 
 
+@pytest.mark.parametrize("h,R,window,extras", [(2, 512, 0, False), (16, 512, 0, True), (3, 128, 150, True)])
+def test_latent_prompt_attention(h, R, window, extras):
+    """Latents projected up to keys and values per head, against the same product in fp32: ragged prompts around tiles of 64 keys
+    and 128 queries, one that continues a cached prefix, sink and gate."""
+    from modular_b200.nn import latent_attention as la
+
+    torch.manual_seed(h)
+    ql, kl = [300, 127, 1, 129, 64, 513], [300, 127, 1, 200, 64, 700]
+    T, page = sum(ql), 64
+    need = [-(-n // page) for n in kl]
+    cache = torch.randn(sum(need) + 1, page, R + 64, device=DEV).to(torch.bfloat16)
+    order = (torch.randperm(sum(need)) + 1).int()
+    bt = torch.zeros(len(ql), max(need), dtype=torch.int32)
+    at = 0
+    for s, n in enumerate(need):
+        bt[s, :n] = order[at: at + n]
+        at += n
+    bt, i32 = bt.to(DEV), lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    q = torch.randn(T, h, 192, device=DEV).to(torch.bfloat16)
+    w_uk, w_uv = ((torch.randn(*s, device=DEV) * R ** -0.5).to(torch.bfloat16) for s in ((h, R, 128), (h, 128, R)))
+    sink = torch.randn(h, device=DEV) if extras else None
+    gate = torch.randn(T, h + 3, device=DEV).to(torch.bfloat16)[:, :h] if extras else None
+    plan = la.prompt_plan(T, i32(ql), i32(kl))
+    assert plan is not None and plan.rows == sum(kl)
+    out = torch.full((T, h * 128 + 8), 7.0, device=DEV, dtype=torch.bfloat16)
+    qs = i32([0] + list(torch.tensor(ql).cumsum(0)[:-1]))
+    la.prompt_attention(plan, q[:, :, :128], q[:, :, 128:], la.stacked_up(w_uk, w_uv), cache, bt, qs, i32(ql), i32(kl), out, 192 ** -0.5, sink, window,
+                        gate)
+    ops.check_device_error()
+    assert (out[:, h * 128:] == 7).all()
+    at = 0
+    for s, (n, k) in enumerate(zip(ql, kl)):
+        rows = cache[bt[s, : need[s]].long()].reshape(-1, R + 64)[:k].float()
+        keys = torch.einsum("kr,hrn->hkn", rows[:, :R], w_uk.float())
+        v = torch.einsum("kr,hvr->hkv", rows[:, :R], w_uv.float())
+        sc = (torch.einsum("qhn,hkn->hqk", q[at: at + n, :, :128].float(), keys) + torch.einsum("qhn,kn->hqk", q[at: at + n, :, 128:].float(), rows[:, R:])) * 192 ** -0.5
+        d = torch.arange(n, device=DEV).unsqueeze(1) + (k - n) - torch.arange(k, device=DEV)
+        sc = sc.masked_fill((d < 0) | (d >= (window or k)), float("-inf"))
+        if sink is not None:
+            sc = torch.cat([sc, sink.view(h, 1, 1).expand(h, n, 1)], -1)
+        o = torch.einsum("hqk,hkv->qhv", torch.softmax(sc, -1)[..., :k], v)
+        if gate is not None:
+            o = o * torch.sigmoid(gate[at: at + n].float()).unsqueeze(2)
+        assert _rel_err(out[at: at + n, : h * 128].float(), o.reshape(n, -1)) < 1e-2, s      # keys, values and P in bf16
+        at += n
+
+
 @pytest.mark.parametrize("counts,N,K,swiglu", [([0, 257, 1, 900, 255, 256, 0, 3], 384, 128, False), ([700, 0, 513], 200, 72, True),
                                               ([300] * 5, 1408, 256, True), ([128, 128], 256, 64, False)])
 def test_grouped_gemm_pairs(counts, N, K, swiglu):
