@@ -537,8 +537,10 @@ static int scan_by_width(const MbDelta& p, int num_sms, cudaStream_t stream) {
   constexpr int max_warps = (RL4 <= 8 ? 512 : 256) / 32;
   const int head_warps = (p.vdim + 7) / 8;
   if (p.one_token && head_warps <= max_warps) return scan_launch<T, RL4, 2, HEADG>(p, head_warps, true, stream);
-  // longer sequences: four columns per lane where the registers allow it (the rows are read once for all of them), and
-  // CTAs of up to four warps as long as the grid has one per SM
+  // longer sequences: four columns per lane where the registers allow it (the rows are read once for all of them) and the
+  // grid still has two warps per scheduler, two columns otherwise: a token is a chain of some 300 instructions for four
+  // columns, and one warp alone issues one in two cycles (four prompts of 3076 tokens at most, 16 heads of 128 x 128:
+  // 1151 us with four, 1065 with two). CTAs have up to four warps as long as the grid has one per SM.
   auto fit = [&](int per_warp) {
     const int hw = (p.vdim + per_warp - 1) / per_warp;
     int w = hw < 4 ? hw : 4;
@@ -546,7 +548,8 @@ static int scan_by_width(const MbDelta& p, int num_sms, cudaStream_t stream) {
     return w;
   };
   if constexpr (RL4 <= 4) {
-    if (p.vdim >= 16) return scan_launch<T, RL4, 4, HEADG>(p, fit(16), false, stream);
+    if (p.vdim >= 16 && static_cast<long long>(p.B) * p.heads * ((p.vdim + 15) / 16) >= 8LL * num_sms)
+      return scan_launch<T, RL4, 4, HEADG>(p, fit(16), false, stream);
   }
   return scan_launch<T, RL4, 2, HEADG>(p, fit(8), false, stream);
 }
