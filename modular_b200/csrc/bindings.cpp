@@ -1233,7 +1233,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                     q.size(0) == M && q.size(1) == I && scales.is_contiguous() && scales.scalar_type() == at::kFloat &&
                     scales.dim() == 2 && scales.size(0) == I / 128 && scales.size(1) >= M,
                 "silu_mul_quant_fp8 layout");
-    check_rc(mb_silu_mul_quant_fp8(gu.data_ptr(), q.data_ptr(), scales.data_ptr<float>(), M, I,
+    const Tensor src = reinterpret_cast<uintptr_t>(gu.data_ptr()) & 15 ? gu.clone() : gu;      // the kernel reads 16 bytes at a time
+    check_rc(mb_silu_mul_quant_fp8(src.data_ptr(), q.data_ptr(), scales.data_ptr<float>(), M, I,
                                    static_cast<int>(scales.size(1)), n_rows ? n_rows->data_ptr<int32_t>() : nullptr,
                                    cur_stream()),
              "silu_mul_quant_fp8");

@@ -171,6 +171,11 @@ class MLP:
         x2 = x.reshape(-1, x.shape[-1])
         if self.gate_up.weight_scale is None and self.gate_up.bias is None:
             act = ops.linear_swiglu(x2, self.gate_up.weight)
+        elif (x2.is_cuda and x2.dtype == torch.bfloat16 and type(self.down) is Linear and self.down.weight_scale is not None
+              and self.down.weight_format is None and self.down.bias is None and self.down.in_dim % 128 == 0):
+            # fp8 down projection: the activation leaves SwiGLU quantised, the same values as in two passes
+            y = ops.linear_fp8_blockscaled(*ops.silu_mul_quant_fp8(self.gate_up(x2)), self.down.weight, self.down.weight_scale, residual)
+            return y.reshape(x.shape)
         else:
             act = ops.silu_mul(self.gate_up(x2))
         return self.down(act, residual=residual).reshape(x.shape)

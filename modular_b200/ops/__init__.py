@@ -448,6 +448,15 @@ def quant_fp8_group128(x):
     return q, s
 
 
+def silu_mul_quant_fp8(gate_up):
+    """``quant_fp8_group128(silu_mul(gate_up))`` in one pass over a CUDA tensor [M, 2 I], I % 128 == 0."""
+    M, I = gate_up.shape[0], gate_up.shape[1] // 2
+    q = torch.empty(M, I, dtype=torch.float8_e4m3fn, device=gate_up.device)
+    s = torch.empty(I // 128, M, dtype=torch.float32, device=gate_up.device)
+    _lib().silu_mul_quant_fp8(gate_up.contiguous(), q, s, None)
+    return q, s
+
+
 def linear_fp8_blockscaled(xq, xs, wq, ws, residual=None, out=None, bn=0, stages=0, splits=0):
     """``(xq * xs) @ (wq * ws).T`` with 128x128 weight-block scales and 1x128 activation scales.
     ``splits``: K splits (0 = chosen by the kernel from the tile count and the SM count)."""

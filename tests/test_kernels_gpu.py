@@ -590,6 +590,31 @@ def test_grouped_gemm_fp8_many_experts_with_row_bound():
         assert torch.all(y[rows:] == 0)
 
 
+@pytest.mark.parametrize("M,K", [(1, 128), (3, 136), (17, 1000), (33, 132), (2050, 384)])
+def test_quant_fp8_group128_widths(M, K):
+    """Sixteen lanes a group where rows are whole 16-byte pieces, one warp a group where not (132): the rows of a tensor and the same
+    rows one element further along, which take the other path, in codes and scales; a silent group has the smallest scale."""
+    torch.manual_seed(K)
+    x = (torch.randn(M, K, device=DEV) * 3).to(torch.bfloat16)
+    x[-1, :128] = 0
+    q, s = ops.quant_fp8_group128(x)
+    shifted = torch.zeros(M * K + 4, device=DEV, dtype=torch.bfloat16)[4:].view(M, K).copy_(x)      # 8 bytes off
+    q2, s2 = ops.quant_fp8_group128(shifted)
+    assert torch.equal(q.view(torch.uint8), q2.view(torch.uint8)) and torch.equal(s, s2)
+    assert s[0, -1] == torch.tensor(1e-12, device=DEV) / 448 and (q.view(torch.uint8)[-1, :128] & 0x7F).eq(0).all()
+
+
+def test_fp8_mlp_equals_its_parts():
+    from modular_b200.nn.layers import MLP
+
+    torch.manual_seed(24)
+    m = MLP.random(256, 384, device=DEV)
+    m.gate_up, m.down = m.gate_up.quantize_fp8(), m.down.quantize_fp8()
+    for T in (1, 150):
+        x, r = (torch.randn(T, 256, device=DEV).to(torch.bfloat16) for _ in range(2))
+        assert torch.equal(m(x, r), m.down(ops.silu_mul(m.gate_up(x)), r))
+
+
 def test_silu_mul_quant_fp8_equals_two_passes_and_respects_row_count():
     from modular_b200._native import lib
 
