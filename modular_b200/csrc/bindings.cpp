@@ -235,6 +235,17 @@ void moe_permute_rows(const Tensor& src, const Tensor& order, const c10::optiona
                                src.size(1) * src.element_size(), top_k, cur_stream()),
            "moe_permute_rows");
 }
+// the same rows quantised on the way: q [n, K] e4m3, scales [ceil(K / 128), n]
+void moe_permute_quant_fp8(const Tensor& src, const Tensor& order, const c10::optional<Tensor>& n_rows, Tensor& q, Tensor& scales, int top_k) {
+  need_cuda(src, "src");
+  TORCH_CHECK(src.is_contiguous() && src.dim() == 2 && src.scalar_type() == at::kBFloat16 && order.scalar_type() == at::kInt && q.is_contiguous() &&
+                  q.dim() == 2 && q.element_size() == 1 && q.size(1) == src.size(1) && order.numel() >= q.size(0) && scales.is_contiguous() &&
+                  scales.scalar_type() == at::kFloat && scales.numel() == (src.size(1) + 127) / 128 * q.size(0),
+              "moe_permute_quant_fp8 layout");
+  check_rc(mb_moe_permute_quant_fp8(src.data_ptr(), order.data_ptr<int32_t>(), static_cast<const int32_t*>(optptr(n_rows)), q.data_ptr(),
+                                    scales.data_ptr<float>(), q.size(0), src.size(1), top_k, cur_stream()),
+           "moe_permute_quant_fp8");
+}
 void moe_combine(const Tensor& expert_out, const Tensor& inverse, const Tensor& w,
                  const c10::optional<Tensor>& shared, Tensor& y, int top_k) {
   need_cuda(expert_out, "expert_out");
@@ -611,6 +622,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_router_softmax_topk", &moe_router_softmax_topk);
   m.def("moe_create_indices", &moe_create_indices);
   m.def("moe_permute_rows", &moe_permute_rows);
+  m.def("moe_permute_quant_fp8", &moe_permute_quant_fp8);
   m.def("moe_combine", &moe_combine);
   m.def("grouped_gemm_bf16", &grouped_gemm_bf16);
   m.def("quant_fp8_group128", &quant_fp8_group128);

@@ -79,6 +79,8 @@ int mb_gemm_dec(const void* X, const void* W, int M, int N, int K, int ldx, int 
                 cudaStream_t stream);
 
 // ---- block-scaled fp8 (gemm_fp8_blockscaled.cu, quant_fp8.cu) ----------------------------
+int mb_moe_permute_quant_fp8(const void* src, const int32_t* order, const int32_t* n_rows_dev, void* q_fp8, float* scales, int max_rows, int K,
+                             int top_k, cudaStream_t stream);
 int mb_quant_fp8_group128(const void* x_bf16, void* q_fp8, float* scales, int M, int K, int ldx,
                           int scale_ld, int scales_k_major, cudaStream_t stream);
 int mb_gemm_fp8_blockscaled(const void* Xq, const float* Xs, const void* Wq, const float* Ws, void* Y,

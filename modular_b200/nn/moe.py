@@ -189,8 +189,14 @@ class MoE:
         L = _lib()
         L.moe_create_indices(ids, self.e_begin, self.e_end, scratch, offsets, order, inverse)
         n_local = offsets[E:E + 1]
-        xp = torch.empty(T * k, cfg.hidden_size, dtype=x.dtype, device=dev)
-        L.moe_permute_rows(x, order, n_local, xp, k)
+        H = cfg.hidden_size
+        if isinstance(self.w_gate_up, Fp8ExpertWeights) and x.dtype == torch.bfloat16 and H % 8 == 0 and x.data_ptr() % 16 == 0 and T * k * H < 1 << 34:
+            # quantised into expert order: the rows are written once, in 8 bits
+            xp = (torch.empty(T * k, H, dtype=torch.float8_e4m3fn, device=dev), torch.empty((H + 127) // 128, T * k, dtype=torch.float32, device=dev))
+            L.moe_permute_quant_fp8(x, order, n_local, *xp, k)
+        else:
+            xp = torch.empty(T * k, H, dtype=x.dtype, device=dev)
+            L.moe_permute_rows(x, order, n_local, xp, k)
         out = self.local_gemms(xp, offsets)
         y = torch.empty(T, cfg.hidden_size, dtype=x.dtype, device=dev)
         L.moe_combine(out, inverse, w, shared_out, y, k)

@@ -590,7 +590,7 @@ def test_grouped_gemm_fp8_many_experts_with_row_bound():
         assert torch.all(y[rows:] == 0)
 
 
-@pytest.mark.parametrize("M,K", [(1, 128), (3, 136), (17, 1000), (33, 132), (2050, 384)])
+@pytest.mark.parametrize("M,K", [(1, 128), (3, 136), (17, 1000), (33, 132), (2050, 384), (20000, 256), (9000, 648)])
 def test_quant_fp8_group128_widths(M, K):
     """Sixteen lanes a group where rows are whole 16-byte pieces, one warp a group where not (132): the rows of a tensor and the same
     rows one element further along, which take the other path, in codes and scales; a silent group has the smallest scale."""
@@ -602,6 +602,23 @@ def test_quant_fp8_group128_widths(M, K):
     q2, s2 = ops.quant_fp8_group128(shifted)
     assert torch.equal(q.view(torch.uint8), q2.view(torch.uint8)) and torch.equal(s, s2)
     assert s[0, -1] == torch.tensor(1e-12, device=DEV) / 448 and (q.view(torch.uint8)[-1, :128] & 0x7F).eq(0).all()
+
+
+@pytest.mark.parametrize("T,H,k,local", [(1, 128, 1, 1), (5, 136, 3, 11), (130, 1000, 8, 700), (64, 384, 2, 0), (3001, 1096, 8, 24003)])
+def test_moe_permute_quant_fp8_equals_two_passes(T, H, k, local):
+    from modular_b200._native import lib
+
+    torch.manual_seed(T)
+    x = (torch.randn(T, H, device=DEV) * 2).to(torch.bfloat16)
+    order = torch.randperm(T * k, device=DEV).int()
+    xp = torch.zeros(T * k, H, dtype=torch.bfloat16, device=DEV)
+    n = torch.tensor([local], dtype=torch.int32, device=DEV)
+    lib().moe_permute_rows(x, order, n, xp, k)
+    want, ws = ops.quant_fp8_group128(xp)
+    q, s = torch.zeros_like(want), torch.zeros_like(ws)
+    lib().moe_permute_quant_fp8(x, order, n, q, s, k)
+    assert torch.equal(q.view(torch.uint8)[:local], want.view(torch.uint8)[:local]) and torch.equal(s[:, :local], ws[:, :local])
+    assert not q.view(torch.uint8)[local:].any() and not s[:, local:].any()
 
 
 def test_fp8_mlp_equals_its_parts():
