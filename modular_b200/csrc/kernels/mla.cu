@@ -92,18 +92,22 @@ __device__ __forceinline__ int swz(int row, int chunk) {
   return row * LD + ((chunk ^ (row & 7)) << 3);
 }
 
+// 64 cache rows, eight lanes a row: a thread looks up two rows and copies every eighth chunk of them
 template <int R>
 __device__ __forceinline__ void load_kv_tile(bf16* sK, const Params& p, const int32_t* bt, int kv0,
                                              int kv_end, int tid) {
-  constexpr int LD = R + DR, CH = LD / 8;
-  for (int idx = tid; idx < 64 * CH; idx += 256) {
-    const int row = idx / CH, chunk = idx % CH;
+  constexpr int LD = R + DR;
+  const int c0 = tid & 7;
+#pragma unroll
+  for (int row = tid >> 3; row < 64; row += 32) {
     const int tok = kv0 + row;
     const bool valid = tok < kv_end;
     const int pg = valid ? bt[tok / p.page_size] : 0;
     const int off = valid ? tok % p.page_size : 0;
-    const bf16* src = p.cache + static_cast<int64_t>(pg) * p.page_stride + static_cast<int64_t>(off) * p.ld_cache + chunk * 8;
-    cp_async16(sK + swz<LD>(row, chunk), src, valid);
+    const bf16* src = p.cache + static_cast<int64_t>(pg) * p.page_stride + static_cast<int64_t>(off) * p.ld_cache + c0 * 8;
+    bf16* dst = sK + swz<LD>(row, c0);
+#pragma unroll
+    for (int j = 0; j < LD / 64; ++j) cp_async16(dst + j * 64, src + j * 64, valid);
   }
 }
 
@@ -290,6 +294,189 @@ __global__ void __launch_bounds__(256, 1) mla_kernel(const Params p) {
   }
 }
 
+// At most 16 query rows a CTA (one token of up to 16 heads, or several tokens of fewer): the 64-row kernel would leave three
+// quarters of its warps without rows and the others 544 MMAs a tile to do one after another (R = 512). Here the eight warps share
+// the tile: a warp scores 8 of its 64 keys (Q in registers, four independent chains), the row maxima meet in shared memory, so do
+// the probabilities, and a warp multiplies them with its eighth of the value columns. Bound by the cache reads after that.
+// 64 sequences of 2048 keys, 16 heads: 144 us with the 64-row kernel, 37 us (23 at the copy rate).
+template <int R>
+__global__ void __launch_bounds__(256, 1) mla_rows16_kernel(const Params p) {
+  constexpr int LD = R + DR, CH = LD / 8, KS = LD / 16, NT = R / 64;   // NT: 8-column tiles of a warp
+  constexpr int LP = 72;                                             // row of probabilities: 16-byte rows in different banks
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  bf16* sQ = reinterpret_cast<bf16*>(smem_raw);  // [16][LD]
+  bf16* sK = sQ + 16 * LD;                       // [2][64][LD]
+  __shared__ __align__(16) bf16 sP[16 * LP];
+  __shared__ float s_red[8][16];
+  __shared__ int s_seq, s_tq0;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tokens_per_tile = 16 / p.HB, rows = tokens_per_tile * p.HB;
+
+  if (warp == 0) {                               // this CTA's (sequence, first query token): tiles follow each other sequence by sequence
+    int acc = 0, seq = -1, tq0 = 0;
+    for (int c = 0; c < p.B && seq < 0; c += 32) {
+      const int nt = c + lane < p.B ? (p.q_len[c + lane] + tokens_per_tile - 1) / tokens_per_tile : 0;
+      int incl = nt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      const int at = static_cast<int>(blockIdx.x) - acc;
+      const uint32_t hit = __ballot_sync(0xffffffffu, at < incl);
+      if (hit) {
+        const int who = __ffs(hit) - 1;
+        seq = c + who;
+        tq0 = (at - __shfl_sync(0xffffffffu, incl - nt, who)) * tokens_per_tile;
+      }
+      acc += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) { s_seq = seq; s_tq0 = tq0; }
+  }
+  __syncthreads();
+  const int seq = s_seq, tq0 = s_tq0;
+  if (seq < 0) return;
+  const int head0 = blockIdx.y * p.HB;
+  const int qs = p.q_start[seq], ql = p.q_len[seq], kl = p.kv_len[seq];
+  const int32_t* bt = p.block_table + static_cast<int64_t>(seq) * p.bt_stride;
+
+  for (int idx = tid; idx < 16 * CH; idx += 256) {
+    const int row = idx / CH, chunk = idx % CH;
+    const int tq = tq0 + row / p.HB, head = head0 + row % p.HB;
+    const bool valid = row < rows && tq < ql;
+    const int64_t tok = qs + (valid ? tq : 0);
+    const bf16* src = chunk < R / 8
+                          ? p.q_lat + tok * p.ld_ql + static_cast<int64_t>(valid ? head : 0) * R + chunk * 8
+                          : p.q_rope + tok * p.ld_qr + static_cast<int64_t>(valid ? head : 0) * p.hs_qr + (chunk - R / 8) * 8;
+    cp_async16(sQ + swz<LD>(row, chunk), src, valid);
+  }
+  const int last_tq = min(tq0 + tokens_per_tile, ql);
+  const int kv_hi = kl - ql + last_tq;  // exclusive bound of the KV positions any row here may see
+  const int kv_lo = kl - ql + tq0 - p.window + 1;  // the first one the tile's first row sees
+  const int t_first = kv_lo > 0 ? kv_lo / 64 : 0, tiles_all = (kv_hi + 63) / 64;
+  const int tiles_per = (tiles_all - t_first + p.nsplit - 1) / p.nsplit;
+  const int t_begin = t_first + static_cast<int>(blockIdx.z) * tiles_per;
+  const int t_end = min(tiles_all, t_begin + tiles_per);     // trailing parts may be empty
+  load_kv_tile<R>(sK, p, bt, t_begin * 64, kv_hi, tid);
+  cp_async_commit();
+  cp_async_wait_all();
+  __syncthreads();
+
+  uint32_t qf[KS][4];
+#pragma unroll
+  for (int ks = 0; ks < KS; ++ks) ldsm_x4(qf[ks], sQ + swz<LD>(lane & 15, 2 * ks + (lane >> 4)));
+  float o[NT][4];
+#pragma unroll
+  for (int i = 0; i < NT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};            // m of all keys so far, l of this warp's keys
+  int limit[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = (lane >> 2) + h * 8, tq = tq0 + r / p.HB;
+    limit[h] = (r < rows && tq < ql) ? kl - ql + tq : -1;
+  }
+
+  for (int it = t_begin; it < t_end; ++it) {
+    const int buf = (it - t_begin) & 1;
+    if (it + 1 < t_end) {
+      load_kv_tile<R>(sK + (buf ^ 1) * 64 * LD, p, bt, (it + 1) * 64, kv_hi, tid);
+      cp_async_commit();
+    }
+    const bf16* tK = sK + buf * 64 * LD;
+    float s4[4][4] = {};
+#pragma unroll
+    for (int ks = 0; ks < KS; ks += 2) {
+      uint32_t b[4];
+      ldsm_x4(b, tK + swz<LD>(warp * 8 + (lane & 7), 2 * ks + (lane >> 3)));
+      mma_bf16(s4[ks & 3], qf[ks], b[0], b[1]);
+      mma_bf16(s4[(ks & 3) + 1], qf[ks + 1], b[2], b[3]);
+    }
+    float s[4], mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int col = it * 64 + warp * 8 + 2 * (lane & 3) + (e & 1), h = e >> 1;
+      const float v = (s4[0][e] + s4[1][e]) + (s4[2][e] + s4[3][e]);
+      s[e] = static_cast<uint32_t>(limit[h] - col) < static_cast<uint32_t>(p.window) ? v * p.scale_log2 : -INFINITY;
+      mx[h] = fmaxf(mx[h], s[e]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+      mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
+      if ((lane & 3) == 0) s_red[warp][(lane >> 2) + h * 8] = mx[h];
+    }
+    __syncthreads();
+    float alpha[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float mn = m[h];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) mn = fmaxf(mn, s_red[w][(lane >> 2) + h * 8]);
+      const float safe = mn == -INFINITY ? 0.f : mn;
+      alpha[h] = exp2f(m[h] - safe);
+      m[h] = mn;
+      const float p0 = exp2f(s[2 * h] - safe), p1 = exp2f(s[2 * h + 1] - safe);
+      l[h] = l[h] * alpha[h] + (p0 + p1);
+      *reinterpret_cast<uint32_t*>(sP + ((lane >> 2) + h * 8) * LP + warp * 8 + 2 * (lane & 3)) = pack_bf16(p0, p1);
+    }
+    __syncthreads();
+    uint32_t a[4][4];
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) ldsm_x4(a[kk], sP + (lane & 15) * LP + kk * 16 + (lane >> 4) * 8);
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      o[nt][0] *= alpha[0]; o[nt][1] *= alpha[0];
+      o[nt][2] *= alpha[1]; o[nt][3] *= alpha[1];
+#pragma unroll
+      for (int k2 = 0; k2 < 2; ++k2) {           // 32 keys of 8 value columns (the first R columns of a key)
+        uint32_t b[4];
+        ldsm_x4_t(b, tK + swz<LD>(k2 * 32 + lane, warp * NT + nt));
+        mma_bf16(o[nt], a[2 * k2], b[0], b[1]);
+        mma_bf16(o[nt], a[2 * k2 + 1], b[2], b[3]);
+      }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+  }
+
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
+    l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
+    if ((lane & 3) == 0) s_red[warp][(lane >> 2) + h * 8] = l[h];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = (lane >> 2) + h * 8;
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) sum += s_red[w][r];
+    const int tq = tq0 + r / p.HB, head = head0 + r % p.HB;
+    if (r >= rows || tq >= ql) continue;
+    if (p.nsplit > 1) {
+      const int64_t row = static_cast<int64_t>(blockIdx.z) * p.T * p.n_heads + static_cast<int64_t>(qs + tq) * p.n_heads + head;
+      float* orow = p.ws + row * R + warp * (R / 8) + 2 * (lane & 3);
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) *reinterpret_cast<float2*>(orow + nt * 8) = make_float2(o[nt][2 * h], o[nt][2 * h + 1]);
+      if (warp == 0 && (lane & 3) == 0)
+        *reinterpret_cast<float2*>(p.ws + static_cast<int64_t>(p.nsplit) * p.T * p.n_heads * R + row * 2) = make_float2(m[h], sum);
+      continue;
+    }
+    float inv = sum > 0.f ? 1.f / sum : 0.f;
+    if (p.sink) {       // the running maximum and the sink share one reference, so neither exponential overflows
+      const float sk = p.sink[head] * 1.4426950408889634f, mm = fmaxf(m[h], sk);
+      const float f = exp2f(m[h] - mm);
+      inv = f / (sum * f + exp2f(sk - mm));
+    }
+    inv *= p.gate(qs + tq, head);
+    bf16* orow = p.out + (static_cast<int64_t>(qs + tq) * p.n_heads + head) * R + warp * (R / 8) + 2 * (lane & 3);
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+      *reinterpret_cast<uint32_t*>(orow + nt * 8) = pack_bf16(o[nt][2 * h] * inv, o[nt][2 * h + 1] * inv);
+  }
+}
+
 // Combines the parts of a KV-split launch: one warp per (token, head) and 64 columns, part weights exp2(m - max).
 __global__ void __launch_bounds__(256)
 mla_combine_kernel(const float* __restrict__ ws, bf16* __restrict__ out, const float* __restrict__ sink, const HeadGate gate, int n_rows,
@@ -432,18 +619,19 @@ __global__ void mla_q_rope_kernel(const bf16* __restrict__ q, int n_heads, int n
 }
 
 template <int R>
-static int launch(const Params& p, int grid_x, cudaStream_t stream) {
+static int launch(const Params& p, int grid_x, bool rows16, cudaStream_t stream) {
   constexpr int LD = R + DR;
-  const size_t smem = static_cast<size_t>(3) * 64 * LD * sizeof(bf16);
-  auto kern = mla_kernel<R>;
+  const size_t smem = static_cast<size_t>(3) * 64 * LD * sizeof(bf16), smem16 = static_cast<size_t>(16 + 2 * 64) * LD * sizeof(bf16);
   static PerDeviceOnce configured;
   if (configured.needed()) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
+    if (cudaFuncSetAttribute(mla_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
+        cudaFuncSetAttribute(mla_rows16_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem16)) != cudaSuccess)
       return MB_ERR_LAUNCH;
     configured.done();
   }
   dim3 grid(grid_x, p.n_heads / p.HB, p.nsplit);
-  if (launch_plain(kern, grid, dim3(256), smem, stream, p) != cudaSuccess) return MB_ERR_LAUNCH;
+  if (launch_plain(rows16 ? mla_rows16_kernel<R> : mla_kernel<R>, grid, dim3(256), rows16 ? smem16 : smem, stream, p) != cudaSuccess)
+    return MB_ERR_LAUNCH;
   if (p.nsplit > 1) {
     const int n_rows = p.T * p.n_heads, units = n_rows * (R / 64);
     if (launch_plain(mla_combine_kernel, dim3((units + 7) / 8), dim3(256), 0, stream, static_cast<const float*>(p.ws), p.out,
@@ -517,8 +705,11 @@ extern "C" int mb_mla_paged_attention_ex(const void* q_lat, long long ld_ql, con
   p.sink = opt ? opt->sink : nullptr; p.gate = HeadGate(opt);
   p.window = opt && opt->window > 0 ? opt->window : 0x7fffffff; p.ld_cache = ld_cache; p.T = T; p.ld_ql = ld_ql; p.ld_qr = ld_qr; p.hs_qr = hs_qr;
   p.ws = static_cast<float*>(ws); p.nsplit = 1;
-  const int tpt = 64 / p.HB;
-  const int grid_x = (T + tpt - 1) / tpt + B;  // >= sum over sequences of ceil(q_len / tpt)
+  // Steps of one token a sequence, of up to 16 heads, take tiles of 16 rows (figures at the kernel); with more tokens or heads
+  // the 64-row tiles have work for more of their warps.
+  const bool rows16 = n_heads <= 16 && T <= B;
+  const int tpt = (rows16 ? 16 : 64) / p.HB;
+  const int grid_x = rows16 ? T : (T + tpt - 1) / tpt + B;  // >= sum over sequences of ceil(q_len / tpt)
   if (ws != nullptr) {
     // decode-sized steps: tiles of the batch that really exist are at most T, so count those
     const long long ctas = static_cast<long long>(T < grid_x ? T : grid_x) * (n_heads / p.HB);
@@ -531,12 +722,12 @@ extern "C" int mb_mla_paged_attention_ex(const void* q_lat, long long ld_ql, con
     if (ns > 1) p.nsplit = static_cast<int>(ns);
   }
   switch (R) {
-    case 64: return mla::launch<64>(p, grid_x, stream);
-    case 128: return mla::launch<128>(p, grid_x, stream);
-    case 192: return mla::launch<192>(p, grid_x, stream);
-    case 256: return mla::launch<256>(p, grid_x, stream);
-    case 384: return mla::launch<384>(p, grid_x, stream);
-    case 512: return mla::launch<512>(p, grid_x, stream);
+    case 64: return mla::launch<64>(p, grid_x, rows16, stream);
+    case 128: return mla::launch<128>(p, grid_x, rows16, stream);
+    case 192: return mla::launch<192>(p, grid_x, rows16, stream);
+    case 256: return mla::launch<256>(p, grid_x, rows16, stream);
+    case 384: return mla::launch<384>(p, grid_x, rows16, stream);
+    case 512: return mla::launch<512>(p, grid_x, rows16, stream);
     default: return MB_ERR_SHAPE;
   }
 }

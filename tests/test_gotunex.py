@@ -246,6 +246,27 @@ def test_attention_kernels_agree(heads, rank, decode):
     assert rel(got, want.cpu()) < 1e-2
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,rank", [(16, 512), (1, 64), (5, 128), (7, 384), (4, 256), (16, 192)])
+@pytest.mark.parametrize("qn", [[1] * 40, [3, 0, 1, 0], [0, 4, 0, 1, 0]])
+def test_attention_of_few_rows(heads, rank, qn):
+    """Tiles of 16 query rows against the CUDA-core kernel: one token a sequence, and as many tokens as sequences in other shares."""
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    lens = [(1 + 67 * i) % 400 + 4 for i in range(len(qn))]
+    need = [-(-n // 16) for n in lens]
+    bt = torch.zeros(len(qn), max(need), dtype=torch.int32)
+    for b, n in enumerate(need):
+        bt[b, :n] = torch.arange(n) + sum(need[:b])
+    rows = lambda *s: torch.randn(*s, generator=g, device="cuda", dtype=torch.float32).bfloat16()
+    cache, q, gate = rows(sum(need), 16, rank + 64), rows(sum(qn), heads, rank + 64), rows(sum(qn), heads)
+    ql, kl = torch.tensor(qn, dtype=torch.int32, device="cuda"), torch.tensor(lens, dtype=torch.int32, device="cuda")
+    for sink, window, gt in ((None, 0, None), (torch.randn(heads, generator=g, device="cuda"), 70, gate)):
+        args = (bt.cuda(), (torch.cumsum(ql, 0) - ql).int(), ql, kl, (rank + 64) ** -0.5, sink, False, window)
+        got = latent_attention(q[..., :rank].contiguous(), q[..., rank:].contiguous(), cache, *args, gt)
+        want = latent_attention(q[..., :rank].float().contiguous(), q[..., rank:].float(), cache.float(), *args, None if gt is None else gt.float())
+        assert rel(got, want.cpu()) < 1e-2                       # P in bf16
+
+
 @pytest.mark.parametrize("device,dtype", RUNS)
 @pytest.mark.parametrize("H,KH,d,dv,taps", [(4, 4, 32, 32, 4), (6, 2, 24, 40, 3), (3, 1, 72, 9, 2), (2, 2, 128, 128, 4), (2, 1, 100, 136, 1),
                                             (1, 1, 300, 16, 5), (2, 2, 200, 264, 4)])
