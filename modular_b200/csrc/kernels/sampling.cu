@@ -495,7 +495,9 @@ __device__ __forceinline__ void load4(const float* __restrict__ row, int i, int 
     for (int e = 0; e < 4; ++e) xv[e] = i + e < end ? row[i + e] : -FLT_MAX;
   }
 }
-__device__ __forceinline__ u64 weight_of(float below) { return __float2ull_rn(__expf(-below) * 4398046511104.f); }
+// 2^-42 is the smallest weight: a token about 29 units below the maximum is not drawn (uniform01 has 24 bits, so that no draw
+// could tell it from one of weight 1e-38). NaN (an infinite maximum minus itself, a NaN logit) weighs nothing.
+__device__ __forceinline__ u64 weight_of(float below) { return __float2ull_rn(fmaxf(__expf(-below) * 4398046511104.f, 0.f)); }
 __device__ __forceinline__ int bin_of(float below) {       // NaN goes to the last bin
   const float b = below * kBinsPerUnit;
   return b < static_cast<float>(kBins - 1) ? static_cast<int>(b) : kBins - 1;
@@ -713,14 +715,14 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
       if (bin_of(__fsub_rn(mx, x)) > last) return;
       const uint32_t pos = first + atomicAdd(&sm->fill, 1u);
       if (pos >= kList) return;    // cannot happen: the same elements were counted
-      st_cluster_u32(lx + 4u * pos, __float_as_uint(x));
+      st_cluster_u32(lx + 4u * pos, __float_as_uint(x == x ? x : -INFINITY));      // ranks need an order: NaN is the lowest
       st_cluster_u32(li + 4u * pos, static_cast<uint32_t>(i));
     });
     cluster_sync_all();
     if (rank != 0) return;
     // one candidate per thread: its rank by value and by index, counted directly
     const int n4 = (n + 3) & ~3;
-    if (tid >= n && tid < n4) { sm->lx[tid] = -FLT_MAX; sm->li[tid] = 0x7fffffff; }
+    if (tid >= n && tid < n4) { sm->lx[tid] = -INFINITY; sm->li[tid] = 0x7fffffff; }   // behind every candidate, masked ones too
     if (tid == 0) sm->cut = -1;
     __syncthreads();
     float x = 0.f;
@@ -752,22 +754,19 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
     if (use_k) thr = fkey(sm->sx[k - 1]);                  // k <= n by the choice of the bins
     if (use_m) thr = max(thr, km);
     if (thr > hi_key) thr = hi_key;                        // a min_p above one keeps the maximum alone
-    int kept = __syncthreads_count(tid < n && mykey >= thr);
-    u64 Z = kept > 0 ? sm->sp[kept - 1] : 0;
+    const int kept = __syncthreads_count(tid < n && mykey >= thr);
     if (use_p && kept > 0) {
-      const u64 target = nucleus ? ptarget : portion(tp, Z);
+      const u64 target = nucleus ? ptarget : portion(tp, sm->sp[kept - 1]);
       if (tid < kept && incl >= target && incl - mine < target) sm->cut = tid;
       __syncthreads();
       const int r = sm->cut >= 0 ? sm->cut : kept - 1;
       thr = max(thr, fkey(sm->sx[r]));
-      kept = __syncthreads_count(tid < n && mykey >= thr);
-      Z = sm->sp[kept - 1];
     }
     // inverse-CDF draw over the kept entries in index order
-    const u64 target = portion(uniform01(seed, step, 0xffffffffull), Z);
     const float xo = tid < n ? sm->ox[tid] : 0.f;
     const u64 w = (tid < n && fkey(xo) >= thr) ? weight_of(__fsub_rn(mx, xo)) : 0;
     const u64 cum = block_before(w, sm->red, total);
+    const u64 target = portion(uniform01(seed, step, 0xffffffffull), total);
     if (w > 0 && cum < target && cum + w >= target) out[rowi] = sm->oi[tid];
     if (total == 0 && tid == 0) out[rowi] = a.i;           // nothing has a weight (infinite or NaN logits)
     return;

@@ -434,6 +434,39 @@ def test_sampler_kept_sets_beyond_the_list(V):
             assert torch.equal(a, again)
 
 
+@pytest.mark.parametrize("V,finite", [(130, 20), (255, 7), (511, 100), (512, 3)])
+def test_sampler_small_vocabulary_with_masked_tokens(V, finite):
+    """Kept sets that reach into the masked tokens (top_k beyond the allowed ones): masked tokens rank behind every allowed one."""
+    torch.manual_seed(83)
+    R = 64
+    lg = torch.randn(R, V, device=DEV) - 5.0
+    order = torch.rand(R, V, device=DEV).argsort(1)
+    lg.scatter_(1, order[:, finite:], float("-inf"))
+    seeds, temp = torch.arange(R, device=DEV, dtype=torch.int64) * 31 + 1, torch.full((R,), 0.9, device=DEV)
+    for k in range(max(2, finite - 1), min(finite + 6, V)):
+        for kw in (dict(), dict(top_p=torch.full((R,), 0.95, device=DEV))):
+            kw["top_k"] = torch.full((R,), k, device=DEV, dtype=torch.int32)
+            got = ops.sample(lg, temperature=temp, seeds=seeds, step=2, **kw)
+            ops.set_sample_cluster(False)
+            want = ops.sample(lg, temperature=temp, seeds=seeds, step=2, **kw)
+            ops.set_sample_cluster(True)
+            assert torch.equal(got, want), (k, list(kw))
+
+
+@pytest.mark.parametrize("V", [300, 50001])
+def test_sampler_never_draws_nan(V):
+    """NaN logits have no weight: the draw is one of the other kept tokens, and is always written."""
+    torch.manual_seed(84)
+    R = 32
+    lg = torch.randn(R, V, device=DEV)
+    lg[:, torch.randperm(V, device=DEV)[: V // 3]] = float("nan")
+    seeds, temp = torch.arange(R, device=DEV, dtype=torch.int64), torch.full((R,), 0.8, device=DEV)
+    for k in (40, V - V // 3 - 5, V - 2):
+        out = torch.full((R,), -7, device=DEV, dtype=torch.long)
+        ops.sample(lg, temperature=temp, seeds=seeds, top_k=torch.full((R,), k, device=DEV, dtype=torch.int32), out=out)
+        assert ((out >= 0) & (out < V)).all() and torch.isfinite(lg.gather(1, out[:, None])).all()
+
+
 def test_penalties():
     torch.manual_seed(9)
     logits = torch.randn(3, 1000, device=DEV)
