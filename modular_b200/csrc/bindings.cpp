@@ -771,6 +771,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("sample", &sample);
   m.def("apply_penalties", &apply_penalties);
   // state-space layers
+  // `t` with its last `inner` dimensions packed, whatever the distance between its rows. A dimension of one element has no
+  // stride to speak of (is_contiguous() ignores it too).
+  static const auto packed_rows = [](const Tensor& t, int64_t inner) {
+    int64_t want = 1;
+    for (int64_t i = t.dim() - 1; i >= t.dim() - inner; want *= t.size(i--))
+      if (t.size(i) != 1 && t.stride(i) != want) return t.contiguous();
+    return t;
+  };
   m.def("causal_conv1d_varlen", [](const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias, Tensor& y,
                                    const c10::optional<Tensor>& conv_state, const Tensor& cu_seqlens,
                                    const c10::optional<Tensor>& state_idx, const c10::optional<Tensor>& has_init,
@@ -796,20 +804,21 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                     const c10::optional<Tensor>& state_idx, const c10::optional<Tensor>& has_init,
                                     bool dt_softplus) {
     need_cuda(u, "u");
-    TORCH_CHECK(u.is_contiguous() && delta.is_contiguous() && y.is_contiguous() && B.dim() == 2 && B.stride(1) == 1 &&
-                    C.dim() == 2 && C.stride(1) == 1 && A.is_contiguous() && A.scalar_type() == at::kFloat &&
-                    u.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16,
-                "selective_scan: contiguous bf16 u/delta, bf16 B/C of contiguous rows, fp32 A");
-    TORCH_CHECK(!z.has_value() || (z->dim() == 2 && z->stride(1) == 1), "selective_scan: rows of z contiguous");
-    check_rc(mb_selective_scan_varlen(u.data_ptr(), delta.data_ptr(), A.data_ptr<float>(), B.data_ptr(),
-                                      C.data_ptr(), D.has_value() ? D->data_ptr<float>() : nullptr, optptr(z),
+    TORCH_CHECK(u.is_contiguous() && delta.is_contiguous() && y.is_contiguous() && A.is_contiguous() &&
+                    A.scalar_type() == at::kFloat && u.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16,
+                "selective_scan: contiguous bf16 u/delta, bf16 B/C, fp32 A");
+    auto rows = [](const Tensor& t) { return packed_rows(t.dim() == 2 ? t : t.reshape({t.size(0), t.numel() / std::max<int64_t>(t.size(0), 1)}), 1); };
+    const Tensor Br = rows(B), Cr = rows(C), zr = z.has_value() ? rows(*z) : Tensor();
+    check_rc(mb_selective_scan_varlen(u.data_ptr(), delta.data_ptr(), A.data_ptr<float>(), Br.data_ptr(),
+                                      Cr.data_ptr(), D.has_value() ? D->data_ptr<float>() : nullptr,
+                                      z.has_value() ? zr.data_ptr() : nullptr,
                                       dt_bias.has_value() ? dt_bias->data_ptr<float>() : nullptr, y.data_ptr(),
                                       ssm_state.has_value() ? ssm_state->data_ptr<float>() : nullptr,
                                       cu_seqlens.data_ptr<int>(),
                                       state_idx.has_value() ? state_idx->data_ptr<int>() : nullptr,
                                       has_init.has_value() ? has_init->data_ptr<int>() : nullptr,
                                       cu_seqlens.numel() - 1, u.size(1), A.size(1), u.size(1),
-                                      z.has_value() ? z->stride(0) : 0, B.stride(0), C.stride(0), dt_softplus ? 1 : 0, cur_stream()),
+                                      z.has_value() ? zr.stride(0) : 0, Br.stride(0), Cr.stride(0), dt_softplus ? 1 : 0, cur_stream()),
              "selective_scan_varlen");
   });
   m.def("ssd_scan_varlen", [](const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C,
@@ -818,11 +827,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                               const c10::optional<Tensor>& state_idx, const c10::optional<Tensor>& has_init,
                               bool dt_softplus) {
     need_cuda(x, "x");
-    auto rows = [](const Tensor& t) { return t.dim() == 3 && t.stride(2) == 1 && t.stride(1) == t.size(2); };
-    TORCH_CHECK(rows(x) && dt.dim() == 2 && dt.stride(1) == 1 && rows(B) && rows(C) && y.is_contiguous() &&
-                    A.scalar_type() == at::kFloat && x.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16,
-                "ssd_scan: x [T, H, P], dt [T, H], B/C [T, G, N] bf16 of contiguous rows, A fp32 [H]");
-    check_rc(mb_ssd_scan_varlen(x.data_ptr(), dt.data_ptr(), A.data_ptr<float>(), B.data_ptr(), C.data_ptr(),
+    TORCH_CHECK(x.dim() == 3 && B.dim() == 3 && C.dim() == 3 && y.is_contiguous() && A.scalar_type() == at::kFloat &&
+                    x.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16,
+                "ssd_scan: x [T, H, P], dt [T, H], B/C [T, G, N] bf16, A fp32 [H]");
+    const Tensor xr = packed_rows(x, 2), Br = packed_rows(B, 2), Cr = packed_rows(C, 2),
+                 dtr = packed_rows(dt.dim() == 2 ? dt : dt.reshape({x.size(0), x.size(1)}), 1);
+    check_rc(mb_ssd_scan_varlen(xr.data_ptr(), dtr.data_ptr(), A.data_ptr<float>(), Br.data_ptr(), Cr.data_ptr(),
                                 D.has_value() ? D->data_ptr<float>() : nullptr,
                                 dt_bias.has_value() ? dt_bias->data_ptr<float>() : nullptr, y.data_ptr(),
                                 ssm_state.has_value() ? ssm_state->data_ptr<float>() : nullptr,
@@ -830,7 +840,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                 state_idx.has_value() ? state_idx->data_ptr<int>() : nullptr,
                                 has_init.has_value() ? has_init->data_ptr<int>() : nullptr,
                                 cu_seqlens.numel() - 1, x.size(0), x.size(1), x.size(2), B.size(2), B.size(1),
-                                x.stride(0), dt.stride(0), B.stride(0), C.stride(0), dt_softplus ? 1 : 0, cur_stream()),
+                                xr.stride(0), dtr.stride(0), Br.stride(0), Cr.stride(0), dt_softplus ? 1 : 0, cur_stream()),
              "ssd_scan_varlen");
   });
   m.def("gated_rms_norm", [](const Tensor& y, const Tensor& z, const Tensor& w, Tensor& out, double eps) {

@@ -116,12 +116,6 @@ def _native_ok(t):
     return t.is_cuda and t.dtype == torch.bfloat16
 
 
-def _rows(t):
-    """``t`` as the kernels take it: any distance between rows (tokens), each row contiguous."""
-    inner = t.stride(-1) == 1 and (t.dim() == 2 or t.stride(1) == t.shape[2])
-    return t if inner else t.contiguous()
-
-
 def causal_conv1d_varlen(x, w, bias, cu_seqlens, conv_state=None, state_idx=None, has_init=None, silu=True):
     """x [T, D]; w [D, W]; conv_state fp32 [slots, D, W-1] holds the last W-1 inputs of each live sequence."""
     if not _native_ok(x) or w.shape[1] not in (2, 3, 4, 8):
@@ -139,9 +133,8 @@ def selective_scan_varlen(u, delta, A, B, C, D=None, z=None, dt_bias=None, cu_se
         return selective_scan_reference(u, delta, A, B, C, D, z, dt_bias, cu_seqlens, ssm_state, state_idx,
                                         has_init, dt_softplus)
     y = torch.empty_like(u)
-    _lib().selective_scan_varlen(u.contiguous(), delta.contiguous(), A.float().contiguous(), _rows(B),
-                                 _rows(C), None if D is None else D.float().contiguous(),
-                                 None if z is None else _rows(z),
+    _lib().selective_scan_varlen(u.contiguous(), delta.contiguous(), A.float().contiguous(), B,
+                                 C, None if D is None else D.float().contiguous(), z,
                                  None if dt_bias is None else dt_bias.float().contiguous(), y, ssm_state,
                                  _opt_i32(cu_seqlens, u.device), _opt_i32(state_idx, u.device),
                                  _opt_i32(has_init, u.device), dt_softplus)
@@ -156,7 +149,7 @@ def ssd_scan_varlen(x, dt, A, B, C, D=None, dt_bias=None, cu_seqlens=None, ssm_s
         return ssd_scan_reference(x, dt, A, B, C, D, dt_bias, cu_seqlens, ssm_state, state_idx, has_init,
                                   dt_softplus)
     y = torch.empty_like(x)
-    _lib().ssd_scan_varlen(_rows(x), _rows(dt), A.float().contiguous(), _rows(B), _rows(C),
+    _lib().ssd_scan_varlen(x, dt, A.float().contiguous(), B, C,           # tokens (rows) at any distance
                            None if D is None else D.float().contiguous(),
                            None if dt_bias is None else dt_bias.float().contiguous(), y, ssm_state,
                            _opt_i32(cu_seqlens, x.device), _opt_i32(state_idx, x.device),

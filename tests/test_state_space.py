@@ -203,3 +203,25 @@ def test_gated_rms_norm(D):
     g = y.double() * z.double() / (1 + torch.exp(-z.double()))
     want = g * torch.rsqrt(g.pow(2).mean(-1, keepdim=True) + 1e-5) * w.double()
     assert _rel(ss.gated_rms_norm(y, z, w, 1e-5), want) < 2 ** -8
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,P,N", [(1, 64, 16), (1, 4, 16), (4, 1, 8), (4, 32, 1)])
+def test_strides_of_single_elements(H, P, N):
+    """Dimensions of one element may have any stride: one head, one group, one value, one channel."""
+    torch.manual_seed(9)
+    dev, lens = "cuda", [40, 1]
+    T, cu = sum(lens), _cu(lens, dev)
+    bf = lambda *s, k=1.0: (torch.randn(*s, device=dev) * k).to(torch.bfloat16)
+    loose = lambda t: torch.as_strided(t, t.shape, [st if n != 1 else 7777 for st, n in zip(t.stride(), t.shape)])
+    x, dt, B, C = bf(T, H, P), bf(T, H, k=0.5), bf(T, 1, N), bf(T, 1, N)
+    A = -torch.rand(H, device=dev) - 0.1
+    want = ss.ssd_scan_varlen(x, dt, A, B, C, None, None, cu)
+    assert torch.equal(ss.ssd_scan_varlen(loose(x), loose(dt), A, loose(B), loose(C), None, None, cu), want)
+    if H == 1:
+        assert torch.equal(ss.ssd_scan_varlen(x, dt.flatten(), A, B, C, None, None, cu), want)
+    u, z, b, c = bf(T, 1), bf(T, 1), bf(T, 8), bf(T, 8)
+    a = -torch.rand(1, 8, device=dev)
+    want = ss.selective_scan_varlen(u, u, a, b, c, None, z, None, cu)
+    assert torch.equal(ss.selective_scan_varlen(u, u, a, b, c, None, loose(z), None, cu), want)
+    assert torch.equal(ss.selective_scan_varlen(u, u, a, b.unsqueeze(2), c, None, z.unsqueeze(2), None, cu), want)
