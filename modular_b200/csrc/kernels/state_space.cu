@@ -408,6 +408,9 @@ __device__ __forceinline__ uint32_t take_bf16(float& x, float& y) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+// the signs' places of two bf16 values set where one is infinite or NaN (an exponent of ones carries into them)
+__device__ __forceinline__ uint32_t mark_special(uint32_t w) { return (w & 0x7f807f80u) + 0x00800080u; }
+
 struct SsdChunk {
   const __nv_bfloat16 *x, *dt, *B, *C;
   const float *A, *Dskip, *dt_bias;
@@ -594,20 +597,44 @@ __global__ void __launch_bounds__(kChunkThreads, 2) ssd_chunk_kernel(const SsdCh
         for (int j = 0; j < 2; ++j) { o[i][j][0] *= f0; o[i][j][1] *= f0; o[i][j][2] *= f1; o[i][j][3] *= f1; }
       }
     }
-    __syncthreads();                                 // the products of every warp are in sP
+    // an infinite or NaN input must not reach the tokens before it, whose products with it are zeros
+    uint32_t odd = 0;
 #pragma unroll
-    for (int kb = 0; kb < 4; ++kb) {
-      uint32_t b[4];
-      ldsm4_t(b, sV + (kb * 16 + (mi & 1) * 8 + r8) * kLdV + warp * 16 + (mi >> 1) * 8);
+    for (int q = 0; q < kChunk * kNV / 8 / kChunkThreads; ++q) {
+      const int at = q * kChunkThreads + tid;
+      const uint4 w = *reinterpret_cast<const uint4*>(sV + at / (kNV / 8) * kLdV + at % (kNV / 8) * 8);
+      odd |= mark_special(w.x) | mark_special(w.y) | mark_special(w.z) | mark_special(w.w);
+    }
+    const bool special = __syncthreads_or(odd & 0x80008000u);      // the products of every warp are in sP
+    if (!special) {
 #pragma unroll
-      for (int half = 0; half < 2; ++half)
+      for (int kb = 0; kb < 4; ++kb) {
+        uint32_t b[4];
+        ldsm4_t(b, sV + (kb * 16 + (mi & 1) * 8 + r8) * kLdV + warp * 16 + (mi >> 1) * 8);
 #pragma unroll
-        for (int i = kb; i < 4; ++i) {
-          uint32_t a[4];
-          ldsm4(a, sP + (half * kChunk + i * 16 + (lane & 15)) * kLdP + kb * 16 + (lane >> 4) * 8);
-          mma(o[i][0], a, b[0], b[1]);
-          mma(o[i][1], a, b[2], b[3]);
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+          for (int i = kb; i < 4; ++i) {
+            uint32_t a[4];
+            ldsm4(a, sP + (half * kChunk + i * 16 + (lane & 15)) * kLdP + kb * 16 + (lane >> 4) * 8);
+            mma(o[i][0], a, b[0], b[1]);
+            mma(o[i][1], a, b[2], b[3]);
+          }
+      }
+    } else {
+      for (int t = 0; t < m; ++t) {
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = __bfloat162float(sV[t * kLdV + warp * 16 + (j >> 1) * 8 + col2 + (j & 1)]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {                // rows i / 2, its lower or upper half
+          const int r = (i >> 1) * 16 + row4 + 8 * (i & 1);
+          if (r < t) continue;
+          const float w = __bfloat162float(sP[r * kLdP + t]) + __bfloat162float(sP[(kChunk + r) * kLdP + t]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o[i >> 1][j >> 1][2 * (i & 1) + (j & 1)] = fmaf(w, v[j], o[i >> 1][j >> 1][2 * (i & 1) + (j & 1)]);
         }
+      }
     }
     bf16* out = p.y + (static_cast<size_t>(t0 + c0) * p.H + h) * P;
 #pragma unroll

@@ -225,3 +225,21 @@ def test_strides_of_single_elements(H, P, N):
     want = ss.selective_scan_varlen(u, u, a, b, c, None, z, None, cu)
     assert torch.equal(ss.selective_scan_varlen(u, u, a, b, c, None, loose(z), None, cu), want)
     assert torch.equal(ss.selective_scan_varlen(u, u, a, b.unsqueeze(2), c, None, z.unsqueeze(2), None, cu), want)
+
+
+@pytest.mark.gpu
+def test_ssd_special_inputs_stay_causal():
+    """An infinite or NaN input of a prompt changes its own row of the state from its token on, and nothing before it."""
+    torch.manual_seed(10)
+    dev, lens, (H, P, N) = "cuda", [150, 64, 70], (3, 32, 16)
+    T = sum(lens)
+    bf = lambda *s, k=1.0: (torch.randn(*s, device=dev) * k).to(torch.bfloat16)
+    x, dt, B, C = bf(T, H, P), bf(T, H, k=0.5), bf(T, 1, N, k=0.3), bf(T, 1, N, k=0.3)
+    x[77, 1, 3], x[5, 0, 8], x[149, 2, 0], x[150 + 63, 2, 31] = float("inf"), float("nan"), -float("inf"), float("nan")
+    A, bias, st = -torch.rand(H, device=dev) - 0.1, torch.randn(H, device=dev) * 0.1, torch.randn(3, H, P, N, device=dev)
+    ref, idx, init = st.clone(), torch.arange(3, dtype=torch.int32, device=dev), torch.ones(3, dtype=torch.int32, device=dev)
+    y = ss.ssd_scan_varlen(x, dt, A, B, C, None, bias, _cu(lens, dev), st, idx, init, True).cpu()
+    want = ss.ssd_scan_reference(x.cpu(), dt.cpu(), A.cpu(), B.cpu(), C.cpu(), None, bias.cpu(), _cu(lens), ref.cpu(), idx.cpu(), init.cpu(), True)
+    ok = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(y), ok) and not ok.all()
+    assert _rel(y[ok], want[ok]) < 2 ** -8
