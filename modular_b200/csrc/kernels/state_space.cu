@@ -419,8 +419,10 @@ struct SsdChunk {
   const int *cu_seqlens, *state_idx, *has_init;
   int H, P, N, G, ldx, ld_dt, ldb, ldc, dt_softplus, col_blocks;
 };
-// per chunk: c_i, 2^(sum beyond j) dt_j, dt_j, 2^c_i
-struct SsdTimes { float cum[kChunk], tail[kChunk], dt[kChunk], grow[kChunk], total; };
+// per chunk: c_i (and what its rounding left), 2^(sum beyond j) dt_j, dt_j, 2^c_i. With c_i alone a difference c_i - c_j would
+// carry the rounding of sums that may be thousands of times larger than it: after a token that decays by 2^-50000 the next ones'
+// weights were off by 2 in 1000.
+struct SsdTimes { float cum[kChunk], rest[kChunk], tail[kChunk], dt[kChunk], grow[kChunk], total; };
 
 // 16 queries (rows 16 W ..) with the keys at or before them, weighted, into sP as hi and lo parts
 template <int W, int DK>
@@ -445,12 +447,13 @@ __device__ __forceinline__ void ssd_products(const __nv_bfloat16* sC, const __nv
 #pragma unroll
   for (int nt = 0; nt < 2 * (W + 1); ++nt) {
     const int j = nt * 8 + col2;
-    const float c0 = tm.cum[j], c1 = tm.cum[j + 1], d0 = tm.dt[j], d1 = tm.dt[j + 1];
+    const float c0 = tm.cum[j], c1 = tm.cum[j + 1], r0 = tm.rest[j], r1 = tm.rest[j + 1], d0 = tm.dt[j], d1 = tm.dt[j + 1];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int i = W * 16 + row4 + 8 * e;
-      const float ci = tm.cum[i];
-      float a0 = i >= j ? sc[nt][2 * e] * (ex2(ci - c0) * d0) : 0.f, a1 = i > j ? sc[nt][2 * e + 1] * (ex2(ci - c1) * d1) : 0.f;
+      const float ci = tm.cum[i], ri = tm.rest[i];
+      float a0 = i >= j ? sc[nt][2 * e] * (ex2((ci - c0) + (ri - r0)) * d0) : 0.f;
+      float a1 = i > j ? sc[nt][2 * e + 1] * (ex2((ci - c1) + (ri - r1)) * d1) : 0.f;
       *reinterpret_cast<uint32_t*>(sP + i * kLdP + j) = take_bf16(a0, a1);
       *reinterpret_cast<uint32_t*>(sP + (kChunk + i) * kLdP + j) = take_bf16(a0, a1);
     }
@@ -505,19 +508,23 @@ __global__ void __launch_bounds__(kChunkThreads, 2) ssd_chunk_kernel(const SsdCh
       if (c0 + 2 * lane + e >= n) dt[e] = 0.f;
       l[e] = dt[e] * a2;
     }
-    const float pair = l[0] + l[1];
-    float up = pair, down = pair;                    // sums up to and from this pair
+    const double pair = static_cast<double>(l[0]) + l[1];
+    double up = pair;                                // sum up to this pair
+    float down = l[0] + l[1];                        // and from it: the large powers are the short sums
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const float u = __shfl_up_sync(0xffffffffu, up, o), w = __shfl_down_sync(0xffffffffu, down, o);
+      const double u = __shfl_up_sync(0xffffffffu, up, o);
+      const float w = __shfl_down_sync(0xffffffffu, down, o);
       if (lane >= o) up += u;
       if (lane + o < 32) down += w;
     }
-    float before = __shfl_up_sync(0xffffffffu, up, 1), after = __shfl_down_sync(0xffffffffu, down, 1);
-    if (lane == 0) before = 0.f;
+    double before = __shfl_up_sync(0xffffffffu, up, 1);
+    float after = __shfl_down_sync(0xffffffffu, down, 1);
+    if (lane == 0) before = 0.;
     if (lane == 31) after = 0.f;
-    const float c0_ = before + l[0], c1_ = before + pair;
+    const float c0_ = static_cast<float>(before + l[0]), c1_ = static_cast<float>(before + pair);
     tm.cum[2 * lane] = c0_; tm.cum[2 * lane + 1] = c1_;
+    tm.rest[2 * lane] = static_cast<float>(before + l[0] - c0_); tm.rest[2 * lane + 1] = static_cast<float>(before + pair - c1_);
     tm.grow[2 * lane] = ex2(c0_); tm.grow[2 * lane + 1] = ex2(c1_);
     tm.tail[2 * lane] = ex2(after + l[1]) * dt[0]; tm.tail[2 * lane + 1] = ex2(after) * dt[1];
     tm.dt[2 * lane] = dt[0]; tm.dt[2 * lane + 1] = dt[1];

@@ -243,3 +243,18 @@ def test_ssd_special_inputs_stay_causal():
     ok = torch.isfinite(want)
     assert torch.equal(torch.isfinite(y), ok) and not ok.all()
     assert _rel(y[ok], want[ok]) < 2 ** -8
+
+
+@pytest.mark.gpu
+def test_ssd_decays_of_many_octaves():
+    """Every eleventh token all but clears the state (2^-94000 and less): what follows it keeps its own, small decays."""
+    torch.manual_seed(11)
+    dev, T, (H, P, N) = "cuda", 200, (4, 32, 64)
+    bf = lambda *s, k=1.0: (torch.randn(*s, device=dev) * k).to(torch.bfloat16)
+    dt = torch.rand(T, H, device=dev) * 2.0 ** -15
+    dt[::11] = 2.0 + torch.rand(H, device=dev)
+    dt = dt.to(torch.bfloat16)
+    x, B, C, A = bf(T, H, P), bf(T, 1, N, k=0.3), bf(T, 1, N, k=0.3), torch.full((H,), -2.0 ** 15, device=dev)
+    y = ss.ssd_scan_varlen(x, dt, A, B, C, None, None, _cu([T], dev), dt_softplus=False)
+    want = ss.ssd_scan_reference(x.cpu().float(), dt.cpu(), A.cpu(), B.cpu(), C.cpu(), None, None, _cu([T]), dt_softplus=False)
+    assert _rel(y.cpu(), want) < 2 ** -8                 # one rounding to bf16
