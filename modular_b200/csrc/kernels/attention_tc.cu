@@ -499,6 +499,7 @@ extern "C" int mb_latent_prefill_tc(const void* q, int ldq, int q_head, const vo
 namespace mb {
 namespace atc {
 // Rows [0, kv_len[s]) of every sequence, out of the pages: latents [rows, R] and rotated parts [rows, 64], 16 bytes a thread.
+// Rows between a sequence's end and the next one's start are zeros.
 __global__ void latent_gather_kernel(const bf16* __restrict__ cache, long long page_stride, int ld, int page, const int32_t* __restrict__ block_table,
                                      int bt_stride, const int32_t* __restrict__ kv_start, const int32_t* __restrict__ kv_len, int B, int R,
                                      bf16* __restrict__ c, bf16* __restrict__ rope, long long rows) {
@@ -512,10 +513,12 @@ __global__ void latent_gather_kernel(const bf16* __restrict__ cache, long long p
     if (kv_start[m] <= row) lo = m; else hi = m - 1;
   }
   const int at = row - kv_start[lo];
-  if (at >= kv_len[lo]) return;
-  const bf16* src = cache + block_table[static_cast<long long>(lo) * bt_stride + at / page] * page_stride + static_cast<long long>(at % page) * ld + col;
+  uint4 v = make_uint4(0, 0, 0, 0);
+  if (at < kv_len[lo])
+    v = *reinterpret_cast<const uint4*>(cache + block_table[static_cast<long long>(lo) * bt_stride + at / page] * page_stride +
+                                        static_cast<long long>(at % page) * ld + col);
   bf16* dst = col < R ? c + static_cast<long long>(row) * R + col : rope + static_cast<long long>(row) * 64 + (col - R);
-  *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
+  *reinterpret_cast<uint4*>(dst) = v;
 }
 }  // namespace atc
 }  // namespace mb

@@ -165,9 +165,11 @@ _PER_ROW, _PER_PAIR = 256 * 512, (512 + 64 + 512) - (128 + 64 + 128)
 
 @dataclass
 class PromptPlan:
-    """Work of a prompt step in the projected form: ``rows`` cache rows, those of sequence s from ``kv_start[s]`` on, and the
-    query tiles of 128 tokens."""
+    """Work of a prompt step in the projected form: ``rows`` cache rows, those of sequence s from row ``kv_start[s]`` of
+    ``scratch`` rows on (a multiple of 64, the keys of a tile: no tile reads another sequence's rows, whose values a
+    product with a probability of zero would let through if they are not finite), and the query tiles of 128 tokens."""
     rows: int
+    scratch: int
     kv_start: torch.Tensor
     tile_seq: torch.Tensor
     tile_q0: torch.Tensor
@@ -187,13 +189,13 @@ def prompt_plan(T: int, q_len, kv_len) -> Optional[PromptPlan]:
         return None
     start, seq, q0 = [0], [], []
     for s, (n, k) in enumerate(zip(ql, kl)):
-        start.append(start[-1] + k)
+        start.append(start[-1] + -(-k // 64) * 64)
         for t in range(0, n, 128):
             seq.append(s)
             q0.append(t)
     B, n = len(ql), len(seq)
     buf = torch.tensor(start[:B] + seq + q0, dtype=torch.int32).to(q_len.device)
-    return PromptPlan(rows, buf[:B], buf[B: B + n], buf[B + n:])
+    return PromptPlan(rows, start[B], buf[:B], buf[B: B + n], buf[B + n:])
 
 
 def stacked_up(w_uk: torch.Tensor, w_uv: torch.Tensor) -> torch.Tensor:
@@ -205,8 +207,8 @@ def stacked_up(w_uk: torch.Tensor, w_uv: torch.Tensor) -> torch.Tensor:
 def prompt_attention(plan: PromptPlan, q, q_rope, w_up, cache, block_table, q_start, q_len, kv_len, out, scale, sink=None, window=0, gate=None):
     """q [T, h, 128], q_rope [T, h, 64] (rotated, any strides), cache [pages, page, latent + 64]; out [T, h * 128 ..]."""
     R, L = w_up.shape[1], _lib()
-    c = torch.empty(plan.rows, R, dtype=q.dtype, device=q.device)
-    k_rope = torch.empty(plan.rows, 64, dtype=q.dtype, device=q.device)
+    c = torch.empty(plan.scratch, R, dtype=q.dtype, device=q.device)
+    k_rope = torch.empty(plan.scratch, 64, dtype=q.dtype, device=q.device)
     L.latent_gather(cache, block_table, plan.kv_start, kv_len, c, k_rope)
     L.latent_prefill(q, q_rope, ops.linear(c, w_up), k_rope, plan.kv_start, q_start, q_len, kv_len, plan.tile_seq, plan.tile_q0, out, scale,
                      sink=sink, window=window, gate=gate)

@@ -310,6 +310,31 @@ def test_latent_prompt_attention(h, R, window, extras):
         at += n
 
 
+def test_latent_prompts_of_one_step_do_not_meet():
+    """A request whose cache rows are not finite leaves the other requests of the step as they are without it."""
+    from modular_b200.nn import latent_attention as la
+
+    torch.manual_seed(5)
+    h, R, page, ql = 4, 128, 64, [420, 421, 444]
+    cache = torch.randn(21, page, R + 64, device=DEV).to(torch.bfloat16)
+    bt = torch.tensor([list(range(7)), list(range(7, 14)), list(range(14, 21))], dtype=torch.int32, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    q = torch.randn(sum(ql), h, 192, device=DEV).to(torch.bfloat16)
+    up = (torch.randn(2 * h * 128, R, device=DEV) * R ** -0.5).to(torch.bfloat16)
+
+    def run():
+        out = torch.zeros(sum(ql), h * 128, device=DEV, dtype=torch.bfloat16)
+        la.prompt_attention(la.prompt_plan(sum(ql), i32(ql), i32(ql)), q[:, :, :128], q[:, :, 128:], up, cache, bt, i32([0, 420, 841]), i32(ql),
+                            i32(ql), out, 192 ** -0.5)
+        return out
+
+    want = run()
+    cache[7:14] = float("nan")                         # the request in the middle
+    got = run()
+    assert torch.equal(got[:420], want[:420]) and torch.equal(got[841:], want[841:]) and not torch.isfinite(got[420:841]).all()
+    ops.check_device_error()
+
+
 @pytest.mark.parametrize("counts,N,K,swiglu", [([0, 257, 1, 900, 255, 256, 0, 3], 384, 128, False), ([700, 0, 513], 200, 72, True),
                                               ([300] * 5, 1408, 256, True), ([128, 128], 256, 64, False)])
 def test_grouped_gemm_pairs(counts, N, K, swiglu):
