@@ -18,6 +18,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "../common/api.h"
 #include "../common/launch.h"
 
@@ -420,7 +422,8 @@ __global__ void ssd_scan_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
 // The chain from chunk to chunk is the bound (one CTA per sequence, head and 64 rows walks the chunks in order, about
 // 7 us each), so it is kept short: two barriers a chunk, tiles and step sizes fetched one chunk ahead.
 // Two sequences, 4096 tokens, 80 heads x 64 x 128: 12742 us token by token (two barriers and a load from global memory on
-// every token's chain), 239 us so.
+// every token's chain), 239 us so (in a row 224, and 231 with `rest` and the check of the products below). Up to 16 tokens a
+// chunk does the work of 16: 64 sequences of 4 tokens 563 us walked, 168 as whole chunks, 111 so. Three CTAs per SM up to 32 states.
 constexpr int kChunk = 64, kNV = 64, kChunkThreads = 128, kLdV = kNV + 8, kLdP = kChunk + 8;
 
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const void* p) {
@@ -445,8 +448,12 @@ __device__ __forceinline__ uint32_t take_bf16(float& x, float& y) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// the signs' places of two bf16 values set where one is infinite or NaN (an exponent of ones carries into them)
-__device__ __forceinline__ uint32_t mark_special(uint32_t w) { return (w & 0x7f807f80u) + 0x00800080u; }
+// a + b, and in `left` what its rounding left (Knuth's exact sum of two floats)
+__device__ __forceinline__ float two_sum(float a, float b, float& left) {
+  const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+  left = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+  return s;
+}
 
 struct SsdChunk {
   const __nv_bfloat16 *x, *dt, *B, *C;
@@ -459,7 +466,7 @@ struct SsdChunk {
 // per chunk: c_i (and what its rounding left), 2^(sum beyond j) dt_j, dt_j, 2^c_i. With c_i alone a difference c_i - c_j would
 // carry the rounding of sums that may be thousands of times larger than it: after a token that decays by 2^-50000 the next ones'
 // weights were off by 2 in 1000.
-struct SsdTimes { float cum[kChunk], rest[kChunk], tail[kChunk], dt[kChunk], grow[kChunk], total; };
+struct alignas(8) SsdTimes { float cum[kChunk], rest[kChunk], tail[kChunk], dt[kChunk], grow[kChunk], total; };
 
 // 16 queries (rows 16 W ..) with the keys at or before them, weighted, into sP as hi and lo parts
 template <int W, int DK>
@@ -481,16 +488,20 @@ __device__ __forceinline__ void ssd_products(const __nv_bfloat16* sC, const __nv
       mma(sc[2 * np + 1], a, b[2], b[3]);
     }
   }
+  const float ci[2] = {tm.cum[W * 16 + row4], tm.cum[W * 16 + row4 + 8]}, ri[2] = {tm.rest[W * 16 + row4], tm.rest[W * 16 + row4 + 8]};
 #pragma unroll
   for (int nt = 0; nt < 2 * (W + 1); ++nt) {
     const int j = nt * 8 + col2;
-    const float c0 = tm.cum[j], c1 = tm.cum[j + 1], r0 = tm.rest[j], r1 = tm.rest[j + 1], d0 = tm.dt[j], d1 = tm.dt[j + 1];
+    const float2 c = *reinterpret_cast<const float2*>(&tm.cum[j]), r = *reinterpret_cast<const float2*>(&tm.rest[j]),
+                 d = *reinterpret_cast<const float2*>(&tm.dt[j]);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int i = W * 16 + row4 + 8 * e;
-      const float ci = tm.cum[i], ri = tm.rest[i];
-      float a0 = i >= j ? sc[nt][2 * e] * (ex2((ci - c0) + (ri - r0)) * d0) : 0.f;
-      float a1 = i > j ? sc[nt][2 * e + 1] * (ex2((ci - c1) + (ri - r1)) * d1) : 0.f;
+      float a0 = sc[nt][2 * e] * (ex2((ci[e] - c.x) + (ri[e] - r.x)) * d.x), a1 = sc[nt][2 * e + 1] * (ex2((ci[e] - c.y) + (ri[e] - r.y)) * d.y);
+      if (nt >= 2 * W) {                             // the block on the diagonal
+        if (i < j) a0 = 0.f;
+        if (i <= j) a1 = 0.f;
+      }
       *reinterpret_cast<uint32_t*>(sP + i * kLdP + j) = take_bf16(a0, a1);
       *reinterpret_cast<uint32_t*>(sP + (kChunk + i) * kLdP + j) = take_bf16(a0, a1);
     }
@@ -498,7 +509,7 @@ __device__ __forceinline__ void ssd_products(const __nv_bfloat16* sC, const __nv
 }
 
 template <int DK>
-__global__ void __launch_bounds__(kChunkThreads, 2) ssd_chunk_kernel(const SsdChunk p) {
+__global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_kernel(const SsdChunk p) {
   typedef __nv_bfloat16 bf16;
   constexpr int LDK = DK + 8, KB = DK / 16, kStage = kChunk * (2 * LDK + kLdV);
   extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -545,23 +556,25 @@ __global__ void __launch_bounds__(kChunkThreads, 2) ssd_chunk_kernel(const SsdCh
       if (c0 + 2 * lane + e >= n) dt[e] = 0.f;
       l[e] = dt[e] * a2;
     }
-    const double pair = static_cast<double>(l[0]) + l[1];
-    double up = pair;                                // sum up to this pair
-    float down = l[0] + l[1];                        // and from it: the large powers are the short sums
+    // sums up to this pair as a float and what its rounding left, and from it (the large powers are the short sums)
+    float rest, hi = two_sum(l[0], l[1], rest), down = hi;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const double u = __shfl_up_sync(0xffffffffu, up, o);
-      const float w = __shfl_down_sync(0xffffffffu, down, o);
-      if (lane >= o) up += u;
+      const float u = __shfl_up_sync(0xffffffffu, hi, o), v = __shfl_up_sync(0xffffffffu, rest, o), w = __shfl_down_sync(0xffffffffu, down, o);
+      if (lane >= o) {
+        float left;
+        hi = two_sum(hi, u, left);
+        rest += v + left;
+      }
       if (lane + o < 32) down += w;
     }
-    double before = __shfl_up_sync(0xffffffffu, up, 1);
-    float after = __shfl_down_sync(0xffffffffu, down, 1);
-    if (lane == 0) before = 0.;
+    float before = __shfl_up_sync(0xffffffffu, hi, 1), before_rest = __shfl_up_sync(0xffffffffu, rest, 1);
+    float after = __shfl_down_sync(0xffffffffu, down, 1), left;
+    if (lane == 0) before = before_rest = 0.f;
     if (lane == 31) after = 0.f;
-    const float c0_ = static_cast<float>(before + l[0]), c1_ = static_cast<float>(before + pair);
+    const float c0_ = two_sum(before, l[0], left), c1_ = hi;
     tm.cum[2 * lane] = c0_; tm.cum[2 * lane + 1] = c1_;
-    tm.rest[2 * lane] = static_cast<float>(before + l[0] - c0_); tm.rest[2 * lane + 1] = static_cast<float>(before + pair - c1_);
+    tm.rest[2 * lane] = before_rest + left; tm.rest[2 * lane + 1] = rest;
     tm.grow[2 * lane] = ex2(c0_); tm.grow[2 * lane + 1] = ex2(c1_);
     tm.tail[2 * lane] = ex2(after + l[1]) * dt[0]; tm.tail[2 * lane + 1] = ex2(after) * dt[1];
     tm.dt[2 * lane] = dt[0]; tm.dt[2 * lane + 1] = dt[1];
@@ -596,139 +609,150 @@ __global__ void __launch_bounds__(kChunkThreads, 2) ssd_chunk_kernel(const SsdCh
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                 // this chunk is in; everyone is done with the last one's stage, times and sP
     if (c0 + kChunk < n) fetch(c0 + kChunk, stages + ((it + 1) & 1) * kStage);
-    switch (warp) {
-      case 0:                                        // the fewest products: this warp also prepares the next chunk's times
-        ssd_products<0, DK>(sC, sB, sP, tm, lane);
-        if (c0 + kChunk < n) {
-          make_times(c0 + kChunk, times[(it + 1) & 1]);
-          read_dt(c0 + 2 * kChunk);
-        }
-        break;
-      case 1: ssd_products<1, DK>(sC, sB, sP, tm, lane); break;
-      case 2: ssd_products<2, DK>(sC, sB, sP, tm, lane); break;
-      default: ssd_products<3, DK>(sC, sB, sP, tm, lane); break;
-    }
-    // what the state before the chunk contributes, for all tokens and this warp's 16 rows
-    float o[4][2][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) o[i][j][0] = o[i][j][1] = o[i][j][2] = o[i][j][3] = 0.f;
-    if (have_state) {
-#pragma unroll
-      for (int kb = 0; kb < KB; ++kb) {
-        uint32_t hi[2][2], lo[2][2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            float u = S[2 * kb + e][2 * j], w = S[2 * kb + e][2 * j + 1];
-            hi[j][e] = take_bf16(u, w);
-            lo[j][e] = take_bf16(u, w);
+    // NB: blocks of 16 tokens that have any
+    auto chunk = [&](auto blocks) {
+      constexpr int NB = decltype(blocks)::value;
+      switch (warp) {
+        case 0:                                        // the fewest products: this warp also prepares the next chunk's times
+          ssd_products<0, DK>(sC, sB, sP, tm, lane);
+          if (c0 + kChunk < n) {
+            make_times(c0 + kChunk, times[(it + 1) & 1]);
+            read_dt(c0 + 2 * kChunk);
           }
-        uint32_t a[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) ldsm4(a[i], sC + (i * 16 + (lane & 15)) * LDK + kb * 16 + (lane >> 4) * 8);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { mma(o[i][0], a[i], hi[0][0], hi[0][1]); mma(o[i][1], a[i], hi[1][0], hi[1][1]); }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { mma(o[i][0], a[i], lo[0][0], lo[0][1]); mma(o[i][1], a[i], lo[1][0], lo[1][1]); }
+          break;
+        case 1: if constexpr (NB > 1) ssd_products<1, DK>(sC, sB, sP, tm, lane); break;
+        case 2: if constexpr (NB > 2) ssd_products<2, DK>(sC, sB, sP, tm, lane); break;
+        default: if constexpr (NB > 3) ssd_products<3, DK>(sC, sB, sP, tm, lane); break;
       }
+      // what the state before the chunk contributes, for all tokens and this warp's 16 rows
+      float o[NB][2][4];
+      auto from_state = [&]() {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float f0 = tm.grow[i * 16 + row4], f1 = tm.grow[i * 16 + row4 + 8];
+        for (int i = 0; i < NB; ++i)
 #pragma unroll
-        for (int j = 0; j < 2; ++j) { o[i][j][0] *= f0; o[i][j][1] *= f0; o[i][j][2] *= f1; o[i][j][3] *= f1; }
-      }
-    }
-    // an infinite or NaN input must not reach the tokens before it, whose products with it are zeros
-    uint32_t odd = 0;
+          for (int j = 0; j < 2; ++j) o[i][j][0] = o[i][j][1] = o[i][j][2] = o[i][j][3] = 0.f;
+        if (have_state) {
 #pragma unroll
-    for (int q = 0; q < kChunk * kNV / 8 / kChunkThreads; ++q) {
-      const int at = q * kChunkThreads + tid;
-      const uint4 w = *reinterpret_cast<const uint4*>(sV + at / (kNV / 8) * kLdV + at % (kNV / 8) * 8);
-      odd |= mark_special(w.x) | mark_special(w.y) | mark_special(w.z) | mark_special(w.w);
-    }
-    const bool special = __syncthreads_or(odd & 0x80008000u);      // the products of every warp are in sP
-    if (!special) {
+          for (int kb = 0; kb < KB; ++kb) {
+            uint32_t hi[2][2], lo[2][2];
 #pragma unroll
-      for (int kb = 0; kb < 4; ++kb) {
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                float u = S[2 * kb + e][2 * j], w = S[2 * kb + e][2 * j + 1];
+                hi[j][e] = take_bf16(u, w);
+                lo[j][e] = take_bf16(u, w);
+              }
+            uint32_t a[NB][4];
+#pragma unroll
+            for (int i = 0; i < NB; ++i) ldsm4(a[i], sC + (i * 16 + (lane & 15)) * LDK + kb * 16 + (lane >> 4) * 8);
+#pragma unroll
+            for (int i = 0; i < NB; ++i) { mma(o[i][0], a[i], hi[0][0], hi[0][1]); mma(o[i][1], a[i], hi[1][0], hi[1][1]); }
+#pragma unroll
+            for (int i = 0; i < NB; ++i) { mma(o[i][0], a[i], lo[0][0], lo[0][1]); mma(o[i][1], a[i], lo[1][0], lo[1][1]); }
+          }
+#pragma unroll
+          for (int i = 0; i < NB; ++i) {
+            const float f0 = tm.grow[i * 16 + row4], f1 = tm.grow[i * 16 + row4 + 8];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) { o[i][j][0] *= f0; o[i][j][1] *= f0; o[i][j][2] *= f1; o[i][j][3] *= f1; }
+          }
+        }
+      };
+      from_state();
+      __syncthreads();                               // the products of every warp are in sP
+#pragma unroll
+      for (int kb = 0; kb < NB; ++kb) {
         uint32_t b[4];
         ldsm4_t(b, sV + (kb * 16 + (mi & 1) * 8 + r8) * kLdV + warp * 16 + (mi >> 1) * 8);
 #pragma unroll
         for (int half = 0; half < 2; ++half)
 #pragma unroll
-          for (int i = kb; i < 4; ++i) {
+          for (int i = kb; i < NB; ++i) {
             uint32_t a[4];
             ldsm4(a, sP + (half * kChunk + i * 16 + (lane & 15)) * kLdP + kb * 16 + (lane >> 4) * 8);
             mma(o[i][0], a, b[0], b[1]);
             mma(o[i][1], a, b[2], b[3]);
           }
       }
-    } else {
-      for (int t = 0; t < m; ++t) {
-        float v[4];
+      // The products with later tokens are zeros, and zero times an infinite or NaN input is NaN: a warp that finds such a result
+      // takes its products again, one token at a time, over the tokens at or before each row.
+      float zero[8] = {};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = __bfloat162float(sV[t * kLdV + warp * 16 + (j >> 1) * 8 + col2 + (j & 1)]);
+      for (int i = 0; i < NB; ++i)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {                // rows i / 2, its lower or upper half
-          const int r = (i >> 1) * 16 + row4 + 8 * (i & 1);
-          if (r < t) continue;
-          const float w = __bfloat162float(sP[r * kLdP + t]) + __bfloat162float(sP[(kChunk + r) * kLdP + t]);
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) o[i >> 1][j >> 1][2 * (i & 1) + (j & 1)] = fmaf(w, v[j], o[i >> 1][j >> 1][2 * (i & 1) + (j & 1)]);
+          for (int e = 0; e < 4; ++e) zero[j * 4 + e] = fmaf(o[i][j][e], 0.f, zero[j * 4 + e]);
+      const float all = ((zero[0] + zero[1]) + (zero[2] + zero[3])) + ((zero[4] + zero[5]) + (zero[6] + zero[7]));
+      if (__any_sync(0xffffffffu, all != 0.f)) {
+        from_state();
+        for (int t = 0; t < m; ++t) {
+          float v[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] = __bfloat162float(sV[t * kLdV + warp * 16 + (j >> 1) * 8 + col2 + (j & 1)]);
+#pragma unroll
+          for (int i = 0; i < 2 * NB; ++i) {           // rows i / 2, its lower or upper half
+            const int r = (i >> 1) * 16 + row4 + 8 * (i & 1);
+            if (r < t) continue;
+            const float w = __bfloat162float(sP[r * kLdP + t]) + __bfloat162float(sP[(kChunk + r) * kLdP + t]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o[i >> 1][j >> 1][2 * (i & 1) + (j & 1)] = fmaf(w, v[j], o[i >> 1][j >> 1][2 * (i & 1) + (j & 1)]);
+          }
         }
       }
-    }
-    bf16* out = p.y + (static_cast<size_t>(t0 + c0) * p.H + h) * P;
+      bf16* out = p.y + (static_cast<size_t>(t0 + c0) * p.H + h) * P;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < NB; ++i)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int r = i * 16 + row4 + 8 * e;
-        if (r >= m) continue;
+        for (int e = 0; e < 2; ++e) {
+          const int r = i * 16 + row4 + 8 * e;
+          if (r >= m) continue;
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int cl = warp * 16 + j * 8 + col2, c = v0 + cl;
-          if (c >= P) continue;
-          const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sV + r * kLdV + cl));
-          *reinterpret_cast<__nv_bfloat162*>(out + static_cast<size_t>(r) * p.H * P + c) =
-              __floats2bfloat162_rn(fmaf(dsk, xv.x, o[i][j][2 * e]), fmaf(dsk, xv.y, o[i][j][2 * e + 1]));
+          for (int j = 0; j < 2; ++j) {
+            const int cl = warp * 16 + j * 8 + col2, c = v0 + cl;
+            if (c >= P) continue;
+            const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sV + r * kLdV + cl));
+            *reinterpret_cast<__nv_bfloat162*>(out + static_cast<size_t>(r) * p.H * P + c) =
+                __floats2bfloat162_rn(fmaf(dsk, xv.x, o[i][j][2 * e]), fmaf(dsk, xv.y, o[i][j][2 * e + 1]));
+          }
+        }
+      // the state after the chunk
+      if (have_state) {
+        const float f = tm.total;
+#pragma unroll
+        for (int t = 0; t < 2 * KB; ++t) { S[t][0] *= f; S[t][1] *= f; S[t][2] *= f; S[t][3] *= f; }
+      }
+      have_state = true;
+#pragma unroll
+      for (int kb = 0; kb < NB; ++kb) {
+        uint32_t a[4], w3[3][4];                       // rows p: transposed fragments of x, weighted, in three parts
+        ldsm4_t(a, sV + (kb * 16 + (mi >> 1) * 8 + r8) * kLdV + warp * 16 + (mi & 1) * 8);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int j = kb * 16 + (q >> 1) * 8 + col2;
+          const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[q]));
+          float u = f.x * tm.tail[j], w = f.y * tm.tail[j + 1];
+#pragma unroll
+          for (int part = 0; part < 3; ++part) w3[part][q] = take_bf16(u, w);
+        }
+#pragma unroll
+        for (int t = 0; t < KB; t += 2) {
+          uint32_t b[4], c[4];
+          ldsm4_t(b, sB + (kb * 16 + (mi & 1) * 8 + r8) * LDK + t * 16 + (mi >> 1) * 8);
+          ldsm4_t(c, sB + (kb * 16 + (mi & 1) * 8 + r8) * LDK + t * 16 + 16 + (mi >> 1) * 8);
+#pragma unroll
+          for (int part = 0; part < 3; ++part) {
+            mma(S[2 * t], w3[part], b[0], b[1]);
+            mma(S[2 * t + 1], w3[part], b[2], b[3]);
+            mma(S[2 * t + 2], w3[part], c[0], c[1]);
+            mma(S[2 * t + 3], w3[part], c[2], c[3]);
+          }
         }
       }
-    // the state after the chunk
-    if (have_state) {
-      const float f = tm.total;
-#pragma unroll
-      for (int t = 0; t < 2 * KB; ++t) { S[t][0] *= f; S[t][1] *= f; S[t][2] *= f; S[t][3] *= f; }
-    }
-    have_state = true;
-#pragma unroll
-    for (int kb = 0; kb < 4; ++kb) {
-      uint32_t a[4], w3[3][4];                       // rows p: transposed fragments of x, weighted, in three parts
-      ldsm4_t(a, sV + (kb * 16 + (mi >> 1) * 8 + r8) * kLdV + warp * 16 + (mi & 1) * 8);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int j = kb * 16 + (q >> 1) * 8 + col2;
-        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[q]));
-        float u = f.x * tm.tail[j], w = f.y * tm.tail[j + 1];
-#pragma unroll
-        for (int part = 0; part < 3; ++part) w3[part][q] = take_bf16(u, w);
-      }
-#pragma unroll
-      for (int t = 0; t < KB; t += 2) {
-        uint32_t b[4], c[4];
-        ldsm4_t(b, sB + (kb * 16 + (mi & 1) * 8 + r8) * LDK + t * 16 + (mi >> 1) * 8);
-        ldsm4_t(c, sB + (kb * 16 + (mi & 1) * 8 + r8) * LDK + t * 16 + 16 + (mi >> 1) * 8);
-#pragma unroll
-        for (int part = 0; part < 3; ++part) {
-          mma(S[2 * t], w3[part], b[0], b[1]);
-          mma(S[2 * t + 1], w3[part], b[2], b[3]);
-          mma(S[2 * t + 2], w3[part], c[0], c[1]);
-          mma(S[2 * t + 3], w3[part], c[2], c[3]);
-        }
-      }
-    }
+    };
+    if (m > 16) chunk(std::integral_constant<int, 4>());
+    else chunk(std::integral_constant<int, 1>());      // a short prompt, or a prompt's end
   }
   if (slot >= 0) {
 #pragma unroll
@@ -864,8 +888,9 @@ extern "C" int mb_ssd_scan_varlen(const void* x, const void* dt, const float* A,
                                   int dt_softplus, cudaStream_t stream) {
   if (n_seqs <= 0 || H <= 0) return MB_OK;
   if (P <= 0 || P > 256 || (P & (P - 1)) || G <= 0 || H % G || N <= 0 || N > 256) return MB_ERR_SHAPE;
-  // A chunk takes 7 us, full or not, a token of the walk 1.5 to 5 us: from four tokens per sequence on, the chunks win (and
-  // earlier where one sequence is much longer than the others). They take 16-byte copies of whole 8-value groups, so sizes and addresses that do not fit stay with the walk.
+  // From four tokens per sequence on, the chunks win (64 sequences of 4 tokens: 80 heads x 64 x 128 563 against 111 us, 24 heads x 64 x
+  // 16 17 against 16.5), and earlier where one sequence is much longer than the others. They take 16-byte copies of whole 8-value
+  // groups, so sizes and addresses that do not fit stay with the walk.
   if (tokens >= 4LL * n_seqs && N <= 128 && N % 8 == 0 && P % 8 == 0 && ldx % 8 == 0 && ldb % 8 == 0 && ldc % 8 == 0 &&
       aligned16(x) && aligned16(B) && aligned16(C) && (reinterpret_cast<uintptr_t>(ssm_state) & 7) == 0) {
     SsdChunk p{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dt), static_cast<const __nv_bfloat16*>(B),
