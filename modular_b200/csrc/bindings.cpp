@@ -629,6 +629,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_fp8_blockscaled", &gemm_fp8_blockscaled, py::arg("xq"), py::arg("xs"), py::arg("wq"),
         py::arg("ws"), py::arg("y"), py::arg("residual") = py::none(), py::arg("bn") = 0,
         py::arg("stages") = 0, py::arg("splits") = 0, py::arg("workspace") = py::none());
+  // (tokens on the MMA's M side, token tile, K splits) of a dense block-scaled product
+  m.def("gemm_fp8_plan", [](int M, int N, int K, int64_t workspace_bytes, int sms) {
+    int bn, splits;
+    const int rows = mb_gemm_fp8_plan(M, N, K, workspace_bytes, sms, &bn, &splits);
+    return py::make_tuple(rows != 0, bn, splits);
+  });
   m.def("gemm_bf16_persistent", &gemm_bf16_persistent, py::arg("x"), py::arg("w"), py::arg("y"),
         py::arg("residual") = py::none(), py::arg("dual") = false, py::arg("ws"), py::arg("counters"),
         py::arg("bn") = 0, py::arg("stages") = 0, py::arg("mode") = -1, py::arg("pdl") = false,

@@ -326,7 +326,7 @@ constexpr int kRowStages = 6, kRowTileN = 256, kMaxRowTiles = 1024;
 // warp 0 TMA, warp 1 MMA, warp 2 the experts' tiles, warps 4-11 promotion (setmaxnreg works on groups of four warps)
 constexpr int kRowThreads = 384;
 constexpr int kAhead = 4;             // K groups whose factors are on their way
-constexpr int kRowsFrom = 128;
+constexpr int kRowsFrom = 128, kRowsAlways = 1024;
 
 struct RowTail {
   uint64_t full[8];
@@ -517,34 +517,34 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
 #pragma unroll
       for (int j = 0; j < kAhead; ++j) fetch(j);
       for (int kb = 0; kb < kb_total; ++kb) {
-          asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
-          const float* at = mine + (kb % kAhead) * 64;
-          const float f = live ? at[0] * at[32] : 0.f;
-          fetch(kb + kAhead);
-          uint64_t f2;
-          asm("mov.b64 %0, {%1, %1};" : "=l"(f2) : "r"(__float_as_uint(f)));
-          const uint32_t buf = g & 1;
-          ok = mbar_wait(&tail->acc_full[buf], (g >> 1) & 1, abort_word, p.err, 514);
-          if (!ok) break;
-          ++g;
-          tc_fence_after();
-          // a load of the next columns is in flight while these are added
-          constexpr int W = 32;
-          uint32_t v[2][W];
-          tmem_ld_32x32(addr + buf * kRowTileN, v[0]);
+        asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
+        const float* at = mine + (kb % kAhead) * 64;
+        const float f = live ? at[0] * at[32] : 0.f;
+        fetch(kb + kAhead);
+        uint64_t f2;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(f2) : "r"(__float_as_uint(f)));
+        const uint32_t buf = g & 1;
+        ok = mbar_wait(&tail->acc_full[buf], (g >> 1) & 1, abort_word, p.err, 514);
+        if (!ok) break;
+        ++g;
+        tc_fence_after();
+        // a load of the next columns is in flight while these are added
+        constexpr int W = 32;
+        uint32_t v[2][W];
+        tmem_ld_32x32(addr + buf * kRowTileN, v[0]);
 #pragma unroll
-          for (int c = 0; c < 128 / W; ++c) {
-            tc_wait_ld();
-            if (c < 128 / W - 1) {
-              tmem_ld_32x32(addr + buf * kRowTileN + (c + 1) * W, v[(c + 1) & 1]);
-            } else {                     // everything is read: the buffer may be overwritten
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive_cluster_relaxed(aempty + 8u * buf);
-            }
-#pragma unroll
-            for (int i = 0; i < W / 2; ++i) acc[c * (W / 2) + i] = fma2(v[c & 1][2 * i], v[c & 1][2 * i + 1], f2, acc[c * (W / 2) + i]);
+        for (int c = 0; c < 128 / W; ++c) {
+          tc_wait_ld();
+          if (c < 128 / W - 1) {
+            tmem_ld_32x32(addr + buf * kRowTileN + (c + 1) * W, v[(c + 1) & 1]);
+          } else {                     // everything is read: the buffer may be overwritten
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster_relaxed(aempty + 8u * buf);
           }
+#pragma unroll
+          for (int i = 0; i < W / 2; ++i) acc[c * (W / 2) + i] = fma2(v[c & 1][2 * i], v[c & 1][2 * i + 1], f2, acc[c * (W / 2) + i]);
+        }
       }
       asm volatile("cp.async.wait_group 0;" ::: "memory");
       if (!ok) break;
@@ -849,6 +849,8 @@ extern "C" int mb_moe_permute_quant_fp8(const void* src, const int32_t* order, c
   return f8::launch_quant_vec(src, q_fp8, scales, max_rows, K, K, 1, order, n_rows_dev, top_k, stream);
 }
 
+namespace mb {
+namespace f8 {
 // Number of K splits for a grid of `ctas` output tiles: the split count (<= 8, at least four K groups
 // each) that fills whole waves of SMs best, with a small bias towards fewer splits.
 static int fp8_pick_splits(int ctas, int kb_total, int num_sms) {
@@ -864,8 +866,51 @@ static int fp8_pick_splits(int ctas, int kb_total, int num_sms) {
   return best;
 }
 
+// Token tile and K splits of the form with weights on M.
+static void fp8_split_plan(int M, int N, int K, size_t workspace_bytes, int num_sms, int* bn, int* splits) {
+  const int kb = K > 0 ? (K + 127) / 128 : 1;
+  if (*bn <= 0) {
+    const int mt = (M + 127) / 128;
+    *bn = ((M + mt - 1) / mt + 31) / 32 * 32;
+  }
+  int s = *splits;
+  if (s <= 0) s = fp8_pick_splits(((M + *bn - 1) / *bn) * ((N + kBM - 1) / kBM), kb, num_sms);
+  if (s > kb) s = kb;
+  if (N % 4 || static_cast<size_t>(s) * M * N * sizeof(float) > workspace_bytes) s = 1;
+  const int per = (kb + s - 1) / s;
+  *splits = (kb + per - 1) / per;
+}
+}  // namespace f8
+}  // namespace mb
+
+// Whether a dense product takes the form with tokens on M (1) or with weights on M (0, with its token tile and K splits): the one whose
+// time is less. Tokens on M give a pair of SMs one 256 x 256 tile for the whole of K, so that a narrow output leaves SMs idle; the
+// other form splits K until they are busy. In us, from 240 shapes (129 to 2048 tokens, 576 to 16384 features, K 2048 to 14336) on 148
+// SMs:  tokens on M  10.5 + 0.55 a K group and round of tiles;  weights on M  4 + 1.5 a wave + 0.64 a K group and wave (0.42 with token
+// tiles of 32), and with splits 3 + 1.7 for every million partial sums. 200 tokens, 1280 x 7168: 41 against 17 us; 512 tokens, 4096 x
+// 14336: 72 against 75; 2048 tokens, 8192 x 14336: 279 against 490. Splits change the order of a sum, so they have to gain 2.8 us, and
+// from 1024 tokens on no sum depends on them: only outputs of fewer than some 700 features would still gain (1024 tokens, 576 x 7168:
+// 42 against 27 us; 1536 tokens 42 against 38). No shape below 1024 tokens takes more than 1.14 of its faster form's time.
+// Up to 128 tokens weights on M stream faster at any width (one token, 57344 x 8192: 113 against 178 us).
+extern "C" int mb_gemm_fp8_plan(int M, int N, int K, size_t workspace_bytes, int num_sms, int* bn, int* splits) {
+  *bn = *splits = 0;
+  mb::f8::fp8_split_plan(M, N, K, workspace_bytes, num_sms, bn, splits);
+  using namespace mb::f8;
+  if (M <= kRowsFrom || N < kRowTileN || num_sms < 2) return 0;
+  if (M >= kRowsAlways) return 1;
+  const int groups = (K + 127) / 128, per = (groups + *splits - 1) / *splits;
+  const long long pairs = num_sms / 2, tiles = static_cast<long long>((M + 2 * kBM - 1) / (2 * kBM)) * ((N + kRowTileN - 1) / kRowTileN);
+  const long long ctas = static_cast<long long>((M + *bn - 1) / *bn) * ((N + kBM - 1) / kBM) * *splits;
+  const double rounds = static_cast<double>((tiles + pairs - 1) / pairs), waves = static_cast<double>((ctas + num_sms - 1) / num_sms);
+  const double rows_us = 10.5 + 0.55 * rounds * groups;
+  double split_us = 4. + waves * (1.5 + (0.34 + 0.3 * *bn / 128.) * per);
+  if (*splits > 1) split_us += 3. + 1.7e-6 * *splits * M * N;
+  return rows_us <= split_us + 2.8;
+}
+
 // flags: bit1 residual add. Xs is K-group-major [ceil(K/128), M]; Ws is [ceil(N/128), ceil(K/128)].
-// splits <= 0: chosen here (1 without a workspace of splits*M*N floats); num_sms is used for that choice.
+// bn, splits <= 0: chosen here (no splits without a workspace of splits*M*N floats) from the sizes and num_sms. A caller that names
+// any of bn, stages or splits gets the form with weights on M, which has them.
 extern "C" int mb_gemm_fp8_blockscaled(const void* Xq, const float* Xs, const void* Wq, const float* Ws,
                                        void* Y, const void* R, int M, int N, int K, int flags, int bn,
                                        int stages, int splits, void* workspace, size_t workspace_bytes,
@@ -876,13 +921,10 @@ extern "C" int mb_gemm_fp8_blockscaled(const void* Xq, const float* Xs, const vo
   if ((reinterpret_cast<uintptr_t>(Xq) | reinterpret_cast<uintptr_t>(Wq) | reinterpret_cast<uintptr_t>(Y) |
        reinterpret_cast<uintptr_t>(R)) & 15)
     return MB_ERR_ALIGN;
-  // Up to 128 tokens the other form streams the weights faster (64 tokens, 57344 x 8192: 157 against 177 us, one token 113
-  // against 178: its narrow token tiles leave room for more stages); at 300 tokens 28672 -> 8192 it takes 301 us, this one 153.
-  const bool rows_form = bn <= 0 && splits <= 0 && M > kRowsFrom && N >= kRowTileN && num_sms >= 2;
-  if (bn <= 0) {
-    const int mt = (M + 127) / 128;
-    bn = ((M + mt - 1) / mt + 31) / 32 * 32;
-  }
+  if (workspace == nullptr) workspace_bytes = 0;
+  bool rows_form = false;
+  if (bn <= 0 && splits <= 0 && stages <= 0) rows_form = mb_gemm_fp8_plan(M, N, K, workspace_bytes, num_sms, &bn, &splits) != 0;
+  else fp8_split_plan(M, N, K, workspace_bytes, num_sms, &bn, &splits);
   if (bn % 32 || bn < 32 || bn > 128) return MB_ERR_SHAPE;
   Params p = {};
   p.Y = static_cast<__nv_bfloat16*>(Y);
@@ -910,14 +952,7 @@ extern "C" int mb_gemm_fp8_blockscaled(const void* Xq, const float* Xs, const vo
   if (rc != MB_OK) return rc;
   const size_t smem = static_cast<size_t>(stages) * stage_bytes + 8 * kStgWarp + sizeof(Tail) + 1024;
   const int kb_all = (K + 127) / 128;
-  const int tiles = ((M + bn - 1) / bn) * ((N + kBM - 1) / kBM);
-  if (splits <= 0) splits = fp8_pick_splits(tiles, kb_all, num_sms);
-  if (splits > kb_all) splits = kb_all;
-  if (workspace == nullptr || N % 4 ||
-      static_cast<size_t>(splits) * M * N * sizeof(float) > workspace_bytes)
-    splits = 1;
   p.kb_per_split = (kb_all + splits - 1) / splits;
-  splits = (kb_all + p.kb_per_split - 1) / p.kb_per_split;
   p.splits = splits;
   p.partial = static_cast<float*>(workspace);
   p.expert_offsets = nullptr; p.w_rows = 0; p.sw_rows = 0; p.n_experts = 0;

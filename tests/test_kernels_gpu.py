@@ -585,6 +585,26 @@ def test_grouped_gemm_fp8_tokens_on_m(counts, N, K):
     ops.check_device_error()
 
 
+@pytest.mark.parametrize("M,N,K", [(1030, 8200, 272), (1100, 384, 640), (1281, 264, 144)])
+def test_gemm_fp8_tokens_on_m_over_many_tiles(M, N, K):
+    """From 1024 tokens on: several tiles for a pair of SMs one after another (165 of them for 74 pairs, three K groups each), ragged
+    edges in tokens, features and K, residual read while the tile before it is written."""
+    from modular_b200._native import lib
+
+    torch.manual_seed(N)
+    assert lib().gemm_fp8_plan(M, N, K, 1 << 30, torch.cuda.get_device_properties(0).multi_processor_count)[0]
+    wq = torch.randn(N, K, device=DEV).mul_(60).clamp_(-448, 448).to(torch.float8_e4m3fn)
+    ws = torch.rand(-(-N // 128), -(-K // 128), device=DEV) * 1e-3
+    xq, xs = ops.quant_fp8_group128(torch.randn(M, K, device=DEV).to(torch.bfloat16))
+    r = torch.randn(M, N, device=DEV).to(torch.bfloat16)
+    for res in (None, r):
+        y = ops.linear_fp8_blockscaled(xq, xs, wq, ws, residual=res)
+        assert torch.equal(y, ops.linear_fp8_blockscaled(xq, xs, wq, ws, residual=res, bn=128, splits=1))
+    ops.linear_fp8_blockscaled(xq, xs, wq, ws, residual=r, out=r)
+    assert torch.equal(r, y)
+    ops.check_device_error()
+
+
 def test_grouped_gemm_fp8_and_fp8_experts():
     """Grouped block-scaled fp8 GEMM against per-expert references, and a MoE layer with fp8 expert weights
     against the same layer with those weights dequantised to bf16."""

@@ -105,3 +105,18 @@ def test_kv_tier_page_copies_run_on_the_native_pool(tmp_path):
         assert store.onload(100 + i, out) is not None and torch.equal(out, p)
     assert store.disk_hits == 2 and store.host_hits == 1
     store.close()
+
+
+def test_fp8_products_of_narrow_outputs_split_k():
+    """A product whose 256 x 256 tiles leave most SMs idle takes the form that splits K; wide ones and long prompts do not."""
+    from modular_b200._native import lib
+
+    plan = lambda m, n, k: lib().gemm_fp8_plan(m, n, k, 1 << 30, 148)
+    for m, n, k in ((129, 576, 7168), (200, 1280, 7168), (256, 1536, 14336), (256, 4096, 14336), (300, 2048, 7168), (129, 4096, 7168)):
+        rows, bn, splits = plan(m, n, k)
+        assert not rows and splits > 1, (m, n, k)
+    for m, n, k in ((300, 8192, 28672), (256, 57344, 8192), (768, 4096, 7168), (2050, 57344, 8192), (2048, 576, 7168)):
+        assert plan(m, n, k)[0], (m, n, k)
+    assert not plan(128, 57344, 8192)[0] and not plan(4096, 128, 8192)[0]
+    rows, bn, splits = lib().gemm_fp8_plan(200, 1280, 7168, 0, 148)           # no workspace: no splits
+    assert splits == 1
