@@ -85,6 +85,7 @@ int mb_quant_fp8_group128(const void* x_bf16, void* q_fp8, float* scales, int M,
                           int scale_ld, int scales_k_major, cudaStream_t stream);
 // the form a dense product takes: 1 tokens on the MMA's M side, 0 weights there, with its token tile and K splits
 int mb_gemm_fp8_plan(int M, int N, int K, size_t workspace_bytes, int num_sms, int* bn, int* splits);
+int mb_grouped_fp8_plan(int n_experts, int total_rows, int max_rows, int N, int num_sms, int* bn);
 int mb_gemm_fp8_blockscaled(const void* Xq, const float* Xs, const void* Wq, const float* Ws, void* Y,
                             const void* R, int M, int N, int K, int flags, int bn, int stages, int splits,
                             void* workspace, size_t workspace_bytes, int num_sms, int* err,

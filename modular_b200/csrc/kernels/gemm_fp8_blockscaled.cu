@@ -976,6 +976,21 @@ extern "C" int mb_gemm_fp8_blockscaled(const void* Xq, const float* Xs, const vo
   return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ERR_LAUNCH;
 }
 
+// Whether a grouped product takes the form with tokens on M: where its 256-wide tiles keep half the SMs busy, or where the other form's
+// grid, sized for any expert taking every row, is six waves and more of CTAs that mostly have nothing to do. Else the twice as many
+// tiles of the other form are faster (148 SMs; 8 experts of 3072 x 7168, one row: 42 against 27 us; of 1536 x 2048, 128 rows: 17
+// against 13; 64 experts of 2816 x 2048, 64 rows: 55 against 71; 256 of 4096 x 7168, 2048 rows: 1303 against 2936). Outputs of 128
+// features fill half a tile (19 against 13 us). `avg` decides the other form's token tile.
+extern "C" int mb_grouped_fp8_plan(int n_experts, int total_rows, int max_rows, int N, int num_sms, int* bn) {
+  using namespace mb::f8;
+  const int avg = (total_rows + n_experts - 1) / n_experts;
+  *bn = avg <= 32 ? 32 : (avg <= 64 ? 64 : 128);
+  if (N < kRowTileN || n_experts + total_rows / kBM > kMaxRowTiles) return 0;
+  const long long tiles = static_cast<long long>((n_experts < total_rows ? n_experts : total_rows) + total_rows / kBM) * ((N + kRowTileN - 1) / kRowTileN);
+  const long long ctas = static_cast<long long>(n_experts) * ((max_rows + *bn - 1) / *bn) * (N / kBM);
+  return 2 * tiles >= num_sms || ctas >= 6ll * num_sms;
+}
+
 // Grouped block-scaled fp8 GEMM for mixture-of-experts layers: rows [offsets[e], offsets[e+1]) of Xq
 // (tokens in expert order, scales Xs K-group-major over all `total_rows`) times expert e's weights
 // Wq[e] ([N, K] e4m3 with 128x128 block scales Ws[e]). N % 128 == 0. `max_rows` bounds the rows of any
@@ -994,14 +1009,11 @@ extern "C" int mb_grouped_gemm_fp8_blockscaled(const void* Xq, const float* Xs, 
   if ((reinterpret_cast<uintptr_t>(Xq) | reinterpret_cast<uintptr_t>(Wq) | reinterpret_cast<uintptr_t>(Y)) & 15)
     return MB_ERR_ALIGN;
   if (max_rows <= 0 || max_rows > total_rows) max_rows = total_rows;
-  // tokens on the M side for any number of rows (256 experts of 4096 x 7168: 48 tokens with 8 experts each 1003 against 1384 us,
-  // 512 tokens 1340 against 2292): the weights' stream is the bound, and tiles of 256 weight rows keep it full
-  const bool rows_form = bn <= 0 && n_experts + total_rows / kBM <= kMaxRowTiles;
-  if (bn <= 0) {
-    // expected rows per expert decide the token tile: small tiles when experts see few tokens
-    const int avg = (total_rows + n_experts - 1) / n_experts;
-    bn = avg <= 32 ? 32 : (avg <= 64 ? 64 : 128);
-  }
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // a caller that names a token tile (expert parallelism does, from the rows it expects) gets the form with weights on M
+  const bool rows_form = bn <= 0 && mb_grouped_fp8_plan(n_experts, total_rows, max_rows, N, sms, &bn) != 0;
   if (bn % 32 || bn < 32 || bn > 128) return MB_ERR_SHAPE;
   Params p = {};
   p.Y = static_cast<__nv_bfloat16*>(Y);
@@ -1018,9 +1030,6 @@ extern "C" int mb_grouped_gemm_fp8_blockscaled(const void* Xq, const float* Xs, 
     if (rc != MB_OK) return rc;
     rc = cached_tmap(&tx, Xq, total_rows, K, ldx, kBM, 1);
     if (rc != MB_OK) return rc;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return launch_rows<false, false>(p, sms, 1 << 30, tw, tx, stream);
   }
   const int stage_bytes = kATile + bn * kBKBytes;

@@ -605,6 +605,26 @@ def test_gemm_fp8_tokens_on_m_over_many_tiles(M, N, K):
     ops.check_device_error()
 
 
+@pytest.mark.parametrize("E,N,K", [(64, 1024, 272), (300, 384, 640), (160, 256, 144)])
+def test_grouped_gemm_fp8_tokens_on_m_over_many_tiles(E, N, K):
+    """More tiles than SMs, odd numbers of K groups, experts without rows, of one row, and around 128 and 256."""
+    from modular_b200._native import lib
+
+    torch.manual_seed(E)
+    counts = [(0, 1, 127, 128, 129, 256, 300, 2, 0, 40)[i % 10] for i in range(E)]
+    n = sum(counts)
+    assert lib().grouped_fp8_plan(E, n + 5, n + 5, N, torch.cuda.get_device_properties(0).multi_processor_count)
+    wq = torch.randint(0, 120, (E, N, K), device=DEV, dtype=torch.uint8).view(torch.float8_e4m3fn)
+    ws = torch.rand(E, N // 128, (K + 127) // 128, device=DEV) * 1e-3
+    xq, xs = ops.quant_fp8_group128(torch.randn(n + 5, K, device=DEV).to(torch.bfloat16))        # five rows of nobody
+    off = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device=DEV)
+    y, want = (torch.full((n + 5, N), 7.0, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    lib().grouped_gemm_fp8(xq, xs, wq, ws, y, off, 0, 0)
+    lib().grouped_gemm_fp8(xq, xs, wq, ws, want, off, 0, 128)                                     # weights on M
+    assert torch.equal(y, want)
+    ops.check_device_error()
+
+
 def test_grouped_gemm_fp8_and_fp8_experts():
     """Grouped block-scaled fp8 GEMM against per-expert references, and a MoE layer with fp8 expert weights
     against the same layer with those weights dequantised to bf16."""

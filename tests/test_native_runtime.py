@@ -120,3 +120,14 @@ def test_fp8_products_of_narrow_outputs_split_k():
     assert not plan(128, 57344, 8192)[0] and not plan(4096, 128, 8192)[0]
     rows, bn, splits = lib().gemm_fp8_plan(200, 1280, 7168, 0, 148)           # no workspace: no splits
     assert splits == 1
+
+
+def test_grouped_products_of_few_tiles_keep_the_smaller_ones():
+    from modular_b200._native import lib
+
+    fp8 = lambda e, rows, n: lib().grouped_fp8_plan(e, rows, rows, n, 148)
+    for e, rows, n in ((8, 1, 3072), (8, 128, 1536), (4, 512, 512), (2, 32, 4096), (64, 4096, 128)):
+        assert not fp8(e, rows, n), (e, rows, n)
+    for e, rows, n in ((256, 384, 4096), (256, 16800, 4096), (64, 64, 2816), (8, 2048, 4096), (128, 8, 2048)):
+        assert fp8(e, rows, n), (e, rows, n)
+    assert not fp8(1000, 8192, 4096)                                          # more token tiles than the table holds
