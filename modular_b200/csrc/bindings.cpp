@@ -639,6 +639,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     int bn;
     return mb_grouped_fp8_plan(experts, rows, max_rows, N, sms, &bn) != 0;
   });
+  m.def("grouped_bf16_plan", [](int experts, int rows, int max_rows, int N, int K, bool dual, int sms) {
+    return mb_grouped_bf16_plan(experts, rows, max_rows, N, K, dual, sms) != 0;
+  });
   m.def("gemm_bf16_persistent", &gemm_bf16_persistent, py::arg("x"), py::arg("w"), py::arg("y"),
         py::arg("residual") = py::none(), py::arg("dual") = false, py::arg("ws"), py::arg("counters"),
         py::arg("bn") = 0, py::arg("stages") = 0, py::arg("mode") = -1, py::arg("pdl") = false,

@@ -451,6 +451,8 @@ int mb_moe_permute_rows(const void* src, const int32_t* order, const int32_t* n_
                         int max_rows, int row_bytes, int top_k, cudaStream_t stream);
 int mb_moe_combine(const void* expert_out, const int32_t* inverse, const float* w, const void* shared,
                    void* y, int T, int H, int top_k, cudaStream_t stream);
+// 1: a grouped bf16 product without a named token tile takes the token-major pairs of SMs
+int mb_grouped_bf16_plan(int n_experts, int total_rows, int max_rows, int N, int K, int dual, int num_sms);
 int mb_grouped_gemm_bf16(const void* X, const void* W, void* Y, const int32_t* expert_offsets,
                          int n_experts, int total_rows, int max_rows, int N, int K, int flags, int bn,
                          int* err, cudaStream_t stream);

@@ -678,6 +678,7 @@ __device__ __forceinline__ void epilogue_rows(uint32_t tmem_acc, int quad, int l
   const uint32_t lane_addr = tmem_acc + (static_cast<uint32_t>(quad * 32) << 16);
   constexpr int kCols = DUAL ? 128 : 256;
   const bool row_ok = token < M;
+  if (!__any_sync(0xffffffffu, row_ok)) return;
   // The residual is fetched one 128-byte line (64 features) ahead. The output is usually written in place over
   // the residual, and a load that follows a store of the same thread to the same line waits for that store to
   // be acknowledged: with a look-ahead of one 16-feature chunk every chunk paid two round trips to L2 (139
@@ -711,8 +712,10 @@ __device__ __forceinline__ void epilogue_rows(uint32_t tmem_acc, int quad, int l
         uint32_t u[16];
         tmem_ld_32x16(lane_addr + 128 + c0, u);
         tc_wait_ld();
+        // rows past the end are zeros, and a division of zero takes the slow path of the divide (13 us of a 35 us launch:
+        // 192 rows, one expert of 2 x 768 x 2048)
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = silu_f(__uint_as_float(g[j])) * __uint_as_float(u[j]);
+        for (int j = 0; j < 16; ++j) v[j] = silu_f(row_ok ? __uint_as_float(g[j]) : 1.f) * __uint_as_float(u[j]);
       } else {
         tc_wait_ld();
 #pragma unroll
@@ -1570,6 +1573,25 @@ extern "C" int mb_batched_gemm_bf16(const void* X, const void* W, void* Y, int B
                                      N, nullptr, 1, 0, 0, B, x_off, y_off);
 }
 
+// Whether a grouped product takes the token-major pairs, from 128 rows an expert on average (below that most of their 256-row tiles is
+// empty; the tile table is bounded, and features narrower than a tile stay with the weight-major tiles). In us, from 550 shapes on 148
+// SMs:  pairs  5 + (0.45 a K block + 2.5) a round of tiles;  weight-major  2.5 + (0.4 a K block, 0.8 with gate and up, + 2.5) a wave of
+// tiles with rows + 0.7 a wave of the others (its grid is sized for `max_rows` in every expert). Chosen so a shape takes 1.002 of its
+// faster form's time on average and 1.21 at most; few tiles are faster weight-major (2 experts of 2048 x 1408, 192 rows each: 14 against
+// 11 us; 128 of 4096 x 4096, 128 rows each, `max_rows` 128: 879 against 773; `max_rows` all: 879 against 3560).
+extern "C" int mb_grouped_bf16_plan(int n_experts, int total_rows, int max_rows, int N, int K, int dual, int num_sms) {
+  const int tile_n = dual ? 128 : 256;
+  if (n_experts <= 0 || total_rows < 128LL * n_experts || N < tile_n || n_experts + total_rows / 256 > kMaxRowTiles || num_sms < 2) return 0;
+  const long long avg = (total_rows + n_experts - 1) / n_experts, kb = (K + kBK - 1) / kBK, pairs = num_sms / 2;
+  const long long pair_tiles = n_experts * ((avg + 255) / 256) * ((N + tile_n - 1) / tile_n);
+  const long long tiles = n_experts * ((avg + 127) / 128) * ((N + 127) / 128);
+  const long long grid = static_cast<long long>(n_experts) * ((max_rows + 127) / 128) * ((N + 127) / 128);
+  const double pairs_us = 5. + static_cast<double>((pair_tiles + pairs - 1) / pairs) * (0.45 * kb + 2.5);
+  const double tiles_us = 2.5 + static_cast<double>((tiles + num_sms - 1) / num_sms) * ((dual ? 0.8 : 0.4) * kb + 2.5) +
+                          0.7 * (grid > tiles ? grid - tiles : 0) / num_sms;
+  return pairs_us <= tiles_us;
+}
+
 extern "C" int mb_grouped_gemm_bf16(const void* X, const void* W, void* Y, const int32_t* expert_offsets,
                                     int n_experts, int total_rows, int max_rows, int N, int K, int flags,
                                     int bn, int* err, cudaStream_t stream) {
@@ -1578,18 +1600,16 @@ extern "C" int mb_grouped_gemm_bf16(const void* X, const void* W, void* Y, const
   if (K % 8 || N % 8) return MB_ERR_SHAPE;
   if ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(Y)) & 15)
     return MB_ERR_ALIGN;
-  // Experts with 128 rows and more on average take the token-major pairs, whose tiles hold 256 rows (below that most of a
-  // tile is empty, and the tile table is bounded); features narrower than a tile stay with the weight-major tiles.
-  if (bn <= 0 && total_rows >= 128LL * n_experts && N >= (dual ? 128 : 256) && n_experts + total_rows / 256 <= kMaxRowTiles) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (bn <= 0 && mb_grouped_bf16_plan(n_experts, total_rows, max_rows, N, K, dual, sms)) {
     const int rows = dual ? 2 * N : N;
     CUtensorMap tw, tx;
     int rc = cached_tmap(&tw, W, static_cast<uint64_t>(rows) * n_experts, K, K, kBM, 2);
     if (rc != MB_OK) return rc;
     rc = cached_tmap(&tx, X, total_rows, K, K, kBM, 2);
     if (rc != MB_OK) return rc;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return dual ? launch_pair_xw<true, EPI_BF16, true>(tw, tx, Y, nullptr, total_rows, N, K, N, 0, N, sms, err, stream, 0, expert_offsets, n_experts, rows)
                 : launch_pair_xw<false, EPI_BF16, true>(tw, tx, Y, nullptr, total_rows, N, K, N, 0, 0, sms, err, stream, 0, expert_offsets, n_experts, rows);
   }

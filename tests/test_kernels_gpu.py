@@ -359,6 +359,25 @@ def test_grouped_gemm_pairs(counts, N, K, swiglu):
     ops.check_device_error()
 
 
+@pytest.mark.parametrize("counts,N,K,swiglu", [([0, 257, 1, 900, 255, 256, 0, 3], 384, 128, False), ([700, 0, 513], 200, 72, True),
+                                              ([128, 128], 256, 64, False), ([300, 0, 129, 512, 1, 270] * 20, 392, 136, True)])
+def test_grouped_gemm_token_major_pairs(counts, N, K, swiglu):
+    """The pairs at edges of their tiles: a bound of the rows of one expert far above the real ones leads to them at any size."""
+    from modular_b200._native import lib
+
+    torch.manual_seed(len(counts))
+    E, n = len(counts), sum(counts)
+    assert lib().grouped_bf16_plan(E, n, 1 << 16, N, K, swiglu, torch.cuda.get_device_properties(0).multi_processor_count)
+    x = torch.randn(n, K, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(E, (2 if swiglu else 1) * N, K, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    off = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device=DEV)
+    y, want = (torch.full((n, N), 7.0, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    lib().grouped_gemm_bf16(x, w, y, off, 1 << 16, swiglu, 0)
+    lib().grouped_gemm_bf16(x, w, want, off, max(counts), swiglu, 128)
+    assert torch.equal(y, want)                        # the same sums in the same order
+    ops.check_device_error()
+
+
 def test_argmax_and_sampling():
     torch.manual_seed(8)
     logits = torch.randn(9, 128256, device=DEV)

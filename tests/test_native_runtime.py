@@ -131,3 +131,9 @@ def test_grouped_products_of_few_tiles_keep_the_smaller_ones():
     for e, rows, n in ((256, 384, 4096), (256, 16800, 4096), (64, 64, 2816), (8, 2048, 4096), (128, 8, 2048)):
         assert fp8(e, rows, n), (e, rows, n)
     assert not fp8(1000, 8192, 4096)                                          # more token tiles than the table holds
+    bf16 = lambda e, per, most, n, k, dual=False: lib().grouped_bf16_plan(e, e * per, most, n, k, dual, 148)
+    for e, per, most, n, k in ((2, 192, 384, 2048, 1408), (1, 257, 257, 4096, 4096), (128, 128, 128, 4096, 4096), (8, 128, 1024, 512, 128)):
+        assert not bf16(e, per, most, n, k), (e, per, n, k)
+    for e, per, most, n, k in ((64, 768, 49152, 2048, 1408), (128, 128, 16384, 4096, 4096), (8, 1024, 8192, 4096, 14336)):
+        assert bf16(e, per, most, n, k), (e, per, n, k)
+    assert bf16(64, 768, 49152, 1408, 2048, True) and not bf16(64, 100, 6400, 1408, 2048, True) and not bf16(8, 1024, 8192, 200, 2048)
