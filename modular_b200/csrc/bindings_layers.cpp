@@ -272,6 +272,16 @@ void latent_prefill(const Tensor& q, const Tensor& q_rope, const Tensor& kv, con
            "latent_prefill");
 }
 
+// w_uk [h, R, 128], w_uv [h, 128, R] -> out [2 h 128, R]
+void latent_stack(const Tensor& w_uk, const Tensor& w_uv, Tensor& out) {
+  const int h = w_uk.size(0), R = w_uk.dim() == 3 ? w_uk.size(1) : 0;
+  auto bf = [](const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.is_contiguous(); };
+  TORCH_CHECK(bf(w_uk) && bf(w_uv) && bf(out) && w_uk.dim() == 3 && w_uk.size(2) == 128 && w_uv.dim() == 3 && w_uv.size(0) == h && w_uv.size(1) == 128 &&
+                  w_uv.size(2) == R && out.dim() == 2 && out.size(0) == 2 * h * 128 && out.size(1) == R,
+              "latent_stack layout");
+  check_rc(mb_latent_stack(w_uk.data_ptr(), w_uv.data_ptr(), out.data_ptr(), h, R, cur_stream()), "latent_stack");
+}
+
 // cache [pages, page, >= R + 64] -> c [rows, R], rope [rows, 64]: the rows of all sequences, one after another
 void latent_gather(const Tensor& cache, const Tensor& block_table, const Tensor& kv_start, const Tensor& kv_len, Tensor& c, Tensor& rope) {
   const int B = kv_len.numel(), R = c.size(1);
@@ -598,6 +608,7 @@ void mb::bind_layers(py::module_& m) {
                              i32(positions, x.size(0), "positions"), f32(cos_sin, 0, "cos_sin"), dtype_of(x, "x"), cur_stream()),
              "rotate_heads");
   });
+  m.def("latent_stack", &latent_stack);
   m.def("latent_gather", &latent_gather);
   m.def("latent_prefill", &latent_prefill, py::arg("q"), py::arg("q_rope"), py::arg("kv"), py::arg("k_rope"), py::arg("kv_start"), py::arg("q_start"),
         py::arg("q_len"), py::arg("kv_len"), py::arg("tile_seq"), py::arg("tile_q0"), py::arg("out"), py::arg("scale"), py::arg("sink") = py::none(),

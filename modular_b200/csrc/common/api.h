@@ -200,6 +200,7 @@ int mb_latent_prefill_tc(const void* q, int ldq, int q_head, const void* q_rope,
                          int ld_kv, const void* k_rope, long long rows, const int32_t* kv_start, const int32_t* q_start, const int32_t* q_len,
                          const int32_t* kv_len, const int32_t* tile_seq, const int32_t* tile_q0, int n_tiles, int n_heads, float scale,
                          const MbAttnOptions* opt, int* err, cudaStream_t stream);
+int mb_latent_stack(const void* w_uk, const void* w_uv, void* out, int heads, int R, cudaStream_t stream);
 int mb_latent_gather(const void* cache, long long page_stride, int ld, int page, const int32_t* block_table, int bt_stride,
                      const int32_t* kv_start, const int32_t* kv_len, int B, int R, void* c, void* rope, long long rows, cudaStream_t stream);
 // tcgen05 prefill attention (attention_tc.cu): same addressing as mb_paged_attention_tma, head_dim 128 only.

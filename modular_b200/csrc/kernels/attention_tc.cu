@@ -520,8 +520,47 @@ __global__ void latent_gather_kernel(const bf16* __restrict__ cache, long long p
   bf16* dst = col < R ? c + static_cast<long long>(row) * R + col : rope + static_cast<long long>(row) * 64 + (col - R);
   *reinterpret_cast<uint4*>(dst) = v;
 }
+
+// Weights of the projection: out rows [h 128 | h 128] x R from w_uk [h, R, 128] (transposed per head, tiles of 64 x 64 through shared
+// memory) and w_uv [h, 128, R] (as it is). Made anew for each layer of a step, in the step's scratch: kept, it would be a second copy of
+// both (2 GB for 61 layers of 128 heads), and an old one once the weights change. 128 heads, R = 512: 48 us as three torch kernels.
+__global__ void __launch_bounds__(256) latent_stack_kernel(const bf16* __restrict__ w_uk, const bf16* __restrict__ w_uv, bf16* __restrict__ out, int h, int R) {
+  __shared__ bf16 tile[64][66];
+  const int head = blockIdx.z, r0 = blockIdx.x * 64, n0 = (blockIdx.y & 1) * 64, tid = threadIdx.x, row = tid >> 3, c = (tid & 7) * 8;
+  if (blockIdx.y >= 2) {                             // 64 value rows of a head
+    const size_t at = (static_cast<size_t>(head) * 128 + n0) * R + r0;
+#pragma unroll
+    for (int q = 0; q < 64; q += 32)
+      *reinterpret_cast<uint4*>(out + static_cast<size_t>(h) * 128 * R + at + static_cast<size_t>(row + q) * R + c) =
+          *reinterpret_cast<const uint4*>(w_uv + at + static_cast<size_t>(row + q) * R + c);
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < 64; q += 32) {
+    const uint4 v = *reinterpret_cast<const uint4*>(w_uk + (static_cast<size_t>(head) * R + r0 + row + q) * 128 + n0 + c);
+    uint32_t* to = reinterpret_cast<uint32_t*>(&tile[row + q][c]);
+    to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 64; q += 32) {
+    __align__(16) bf16 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = tile[c + i][row + q];
+    *reinterpret_cast<uint4*>(out + (static_cast<size_t>(head) * 128 + n0 + row + q) * R + r0 + c) = *reinterpret_cast<const uint4*>(v);
+  }
+}
 }  // namespace atc
 }  // namespace mb
+
+extern "C" int mb_latent_stack(const void* w_uk, const void* w_uv, void* out, int heads, int R, cudaStream_t stream) {
+  using namespace mb::atc;
+  if (heads <= 0 || R <= 0) return MB_OK;
+  if (R % 64 || heads > 65535) return MB_ERR_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(w_uk) | reinterpret_cast<uintptr_t>(w_uv) | reinterpret_cast<uintptr_t>(out)) & 15) return MB_ERR_ALIGN;
+  latent_stack_kernel<<<dim3(R / 64, 4, heads), 256, 0, stream>>>(static_cast<const bf16*>(w_uk), static_cast<const bf16*>(w_uv), static_cast<bf16*>(out), heads, R);
+  return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ERR_LAUNCH;
+}
 
 extern "C" int mb_latent_gather(const void* cache, long long page_stride, int ld, int page, const int32_t* block_table, int bt_stride,
                                 const int32_t* kv_start, const int32_t* kv_len, int B, int R, void* c, void* rope, long long rows,

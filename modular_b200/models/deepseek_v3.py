@@ -192,7 +192,6 @@ class DSLayer:
     w_uv: torch.Tensor               # [h, v_dim, kv_lora]  applied to the latent output  (N=v_dim, K=kv_lora)
     wo: object                       # [H, h * v_dim]
     mlp_norm: torch.Tensor
-    w_up: Optional[torch.Tensor] = None  # [2 * h * 128, kv_lora]: both halves of kv_b stacked, for prompts
     w_a: Optional[torch.Tensor] = None   # [q_lora + kv_lora + rope, H]: q_a and kv_a stacked (bf16 weights only)
     wgu: Optional[object] = None     # dense layers: [2 * inter, H]
     wd: Optional[object] = None      # dense layers: [H, inter]
@@ -429,9 +428,9 @@ class DeepseekV3Model:
                 if l.q_a is not None:
                     ql = l.q_a.shape[0]
                     l.q_a, l.kv_a = l.w_a[:ql], l.w_a[ql:]
-            if (l.w_up is None and self.device.type == "cuda" and self.dtype == torch.bfloat16 and cfg.qk_nope_head_dim == cfg.v_head_dim == 128
-                    and cfg.qk_rope_head_dim == 64):
-                l.w_up = stacked_up(l.w_uk, l.w_uv)
+        # prompts project latents up to keys and values where the sizes are those of the kernel (:meth:`_attention_fused`)
+        self.projects = (self.device.type == "cuda" and self.dtype == torch.bfloat16 and cfg.qk_nope_head_dim == cfg.v_head_dim == 128
+                         and cfg.qk_rope_head_dim == 64 and any(self._fused(l) for l in weights.layers))
         self.ep = ep
         self._ep_layers = {}
         if ep is not None:
@@ -558,11 +557,11 @@ class DeepseekV3Model:
         q = lin(q_a if ql else x, l.q_b)                                      # [T, h * (nope + rope)]
         q_rope = torch.empty(T, h, c.qk_rope_head_dim, dtype=x.dtype, device=dev)
         L.mla_q_rope(q, h, c.qk_nope_head_dim, positions, self.cos_sin, q_rope)
-        if plan is not None and l.w_up is not None:
+        if plan is not None:
             # long prompts: the cached latents projected up to keys and values per head
             o = torch.empty(T, h * c.v_head_dim, dtype=x.dtype, device=dev)
-            prompt_attention(plan, q.view(T, h, c.qk_head_dim)[:, :, : c.qk_nope_head_dim], q_rope, l.w_up, cache, block_table, q_start, q_len,
-                             kv_len, o, self.scale)
+            prompt_attention(plan, q.view(T, h, c.qk_head_dim)[:, :, : c.qk_nope_head_dim], q_rope, stacked_up(l.w_uk, l.w_uv), cache, block_table,
+                             q_start, q_len, kv_len, o, self.scale)
             return o
         q_lat = torch.empty(T, h * R, dtype=x.dtype, device=dev)
         ops.batched_linear_heads(q, l.w_uk, q_lat, c.qk_head_dim, R)          # absorb W_uk per head
@@ -572,10 +571,13 @@ class DeepseekV3Model:
         ops.batched_linear_heads(o_lat.view(T, h * R), l.w_uv, o, R, c.v_head_dim)   # apply W_uv per head
         return o
 
+    @staticmethod
+    def _fused(l: DSLayer) -> bool:
+        return l.w_a is not None and torch.is_tensor(l.q_b)
+
     def _attention(self, li: int, l: DSLayer, x, positions, slots, block_table, q_start, q_len, kv_len, plan=None):
         c = self.cfg
-        if (x.is_cuda and x.dtype == torch.bfloat16 and l.w_a is not None and torch.is_tensor(l.q_b)
-                and c.qk_rope_head_dim == 64 and positions.dtype == torch.int32):
+        if x.is_cuda and x.dtype == torch.bfloat16 and self._fused(l) and c.qk_rope_head_dim == 64 and positions.dtype == torch.int32:
             return self._attention_fused(li, l, x, positions, slots, block_table, q_start, q_len, kv_len, plan)
         T, h = x.shape[0], c.num_attention_heads
         if l.q_a is not None:
@@ -617,7 +619,7 @@ class DeepseekV3Model:
         # decode-sized steps on the GPU use the GEMM that carries the residual add and the next norm in its tail
         small = h.is_cuda and h.dtype == torch.bfloat16 and h.shape[0] <= ops.DECODE_GEMM_MAX_TOKENS
         x = ops.rms_norm(h, layers[0].attn_norm, eps)
-        plan = prompt_plan(tokens.shape[0], q_len, kv_len) if layers[0].w_up is not None else None
+        plan = prompt_plan(tokens.shape[0], q_len, kv_len) if self.projects else None
         for li, l in enumerate(layers):
             a = self._attention(li, l, x, positions, slots, block_table, q_start, q_len, kv_len, plan)
             if small and torch.is_tensor(l.wo):

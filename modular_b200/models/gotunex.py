@@ -356,7 +356,7 @@ class GotunexModel:
         # the tiled GEMM for every step size: the decode-step GEMM measured 2 to 29 % slower per step at these widths
         lin = ops.linear
         one_token = T == q_len.shape[0]
-        plan = prompt_plan(T, q_len, kv_len) if any(getattr(l.mixer, "w_up", None) is not None for l in w.layers) else None
+        plan = prompt_plan(T, q_len, kv_len) if any(getattr(l.mixer, "projects", False) for l in w.layers) else None
         routes = w.router.route(tokens)
         x = torch.empty(T, Wp, dtype=torch.float32, device=dev)
         # what the next seam adds to the stream: the embedding first, then both branches of a layer

@@ -414,7 +414,7 @@ class MavidraModel:
         new = lambda rows: torch.empty(rows, Wp, dtype=self.dtype, device=dev)
         seam = lambda x, **kw: sandwich_norm(x, cols=c.hidden_size, eps=c.norm_eps, **kw)
         one_token = T == q_len.shape[0]
-        plan = prompt_plan(T, q_len, kv_len) if any(getattr(l.mixer, "w_up", None) is not None for l in w.layers) else None
+        plan = prompt_plan(T, q_len, kv_len) if any(getattr(l.mixer, "projects", False) for l in w.layers) else None
         plans = {g: tensor_core_plan(g, self.kv.shape[5], self.dtype, self.page_size, q_start, q_len, T, one_token)
                  for g in self.groups}
         counts = torch.zeros(len(self.moe_layers), self.max_experts, dtype=torch.int32, device=dev)

@@ -122,8 +122,7 @@ class LatentAttention:
         uv[:, : c.vdim, : c.kv_rank] = t["uv"].view(H, c.vdim, c.kv_rank)
         self.w_uv = put(uv)                                          # [h, vdim, latent]: latent outputs to values
         # prompts project latents up to keys and values where the sizes are those of the kernel
-        self.w_up = stacked_up(self.w_uk, self.w_uv) if (up64(d) == vp == 128 and rot_pad(r) == 64 and self.w_uk.is_cuda
-                                                         and dtype == torch.bfloat16) else None
+        self.projects = up64(d) == vp == 128 and rot_pad(r) == 64 and self.w_uk.is_cuda and dtype == torch.bfloat16
         self.sink = put(t["sink"], torch.float32) if c.sink else None
         self.w_o = put(pad_to(pad_heads(t["o"].t().contiguous(), H, c.vdim, vp).t(), width_pad, gemm_k(H * vp)))
 
@@ -144,9 +143,9 @@ class LatentAttention:
         o = torch.empty(T, self.w_o.shape[1], dtype=x.dtype, device=x.device)
         if o.shape[1] != width:
             o[:, width:].zero_()
-        if plan is not None and self.w_up is not None and (c.window == 0 or c.window > 256):
-            prompt_attention(plan, q.view(T, H, c.head_width)[:, :, :dp], q_rope, self.w_up, cache, block_table, q_start, q_len, kv_len, o,
-                             c.scale, self.sink, c.window, gate)
+        if plan is not None and self.projects and (c.window == 0 or c.window > 256):
+            prompt_attention(plan, q.view(T, H, c.head_width)[:, :, :dp], q_rope, stacked_up(self.w_uk, self.w_uv), cache, block_table, q_start,
+                             q_len, kv_len, o, c.scale, self.sink, c.window, gate)
         else:
             q_lat = torch.empty(T, H * Rp, dtype=x.dtype, device=x.device)
             ops.batched_linear_heads(q, self.w_uk, q_lat, c.head_width, Rp)
@@ -199,8 +198,13 @@ def prompt_plan(T: int, q_len, kv_len) -> Optional[PromptPlan]:
 
 
 def stacked_up(w_uk: torch.Tensor, w_uv: torch.Tensor) -> torch.Tensor:
-    """[heads * 128 | heads * 128, latent] from ``w_uk`` [heads, latent, 128] and ``w_uv`` [heads, 128, latent]."""
-    R = w_uk.shape[1]
+    """[heads * 128 | heads * 128, latent] from ``w_uk`` [heads, latent, 128] and ``w_uv`` [heads, 128, latent]: scratch of one
+    layer's step, so that it is never older than the weights."""
+    h, R = w_uk.shape[:2]
+    if w_uk.is_cuda and w_uk.dtype == torch.bfloat16 and R % 64 == 0 and w_uk.shape[2] == 128:
+        out = torch.empty(2 * h * 128, R, dtype=w_uk.dtype, device=w_uk.device)
+        _lib().latent_stack(w_uk.contiguous(), w_uv.contiguous(), out)
+        return out
     return torch.cat((w_uk.transpose(1, 2).reshape(-1, R), w_uv.reshape(-1, R))).contiguous()
 
 

@@ -250,3 +250,43 @@ def test_mla_decode_tcgen05_matches_reference(h, page, kv_lens):
     assert (unsplit.float() - want).abs().max() / want.abs().max() < 2e-2
     err = (got.float() - want).abs().max() / want.abs().max()
     assert err < 2e-2, err
+
+
+def test_layers_take_the_stacked_down_projection_as_their_eleventh_argument():
+    import dataclasses
+
+    from modular_b200.models.deepseek_v3 import DSLayer
+
+    assert [f.name for f in dataclasses.fields(DSLayer)][8:12] == ["wo", "mlp_norm", "w_a", "wgu"]
+
+
+@pytest.mark.gpu
+def test_prompts_follow_weights_that_change_in_place():
+    """A step whose latents are projected uses the weights as they are, not as they were when the model was made."""
+    from modular_b200.nn.latent_attention import prompt_plan
+
+    dev = "cuda"
+    cfg = DeepseekV3Config.tiny(q_lora_rank=64, kv_lora_rank=128, qk_nope_head_dim=128, qk_rope_head_dim=64, v_head_dim=128)
+    w = DeepseekV3Weights.random_init(cfg, dev, torch.bfloat16, seed=7, std=0.05)
+    T, page = 600, 64
+    tok = torch.randint(0, cfg.vocab_size, (T,), generator=torch.Generator().manual_seed(3)).to(dev)
+    pos, slots, bt = _single_seq_inputs(T, page, dev)
+    step = lambda m: m.forward_tensors(tok, pos, slots, bt, i32(0, dev=dev), i32(T, dev=dev), i32(T, dev=dev), i32(T - 1, dev=dev))
+    make = lambda: DeepseekV3Model(cfg, w, _new_kv(cfg, 12, page, dev, torch.bfloat16))
+    m = make()
+    assert m.projects and prompt_plan(T, i32(T, dev=dev), i32(T, dev=dev)) is not None
+    before = step(m)
+    for l in w.layers:
+        l.w_uk.mul_(-0.5)
+        l.w_uv.mul_(2.0)
+    after = step(m)
+    assert torch.equal(after, step(make())) and not torch.equal(after, before)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h,R", [(1, 64), (3, 192), (16, 512), (128, 512)])
+def test_stacked_projection(h, R):
+    from modular_b200.nn.latent_attention import stacked_up
+
+    w_uk, w_uv = torch.randn(h, R, 128, device="cuda").bfloat16(), torch.randn(h, 128, R, device="cuda").bfloat16()
+    assert torch.equal(stacked_up(w_uk, w_uv), torch.cat((w_uk.transpose(1, 2).reshape(-1, R), w_uv.reshape(-1, R))))
