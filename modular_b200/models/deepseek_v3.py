@@ -499,14 +499,15 @@ class DeepseekV3Model:
         return fit if (fit and T == n_seqs == n_logits) else 0
 
     def forward_tensors(self, tokens, positions, slots, block_table, q_start, q_len, kv_len,
-                        logit_rows, plan=None) -> torch.Tensor:
-        """One ragged step. Returns fp32 logits ``[len(logit_rows), vocab]``. Decode-only steps replay a captured
+                        logit_rows, plan=None, lengths=None) -> torch.Tensor:
+        """One ragged step. Returns fp32 logits ``[len(logit_rows), vocab]``. ``lengths``: (q_len, kv_len) as lists on the host,
+        where the caller has them (prompt steps read them back otherwise). Decode-only steps replay a captured
         graph when one of a fitting size exists (sequences beyond the real ones are dummies that write no KV)."""
         T, n = tokens.shape[0], q_len.shape[0]
         self.forward_calls += 1
         B = self._graph_for(T, n, logit_rows.shape[0]) if (self._graphs or self.ep is not None) else 0
         if not B:
-            return self._forward(tokens, positions, slots, block_table, q_start, q_len, kv_len, logit_rows)
+            return self._forward(tokens, positions, slots, block_table, q_start, q_len, kv_len, logit_rows, lengths)
         g, st, logits = self._graphs[B]
         st["tokens"][:n].copy_(tokens)
         st["positions"][:n].copy_(positions)
@@ -612,14 +613,14 @@ class DeepseekV3Model:
         return l.moe(x)
 
     # ------------------------------------------------------------ step
-    def _forward(self, tokens, positions, slots, block_table, q_start, q_len, kv_len, logit_rows) -> torch.Tensor:
+    def _forward(self, tokens, positions, slots, block_table, q_start, q_len, kv_len, logit_rows, lengths=None) -> torch.Tensor:
         c, eps = self.cfg, self.cfg.rms_norm_eps
         layers = self.w.layers
         h = ops.embedding(tokens, self.w.embed)
         # decode-sized steps on the GPU use the GEMM that carries the residual add and the next norm in its tail
         small = h.is_cuda and h.dtype == torch.bfloat16 and h.shape[0] <= ops.DECODE_GEMM_MAX_TOKENS
         x = ops.rms_norm(h, layers[0].attn_norm, eps)
-        plan = prompt_plan(tokens.shape[0], q_len, kv_len) if self.projects else None
+        plan = prompt_plan(tokens.shape[0], q_len, kv_len, 0, lengths) if self.projects else None
         for li, l in enumerate(layers):
             a = self._attention(li, l, x, positions, slots, block_table, q_start, q_len, kv_len, plan)
             if small and torch.is_tensor(l.wo):

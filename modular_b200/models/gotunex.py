@@ -22,7 +22,7 @@ import torch
 
 from .. import ops
 from ..nn.delta_rule import DeltaRule, DeltaRuleConfig, gemm_k, pad_to, up8
-from ..nn.latent_attention import LatentAttention, LatentAttentionConfig, prompt_plan
+from ..nn.latent_attention import LatentAttention, LatentAttentionConfig, prompt_plans
 from ..nn.moe import TableRouter, expert_mlp
 from ..nn.residual import residual_norm
 from ..nn.rotary_embedding import cos_sin_table
@@ -333,8 +333,9 @@ class GotunexModel:
 
     @torch.no_grad()
     def forward_tensors(self, tokens, positions, slots, block_table, q_start, q_len, kv_len, logit_rows, plan=None,
-                        state_slot=None, lora=None) -> torch.Tensor:
-        """fp32 logits [len(logit_rows), vocab] of a ragged step."""
+                        state_slot=None, lora=None, lengths=None) -> torch.Tensor:
+        """fp32 logits [len(logit_rows), vocab] of a ragged step. ``lengths``: (q_len, kv_len) as lists on the host, where the
+        caller has them (prompt steps read them back otherwise)."""
         if lora is not None:
             raise ValueError("LoRA adapters are not implemented for this family")
         self.forward_calls += 1
@@ -343,12 +344,12 @@ class GotunexModel:
             if size:
                 return self.graphs.replay(size, block_table, tokens=tokens, positions=positions, slots=slots, kv_len=kv_len,
                                           state_slot=state_slot)
-        return self._forward(tokens, positions, slots, block_table, q_start, q_len, kv_len, logit_rows, state_slot)
+        return self._forward(tokens, positions, slots, block_table, q_start, q_len, kv_len, logit_rows, state_slot, lengths=lengths)
 
     # ------------------------------------------------------------ step
     @torch.no_grad()
     def _forward(self, tokens, positions, slots, block_table, q_start, q_len, kv_len, logit_rows, state_slot=None,
-                 stream: Optional[list] = None) -> torch.Tensor:
+                 stream: Optional[list] = None, lengths=None) -> torch.Tensor:
         """``stream`` (a list) collects a copy of the residual stream after every layer."""
         c, w, T, Wp = self.cfg, self.w, tokens.shape[0], self.cfg.width_pad
         dev, eps = self.device, self.cfg.rms_norm_eps
@@ -356,7 +357,7 @@ class GotunexModel:
         # the tiled GEMM for every step size: the decode-step GEMM measured 2 to 29 % slower per step at these widths
         lin = ops.linear
         one_token = T == q_len.shape[0]
-        plan = prompt_plan(T, q_len, kv_len) if any(getattr(l.mixer, "projects", False) for l in w.layers) else None
+        projected = prompt_plans({l.mixer.cfg.window for l in w.layers if getattr(l.mixer, "projects", False)}, T, q_len, kv_len, lengths)
         routes = w.router.route(tokens)
         x = torch.empty(T, Wp, dtype=torch.float32, device=dev)
         # what the next seam adds to the stream: the embedding first, then both branches of a layer
@@ -370,7 +371,7 @@ class GotunexModel:
             residual_norm(x, w1=l.norm1, n1=n1, w2=l.norm2, n2=n2, scatter=inverse, cols=c.hidden_size, eps=eps, **pending)
             if c.is_attention(i):
                 y = l.mixer(n1, lin, self.kv[:, 0, self.plane[i], 0], self.cos_sin[i], positions, slots, block_table, q_start,
-                            q_len, kv_len, one_token, plan)
+                            q_len, kv_len, one_token, projected.get(l.mixer.cfg.window))
             else:
                 y = l.mixer(n1, lin, self.state[f"l{i}.delta"], self.state[f"l{i}.conv"], state_slot, q_start, q_len, kv_len,
                             one_token)

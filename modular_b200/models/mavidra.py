@@ -26,7 +26,7 @@ from ..nn.bigram import STATE as BIGRAM_STATE
 from ..nn.bigram import BigramConfig, bigram_rows
 from ..nn.delta_rule import DeltaRule, DeltaRuleConfig, gemm_k, pad_to, up8
 from ..nn.gated_linear_attention import GatedLinearAttention, GatedLinearConfig
-from ..nn.latent_attention import LatentAttention, LatentAttentionConfig, prompt_plan
+from ..nn.latent_attention import LatentAttention, LatentAttentionConfig, prompt_plans
 from ..nn.moe import ScoreRouter, ScoreRouterConfig, expert_mlp
 from ..nn.parallel_mixer import ParallelMixer
 from ..nn.residual import sandwich_norm
@@ -393,8 +393,9 @@ class MavidraModel:
 
     @torch.no_grad()
     def forward_tensors(self, tokens, positions, slots, block_table, q_start, q_len, kv_len, logit_rows, plan=None,
-                        state_slot=None, lora=None) -> torch.Tensor:
-        """fp32 logits [len(logit_rows), vocab] of a ragged step."""
+                        state_slot=None, lora=None, lengths=None) -> torch.Tensor:
+        """fp32 logits [len(logit_rows), vocab] of a ragged step. ``lengths``: (q_len, kv_len) as lists on the host, where the
+        caller has them (prompt steps read them back otherwise)."""
         if lora is not None:
             raise ValueError("LoRA adapters are not implemented for this family")
         self.forward_calls += 1
@@ -403,18 +404,18 @@ class MavidraModel:
             if size:
                 return self.graphs.replay(size, block_table, tokens=tokens, positions=positions, slots=slots, kv_len=kv_len,
                                           state_slot=state_slot)
-        return self._forward(tokens, positions, slots, block_table, q_start, q_len, kv_len, logit_rows, state_slot)
+        return self._forward(tokens, positions, slots, block_table, q_start, q_len, kv_len, logit_rows, state_slot, lengths=lengths)
 
     # ------------------------------------------------------------ step
     @torch.no_grad()
     def _forward(self, tokens, positions, slots, block_table, q_start, q_len, kv_len, logit_rows, state_slot=None,
-                 stream: Optional[list] = None) -> torch.Tensor:
+                 stream: Optional[list] = None, lengths=None) -> torch.Tensor:
         """``stream`` (a list) collects a copy of the residual stream after every layer."""
         c, w, T, Wp, dev = self.cfg, self.w, tokens.shape[0], self.cfg.width_pad, self.device
         new = lambda rows: torch.empty(rows, Wp, dtype=self.dtype, device=dev)
         seam = lambda x, **kw: sandwich_norm(x, cols=c.hidden_size, eps=c.norm_eps, **kw)
         one_token = T == q_len.shape[0]
-        plan = prompt_plan(T, q_len, kv_len) if any(getattr(l.mixer, "projects", False) for l in w.layers) else None
+        projected = prompt_plans({l.mixer.cfg.window for l in w.layers if getattr(l.mixer, "projects", False)}, T, q_len, kv_len, lengths)
         plans = {g: tensor_core_plan(g, self.kv.shape[5], self.dtype, self.page_size, q_start, q_len, T, one_token)
                  for g in self.groups}
         counts = torch.zeros(len(self.moe_layers), self.max_experts, dtype=torch.int32, device=dev)
@@ -432,7 +433,7 @@ class MavidraModel:
                 y = l.mixer(h, ops.linear, self.state[f"l{i}.gla"], state_slot, q_start, q_len, kv_len, one_token)
             elif kind == LATENT:
                 y = l.mixer(h, ops.linear, self.paged["latent"][:, self.plane[i]], self.cos_sin[i], positions, slots, block_table,
-                            q_start, q_len, kv_len, one_token, plan)
+                            q_start, q_len, kv_len, one_token, projected.get(l.mixer.cfg.window))
             else:
                 y = l.mixer(h, ops.linear, self.kv, self.plane[i], self.state[f"l{i}.delta"], self.state[f"l{i}.conv"], self.cos_sin[i],
                             positions, slots, block_table, q_start, q_len, kv_len, state_slot, plans[l.mixer.left.cfg.group_pad],

@@ -129,7 +129,7 @@ class LatentAttention:
     def __call__(self, x, lin, cache, cos_sin, positions, slots, block_table, q_start, q_len, kv_len, one_token: bool,
                  plan: Optional["PromptPlan"] = None):
         """x [T, width] -> [T, width]; ``cache`` [pages, page, >= cache_width] is this layer's (or the shared) plane.
-        ``plan``: :func:`prompt_plan` of the step."""
+        ``plan``: :func:`prompt_plan` of the step for this layer's window."""
         c, T = self.cfg, x.shape[0]
         H, dp, Dp, Rp = c.heads, up64(c.dim), rot_pad(c.rot_dim), latent_pad(c.kv_rank)
         px = lin(x, self.w_in)
@@ -143,7 +143,7 @@ class LatentAttention:
         o = torch.empty(T, self.w_o.shape[1], dtype=x.dtype, device=x.device)
         if o.shape[1] != width:
             o[:, width:].zero_()
-        if plan is not None and self.projects and (c.window == 0 or c.window > 256):
+        if plan is not None and self.projects:
             prompt_attention(plan, q.view(T, H, c.head_width)[:, :, :dp], q_rope, stacked_up(self.w_uk, self.w_uv), cache, block_table, q_start,
                              q_len, kv_len, o, c.scale, self.sink, c.window, gate)
         else:
@@ -174,27 +174,54 @@ class PromptPlan:
     tile_q0: torch.Tensor
 
 
-def prompt_plan(T: int, q_len, kv_len) -> Optional[PromptPlan]:
-    """The plan of a step whose latents are better projected up to keys and values per head, or None. A query and a key then
-    meet in 320 products a head instead of 1088, but every cache row costs 256 x 512 a head first: it pays where a row is
-    seen by more than 171 queries. Steps below 256 tokens, captured steps and rows beyond the scratch limit stay absorbed.
-    Reads both lengths back (one synchronisation a step)."""
-    if not q_len.is_cuda or T < 256 or T == q_len.numel() or torch.cuda.is_current_stream_capturing():
-        return None
-    ql, kl = torch.stack((q_len.int(), kv_len.int())).tolist()
-    pairs = sum(n * (k - n) + n * (n + 1) // 2 for n, k in zip(ql, kl))
-    rows = sum(kl)
-    if rows > PROMPT_ROWS or pairs * _PER_PAIR <= rows * _PER_ROW:
+def prompt_tiles(q_len, kv_len, window: int = 0):
+    """(rows, first scratch row of every sequence and the end, tiles' sequences, tiles' first queries) of a step with these
+    lengths, or None where the absorbed form is better. A query and a key meet in 320 products a head instead of 1088, but every
+    cache row costs 256 x 512 a head first. ``pairs`` are the queries' keys (no more than ``window`` of them each), so the
+    products are equal at a ratio of 1; measured at 16, 64 and 128 heads, the projected form takes 0.77 of the time and less from
+    a ratio of 0.4 on (256 queries without a cache 39 against 51 us at 16 heads, 46 against 111 at 128), about the same at 0.2 to
+    0.35, and more below (300 queries after 15000 cached rows, window 512, ratio 0.06: 135 against 81 and 660 against 269 us)."""
+    pairs = 0
+    for n, k in zip(q_len, kv_len):
+        first, w = k - n, window or k
+        short = max(0, min(k, w) - first)                    # queries that see fewer than ``w`` keys
+        pairs += short * first + short * (short + 1) // 2 + (n - short) * w
+    rows = sum(kv_len)
+    if 5 * pairs * _PER_PAIR <= 2 * rows * _PER_ROW:
         return None
     start, seq, q0 = [0], [], []
-    for s, (n, k) in enumerate(zip(ql, kl)):
+    for s, (n, k) in enumerate(zip(q_len, kv_len)):
         start.append(start[-1] + -(-k // 64) * 64)
         for t in range(0, n, 128):
             seq.append(s)
             q0.append(t)
-    B, n = len(ql), len(seq)
-    buf = torch.tensor(start[:B] + seq + q0, dtype=torch.int32).to(q_len.device)
-    return PromptPlan(rows, start[B], buf[:B], buf[B: B + n], buf[B + n:])
+    return (rows, start, seq, q0) if start[-1] <= PROMPT_ROWS else None
+
+
+def prompt_plans(windows, T: int, q_len, kv_len, lengths=None) -> dict:
+    """The plan of a step for layers of each window (0: none), where their latents are better projected up to keys and values per
+    head. Steps below 256 tokens, captured steps and rows beyond the scratch limit stay absorbed. ``lengths``: (q_len, kv_len) on
+    the host; without it both are read back, which waits for all that is queued."""
+    if not windows or not q_len.is_cuda or T < 256 or T == q_len.numel() or torch.cuda.is_current_stream_capturing():
+        return {}
+    if lengths is None:
+        lengths = torch.stack((q_len.int(), kv_len.int())).tolist()
+    out = {}
+    for w in set(windows):
+        tiles = prompt_tiles(*lengths, w)
+        if tiles is None:
+            continue
+        rows, start, seq, q0 = tiles
+        B, n = len(start) - 1, len(seq)
+        # from pinned memory: a copy out of pageable memory would wait for the stream
+        buf = torch.tensor(start[:B] + seq + q0, dtype=torch.int32).pin_memory().to(q_len.device, non_blocking=True)
+        out[w] = PromptPlan(rows, start[B], buf[:B], buf[B: B + n], buf[B + n:])
+    return out
+
+
+def prompt_plan(T: int, q_len, kv_len, window: int = 0, lengths=None) -> Optional[PromptPlan]:
+    """:func:`prompt_plans` of one window."""
+    return prompt_plans((window,), T, q_len, kv_len, lengths).get(window)
 
 
 def stacked_up(w_uk: torch.Tensor, w_uv: torch.Tensor) -> torch.Tensor:

@@ -290,3 +290,17 @@ def test_stacked_projection(h, R):
 
     w_uk, w_uv = torch.randn(h, R, 128, device="cuda").bfloat16(), torch.randn(h, 128, R, device="cuda").bfloat16()
     assert torch.equal(stacked_up(w_uk, w_uv), torch.cat((w_uk.transpose(1, 2).reshape(-1, R), w_uv.reshape(-1, R))))
+
+
+def test_prompt_plan_counts_the_keys_that_are_seen():
+    """A window bounds the pairs, not the rows that have to be projected: long prefixes with a short window stay absorbed."""
+    from modular_b200.nn.latent_attention import PROMPT_ROWS, prompt_tiles
+
+    assert prompt_tiles([300], [15300], 512) is None and prompt_tiles([300], [15300]) is not None
+    assert prompt_tiles([1024], [5120], 512) is not None and prompt_tiles([512], [512], 32) is None
+    assert prompt_tiles([1] * 300, [2000] * 8 + [1] * 292) is None and prompt_tiles([512], [PROMPT_ROWS + 1]) is None
+    rows, start, seq, q0 = prompt_tiles([300, 127, 1, 513], [300, 127, 1, 700])
+    assert rows == 1128 and start == [0, 320, 448, 512, 1216] and seq == [0] * 3 + [1, 2] + [3] * 5 and q0 == [0, 128, 256, 0, 0, 0, 128, 256, 384, 512]
+    for n, k, w in ((5, 5, 3), (7, 20, 4), (300, 300, 100), (4, 9, 6)):          # the closed form of the pairs, through the ratio
+        pairs = sum(min(w, k - n + i + 1) for i in range(n))
+        assert (prompt_tiles([n] * 1, [k], w) is not None) == (5 * pairs * 768 > 2 * k * 131072)
