@@ -406,6 +406,7 @@ class DeepseekV3Model:
     """
 
     use_executor = False      # the step is a sequence of this package's kernels driven from Python
+    takes_lengths = True      # forward_tensors(lengths=...)
 
     def __init__(self, cfg: DeepseekV3Config, weights: DeepseekV3Weights, kv_cache: torch.Tensor,
                  max_tokens: int = 8192, max_seqs: int = 256, max_position: Optional[int] = None, ep=None):

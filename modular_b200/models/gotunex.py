@@ -288,6 +288,7 @@ class GotunexModel:
     graphs. ``kv_cache``: [pages, 1, cache layers, 1, page, cache width]; ``state``: the cache manager's state tensors."""
 
     use_executor = False
+    takes_lengths = True      # forward_tensors(lengths=...)
     executor = None
     logits_buf = None
 

@@ -344,6 +344,7 @@ class MavidraModel:
     (latent rows); ``state``: its state tensors."""
 
     use_executor = False
+    takes_lengths = True      # forward_tensors(lengths=...)
     executor = None
     logits_buf = None
 

@@ -230,6 +230,13 @@ class BatchPacker:
         self._events[si] = ev
         return self.meta_dev
 
+    @staticmethod
+    def host_lengths(sb: StepBatch, model) -> dict:
+        """``lengths`` of a step for models that would read them back from the device otherwise."""
+        if not getattr(model, "takes_lengths", False):
+            return {}
+        return {"lengths": tuple(sb.arr(n, np.int32, sb.B).tolist() for n in ("q_len", "kv_len"))}
+
     def step_tensors(self, sb: StepBatch) -> dict:
         """Per-array tensors of a step for models that run op by op: on the GPU, views of the packed buffer after its
         single upload."""

@@ -106,7 +106,8 @@ class _SeqCache:
         old_kv, self.model.kv = self.model.kv, self.kv
         try:
             logits = self.model.forward_tensors(torch.tensor(list(tokens), dtype=torch.long, device=dev), pos,
-                                                (pos.long() + self.page), self.bt, i32(0), i32(n), i32(self.len + n), rows)
+                                                (pos.long() + self.page), self.bt, i32(0), i32(n), i32(self.len + n), rows,
+                                                **({"lengths": ([n], [self.len + n])} if getattr(self.model, "takes_lengths", False) else {}))
         finally:
             self.model.kv = old_kv
         self.len += n
@@ -214,7 +215,7 @@ class BatchedDraftProposer:
             return [int(v) for v in self.model.sampled[: sb.n_logits].cpu().numpy()]
         t = BatchPacker.tensors(sb, self.device)
         logits = self.model.forward_tensors(t["tokens"], t["positions"], t["slots"], t["block_table"], t["q_start"],
-                                            t["q_len"], t["kv_len"], t["logit_rows"])
+                                            t["q_len"], t["kv_len"], t["logit_rows"], **BatchPacker.host_lengths(sb, self.model))
         return [int(v) for v in ops.argmax(logits).cpu().numpy()]
 
     def propose_batch(self, batch, rooms: Sequence[int]) -> list:

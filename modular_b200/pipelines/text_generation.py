@@ -252,7 +252,7 @@ class TextGenerationPipeline:
                 extra["lora"] = LoRABatch(self.lora_manager, token_slots_for(
                     self.lora_manager, [c.tokens.active_length for c in sb.ctxs], [c.lora_name for c in sb.ctxs],
                     self.device))
-            logits = self._forward_step(t, **extra)
+            logits = self._forward_step(t, **BatchPacker.host_lengths(sb, self.model), **extra)
             mask = self._grammar_bitmask(sb) if self.structured is not None else None
             if mask is not None:
                 ops.apply_token_bitmask(logits, mask)
@@ -284,7 +284,7 @@ class TextGenerationPipeline:
         sb = self.packer.pack(batch, self.kv, want=want)
         if self.on_gpu and self.model.use_executor:
             raise NotImplementedError(f"{type(self.model).__name__} steps run in the native executor, which samples")
-        logits = self._forward_step(self.packer.step_tensors(sb))
+        logits = self._forward_step(self.packer.step_tensors(sb), **BatchPacker.host_lengths(sb, self.model))
         self.stats.tokens_in += sb.T
         for c in sb.ctxs:
             c.tokens.advance_processed()
@@ -458,7 +458,7 @@ class TextGenerationPipeline:
         else:
             t = BatchPacker.tensors(sb, self.device)
             logits = self.model.forward_tensors(t["tokens"], t["positions"], t["slots"], t["block_table"], t["q_start"],
-                                                t["q_len"], t["kv_len"], t["logit_rows"])
+                                                t["q_len"], t["kv_len"], t["logit_rows"], **BatchPacker.host_lengths(sb, self.model))
             vals = ops.argmax(logits).cpu().numpy()
         self.stats.tokens_in += sb.T
         out: dict[str, TextGenerationOutput] = {}

@@ -304,3 +304,22 @@ def test_prompt_plan_counts_the_keys_that_are_seen():
     for n, k, w in ((5, 5, 3), (7, 20, 4), (300, 300, 100), (4, 9, 6)):          # the closed form of the pairs, through the ratio
         pairs = sum(min(w, k - n + i + 1) for i in range(n))
         assert (prompt_tiles([n] * 1, [k], w) is not None) == (5 * pairs * 768 > 2 * k * 131072)
+
+
+def test_engine_steps_bring_their_lengths():
+    """No prompt step of the engine has to read the lengths back from the device."""
+    from modular_b200.entrypoints.llm import LLM
+    from modular_b200.pipelines.context import SamplingParams
+
+    cfg = DeepseekV3Config.tiny()
+    llm = LLM(cfg, DeepseekV3Weights.random_init(cfg, "cpu", torch.float32, seed=5, std=0.05), device="cpu", dtype=torch.float32, max_length=128,
+              max_batch_size=4, max_batch_input_tokens=64, page_size=16, num_kv_pages=32)
+    seen, forward = [], llm.model.forward_tensors
+
+    def spy(*args, lengths=None, **kw):
+        seen.append((lengths, args[5].tolist(), args[6].tolist()))
+        return forward(*args, lengths=lengths, **kw)
+
+    llm.model.forward_tensors = spy
+    llm.generate([list(range(5, 90)), list(range(3, 20))], SamplingParams(temperature=0.0, max_new_tokens=3, ignore_eos=True))
+    assert seen and all(tuple(l) == (q, k) for l, q, k in seen)
