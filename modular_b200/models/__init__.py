@@ -41,6 +41,7 @@ def _llama_family() -> ModelFamily:
 
 def _deepseek_family() -> ModelFamily:
     from ..kv_cache import KVCacheParams
+    from ..nn.latent_attention import prompt_scratch_bytes
     from .deepseek_v3 import DeepseekV3Config, DeepseekV3Model, DeepseekV3Weights
 
     def kv(cfg, page, dtype, prefix):
@@ -50,7 +51,8 @@ def _deepseek_family() -> ModelFamily:
         h = cfg.num_attention_heads
         per_tok = (4 * cfg.hidden_size + 2 * h * (cfg.qk_head_dim + cfg.kv_lora_rank + cfg.v_head_dim)
                    + 3 * max(cfg.intermediate_size, cfg.num_experts_per_tok * cfg.moe_intermediate_size))
-        return T * per_tok * 2 + B * cfg.vocab_size * 4 + (256 << 20)
+        fits = cfg.qk_nope_head_dim == cfg.v_head_dim == 128 and cfg.qk_rope_head_dim == 64
+        return T * per_tok * 2 + B * cfg.vocab_size * 4 + prompt_scratch_bytes(h, cfg.kv_lora_rank, T, fits) + (256 << 20)
 
     return ModelFamily("deepseek_v3", DeepseekV3Config, DeepseekV3Weights, DeepseekV3Model, kv, act, supports_ep=True)
 
@@ -109,7 +111,8 @@ def _gotunex_family() -> ModelFamily:
                 n += ff["ff"] if ff["kind"] == "dense" else ff["router"]["top"] * (2 * cfg.width_pad + ff["expert"]["ff"])
             per_tok = max(per_tok, 4 * cfg.width_pad + n)
         state = kv(cfg, 64, torch.bfloat16, False).state_bytes_per_slot
-        return T * per_tok * 4 + B * cfg.vocab_size * 4 + B * state + (256 << 20)
+        scratch = max((a.prompt_scratch_bytes(T) for a in (cfg.attention(i) for i in range(len(cfg.layers)) if cfg.is_attention(i))), default=0)
+        return T * per_tok * 4 + B * cfg.vocab_size * 4 + B * state + scratch + (256 << 20)
 
     return ModelFamily("gotunex", GotunexConfig, GotunexWeights, GotunexModel, kv, act)
 
@@ -161,7 +164,8 @@ def _mavidra_family() -> ModelFamily:
                 n = max(n, l["mlp"]["router"]["top"] * (2 * cfg.width_pad + l["mlp"]["expert"]["ff"]))
             per_tok = max(per_tok, 6 * cfg.width_pad + n)
         state = kv(cfg, 64, torch.bfloat16, False).state_bytes_per_slot
-        return T * per_tok * 4 + B * cfg.vocab_size * 4 + B * state + (256 << 20)
+        scratch = max((a.prompt_scratch_bytes(T) for a in (cfg.latent(i) for i, l in enumerate(cfg.layers) if l["type"] == LATENT)), default=0)
+        return T * per_tok * 4 + B * cfg.vocab_size * 4 + B * state + scratch + (256 << 20)
 
     return ModelFamily("mavidra", MavidraConfig, MavidraWeights, MavidraModel, kv, act)
 

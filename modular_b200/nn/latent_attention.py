@@ -64,6 +64,14 @@ class LatentAttentionConfig:
         return up64(self.dim) + rot_pad(self.rot_dim)
 
     @property
+    def projects(self) -> bool:
+        """Whether prompts may run on projected keys and values (bf16 on the GPU)."""
+        return up64(self.dim) == self.vdim_pad == 128 and rot_pad(self.rot_dim) == 64
+
+    def prompt_scratch_bytes(self, T: int) -> int:
+        return prompt_scratch_bytes(self.heads, latent_pad(self.kv_rank), T, self.projects)
+
+    @property
     def cache_width(self) -> int:
         return latent_pad(self.kv_rank) + rot_pad(self.rot_dim)
 
@@ -122,7 +130,7 @@ class LatentAttention:
         uv[:, : c.vdim, : c.kv_rank] = t["uv"].view(H, c.vdim, c.kv_rank)
         self.w_uv = put(uv)                                          # [h, vdim, latent]: latent outputs to values
         # prompts project latents up to keys and values where the sizes are those of the kernel
-        self.projects = up64(d) == vp == 128 and rot_pad(r) == 64 and self.w_uk.is_cuda and dtype == torch.bfloat16
+        self.projects = c.projects and self.w_uk.is_cuda and dtype == torch.bfloat16
         self.sink = put(t["sink"], torch.float32) if c.sink else None
         self.w_o = put(pad_to(pad_heads(t["o"].t().contiguous(), H, c.vdim, vp).t(), width_pad, gemm_k(H * vp)))
 
@@ -172,6 +180,13 @@ class PromptPlan:
     kv_start: torch.Tensor
     tile_seq: torch.Tensor
     tile_q0: torch.Tensor
+
+
+def prompt_scratch_bytes(heads: int, latent: int, T: int, dims_fit: bool = True) -> int:
+    """Most scratch of a layer in a prompt step of ``T`` tokens: keys and values, gathered rows, stacked weights."""
+    if T < 256 or not dims_fit:
+        return 0
+    return 2 * (PROMPT_ROWS * (2 * heads * 128 + latent + 64) + 2 * heads * 128 * latent)
 
 
 def prompt_tiles(q_len, kv_len, window: int = 0):

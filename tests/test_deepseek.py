@@ -323,3 +323,16 @@ def test_engine_steps_bring_their_lengths():
     llm.model.forward_tensors = spy
     llm.generate([list(range(5, 90)), list(range(3, 20))], SamplingParams(temperature=0.0, max_new_tokens=3, ignore_eos=True))
     assert seen and all(tuple(l) == (q, k) for l, q, k in seen)
+
+
+def test_projected_prompts_are_in_the_memory_plan():
+    from modular_b200.models import family_for
+    from modular_b200.nn.latent_attention import PROMPT_ROWS
+
+    cfg = DeepseekV3Config.deepseek_v3()
+    act = family_for(cfg).activation_bytes
+    h, R = cfg.num_attention_heads, cfg.kv_lora_rank
+    need = 2 * (PROMPT_ROWS * (2 * h * 128 + R + 64) + 2 * h * 128 * R)              # keys and values, latents, rotated keys, weights
+    assert act(cfg, 256, 8) - act(cfg, 255, 8) >= need                               # such steps begin at 256 tokens
+    big = DeepseekV3Config.tiny()                                                    # heads of 64: prompts stay absorbed
+    assert family_for(big).activation_bytes(big, 256, 8) - family_for(big).activation_bytes(big, 255, 8) < 1 << 20
