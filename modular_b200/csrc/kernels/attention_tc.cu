@@ -1,23 +1,25 @@
 // Prefill attention on the 5th-generation tensor cores (tcgen05 + TMEM + TMA): paged grouped-query heads of width 128, and
 // latent heads projected up to keys of 192 and values of 128 (contiguous rows).
 //
-// One CTA owns two tiles of 128 query rows of one (sequence, KV head): 256/G consecutive tokens x the G query heads that
-// share the KV head (GQA packing puts them on the MMA M dimension). It walks the sequence's keys BN at a time:
+// A tile is 128 query rows of one (sequence, KV head): 128/G consecutive tokens x the G query heads that share the KV head (GQA
+// packing puts them on the MMA M dimension). A CTA owns one tile (paged heads; two CTAs an SM) or two (latent heads, whose
+// operands fill an SM's shared memory) and walks the sequence's keys 64 at a time:
 //
 //   warp 0      TMA producer: K tiles and V tiles (boxes of 64 rows x 64 columns, 128B swizzle) into a ring of five slots
-//   warp 1      MMA issuer, for tile g in turn:  O_g += P_g . V   (P_g read from TMEM, V an MN-major operand straight from
-//               the row-major rows), then S_g = Q_g . K^T of the next keys into the columns P_g was read from (MMAs of
-//               one thread run in order)
+//   warp 1      MMA issuer. One tile: S = Q . K^T of the next keys into the other of two score buffers, while the softmax has this
+//               one; then O += P . V (P read from TMEM, V an MN-major operand straight from the row-major rows). Two tiles, for
+//               tile g in turn: O_g += P_g . V, then S_g of the next keys into the columns P_g was read from. (MMAs of one
+//               thread run in order.)
 //   warps 4-7   softmax of tile 0, warps 8-11 of tile 1: one query row per thread (TMEM lane = row). Read S, mask, row
 //               maximum, exponentials, P (bf16) back into the columns of S. The output stays in TMEM; it is rescaled only
 //               when a row's maximum has grown by more than 2^8 since the reference maximum was taken (exact after the
 //               final 1/l normalisation, because P is always computed against that reference)
 //
-// While one tile's softmax runs, the tensor pipe works for the other tile. Per 256 x 128 scores the four MMAs take 2048
-// cycles and the exponentials as many (16 a cycle and SM), so both pipes bound it together; what the form before this one
-// (one tile of 128 rows, 64 keys, P through shared memory, a third MMA wait per tile) lost was the chain between them:
-// 2600 cycles for 128 x 64. 12001 tokens, 32 heads over 8, causal: 2608 us then, 1206 us (980 TFLOP/s) now.
-// CTAs with the most keys start first.
+// While one tile's softmax runs, the tensor pipe works for the other tile, of this CTA or of the other on the SM. Per 256 x 128 scores
+// the four MMAs take 2048 cycles and the exponentials as many (16 a cycle and SM), so both pipes bound it together; what is lost is the
+// chain between them. 32 heads over 8, causal: 8000 tokens 927 us with one tile an SM, P through shared memory and a third wait a tile;
+// 570 with two tiles of 256 rows a CTA and 128 keys; 508 so, and short prompts, of which a pair of tiles was mostly empty, gain more
+// (64 of 64 tokens 65, 65 and 48 us; 16 heads of 64 x 64 tokens 47, 54 and 29).
 //
 // A sliding window of W keys (itself and the W - 1 before it) starts the walk at the first tile any row of the CTA
 // sees and masks the edge; a sink score per head only adds exp(sink) to the denominator.
@@ -44,8 +46,6 @@ namespace atc {
 typedef __nv_bfloat16 bf16;
 constexpr int HD = 128;        // values, and keys without a rotated part of their own
 constexpr int kSlots = 5;      // K and V tiles in turn
-constexpr int kThreads = 384;  // warps 2 and 3 idle: register budgets belong to groups of four warps
-constexpr uint32_t kTmemCols = 512;           // S / P of tile 0 | of tile 1 | O of tile 0 | of tile 1 (128 each)
 
 struct Params {
   const bf16* q;
@@ -73,6 +73,8 @@ struct Bars {
   uint64_t s_full[2];
   uint64_t p_full[2];
   uint64_t o_done[2];
+  uint64_t pv_done[2];     // one tile: the products with V, in turn. A wait for one of them is not confused by the phases around it:
+                           // the product two before it ended before the scores that the waiting warp has, the one two after cannot begin
   uint32_t tmem_base;
   int abort_word;
 };
@@ -110,20 +112,24 @@ __device__ __forceinline__ float ex2(float x) {
 
 template <bool LATENT>
 struct Shape {
+  static constexpr int TILES = LATENT ? 2 : 1;                    // query tiles of a CTA
   static constexpr int NC = LATENT ? 3 : 2;                       // 64-column chunks of a key
-  static constexpr int BN = LATENT ? 64 : 128;                    // keys per tile
+  static constexpr int BN = 64;                                   // keys per tile
+  static constexpr int kThreads = 128 + TILES * 128;              // warps 2 and 3 idle: register budgets belong to groups of four warps
+  static constexpr uint32_t kTmemCols = TILES * 256;              // S / P of tile 0 | of tile 1 | O of tile 0 | of tile 1 (128 each)
+  static constexpr int kScoreCols = TILES == 1 ? 64 : 128;        // one tile: S / P of even keys' tiles | of odd ones | O
   static constexpr int kQTile = NC * 128 * 128;                   // 128 rows
   static constexpr int kKBytes = NC * BN * 128, kVBytes = 2 * BN * 128;
   static constexpr int kSlot = kKBytes > kVBytes ? kKBytes : kVBytes;
-  static constexpr size_t kSmem = 2 * kQTile + kSlots * kSlot + sizeof(Bars);
+  static constexpr size_t kSmem = TILES * kQTile + kSlots * kSlot + sizeof(Bars);
 };
 
 template <bool LATENT>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(Shape<LATENT>::kThreads, LATENT ? 1 : 2)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmR, const __grid_constant__ CUtensorMap tmV,
                const Params p) {
   using Sh = Shape<LATENT>;
-  constexpr int BN = Sh::BN, NC = Sh::NC;
+  constexpr int BN = Sh::BN, NC = Sh::NC, TILES = Sh::TILES;
   // No alignment slack. The dynamic shared memory window starts 1024-byte aligned (there is no static shared memory in
   // this kernel); should a future toolchain place it elsewhere the kernel reports it instead of computing garbage.
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -132,21 +138,24 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     return;
   }
   uint8_t* sQ = smem_raw;                           // [tile][chunk][128 rows x 128 B]
-  uint8_t* sRing = sQ + 2 * Sh::kQTile;             // [slot][chunk][BN rows x 128 B]
+  uint8_t* sRing = sQ + TILES * Sh::kQTile;         // [slot][chunk][BN rows x 128 B]
   Bars* bars = reinterpret_cast<Bars*>(sRing + kSlots * Sh::kSlot);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int kvh = blockIdx.y;
+  const int kvh = blockIdx.x;
   const int G = p.G;
   const int tok_per_tile = 128 / G;
 
-  const int tile = gridDim.x - 1 - blockIdx.x;      // later tiles of a prompt see more keys
+  // A CTA covers two tiles of the plan as a rule, and leaves at the second. First come those that have work (the even ones, where
+  // sequences have even numbers of tiles), spread over all SMs; in each half the later tiles of a prompt, which see more keys.
+  const int n_tiles = gridDim.y, even = (n_tiles + 1) >> 1, at = blockIdx.y;
+  const int tile = at < even ? 2 * (even - 1 - at) : 2 * (n_tiles - 1 - at) + 1;
   const int seq = p.tile_seq[tile];
   if (seq < 0) return;                 // an unused tile of a plan made on the device
   const int tq0 = p.tile_q0[tile];
-  if (tq0 % (2 * tok_per_tile) != 0) return;  // the plan lists 64- or 128-row tiles: the others are covered by this one
+  if (tq0 % (TILES * tok_per_tile) != 0) return;  // covered by the CTA of a tile before it
   const int qs = p.q_start[seq], ql = p.q_len[seq], kl = p.kv_len[seq];
-  const bool two = tq0 + tok_per_tile < ql;         // the second tile has rows
-  const int last_tq = min(tq0 + 2 * tok_per_tile, ql);
+  const bool two = TILES == 2 && tq0 + tok_per_tile < ql;         // the second tile has rows
+  const int last_tq = min(tq0 + TILES * tok_per_tile, ql);
   const int kv_hi = kl - ql + last_tq;
   const int kv_lo = kl - ql + tq0 - p.window + 1;        // first key the CTA's first row sees
   const int t_first = kv_lo > 0 ? kv_lo / BN : 0;
@@ -161,12 +170,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
       mbar_init(&bars->s_full[g], 1);
       mbar_init(&bars->p_full[g], 4);
       mbar_init(&bars->o_done[g], 1);
+      mbar_init(&bars->pv_done[g], 1);
     }
     bars->abort_word = 0;
     fence_mbar_init();
   }
   if (warp == 1) {
-    tmem_alloc(&bars->tmem_base, kTmemCols);
+    tmem_alloc(&bars->tmem_base, Sh::kTmemCols);
     tmem_relinquish();
   }
   if (warp >= 4) {
@@ -194,7 +204,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
   const uint32_t tmem_base = bars->tmem_base;
   volatile int* abort_word = &bars->abort_word;
 
-  // 384 x 168 registers at launch: four warps give theirs up, eight take them (128 x 56 + 256 x 224 is the same sum)
+  // Two tiles: 384 x 168 registers at launch, four warps give theirs up, eight take them (128 x 56 + 256 x 224 is the same sum). One
+  // tile: 256 x 128, of which four warps take 200 (128 x 56 + 128 x 200).
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == 0 && lane == 0) {
@@ -242,16 +253,17 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
       const int last = two ? 1 : 0;
       bool ok = true;
       auto wait_item = [&](int i) { ok = ok && mbar_wait(&bars->full[i % kSlots], (i / kSlots) & 1, abort_word, p.err, 702); };
-      auto scores = [&](int i, int g) {            // S_g from ring item i
+      // S_g from ring item i; with one tile, S into buffer g
+      auto scores = [&](int i, int g) {
         const uint8_t* sK = sRing + (i % kSlots) * Sh::kSlot;
 #pragma unroll
         for (int k = 0; k < NC * 4; ++k) {
-          const uint64_t da = umma_desc_sw128(sQ + g * Sh::kQTile + (k >> 2) * 16384) + static_cast<uint64_t>((k & 3) * 2);
+          const uint64_t da = umma_desc_sw128(sQ + (TILES == 2 ? g * Sh::kQTile : 0) + (k >> 2) * 16384) + static_cast<uint64_t>((k & 3) * 2);
           const uint64_t db = umma_desc_sw128(sK + (k >> 2) * (BN * 128)) + static_cast<uint64_t>((k & 3) * 2);
-          umma_bf16(tmem_base + g * 128, da, db, idesc_s, k > 0 ? 1u : 0u);
+          umma_bf16(tmem_base + g * Sh::kScoreCols, da, db, idesc_s, k > 0 ? 1u : 0u);
         }
         tc_commit(&bars->s_full[g]);
-        if (g == last) tc_commit(&bars->empty[i % kSlots]);
+        if (TILES == 1 || g == last) tc_commit(&bars->empty[i % kSlots]);
       };
       if (ntiles > 0) {
         wait_item(0);
@@ -261,7 +273,29 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
           if (two) scores(0, 1);
         }
       }
-      for (int t = 0; t < ntiles && ok; ++t) {
+      for (int t = 0; t < ntiles && ok && TILES == 1; ++t) {
+        // the next scores go into the other buffer while the softmax has this one (the product that read P there was issued before)
+        if (t + 1 < ntiles) {
+          wait_item(2 * t + 2);
+          if (!ok) break;
+          tc_fence_after();
+          scores(2 * t + 2, (t + 1) & 1);
+        }
+        wait_item(2 * t + 1);
+        // (a barrier per buffer: the softmax may be through with the next tile before this one's values are there)
+        ok = ok && mbar_wait(&bars->p_full[t & 1], (t >> 1) & 1, abort_word, p.err, 704);
+        if (!ok) break;
+        tc_fence_after();
+        const uint8_t* sV = sRing + ((2 * t + 1) % kSlots) * Sh::kSlot;
+#pragma unroll
+        for (int k = 0; k < BN / 16; ++k)
+          umma_bf16_ts(tmem_base + 128, tmem_base + (t & 1) * Sh::kScoreCols + k * 8, umma_desc_mn_sw128(sV + k * 2048, BN * 128, 1024), idesc_pv,
+                       (t > 0 || k > 0) ? 1u : 0u);
+        tc_commit(&bars->empty[(2 * t + 1) % kSlots]);
+        tc_commit(&bars->pv_done[t & 1]);
+        if (t + 1 == ntiles) tc_commit(&bars->o_done[0]);
+      }
+      for (int t = 0; t < ntiles && ok && TILES == 2; ++t) {
         for (int g = 0; g <= last && ok; ++g) {
           if (g == 0) wait_item(2 * t + 1);
           ok = ok && mbar_wait(&bars->p_full[g], t & 1, abort_word, p.err, 704);
@@ -287,18 +321,20 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    if constexpr (TILES == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    else asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
     // ---------------------------------------------------------------- softmax
-    const int g = (warp - 4) >> 2, quad = warp & 3, r = quad * 32 + lane;
+    const int g = TILES == 1 ? 0 : (warp - 4) >> 2, quad = warp & 3, r = quad * 32 + lane;
     const int tq = tq0 + g * tok_per_tile + r / G, head = kvh * G + r % G;
     const int limit = tq < ql ? kl - ql + tq : -1;
-    const uint32_t s_addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + g * 128, o_addr = s_addr + 256;
+    const uint32_t s_tile = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + g * 128, o_addr = s_tile + TILES * 128;
     float m_ref = 0.f, l = 0.f;       // P and l are relative to m_ref (a lagging running maximum)
     bool ok = true, unset = true;     // unset: no key has been visible to the row yet
     const int mine = g == 0 || two ? ntiles : 0;
     for (int t = 0; t < mine; ++t) {
-      // the scores are there; so is everything issued before them: the last P . V has retired, O is at rest
-      ok = mbar_wait(&bars->s_full[g], t & 1, abort_word, p.err, 706);
+      // the scores are there; with two tiles, so is everything issued before them: the last P . V has retired, O is at rest
+      const uint32_t s_addr = TILES == 1 ? s_tile + (t & 1) * Sh::kScoreCols : s_tile;
+      ok = TILES == 1 ? mbar_wait(&bars->s_full[t & 1], (t >> 1) & 1, abort_word, p.err, 706) : mbar_wait(&bars->s_full[g], t & 1, abort_word, p.err, 706);
       if (!ok) break;
       tc_fence_after();
       uint32_t sr[BN / 32][32];
@@ -325,6 +361,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
         grow = mx - m_ref > 8.0f;      // probabilities would exceed 2^8: move the reference
       }
       if (__any_sync(0xffffffffu, grow)) {
+        if (TILES == 1) {              // the last P . V may still be adding (this tile's cannot have begun, the one before it is done)
+          ok = t == 0 || mbar_wait(&bars->pv_done[(t - 1) & 1], ((t - 1) >> 1) & 1, abort_word, p.err, 707);
+          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          tc_fence_after();
+        }
         // rescale this warp's 32 accumulator rows (factor 1 for rows whose reference stays)
         const float factor = grow ? exp2f(m_ref - mx) : 1.0f;
         if (grow) { m_ref = mx; l *= factor; }
@@ -356,7 +397,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->p_full[g]);
+      if (lane == 0) mbar_arrive(&bars->p_full[TILES == 1 ? t & 1 : g]);
     }
     if (ok && mine > 0) ok = mbar_wait(&bars->o_done[g], 0, abort_word, p.err, 708);
     if (ok && mine > 0) {
@@ -396,13 +437,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTmemCols);
+    tmem_dealloc(tmem_base, Sh::kTmemCols);
   }
 }
 
-// An ordinary launch, and no early start of the next kernel either: both would hide a few microseconds of hundreds, and a
-// CTA takes all registers and shared memory of its SM, so that a grid of them that waits for the kernel before it leaves no
-// room for anything else.
+// An ordinary launch, and no early start of the next kernel either: both would hide a microsecond or two, and these CTAs take
+// all registers and shared memory of their SM, so that a grid of them that waits for the kernel before it leaves no room for
+// anything else.
 template <bool LATENT>
 static int launch(const CUtensorMap& tk, const CUtensorMap& tr, const CUtensorMap& tv, const Params& p, int heads, cudaStream_t stream) {
   static PerDeviceOnce configured;
@@ -412,7 +453,8 @@ static int launch(const CUtensorMap& tk, const CUtensorMap& tr, const CUtensorMa
       return MB_ERR_LAUNCH;
     configured.done();
   }
-  return launch_plain(attn_tc_kernel<LATENT>, dim3(p.n_tiles, heads), dim3(kThreads), Shape<LATENT>::kSmem, stream, tk, tr, tv, p) == cudaSuccess
+  using Sh = Shape<LATENT>;
+  return launch_plain(attn_tc_kernel<LATENT>, dim3(heads, p.n_tiles), dim3(Sh::kThreads), Sh::kSmem, stream, tk, tr, tv, p) == cudaSuccess
              ? MB_OK
              : MB_ERR_LAUNCH;
 }
@@ -424,8 +466,8 @@ using namespace mb;
 
 // Prefill tiles of a ragged batch on the tcgen05 kernel. Same KV addressing as mb_paged_attention_tma
 // (kv_base viewed as [total_rows, 128]); head_dim 128, G = n_q / n_kv in {1, 2, 4, 8, 16}, page_size % 64 == 0.
-// tile_seq / tile_q0 is the plan of 64-row tiles (CTAs take four of them) or of 128-row tiles (two); a negative sequence is
-// an unused tile.
+// tile_seq / tile_q0 is the plan of 64-row tiles (CTAs take two of them) or of 128-row tiles; a negative sequence is an unused
+// tile.
 extern "C" int mb_paged_attention_prefill_tc(const void* q, int ldq, void* out, int ldo, const void* kv_base,
                                              long long total_rows, long long k_off_rows, long long v_off_rows,
                                              long long page_rows, const int32_t* block_table, int bt_stride,

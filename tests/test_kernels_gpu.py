@@ -263,6 +263,36 @@ def test_paged_attention_mixed_batch(n_q, n_kv, hd, ps, tma):
     assert (o.float() - o_ref.float()).abs().max() < 3e-2
 
 
+def test_prompt_attention_of_many_short_and_long_walks():
+    """Walks of 1 to 21 key tiles beside each other, more CTAs than fit at once, maxima that grow all along a walk; twice the same."""
+    from modular_b200._native import lib
+
+    torch.manual_seed(11)
+    n_q, n_kv, hd, ps = 8, 4, 128, 64
+    q_lens = [20 + (37 * i) % 90 for i in range(80)]
+    kv_lens = [n + (0, 17, 64, 300, 700, 1230)[i % 6] for i, n in enumerate(q_lens)]
+    B, T, pages = len(q_lens), sum(q_lens), [-(-k // ps) for k in kv_lens]
+    kv = torch.randn(sum(pages), 2, 1, n_kv, ps, hd, device=DEV)
+    kv[:, 0] *= torch.linspace(0.5, 4.0, ps, device=DEV).view(1, 1, 1, ps, 1)
+    kv = kv.to(torch.bfloat16)
+    bt, at = torch.zeros(B, max(pages), dtype=torch.int32), 0
+    for b, n in enumerate(pages):
+        bt[b, :n] = torch.arange(at, at + n)
+        at += n
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    q = torch.randn(T, n_q * hd, device=DEV).to(torch.bfloat16)
+    args = (bt.to(DEV), i32([0] + list(torch.tensor(q_lens).cumsum(0)[:-1])), i32(q_lens), i32(kv_lens), n_q, n_kv, hd, hd ** -0.5)
+    was = lib().get_attn_tc()
+    lib().set_attn_tc(1)
+    try:
+        got = ops.paged_attention(q, kv[:, 0, 0], kv[:, 1, 0], *args, kv=kv, layer=0)
+        again = ops.paged_attention(q, kv[:, 0, 0], kv[:, 1, 0], *args, kv=kv, layer=0)
+    finally:
+        lib().set_attn_tc(was)
+    assert torch.equal(got, again)
+    assert _rel_err(got, ref.paged_attention(q, kv[:, 0, 0], kv[:, 1, 0], *args)) < 1e-2
+
+
 @pytest.mark.parametrize("h,R,window,extras", [(2, 512, 0, False), (16, 512, 0, True), (3, 128, 150, True)])
 def test_latent_prompt_attention(h, R, window, extras):
     """Latents projected up to keys and values per head, against the same product in fp32: ragged prompts around tiles of 64 keys
