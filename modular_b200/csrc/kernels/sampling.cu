@@ -4,8 +4,8 @@
 // sample_kernel: one CTA of 1024 threads owns one batch row. Top-k and top-p cut-offs are found by
 // bisection on the order-preserving integer image of the fp32 logits, so no sort and
 // no scratch memory is needed; pure temperature sampling takes the one-pass Gumbel-max
-// route. sample_cluster_kernel spreads a row over a thread-block cluster and is the one that runs; sample_kernel is for
-// devices that cannot place such clusters. Behavioural counterparts in the reference: max/kernels/src/nn/topk.mojo
+// route. sample_cluster_kernel spreads a row over a thread-block cluster and runs for all but large batches without a filter;
+// sample_kernel is for those and for devices that cannot place such clusters. Behavioural counterparts in the reference: max/kernels/src/nn/topk.mojo
 // (fused token sampling :2037, Gumbel argmax :2369), nn/sampling/topk_fi.mojo,
 // nn/sampling/sampling.mojo:31 (penalties).
 #include <cuda_runtime.h>
@@ -457,6 +457,8 @@ sample_kernel(const float* __restrict__ logits, int64_t* __restrict__ out, int v
 // Masses are integers, so sums do not depend on their order: 42 fractional bits where few weights meet in registers, and
 // per bin the weights relative to the bin's upper edge as 26-bit numbers in two halves, because 32-bit atomics on shared
 // memory are native and 64-bit ones are not (with those 64 nucleus rows took 122 us, with these 101).
+// (One or four rows with a nucleus over the whole row and nothing else, of a spread of 3.75: 45 us when unit bins were counted in registers,
+// 49 so; counts alone here and masses only where a long nucleus is cut: 55, and 78 for the mixed 64 rows below.)
 // 64 rows of 128256 logits, a quarter of the rows with a nucleus of thousands of tokens: 364 us when such rows (and
 // confident ones, whose k-th token lies far below the first) were left to sample_kernel, which walks a row with one
 // CTA, 58 to 66 us so (127 us before where all kept sets were short); one row 28 us, 64 greedy rows 11 us.
@@ -901,7 +903,10 @@ extern "C" int mb_sample_topk_topp(const float* logits, int64_t* out, int rows, 
                                    const float* top_p, const float* min_p, const uint64_t* seeds,
                                    uint64_t step, cudaStream_t stream) {
   if (rows <= 0) return MB_OK;
-  if (g_sample_cluster && rows <= 65535 && vocab <= kClu * kMaxShare) {
+  // Without any filter a row is one pass, and a batch that fills the SMs is faster with a large CTA a row: 128256 logits, 128 rows greedy 10
+  // us, 18 on clusters, sampled 29 and 40; 64 rows 9 and 11, 29 and 23; 1 row 9 and 9, 29 and 10.
+  const bool one_pass = top_k == nullptr && top_p == nullptr && min_p == nullptr && rows >= 128;
+  if (g_sample_cluster && !one_pass && rows <= 65535 && vocab <= kClu * kMaxShare) {
     static PerDeviceOnce once;
     if (once.needed()) {
       if (cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

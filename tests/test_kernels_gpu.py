@@ -466,7 +466,7 @@ def test_cluster_sampler_matches_one_cta_sampler():
              dict(min_p=torch.full((R,), 0.05, device=DEV)),
              dict(top_k=torch.randint(0, 300, (R,), device=DEV, dtype=torch.int32),
                   top_p=torch.rand(R, device=DEV) * 0.6 + 0.4, min_p=torch.rand(R, device=DEV) * 0.02),
-             dict(top_k=torch.full((R,), 20000, device=DEV, dtype=torch.int32))]   # too wide: left to the other kernel
+             dict(top_k=torch.full((R,), 20000, device=DEV, dtype=torch.int32))]   # too wide: refined in passes
     for kw in cases:
         for lg in (logits, logits[:, :50001]):                           # second view: rows off a 16-byte boundary
             ops.set_sample_cluster(True)
@@ -525,6 +525,16 @@ def test_sampler_small_vocabulary_with_masked_tokens(V, finite):
             want = ops.sample(lg, temperature=temp, seeds=seeds, step=2, **kw)
             ops.set_sample_cluster(True)
             assert torch.equal(got, want), (k, list(kw))
+
+
+def test_sampling_without_filters_is_the_same_in_any_batch():
+    """Large batches take the kernel of one CTA a row, small ones clusters: a row's draw depends on neither."""
+    torch.manual_seed(85)
+    lg = torch.randn(300, 32001, device=DEV)
+    seeds, temp = torch.arange(300, device=DEV, dtype=torch.int64) + 9, torch.linspace(0.0, 1.5, 300, device=DEV)
+    whole = ops.sample(lg, temperature=temp, seeds=seeds, step=3)
+    parts = [ops.sample(lg[a: a + 20], temperature=temp[a: a + 20], seeds=seeds[a: a + 20], step=3) for a in range(0, 300, 20)]
+    assert torch.equal(whole, torch.cat(parts))
 
 
 @pytest.mark.parametrize("V", [300, 50001])
