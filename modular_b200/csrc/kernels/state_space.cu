@@ -292,17 +292,24 @@ __global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(const __nv
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                 // this tile is in; everyone is done with the one before
     if (c0 + TT < n) fetch(c0 + TT, stages[(it + 1) & 1]);
-#pragma unroll
-    for (int j = tid >> 5; j < TT; j += kScanThreads / 32) {
-      if (j >= mm) break;
+    auto step = [&](int j) {
       float dt = __bfloat162float(g.dl[j][pc]) + pb;
       if (dt_softplus) dt = softplus(dt);
       if (j >= m) dt = 0.f;                          // tokens beyond the sequence leave the state alone
       sdt[j][pc] = make_float2(dt, dt * __bfloat162float(g.u[j][pc]));
-    }
-    for (int i = tid; i < mm * N; i += kScanThreads) {
+    };
+    auto widen = [&](int i) {
       (&sB[0][0])[i] = __bfloat162float((&g.B[0][0])[i]);
       (&sC[0][0])[i] = __bfloat162float((&g.C[0][0])[i]);
+    };
+    if (m == TT) {
+#pragma unroll
+      for (int j = 0; j < TT; j += kScanThreads / 32) step(j + (tid >> 5));
+#pragma unroll
+      for (int i = 0; i < TT * N; i += kScanThreads) widen(i + tid);
+    } else {
+      for (int j = tid >> 5; j < mm; j += kScanThreads / 32) step(j);
+      for (int i = tid; i < mm * N; i += kScanThreads) widen(i);
     }
     __syncthreads();
     for (int j0 = 0; j0 < m; j0 += 8) {
