@@ -21,6 +21,9 @@
 // 570 with two tiles of 256 rows a CTA and 128 keys; 508 so, and short prompts, of which a pair of tiles was mostly empty, gain more
 // (64 of 64 tokens 65, 65 and 48 us; 16 heads of 64 x 64 tokens 47, 54 and 29).
 //
+// (Exponentials of one tile under the products of another, and the lazy rescaling, are the schedule that FlashAttention-3 and -4
+// published.)
+//
 // A sliding window of W keys (itself and the W - 1 before it) starts the walk at the first tile any row of the CTA
 // sees and masks the edge; a sink score per head only adds exp(sink) to the denominator.
 //

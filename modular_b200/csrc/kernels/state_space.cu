@@ -417,7 +417,7 @@ __global__ void ssd_scan_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
   }
 }
 
-// The SSD recurrence 64 tokens at a time. With l_i = log2 of the decay of token i of a chunk, c_i = l_0 + .. + l_i and
+// The SSD recurrence 64 tokens at a time (the chunked form of Dao and Gu, "Transformers are SSMs", 2024). With l_i = log2 of the decay of token i of a chunk, c_i = l_0 + .. + l_i and
 // the state S before the chunk:
 //   y_i = 2^c_i S C_i + sum_{j <= i} 2^(c_i - c_j) dt_j (C_i . B_j) x_j + D x_i
 //   S'  = 2^c_m S + sum_j 2^(l_(j+1) + .. + l_m) dt_j x_j B_j^T
@@ -454,6 +454,9 @@ __device__ __forceinline__ uint32_t take_bf16(float& x, float& y) {
   y -= f.y;
   return *reinterpret_cast<const uint32_t*>(&h);
 }
+
+// the signs' places of two bf16 values set where one is infinite or NaN (an exponent of ones carries into them)
+__device__ __forceinline__ uint32_t mark_special(uint32_t w) { return (w & 0x7f807f80u) + 0x00800080u; }
 
 // a + b, and in `left` what its rounding left (Knuth's exact sum of two floats)
 __device__ __forceinline__ float two_sum(float a, float b, float& left) {
@@ -633,67 +636,60 @@ __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_ker
       }
       // what the state before the chunk contributes, for all tokens and this warp's 16 rows
       float o[NB][2][4];
-      auto from_state = [&]() {
-#pragma unroll
-        for (int i = 0; i < NB; ++i)
-#pragma unroll
-          for (int j = 0; j < 2; ++j) o[i][j][0] = o[i][j][1] = o[i][j][2] = o[i][j][3] = 0.f;
-        if (have_state) {
-#pragma unroll
-          for (int kb = 0; kb < KB; ++kb) {
-            uint32_t hi[2][2], lo[2][2];
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-#pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                float u = S[2 * kb + e][2 * j], w = S[2 * kb + e][2 * j + 1];
-                hi[j][e] = take_bf16(u, w);
-                lo[j][e] = take_bf16(u, w);
-              }
-            uint32_t a[NB][4];
-#pragma unroll
-            for (int i = 0; i < NB; ++i) ldsm4(a[i], sC + (i * 16 + (lane & 15)) * LDK + kb * 16 + (lane >> 4) * 8);
-#pragma unroll
-            for (int i = 0; i < NB; ++i) { mma(o[i][0], a[i], hi[0][0], hi[0][1]); mma(o[i][1], a[i], hi[1][0], hi[1][1]); }
-#pragma unroll
-            for (int i = 0; i < NB; ++i) { mma(o[i][0], a[i], lo[0][0], lo[0][1]); mma(o[i][1], a[i], lo[1][0], lo[1][1]); }
-          }
-#pragma unroll
-          for (int i = 0; i < NB; ++i) {
-            const float f0 = tm.grow[i * 16 + row4], f1 = tm.grow[i * 16 + row4 + 8];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) { o[i][j][0] *= f0; o[i][j][1] *= f0; o[i][j][2] *= f1; o[i][j][3] *= f1; }
-          }
-        }
-      };
-      from_state();
-      __syncthreads();                               // the products of every warp are in sP
-#pragma unroll
-      for (int kb = 0; kb < NB; ++kb) {
-        uint32_t b[4];
-        ldsm4_t(b, sV + (kb * 16 + (mi & 1) * 8 + r8) * kLdV + warp * 16 + (mi >> 1) * 8);
-#pragma unroll
-        for (int half = 0; half < 2; ++half)
-#pragma unroll
-          for (int i = kb; i < NB; ++i) {
-            uint32_t a[4];
-            ldsm4(a, sP + (half * kChunk + i * 16 + (lane & 15)) * kLdP + kb * 16 + (lane >> 4) * 8);
-            mma(o[i][0], a, b[0], b[1]);
-            mma(o[i][1], a, b[2], b[3]);
-          }
-      }
-      // The products with later tokens are zeros, and zero times an infinite or NaN input is NaN: a warp that finds such a result
-      // takes its products again, one token at a time, over the tokens at or before each row.
-      float zero[8] = {};
 #pragma unroll
       for (int i = 0; i < NB; ++i)
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < 2; ++j) o[i][j][0] = o[i][j][1] = o[i][j][2] = o[i][j][3] = 0.f;
+      if (have_state) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) zero[j * 4 + e] = fmaf(o[i][j][e], 0.f, zero[j * 4 + e]);
-      const float all = ((zero[0] + zero[1]) + (zero[2] + zero[3])) + ((zero[4] + zero[5]) + (zero[6] + zero[7]));
-      if (__any_sync(0xffffffffu, all != 0.f)) {
-        from_state();
+        for (int kb = 0; kb < KB; ++kb) {
+          uint32_t hi[2][2], lo[2][2];
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              float u = S[2 * kb + e][2 * j], w = S[2 * kb + e][2 * j + 1];
+              hi[j][e] = take_bf16(u, w);
+              lo[j][e] = take_bf16(u, w);
+            }
+          uint32_t a[NB][4];
+#pragma unroll
+          for (int i = 0; i < NB; ++i) ldsm4(a[i], sC + (i * 16 + (lane & 15)) * LDK + kb * 16 + (lane >> 4) * 8);
+#pragma unroll
+          for (int i = 0; i < NB; ++i) { mma(o[i][0], a[i], hi[0][0], hi[0][1]); mma(o[i][1], a[i], hi[1][0], hi[1][1]); }
+#pragma unroll
+          for (int i = 0; i < NB; ++i) { mma(o[i][0], a[i], lo[0][0], lo[0][1]); mma(o[i][1], a[i], lo[1][0], lo[1][1]); }
+        }
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+          const float f0 = tm.grow[i * 16 + row4], f1 = tm.grow[i * 16 + row4 + 8];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) { o[i][j][0] *= f0; o[i][j][1] *= f0; o[i][j][2] *= f1; o[i][j][3] *= f1; }
+        }
+      }
+      __syncthreads();                               // the products of every warp are in sP
+      // The products with later tokens are zeros, and zero times an infinite or NaN input is NaN: a warp that finds such an input
+      // takes its products one token at a time, over the tokens at or before each row.
+      uint32_t bv[NB][4], marks = 0;
+#pragma unroll
+      for (int kb = 0; kb < NB; ++kb) {
+        ldsm4_t(bv[kb], sV + (kb * 16 + (mi & 1) * 8 + r8) * kLdV + warp * 16 + (mi >> 1) * 8);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) marks |= mark_special(bv[kb][q]);
+      }
+      if (!__any_sync(0xffffffffu, marks & 0x80008000u)) {
+#pragma unroll
+        for (int kb = 0; kb < NB; ++kb)
+#pragma unroll
+          for (int half = 0; half < 2; ++half)
+#pragma unroll
+            for (int i = kb; i < NB; ++i) {
+              uint32_t a[4];
+              ldsm4(a, sP + (half * kChunk + i * 16 + (lane & 15)) * kLdP + kb * 16 + (lane >> 4) * 8);
+              mma(o[i][0], a, bv[kb][0], bv[kb][1]);
+              mma(o[i][1], a, bv[kb][2], bv[kb][3]);
+            }
+      } else {
         for (int t = 0; t < m; ++t) {
           float v[4];
 #pragma unroll
