@@ -111,8 +111,7 @@ def _gotunex_family() -> ModelFamily:
                 n += ff["ff"] if ff["kind"] == "dense" else ff["router"]["top"] * (2 * cfg.width_pad + ff["expert"]["ff"])
             per_tok = max(per_tok, 4 * cfg.width_pad + n)
         state = kv(cfg, 64, torch.bfloat16, False).state_bytes_per_slot
-        latent = [cfg.attention(i) for i in range(len(cfg.layers)) if cfg.is_attention(i)]
-        scratch = max((a.prompt_scratch_bytes(T) for a in latent), default=0) + sum(a.prompt_weight_bytes for a in latent)
+        scratch = max((a.prompt_scratch_bytes(T) for a in (cfg.attention(i) for i in range(len(cfg.layers)) if cfg.is_attention(i))), default=0)
         return T * per_tok * 4 + B * cfg.vocab_size * 4 + B * state + scratch + (256 << 20)
 
     return ModelFamily("gotunex", GotunexConfig, GotunexWeights, GotunexModel, kv, act)
@@ -165,8 +164,7 @@ def _mavidra_family() -> ModelFamily:
                 n = max(n, l["mlp"]["router"]["top"] * (2 * cfg.width_pad + l["mlp"]["expert"]["ff"]))
             per_tok = max(per_tok, 6 * cfg.width_pad + n)
         state = kv(cfg, 64, torch.bfloat16, False).state_bytes_per_slot
-        latent = [cfg.latent(i) for i, l in enumerate(cfg.layers) if l["type"] == LATENT]
-        scratch = max((a.prompt_scratch_bytes(T) for a in latent), default=0) + sum(a.prompt_weight_bytes for a in latent)
+        scratch = max((a.prompt_scratch_bytes(T) for a in (cfg.latent(i) for i, l in enumerate(cfg.layers) if l["type"] == LATENT)), default=0)
         return T * per_tok * 4 + B * cfg.vocab_size * 4 + B * state + scratch + (256 << 20)
 
     return ModelFamily("mavidra", MavidraConfig, MavidraWeights, MavidraModel, kv, act)

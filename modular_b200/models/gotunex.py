@@ -313,7 +313,6 @@ class GotunexModel:
             self.cos_sin[i] = tables[key]
         self.graphs: Optional[DecodeGraphs] = None
         self.forward_calls = 0
-        self.projected_windows = {l.mixer.cfg.window for l in weights.layers if getattr(l.mixer, "projects", False)}
 
     # ------------------------------------------------------------ CUDA graphs of decode steps
     def capture_decode_graphs(self, batch_sizes) -> None:
@@ -359,7 +358,7 @@ class GotunexModel:
         # the tiled GEMM for every step size: the decode-step GEMM measured 2 to 29 % slower per step at these widths
         lin = ops.linear
         one_token = T == q_len.shape[0]
-        projected = prompt_plans(self.projected_windows, T, q_len, kv_len, lengths)
+        projected = prompt_plans({l.mixer.cfg.window for l in w.layers if getattr(l.mixer, "projects", False)}, T, q_len, kv_len, lengths)
         routes = w.router.route(tokens)
         x = torch.empty(T, Wp, dtype=torch.float32, device=dev)
         # what the next seam adds to the stream: the embedding first, then both branches of a layer

@@ -374,7 +374,6 @@ class MavidraModel:
         self.max_experts = max([cfg.router(i).experts for i in self.moe_layers], default=0)
         self.graphs: Optional[DecodeGraphs] = None
         self.forward_calls = 0
-        self.projected_windows = {l.mixer.cfg.window for l in weights.layers if getattr(l.mixer, "projects", False)}
 
     # ------------------------------------------------------------ CUDA graphs of decode steps
     def capture_decode_graphs(self, batch_sizes) -> None:
@@ -417,7 +416,7 @@ class MavidraModel:
         new = lambda rows: torch.empty(rows, Wp, dtype=self.dtype, device=dev)
         seam = lambda x, **kw: sandwich_norm(x, cols=c.hidden_size, eps=c.norm_eps, **kw)
         one_token = T == q_len.shape[0]
-        projected = prompt_plans(self.projected_windows, T, q_len, kv_len, lengths)
+        projected = prompt_plans({l.mixer.cfg.window for l in w.layers if getattr(l.mixer, "projects", False)}, T, q_len, kv_len, lengths)
         plans = {g: tensor_core_plan(g, self.kv.shape[5], self.dtype, self.page_size, q_start, q_len, T, one_token)
                  for g in self.groups}
         counts = torch.zeros(len(self.moe_layers), self.max_experts, dtype=torch.int32, device=dev)

@@ -72,11 +72,6 @@ class LatentAttentionConfig:
         return prompt_scratch_bytes(self.heads, latent_pad(self.kv_rank), T, self.projects)
 
     @property
-    def prompt_weight_bytes(self) -> int:
-        """What a layer keeps for prompts beside its weights: its key projection once more, transposed."""
-        return 2 * self.heads * 128 * latent_pad(self.kv_rank) if self.projects else 0
-
-    @property
     def cache_width(self) -> int:
         return latent_pad(self.kv_rank) + rot_pad(self.rot_dim)
 
@@ -135,11 +130,7 @@ class LatentAttention:
         uv[:, : c.vdim, : c.kv_rank] = t["uv"].view(H, c.vdim, c.kv_rank)
         self.w_uv = put(uv)                                          # [h, vdim, latent]: latent outputs to values
         # prompts project latents up to keys and values where the sizes are those of the kernel
-        # (w_uv is the stack's second half; the stack is made with the weights, before cache pages take what memory is left)
         self.projects = c.projects and self.w_uk.is_cuda and dtype == torch.bfloat16
-        self.w_up = stacked_up(self.w_uk, self.w_uv) if self.projects else None
-        if self.projects:
-            self.w_uv = self.w_up[H * vp:].view(H, vp, Rp)
         self.sink = put(t["sink"], torch.float32) if c.sink else None
         self.w_o = put(pad_to(pad_heads(t["o"].t().contiguous(), H, c.vdim, vp).t(), width_pad, gemm_k(H * vp)))
 
@@ -161,8 +152,8 @@ class LatentAttention:
         if o.shape[1] != width:
             o[:, width:].zero_()
         if plan is not None and self.projects:
-            prompt_attention(plan, q.view(T, H, c.head_width)[:, :, :dp], q_rope, self.w_up, cache, block_table, q_start, q_len, kv_len, o,
-                             c.scale, self.sink, c.window, gate)
+            prompt_attention(plan, q.view(T, H, c.head_width)[:, :, :dp], q_rope, stacked_up(self.w_uk, self.w_uv), cache, block_table, q_start,
+                             q_len, kv_len, o, c.scale, self.sink, c.window, gate)
         else:
             q_lat = torch.empty(T, H * Rp, dtype=x.dtype, device=x.device)
             ops.batched_linear_heads(q, self.w_uk, q_lat, c.head_width, Rp)
@@ -249,8 +240,8 @@ def prompt_plan(T: int, q_len, kv_len, window: int = 0, lengths=None) -> Optiona
 
 
 def stacked_up(w_uk: torch.Tensor, w_uv: torch.Tensor) -> torch.Tensor:
-    """[heads * 128 | heads * 128, latent] from ``w_uk`` [heads, latent, 128] and ``w_uv`` [heads, 128, latent]: a model whose
-    weights may change under it makes it anew for each layer of a step."""
+    """[heads * 128 | heads * 128, latent] from ``w_uk`` [heads, latent, 128] and ``w_uv`` [heads, 128, latent]: scratch of one
+    layer's step, so that it is never older than the weights."""
     h, R = w_uk.shape[:2]
     if w_uk.is_cuda and w_uk.dtype == torch.bfloat16 and R % 64 == 0 and w_uk.shape[2] == 128:
         out = torch.empty(2 * h * 128, R, dtype=w_uk.dtype, device=w_uk.device)
