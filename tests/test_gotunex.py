@@ -167,34 +167,37 @@ def test_latent_attention_mixer(m, device, dtype):
 
 @pytest.mark.gpu
 def test_projected_prompts_follow_weights_that_change_in_place():
-    """Both forms of a prompt read the mixer's weights as they are: after a change they agree as two roundings to bf16 do."""
+    """A step whose latents are projected uses the mixer's weights as they are: bit for bit what a mixer made from the changed ones gives."""
     from modular_b200 import ops
     from modular_b200.nn.latent_attention import prompt_plan
 
     device, dtype, T, page = "cuda:0", torch.bfloat16, 300, 64
     l = latent(heads=3, dim=128, rot_dim=64, vdim=128, kv_rank=128, q_rank=64)
     t, m = weights_for(config((l, None), width=104), seed=1), l["mixer"]
+    t = {k[len("l0.mix."):]: v for k, v in t.items() if k.startswith("l0.mix.")}
     c = LatentAttentionConfig(m["heads"], m["dim"], m["rot_dim"], m["rot"]["dims"], m["vdim"], m["kv_rank"], m["q_rank"], m["scale"],
                               m["rot"]["base"], 1e-5)
-    mix = LatentAttention(c, {k[len("l0.mix."):]: v for k, v in t.items() if k.startswith("l0.mix.")}, 104, device, dtype)
     x = torch.randn(T, 104, generator=torch.Generator().manual_seed(2)).to(device, dtype)
     bt, pages, slots = paged(T, page)
-    cache = torch.zeros(pages, page, c.cache_width, dtype=dtype, device=device)
     cs = cos_sin_table(c.rot_dims, T, c.rope_base, None, device)
     n = i32(T).to(device)
     plan = prompt_plan(T, n, n)
-    assert mix.projects and plan is not None
 
-    def step(plan):
+    def step(mix):
+        cache = torch.zeros(pages, page, c.cache_width, dtype=dtype, device=device)
         return mix(x, ops.linear, cache, cs, torch.arange(T, dtype=torch.int32, device=device), slots.to(device), bt.to(device),
                    i32(0).to(device), n, n, False, plan)
 
-    before = step(plan)
-    assert rel(before, step(None).cpu()) < 2e-2
-    mix.w_uk.mul_(-4.0)
+    mix = LatentAttention(c, t, 104, device, dtype)
+    assert mix.projects and plan is not None
+    before = step(mix)
+    mix.w_uk.mul_(-4.0)                 # powers of two: the same values as from changed tensors
+    after = step(mix)
+    fresh = dict(t, uk=t["uk"] * -4.0)
+    assert torch.equal(after, step(LatentAttention(c, fresh, 104, device, dtype))) and not torch.equal(after, before)
     mix.w_uv.mul_(0.5)
-    after = step(plan)
-    assert rel(after, step(None).cpu()) < 2e-2 and rel(after, before.cpu()) > 0.1
+    fresh["uv"] = t["uv"] * 0.5
+    assert torch.equal(step(mix), step(LatentAttention(c, fresh, 104, device, dtype)))
 
 
 @pytest.mark.parametrize("device,dtype", RUNS)
