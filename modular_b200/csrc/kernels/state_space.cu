@@ -33,6 +33,9 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cas
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
+// A rate of minus infinity (a decay of zero) as the lowest finite one: rows past a sequence's end take steps of zero, and a product of the
+// two would be NaN.
+__device__ __forceinline__ float finite_rate(float a) { return a < -3.402823466e38f ? -3.402823466e38f : a; }
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -237,7 +240,7 @@ __global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(const __nv
   float* st = ssm_state + (static_cast<size_t>(slot >= 0 ? slot : 0) * D + (live ? d : 0)) * N + q * NS;
 #pragma unroll
   for (int i = 0; i < NS; ++i) {
-    a2[i] = live ? A[static_cast<size_t>(d) * N + q * NS + i] * kLog2e : 0.f;
+    a2[i] = live ? finite_rate(A[static_cast<size_t>(d) * N + q * NS + i] * kLog2e) : 0.f;
     h[i] = resume ? st[i] : 0.f;
   }
   const float dsk = (live && Dskip) ? Dskip[d] : 0.f;
@@ -551,7 +554,7 @@ __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_ker
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   // warp 0 makes the step sizes and their sums, two tokens per lane; the raw values are read one chunk earlier
-  const float a2 = p.A[h] * kLog2e, dtb = p.dt_bias ? p.dt_bias[h] : 0.f;
+  const float a2 = finite_rate(p.A[h] * kLog2e), dtb = p.dt_bias ? p.dt_bias[h] : 0.f;
   float raw[2];
   auto read_dt = [&](int c0) {
 #pragma unroll
@@ -565,6 +568,7 @@ __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_ker
       if (p.dt_softplus) dt[e] = softplus(dt[e]);
       if (c0 + 2 * lane + e >= n) dt[e] = 0.f;
       l[e] = dt[e] * a2;
+      if (l[e] < -1e6f) l[e] = -1e6f;                // zero either way, and the sums stay finite
     }
     // sums up to this pair as a float and what its rounding left, and from it (the large powers are the short sums)
     float rest, hi = two_sum(l[0], l[1], rest), down = hi;

@@ -258,3 +258,25 @@ def test_ssd_decays_of_many_octaves():
     y = ss.ssd_scan_varlen(x, dt, A, B, C, None, None, _cu([T], dev), dt_softplus=False)
     want = ss.ssd_scan_reference(x.cpu().float(), dt.cpu(), A.cpu(), B.cpu(), C.cpu(), None, None, _cu([T]), dt_softplus=False)
     assert _rel(y.cpu(), want) < 2 ** -8                 # one rounding to bf16
+
+
+@pytest.mark.gpu
+def test_decays_of_zero():
+    """Rates so large that a decay is zero (A = -exp(A_log) of minus infinity, sums beyond the largest float): each token alone is left."""
+    torch.manual_seed(12)
+    dev, T, (H, P, N) = "cuda", 133, (3, 32, 16)
+    bf = lambda *s, k=1.0: (torch.randn(*s, device=dev) * k).to(torch.bfloat16)
+    A = torch.tensor([-float("inf"), -3e38, -0.5], device=dev)
+    x, dt, B, C, st = bf(T, H, P), bf(T, H, k=0.3), bf(T, 1, N, k=0.3), bf(T, 1, N, k=0.3), torch.randn(1, H, P, N, device=dev)
+    ref, idx, init = st.clone().cpu(), torch.zeros(1, dtype=torch.int32, device=dev), torch.ones(1, dtype=torch.int32, device=dev)
+    y = ss.ssd_scan_varlen(x, dt, A, B, C, None, None, _cu([T], dev), st, idx, init, True)
+    want = ss.ssd_scan_reference(x.cpu().float(), dt.cpu(), A.cpu(), B.cpu(), C.cpu(), None, None, _cu([T]), ref, idx.cpu(), init.cpu(), True)
+    for h in range(H):
+        assert _rel(y[:, h].cpu(), want[:, h]) < 2 ** -8 and _rel(st[0, h].cpu(), ref[0, h]) < 1e-5, h
+    D = 40
+    u, delta, b, c = bf(T, D), bf(T, D, k=0.3), bf(T, N, k=0.3), bf(T, N, k=0.3)
+    a = -torch.rand(D, N, device=dev) - 0.1
+    a[::3], a[1, 2] = -float("inf"), -3e38
+    got = ss.selective_scan_varlen(u, delta, a, b, c, None, None, None, _cu([T], dev))
+    want = ss.selective_scan_reference(u.cpu().float(), delta.cpu(), a.cpu(), b.cpu(), c.cpu(), None, None, None, _cu([T]))
+    assert _rel(got.cpu(), want) < 2 ** -8
