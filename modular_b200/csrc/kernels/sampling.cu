@@ -448,25 +448,29 @@ sample_kernel(const float* __restrict__ logits, int64_t* __restrict__ out, int v
 
 // ---- a row spread over a cluster of CTAs
 // The 16 c warps of a cluster each own a contiguous share of the row and read it two or three times (L2 hits after the
-// first). Greedy and plain-temperature rows are one pass. Rows with a filter take the maximum, then a histogram of
-// mx - x / T in shared memory (bins of 1/32, counts and, for a nucleus over the whole row, softmax mass; bins that
-// narrow spread the bulk of the row over hundreds of counters, so the atomics hardly meet). If the bins that provably
-// hold the kept set have at most kList elements, those go to the first CTA, which ranks them by counting and reads both
-// cut-offs off the sorted values. Otherwise the cut-off is found exactly by refining the bin it lies in, 2048 buckets
-// of keys at a time (a few more passes), and the draw is a prefix sum over the warps' shares.
+// first). Greedy and plain-temperature rows are one pass. Top-k and min-p rows take the maximum and then go straight to the
+// elements of the bins of mx - x / T (1/32 wide) that can hold the kept set; those (at most kList) go to the first CTA, which
+// ranks them by counting and reads both cut-offs off the sorted values. A nucleus over the whole row takes the maximum, then a
+// histogram of the bins' softmax mass in shared memory (bins that narrow spread the bulk of the row over hundreds of counters,
+// so the atomics hardly meet), then the weight above the bin in which it ends and that bin's elements, among which the first
+// CTA finds the cut-off by their keys. What does not fit (more candidates than the lists hold, cut-offs in the open last bin, a
+// nucleus within a long top-k) is found exactly by refining the bin it lies in, 1024 buckets of keys at a time (a few more
+// passes), and the draw is a prefix sum over the warps' shares.
 // Masses are integers, so sums do not depend on their order: 42 fractional bits where few weights meet in registers, and
 // per bin the weights relative to the bin's upper edge as 26-bit numbers in two halves, because 32-bit atomics on shared
 // memory are native and 64-bit ones are not (with those 64 nucleus rows took 122 us, with these 101).
-// (One or four rows with a nucleus over the whole row and nothing else, of a spread of 3.75: 45 us when unit bins were counted in registers,
-// 49 so; counts alone here and masses only where a long nucleus is cut: 55, and 78 for the mixed 64 rows below.)
-// 64 rows of 128256 logits, a quarter of the rows with a nucleus of thousands of tokens: 364 us when such rows (and
-// confident ones, whose k-th token lies far below the first) were left to sample_kernel, which walks a row with one
-// CTA, 58 to 66 us so (127 us before where all kept sets were short); one row 28 us, 64 greedy rows 11 us.
+// What bounds it: the chain of a nucleus row. Of its 51 thousand cycles (64 rows, two CTAs an SM) the histogram takes 20, nine
+// cycles an atomic and SM; the passes over the row 6 (from memory) and 9; the rest are barriers of the cluster and round trips
+// between its CTAs, each about one.
+// 64 rows of 128256 logits with top-k, top-p and min-p mixed: 31 us (64 when every row was counted, elements in the order of a
+// long list were ranked one by one, and a bin refined over the cluster), 20 rows 25 us (54), one row 19 us (28); 64 greedy
+// rows 11 us.
 constexpr int kClu = 8;          // largest cluster; the launcher picks 8, 4, 2 or 1 CTAs per row from the batch size
 constexpr int kCluThreads = 512, kCluWarps = kCluThreads / 32;
-constexpr int kBins = 2048, kOwn = kBins / kCluThreads;
-static_assert(kOwn == 4, "a thread reads its bins as one vector");
+constexpr int kBins = 1024, kOwn = kBins / kCluThreads;   // 32 units: what lies below weighs nothing
+static_assert(kOwn == 2, "a thread reads its bins as one vector");
 constexpr int kList = kCluThreads;
+constexpr int kBinList = 2048;   // halves of 2^11 weights below 2^42 add up below 2^32
 constexpr float kBinsPerUnit = 32.f;
 constexpr int kMaxShare = 1 << 18;   // elements per CTA: the halves of 2^18 weights of one bin still add up below 2^32
 typedef unsigned long long u64;
@@ -479,6 +483,9 @@ struct ClusterSmem {
   u64 sp[kList];                // by rank: inclusive prefix of the masses
   float ox[kList];              // by index
   int oi[kList];
+  float bx[kBinList];           // elements of the bin in which a nucleus ends and their indices (first CTA only)
+  int bi[kBinList];
+  uint32_t kept_hi[kClu * kCluWarps], kept_lo[kClu * kCluWarps];   // their weights by owning warp, in two halves
   ArgMax cmax;                  // maximum of this CTA's share
   u64 wsum[kCluWarps];          // kept mass of every warp's share
   u64 all[kClu * kCluWarps];
@@ -500,14 +507,33 @@ __device__ __forceinline__ void load4(const float* __restrict__ row, int i, int 
 // 2^-42 is the smallest weight: a token about 29 units below the maximum is not drawn (uniform01 has 24 bits, so that no draw
 // could tell it from one of weight 1e-38). NaN (an infinite maximum minus itself, a NaN logit) weighs nothing.
 __device__ __forceinline__ u64 weight_of(float below) { return __float2ull_rn(fmaxf(__expf(-below) * 4398046511104.f, 0.f)); }
-__device__ __forceinline__ int bin_of(float below) {       // NaN goes to the last bin
-  const float b = below * kBinsPerUnit;
+// The bin of an element `below` >= 0 under the maximum; NaN goes to the last bin. Rounding down while adding 2^23 leaves the
+// integer in the low bits: conversions run on the unit of the exponentials, 16 lanes a cycle, and four of those per element
+// were what a counting pass took its time for (31 cycles per 32 elements and scheduler).
+__device__ __forceinline__ int bin_of(float below) {
+  return __float_as_int(__fadd_rd(fminf(below * kBinsPerUnit, static_cast<float>(kBins - 1)), 8388608.f)) - 0x4b000000;
+}
+// the lowest bin that min-p reaches (negative: none but the maximum's)
+__device__ __forceinline__ int min_p_bin(float mp) {
+  const float b = (0.01f - __logf(mp)) * kBinsPerUnit;
   return b < static_cast<float>(kBins - 1) ? static_cast<int>(b) : kBins - 1;
 }
-__device__ __forceinline__ uint4 ld_cluster_v4(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared::cluster.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+// e^-y as a 26-bit fraction. Elements of one bin have y below 1/32, where four terms of the series are within 2^-25 and the
+// sum's own bits are the fraction.
+__device__ __forceinline__ uint32_t fraction26(float y) {
+  if (y < 0.0625f) {
+    const float e = fmaf(-y, fmaf(-y, fmaf(-y, fmaf(-y, 1.f / 24.f, 1.f / 6.f), 0.5f), 1.f), 1.f);
+    return e < 1.f ? ((__float_as_uint(e) & 0x7fffffu) | 0x800000u) << 2 : 1u << 26;
+  }
+  return __float2uint_rn(__expf(-y) * 67108864.f);
+}
+__device__ __forceinline__ uint2 ld_cluster_v2(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared::cluster.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
   return v;
+}
+__device__ __forceinline__ void st_cluster_u64(uint32_t addr, u64 v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
 }
 __device__ __forceinline__ u64 ld_cluster_u64(uint32_t addr) {
   u64 v;
@@ -570,7 +596,21 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
   // f(x / T, index) for every element of this warp's share, sixteen loads in flight per lane (-0 as 0: equal values are
   // one tie, whatever their sign bit)
   auto visit = [&](auto&& f) {
-    for (int i0 = beg; i0 < end; i0 += 512) {
+    int i0 = beg;
+    for (; vec && i0 + 512 <= end; i0 += 512) {
+      float4 q[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) q[u] = *reinterpret_cast<const float4*>(row + i0 + u * 128 + 4 * lane);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + u * 128 + 4 * lane;
+        f(__fadd_rn(__fmul_rn(q[u].x, invT), 0.f), i);
+        f(__fadd_rn(__fmul_rn(q[u].y, invT), 0.f), i + 1);
+        f(__fadd_rn(__fmul_rn(q[u].z, invT), 0.f), i + 2);
+        f(__fadd_rn(__fmul_rn(q[u].w, invT), 0.f), i + 3);
+      }
+    }
+    for (; i0 < end; i0 += 512) {
       float xv[4][4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) load4(row, i0 + u * 128 + 4 * lane, end, vec, xv[u]);
@@ -584,6 +624,15 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
     }
   };
 
+  auto clear_bins = [&](int want) {
+    for (int i = 4 * tid; i < kBins; i += 4 * kCluThreads) {
+      const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+      if (want & 1) *reinterpret_cast<uint4*>(&sm->cnt[i]) = z;
+      if (want & 2) { *reinterpret_cast<uint4*>(&sm->hi[i]) = z; *reinterpret_cast<uint4*>(&sm->lo[i]) = z; }
+    }
+  };
+  if (!greedy && !plain) clear_bins(3);
+
   // 1. maximum of x / T (greedy: of x; no filter: of x / T + Gumbel noise, which is the draw)
   ArgMax a{-FLT_MAX, 0x7fffffff};
   if (plain) {
@@ -591,17 +640,26 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
   } else {
     visit([&](float x, int i) { a = amax2(a, ArgMax{x, i}); });
   }
+  const float lane_max = a.v;
   a = block_argmax(a, sh_am);
-  if (tid == 0) sm->cmax = a;
+  if (tid == 0) { sm->cmax = a; sm->fill = 0; }
   cluster_sync_all();
   {
+    // lane r asks CTA r: one round trip, where a loop over the CTAs would take one each
     ArgMax g{-FLT_MAX, 0x7fffffff};
-    for (uint32_t r = 0; r < nclu; ++r) {
+    if (lane < static_cast<int>(nclu)) {
+      g.v = __uint_as_float(ld_cluster_u32(mapa_shared(&sm->cmax.v, lane)));
+      g.i = static_cast<int>(ld_cluster_u32(mapa_shared(&sm->cmax.i, lane)));
+    }
+#pragma unroll
+    for (int o = 1; o < kClu; o <<= 1) {
       ArgMax b;
-      b.v = __uint_as_float(ld_cluster_u32(mapa_shared(&sm->cmax.v, r)));
-      b.i = static_cast<int>(ld_cluster_u32(mapa_shared(&sm->cmax.i, r)));
+      b.v = __shfl_xor_sync(0xffffffffu, g.v, o);
+      b.i = __shfl_xor_sync(0xffffffffu, g.i, o);
       g = amax2(g, b);
     }
+    g.v = __shfl_sync(0xffffffffu, g.v, 0);
+    g.i = __shfl_sync(0xffffffffu, g.i, 0);
     a = g;
   }
   if (greedy || plain) {           // the same decision in all CTAs of the cluster
@@ -613,43 +671,54 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
   const uint32_t hi_key = fkey(mx);
   const uint32_t km = use_m ? fkey(mx + __logf(mp)) : 0u;
 
-  // Histogram over the cluster: place(x, below, key) gives an element's bin or -1. This thread's kOwn bins come back as
-  // counts (want & 1) and masses (want & 2).
-  // `all_in`: the unit bin that holds every element placed, or -1 when the bins are the unit bins themselves.
-  auto histogram = [&](int want, int all_in, auto&& place, u64 (&c)[kOwn], u64 (&m)[kOwn]) {
-    cluster_sync_all();            // peers are done reading the bins of the pass before
-    for (int i = tid; i < kBins; i += kCluThreads) { sm->cnt[i] = 0; sm->hi[i] = 0; sm->lo[i] = 0; }
-    __syncthreads();
+  // Weights relative to the edge of unit bin b (or of bin `all_in`, where every element placed lies), 26 bits, in units of
+  // 2^-42 under the maximum: 2^16 e^(-b / 32). One exponential per thread covers its bins.
+  constexpr double kStep[kOwn] = {1.0, 0.9692332344763441};                  // e^(-j / 32)
+  auto edge = [](int b) { return 65536.0 * exp(-b / static_cast<double>(kBinsPerUnit)); };
+  auto count_in = [&](int want, int b, int rel, float below) {
+    if (want & 1) atomicAdd(&sm->cnt[b], 1u);
+    if (want & 2) {
+      const uint32_t q = fraction26(below - rel / kBinsPerUnit);
+      atomicAdd(&sm->hi[b], q >> 13);
+      atomicAdd(&sm->lo[b], q & 0x1fffu);
+    }
+  };
+  // This thread's kOwn bins, added up over CTAs [r0, r1), as counts (want & 1) and masses (want & 2).
+  auto add_bins = [&](int want, bool scaled, double unit, uint32_t r0, uint32_t r1, u64 (&c)[kOwn], u64 (&m)[kOwn]) {
+#pragma unroll
+    for (int j = 0; j < kOwn; ++j) c[j] = m[j] = 0;
+#pragma unroll 4
+    for (uint32_t r = r0; r < r1; ++r) {
+      if (want & 1) {
+        const uint2 v = ld_cluster_v2(mapa_shared(&sm->cnt[tid * kOwn], r));
+        c[0] += v.x; c[1] += v.y;
+      }
+      if (want & 2) {
+        const uint2 h = ld_cluster_v2(mapa_shared(&sm->hi[tid * kOwn], r)), l = ld_cluster_v2(mapa_shared(&sm->lo[tid * kOwn], r));
+        m[0] += (static_cast<u64>(h.x) << 13) + l.x; m[1] += (static_cast<u64>(h.y) << 13) + l.y;
+      }
+    }
+    if (want & 2) {
+#pragma unroll
+      for (int j = 0; j < kOwn; ++j)
+        if (m[j]) m[j] = static_cast<u64>(static_cast<double>(m[j]) * (scaled ? unit * kStep[j] : unit));
+    }
+  };
+  // Histogram over the cluster: place(x, below, key) gives an element's bin or -1; `all_in` is the unit bin that holds every
+  // element placed, or -1 when the bins are the unit bins themselves. `fresh`: the bins are still those cleared at the start.
+  auto histogram = [&](int want, int all_in, double unit, bool fresh, auto&& place, u64 (&c)[kOwn], u64 (&m)[kOwn]) {
+    if (!fresh) {
+      cluster_sync_all();          // peers are done reading the bins of the pass before
+      clear_bins(want);
+      __syncthreads();
+    }
     visit([&](float x, int) {
       const float below = __fsub_rn(mx, x);
       const int b = place(below, fkey(x));
-      if (b < 0) return;
-      if (want & 1) atomicAdd(&sm->cnt[b], 1u);
-      if (want & 2) {
-        const uint32_t q = __float2uint_rn(__expf((all_in < 0 ? b : all_in) / kBinsPerUnit - below) * 67108864.f);
-        atomicAdd(&sm->hi[b], q >> 13);
-        atomicAdd(&sm->lo[b], q & 0x1fffu);
-      }
+      if (b >= 0) count_in(want, b, all_in < 0 ? b : all_in, below);
     });
     cluster_sync_all();
-#pragma unroll
-    for (int j = 0; j < kOwn; ++j) c[j] = m[j] = 0;
-    for (uint32_t r = 0; r < nclu; ++r) {
-      if (want & 1) {
-        const uint4 v = ld_cluster_v4(mapa_shared(&sm->cnt[tid * kOwn], r));
-        c[0] += v.x; c[1] += v.y; c[2] += v.z; c[3] += v.w;
-      }
-      if (want & 2) {
-        const uint4 h = ld_cluster_v4(mapa_shared(&sm->hi[tid * kOwn], r)), l = ld_cluster_v4(mapa_shared(&sm->lo[tid * kOwn], r));
-        m[0] += (static_cast<u64>(h.x) << 13) + l.x; m[1] += (static_cast<u64>(h.y) << 13) + l.y;
-        m[2] += (static_cast<u64>(h.z) << 13) + l.z; m[3] += (static_cast<u64>(h.w) << 13) + l.w;
-      }
-    }
-    if (want & 2) {                // from 26 bits under the bin's edge to 42 under the maximum
-#pragma unroll
-      for (int j = 0; j < kOwn; ++j)
-        if (m[j]) m[j] = static_cast<u64>(static_cast<double>(m[j]) * (65536.0 * exp(-(all_in < 0 ? tid * kOwn + j : all_in) / static_cast<double>(kBinsPerUnit))));
-    }
+    add_bins(want, all_in < 0, unit, 0, nclu, c, m);
   };
   // the first bin where the running sum of v reaches `target` (-1: none) and the sum before it
   auto cross = [&](const u64 (&v)[kOwn], u64 target, int& bin, u64& above) {
@@ -675,53 +744,217 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
     return r > whole ? whole : r;
   };
 
-  // 2. bins under the maximum
+  // 2. The bins that hold the kept set. A top-k set lies in the bins that reach k when every lane of the cluster counts only its
+  // maximum, and what min-p keeps is known from the maximum, so such rows go straight to the elements of those bins (2a): a
+  // pass less than counting the row first, and no atomics for what cannot be kept (20 of 60 thousand cycles). Up to half a list:
+  // the bins that the lanes' maxima reach hold more than k elements, and a list that runs over costs its pass. Where they are
+  // too many, and for a nucleus over the whole row, the row is counted (2b).
   u64 c[kOwn], m[kOwn], z_all = 0;
   const bool nucleus = use_p && !use_k && !use_m;
-  histogram(nucleus ? 3 : 1, -1, [](float below, uint32_t) { return bin_of(below); }, c, m);
-  int last = -1, kbin = -1;
+  int last = -1, kbin = -1, n = 0x7fffffff;
   u64 kabove = 0, pabove = 0, ptarget = 0;
-  if (use_k) { cross(c, static_cast<u64>(k), kbin, kabove); last = kbin; }
-  if (use_m) last = max(last, bin_of(-__logf(mp) + 0.01f));
-  if (nucleus) {
-    block_before(m[0] + m[1] + m[2] + m[3], sm->red, z_all);
-    ptarget = portion(tp, z_all);
-    cross(m, ptarget, last, pabove);
-  }
-  int n = 0x7fffffff;
-  {
-    u64 sum = c[0] + c[1] + c[2] + c[3], total, run = block_before(sum, sm->red, total);
-#pragma unroll
-    for (int j = 0; j < kOwn; ++j) {
-      run += c[j];
-      if (tid * kOwn + j == last) sm->n = run > 0x7fffffffu ? 0x7fffffff : static_cast<int>(run);
+  bool listed = false;
+  // a bound under every element of bins 0 .. b (none for the last bin, which is open): most elements need no look at their bin
+  auto under = [&](int b) { return b >= kBins - 1 ? -INFINITY : mx - (b + 1) / kBinsPerUnit - fmaxf(fabsf(mx), 64.f) * 2e-6f; };
+  // an element of the list in the first CTA
+  auto push = [&](float* xs, int* is, uint32_t pos, float x, int i) {
+    st_cluster_u32(mapa_shared(xs, 0) + 4u * pos, __float_as_uint(x == x ? x : -INFINITY));      // ranks need an order: NaN is the lowest
+    st_cluster_u32(mapa_shared(is, 0) + 4u * pos, static_cast<uint32_t>(i));
+  };
+  if (!nucleus && k <= kList / 2) {
+    if (use_k) {
+      atomicAdd(&sm->cnt[bin_of(__fsub_rn(mx, lane_max))], 1u);
+      cluster_sync_all();
+      add_bins(1, false, 0.0, 0, nclu, c, m);
+      cross(c, static_cast<u64>(k), last, kabove);
     }
-    __syncthreads();
-    if (last >= 0) n = sm->n;
+    if (use_m && (last >= 0 || !use_k)) last = max(last, min_p_bin(mp));
+    if (last >= 0) {
+      const float least = under(last);
+      visit([&](float x, int i) {
+        if (x < least || bin_of(__fsub_rn(mx, x)) > last) return;
+        const uint32_t pos = atomicAdd(&sm->fill, 1u);
+        if (pos < kList) { sm->sx[pos] = x; sm->oi[pos] = i; }
+      });
+      cluster_sync_all();
+      const uint32_t there = lane < static_cast<int>(nclu) ? ld_cluster_u32(mapa_shared(&sm->fill, lane)) : 0u;
+      const uint32_t first = __reduce_add_sync(0xffffffffu, lane < static_cast<int>(rank) ? there : 0u);
+      const uint32_t all = __reduce_add_sync(0xffffffffu, there);
+      if (all <= kList && static_cast<int>(all) >= (use_k ? k : 1)) {
+        listed = true;
+        n = static_cast<int>(all);
+        if (tid < static_cast<int>(sm->fill)) push(sm->lx, sm->li, first + tid, sm->sx[tid], sm->oi[tid]);
+        cluster_sync_all();
+        if (rank != 0) return;
+      }
+    }
+  }
+  if (!listed) {
+    // 2b. bins under the maximum
+    const double unit = nucleus ? edge(tid * kOwn) : 0.0;
+    const bool fresh = nucleus || k > kList / 2;
+    // (the last bin's elements have no weight)
+    if (nucleus) histogram(2, -1, unit, fresh, [](float below, uint32_t) { const int b = bin_of(below); return b < kBins - 1 ? b : -1; }, c, m);
+    else histogram(1, -1, unit, fresh, [](float below, uint32_t) { return bin_of(below); }, c, m);
+    last = -1;
+    if (nucleus) {
+      block_before(m[0] + m[1], sm->red, z_all);
+      ptarget = portion(tp, z_all);
+      cross(m, ptarget, last, pabove);
+    } else {
+      if (use_k) { cross(c, static_cast<u64>(k), kbin, kabove); last = kbin; }
+      if (use_m) last = max(last, min_p_bin(mp));
+      u64 total, run = block_before(c[0] + c[1], sm->red, total);
+#pragma unroll
+      for (int j = 0; j < kOwn; ++j) {
+        run += c[j];
+        if (tid * kOwn + j == last) sm->n = run > 0x7fffffffu ? 0x7fffffff : static_cast<int>(run);
+      }
+      __syncthreads();
+      if (last >= 0) n = sm->n;
+    }
+    uint32_t all = 0x7fffffffu;
+    if (nucleus && last >= 0 && last < kBins - 1) {
+      // One more pass takes the weight of the bins above the last one, warp by warp, and the last bin's elements, which go to
+      // the first CTA: it finds the cut-off among them and draws.
+      const float least = under(last);
+      u64 mass = 0;
+      // a lane marks its elements that can be kept, then takes them one by one: a few of sixteen, in other places in every lane
+      auto take = [&](float x, int i) {
+        const float below = __fsub_rn(mx, x);
+        const int b = bin_of(below);
+        if (b > last) return;
+        if (b < last) { mass += weight_of(below); return; }
+        const uint32_t pos = atomicAdd(&sm->fill, 1u);
+        if (pos < kBinList) { sm->bx[pos] = x; sm->bi[pos] = i; }
+      };
+      for (int i0 = beg; i0 < end; i0 += 512) {
+        float xv[4][4];
+        uint32_t mark = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) load4(row, i0 + u * 128 + 4 * lane, end, vec, xv[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (__fmul_rn(xv[u][e], invT) >= least) mark |= 1u << (4 * u + e);
+        while (mark) {
+          const int j = __ffs(mark) - 1, i = i0 + (j >> 2) * 128 + 4 * lane + (j & 3);
+          mark &= mark - 1;
+          if (i < end) take(__fadd_rn(__fmul_rn(row[i], invT), 0.f), i);
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, o);
+      if (lane == 0) st_cluster_u64(mapa_shared(&sm->all[gw], 0), mass);
+      cluster_sync_all();
+      const uint32_t there = lane < static_cast<int>(nclu) ? ld_cluster_u32(mapa_shared(&sm->fill, lane)) : 0u;
+      const uint32_t first = __reduce_add_sync(0xffffffffu, lane < static_cast<int>(rank) ? there : 0u);
+      all = __reduce_add_sync(0xffffffffu, there);
+      if (all < kBinList && rank != 0)                 // the first CTA's own elements lie at the front already
+        for (uint32_t j = tid; j < sm->fill; j += kCluThreads) push(sm->bx, sm->bi, first + j, sm->bx[j], sm->bi[j]);
+    }
+    if (all < kBinList) {
+      cluster_sync_all();
+      if (rank != 0) return;
+      const int in_last = static_cast<int>(all);
+      const float slack = fmaxf(fabsf(mx), 64.f) * 2e-6f;    // rounding of mx - x
+      uint32_t khi = min(hi_key, fkey(mx - last / kBinsPerUnit + slack));
+      uint32_t klo = min(fkey(mx - (last + 1) / kBinsPerUnit - slack), khi);
+      uint32_t from = 0u, to = 0xffffffffu, thr = klo;
+      const double at = edge(last);
+      if (tid < kClu * kCluWarps) { sm->kept_hi[tid] = 0; sm->kept_lo[tid] = 0; }
+      for (;;) {
+        const uint32_t range = khi - klo;
+        const int sh = range < static_cast<uint32_t>(kBins) ? 0 : 22 - __clz(range);
+        clear_bins(2);
+        __syncthreads();
+        for (int j = tid; j < in_last; j += kCluThreads) {
+          const float x = sm->bx[j];
+          const uint32_t key = fkey(x);
+          if (key >= from && key <= to) count_in(2, static_cast<int>((khi - min(max(key, klo), khi)) >> sh), last, __fsub_rn(mx, x));
+        }
+        __syncthreads();
+        add_bins(2, false, at, 0, 1, c, m);
+        int b;
+        u64 before;
+        cross(m, ptarget - pabove, b, before);
+        thr = klo;
+        if (b < 0) break;
+        pabove += before;
+        const uint32_t top = khi - (static_cast<uint32_t>(b) << sh);
+        thr = top;
+        if (sh == 0) break;
+        const uint32_t width = (1u << sh) - 1;
+        klo = top - klo < width ? klo : top - width;
+        khi = top;
+        from = klo;
+        to = khi;
+      }
+      // inverse-CDF draw in index order: the shares' masses, then the share that holds the target
+      for (int j = tid; j < in_last; j += kCluThreads) {
+        if (fkey(sm->bx[j]) < thr) continue;
+        const u64 w = weight_of(__fsub_rn(mx, sm->bx[j]));
+        atomicAdd(&sm->kept_hi[sm->bi[j] / seg], static_cast<uint32_t>(w >> 21));
+        atomicAdd(&sm->kept_lo[sm->bi[j] / seg], static_cast<uint32_t>(w) & 0x1fffffu);
+      }
+      __syncthreads();
+      u64 Z;
+      const u64 mine = tid < nwarps ? sm->all[tid] + (static_cast<u64>(sm->kept_hi[tid]) << 21) + sm->kept_lo[tid] : 0;
+      const u64 base = block_before(mine, sm->red, Z);
+      if (Z == 0) {
+        if (tid == 0) out[rowi] = a.i;
+        return;
+      }
+      const u64 target = portion(uniform01(seed, step, 0xffffffffull), Z);
+      if (base < target && base + mine >= target) { sm->bin = tid; sm->above = base; }
+      __syncthreads();
+      const int s0 = sm->bin * seg, s1 = vocab - s0 < seg ? vocab : s0 + seg;
+      u64 run = sm->above;
+      for (int i0 = s0; i0 < s1 && run < target; i0 += 4 * kCluThreads) {
+        float xv[4];
+        load4(row, i0 + 4 * tid, s1, vec, xv);
+        u64 w[4], four = 0, total;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float x = __fadd_rn(__fmul_rn(xv[e], invT), 0.f);
+          w[e] = (i0 + 4 * tid + e < s1 && fkey(x) >= thr) ? weight_of(__fsub_rn(mx, x)) : 0;
+          four += w[e];
+        }
+        u64 cum = run + block_before(four, sm->red, total);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (w[e] > 0 && cum < target && cum + w[e] >= target) out[rowi] = i0 + 4 * tid + e;
+          cum += w[e];
+        }
+        run += total;
+      }
+      return;
+    } else if (n <= kList) {
+      // elements of the bins up to the last into a list of the first CTA, in any order within a CTA's part of it. The positions
+      // come from a local counter: one shared by the cluster is a queue of remote atomics (512 of them took 25 us).
+      u64 part = 0, here;
+#pragma unroll
+      for (int j = 0; j < kOwn; ++j)
+        if (tid * kOwn + j <= last) part += sm->cnt[tid * kOwn + j];
+      block_before(part, sm->red, here);
+      if (tid == 0) { sm->wsum[0] = here; sm->fill = 0; }
+      cluster_sync_all();
+      const uint32_t first = __reduce_add_sync(0xffffffffu, lane < static_cast<int>(rank) ? static_cast<uint32_t>(ld_cluster_u64(mapa_shared(&sm->wsum[0], lane))) : 0u);
+      const float least = under(last);
+      visit([&](float x, int i) {
+        if (x < least || bin_of(__fsub_rn(mx, x)) > last) return;
+        const uint32_t pos = first + atomicAdd(&sm->fill, 1u);
+        if (pos < kList) push(sm->lx, sm->li, pos, x, i);      // always: the same elements were counted
+      });
+      cluster_sync_all();
+      if (rank != 0) return;
+      listed = true;
+    }
   }
 
-  if (n <= kList) {
-    // 3a. candidates into the first CTA's list, in any order within a CTA's part of it. The positions come from a local
-    // counter: one shared by the cluster is a queue of remote atomics (512 of them took 25 us).
-    u64 part = 0, here;
-#pragma unroll
-    for (int j = 0; j < kOwn; ++j)
-      if (tid * kOwn + j <= last) part += sm->cnt[tid * kOwn + j];
-    block_before(part, sm->red, here);
-    if (tid == 0) { sm->wsum[0] = here; sm->fill = 0; }
-    cluster_sync_all();
-    uint32_t first = 0;
-    for (uint32_t r = 0; r < rank; ++r) first += static_cast<uint32_t>(ld_cluster_u64(mapa_shared(&sm->wsum[0], r)));
-    const uint32_t lx = mapa_shared(&sm->lx[0], 0), li = mapa_shared(&sm->li[0], 0);
-    visit([&](float x, int i) {
-      if (bin_of(__fsub_rn(mx, x)) > last) return;
-      const uint32_t pos = first + atomicAdd(&sm->fill, 1u);
-      if (pos >= kList) return;    // cannot happen: the same elements were counted
-      st_cluster_u32(lx + 4u * pos, __float_as_uint(x == x ? x : -INFINITY));      // ranks need an order: NaN is the lowest
-      st_cluster_u32(li + 4u * pos, static_cast<uint32_t>(i));
-    });
-    cluster_sync_all();
-    if (rank != 0) return;
+  if (listed) {
+    // 3a. the first CTA alone
     // one candidate per thread: its rank by value and by index, counted directly
     const int n4 = (n + 3) & ~3;
     if (tid >= n && tid < n4) { sm->lx[tid] = -INFINITY; sm->li[tid] = 0x7fffffff; }   // behind every candidate, masked ones too
@@ -781,10 +1014,11 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
     uint32_t klo = bin == kBins - 1 ? 0u : fkey(mx - (bin + 1) / kBinsPerUnit - slack);
     klo = min(max(klo, least), khi);
     uint32_t from = 0u, to = 0xffffffffu;
+    const double at = want & 2 ? edge(bin) : 0.0;
     for (;;) {
       const uint32_t range = khi - klo;
-      const int sh = range < static_cast<uint32_t>(kBins) ? 0 : 21 - __clz(range);
-      histogram(want, bin, [&](float below, uint32_t key) {
+      const int sh = range < static_cast<uint32_t>(kBins) ? 0 : 22 - __clz(range);
+      histogram(want, bin, at, false, [&](float below, uint32_t key) {
         if (key < from || key > to || key < least || bin_of(below) != bin) return -1;
         return static_cast<int>((khi - min(max(key, klo), khi)) >> sh);
       }, c, m);
@@ -810,8 +1044,8 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
     int bin = last;
     if (!nucleus) {                                        // the mass of what the other filters keep
       const uint32_t least = thr;
-      histogram(2, -1, [&](float below, uint32_t key) { return key >= least ? bin_of(below) : -1; }, c, m);
-      block_before(m[0] + m[1] + m[2] + m[3], sm->red, z_all);
+      histogram(2, -1, edge(tid * kOwn), false, [&](float below, uint32_t key) { return key >= least ? bin_of(below) : -1; }, c, m);
+      block_before(m[0] + m[1], sm->red, z_all);
       ptarget = portion(tp, z_all);
       cross(m, ptarget, bin, pabove);
     }

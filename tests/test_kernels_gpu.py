@@ -527,6 +527,31 @@ def test_sampler_small_vocabulary_with_masked_tokens(V, finite):
             assert torch.equal(got, want), (k, list(kw))
 
 
+@pytest.mark.parametrize("rows", [1, 40, 200])           # clusters of 8, 4 and 1
+def test_sampler_lists_at_their_limits(rows):
+    """Kept sets around the sizes of the cluster sampler's lists: 256 and 512 candidates, 2047 elements in a nucleus' last bin."""
+    torch.manual_seed(86)
+    V = 40000
+    seeds, temp = torch.arange(rows, device=DEV, dtype=torch.int64) * 13 + 5, torch.full((rows,), 0.9, device=DEV)
+    i32 = lambda v: torch.full((rows,), v, device=DEV, dtype=torch.int32)
+    f32 = lambda v: torch.full((rows,), v, device=DEV)
+    kws = [dict(top_k=i32(k), **kw) for k in (255, 256, 257, 511, 513) for kw in (dict(), dict(top_p=f32(0.7), min_p=f32(1e-3)))]
+    kws += [dict(top_p=f32(p)) for p in (0.05, 0.6, 0.95, 0.9999)] + [dict(min_p=f32(0.3)), dict(top_p=f32(0.5), min_p=f32(0.01))]
+    for crowd in (0, 200, 513, 2046, 2047, 2048, 5000):
+        lg = torch.randn(rows, V, device=DEV)
+        # `crowd` values of one bin (1 / 32 of T wide) or one value above the bulk, in one stretch or all over the row
+        at = torch.arange(1000, 1000 + crowd, device=DEV) if crowd % 2 else torch.randperm(V, device=DEV)[:crowd]
+        lg[:, at] = 6.0 + (0.0 if crowd == 513 else 0.02) * torch.rand(rows, crowd, device=DEV)
+        for kw in kws:
+            a = ops.sample(lg, temperature=temp, seeds=seeds, step=7, **kw)
+            ops.set_sample_cluster(False)
+            b = ops.sample(lg, temperature=temp, seeds=seeds, step=7, **kw)
+            ops.set_sample_cluster(True)
+            # a row may meet a bucket edge within the rounding of the other kernel's fp32 sums over up to 40000 terms: ~1e-5
+            # of a draw each, times the width of a kept token in it; 3 of 200 rows is that many times over
+            assert (a != b).sum().item() <= max(1, rows // 66), (crowd, list(kw), a.tolist(), b.tolist())
+
+
 def test_sampling_without_filters_is_the_same_in_any_batch():
     """Large batches take the kernel of one CTA a row, small ones clusters: a row's draw depends on neither."""
     torch.manual_seed(85)
