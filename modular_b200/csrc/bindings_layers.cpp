@@ -380,11 +380,15 @@ void delta_rule(const Tensor& x, int q_off, int k_off, int v_off, int b_off, con
   TORCH_CHECK(gate.size(0) >= T && gate.size(1) >= heads * vdim, "delta_rule: gate");
   TORCH_CHECK(norm_w.is_contiguous() && norm_w.scalar_type() == st && norm_w.numel() >= vdim, "delta_rule: norm_w");
   p.norm_w = norm_w.data_ptr(); p.eps = static_cast<float>(eps);
-  TORCH_CHECK(scratch.size() == 7, "delta_rule: scratch is {q, k, g, v, beta, kq, o}");
+  TORCH_CHECK(scratch.size() == 7 || scratch.size() == 8, "delta_rule: scratch is {q, k, g, v, beta, kq, o[, chunks]}");
   const int64_t need[7] = {T * kv_heads * p.dim_pad, T * kv_heads * p.dim_pad, T * heads * (given(z) ? p.dim_pad : 1), T * heads * vdim,
                            T * heads, T * kv_heads, T * heads * vdim};
   float** dst[7] = {&p.q, &p.k, &p.g, &p.v, &p.beta, &p.kq, &p.o};
   for (int i = 0; i < 7; ++i) *dst[i] = const_cast<float*>(f32(scratch[i], need[i], "delta_rule scratch"));
+  if (scratch.size() == 8) {
+    const long long n = mb_delta_chunk_floats(p.T, p.B, heads, kv_heads, dim, vdim, !given(z), dt);
+    if (n > 0) p.chunk = const_cast<float*>(f32(scratch[7], n, "delta_rule scratch"));
+  }
   p.ld_out = ld_of(out, st, "out"); p.out = out.data_ptr();
   TORCH_CHECK(out.size(0) >= T && out.size(1) >= heads * vdim, "delta_rule: out");
   TORCH_CHECK(state.is_contiguous() && state.scalar_type() == at::kFloat && state.dim() == 4 && state.size(1) == heads &&
@@ -641,6 +645,9 @@ void mb::bind_layers(py::module_& m) {
                                dtype_of(o, "o"), cur_stream()), "lightning_norm");
   });
   m.def("delta_dim_pad", [](int dim) { return mb_delta_dim_pad(dim); });
+  m.def("delta_chunk_floats", [](int T, int B, int heads, int kv_heads, int dim, int vdim, bool head_decay, const Tensor& x) {
+    return mb_delta_chunk_floats(T, B, heads, kv_heads, dim, vdim, head_decay, dtype_of(x, "x"));
+  });
   m.def("delta_rule", &delta_rule, py::arg("x"), py::arg("q_off"), py::arg("k_off"), py::arg("v_off"), py::arg("b_off"), py::arg("conv_w"),
         py::arg("z"), py::arg("A_log"), py::arg("dt_bias"), py::arg("gate"), py::arg("norm_w"), py::arg("eps"), py::arg("scratch"),
         py::arg("out"), py::arg("state"), py::arg("conv_state"), py::arg("state_idx"), py::arg("q_start"), py::arg("q_len"),

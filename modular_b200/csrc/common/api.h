@@ -332,6 +332,8 @@ typedef struct {
   int gate_silu; float out_mult;                         // output: norm(o) * out_mult * (sigmoid or silu)(gate)
   const void* norm_w; float eps;                         // [vdim]
   float *q, *k, *g, *v, *beta, *kq, *o;                  // fp32 scratch (q, k, g rows are dim_pad wide)
+  float* chunk;                                          // mb_delta_chunk_floats of scratch, or null: token by token
+  float* chunk_rows;                                     // set by mb_delta_rule
   void* out; int ld_out;                                 // [T, heads * vdim]
   float* state;                                          // [slots, heads, vdim, dim_pad]
   float* conv_state;                                     // [slots, channels, taps - 1]
@@ -339,6 +341,7 @@ typedef struct {
   int T, B, heads, kv_heads, dim, dim_pad, vdim, one_token;
 } MbDelta;
 int mb_delta_dim_pad(int dim);
+long long mb_delta_chunk_floats(int T, int B, int heads, int kv_heads, int dim, int vdim, int head_decay, int dtype);
 int mb_delta_rule(const MbDelta* p, int dtype, int num_sms, cudaStream_t stream);
 // out[t, h * vdim ..] = rms_norm(o[t, h]) * w * mult * (sigmoid or silu)(gate[t, h * vdim ..]); o fp32 [T, heads, vdim]; the
 // norm divides by n <= vdim (columns beyond n hold zeros)

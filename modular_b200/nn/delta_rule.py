@@ -144,6 +144,9 @@ def delta_rule_cuda(m: DeltaRule, px, z, gate, out, state, conv_state, state_idx
     dp = dim_pad(c.dim)
     sizes = (T * c.kv_heads * dp, T * c.kv_heads * dp, T * c.heads * (1 if c.head_decay else dp), T * c.heads * c.vdim, T * c.heads, T * c.kv_heads,
              T * c.heads * c.vdim)
+    # prompts run in chunks where the kernels take them, which need some more
+    chunks = _lib().delta_chunk_floats(T, q_len.numel(), c.heads, c.kv_heads, c.dim, c.vdim, c.head_decay, px)
+    sizes += (chunks,) * (chunks > 0)
     ends, at = [], 0
     for n in sizes:                       # one allocation, every part 16-byte aligned
         ends.append((at, n))

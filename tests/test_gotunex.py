@@ -338,6 +338,93 @@ def test_delta_rule_mixer(H, KH, d, dv, taps, device, dtype):
     assert (state[0] == 3.0).all() and (conv[4] == -2.0).all()       # nobody else's slot was written
 
 
+def delta_step(lens, H, d, dv, taps, resume, seed=0, change=None):
+    """One step of the delta rule on its kernels, and token by token on the CPU in 64 bits: (out, state) of each."""
+    from types import SimpleNamespace
+
+    from modular_b200.nn.delta_rule import delta_rule_cuda, delta_rule_reference, dim_pad
+
+    g = torch.Generator().manual_seed(seed)
+    rn = lambda *s: torch.randn(*s, generator=g)
+    T, C, B = sum(lens), 2 * H * d + H * dv, len(lens)
+    px, gate, conv_w = (rn(*s).bfloat16() for s in ((T, (C + H + 7) // 8 * 8), (T, H * dv), (C, taps)))
+    t = dict(z=rn(T, H * d), A_log=-2 * torch.rand(H, generator=g), dt_bias=rn(H * d) - 3, norm=(1 + 0.1 * rn(dv)).bfloat16(),
+             state=0.05 * rn(B + 1, H, dv, dim_pad(d)), conv=rn(B + 1, C, taps - 1), px=px, gate=gate, conv_w=conv_w * 0.5)
+    t["state"][..., d:] = 0
+    if change:
+        change(t, H, d)
+    meta = [i32(*v) for v in ([B - i for i in range(B)], [sum(lens[:i]) for i in range(B)], lens, [n + 9 * resume for n in lens])]
+    cfg = SimpleNamespace(dim=d, kv_heads=H, heads=H, vdim=dv, taps=taps, channels=C, head_decay=False, eps=1e-5, out_mult=1.0,
+                          blocks=[("q", H * d, 0), ("k", H * d, 0), ("v", H * dv, 0)])
+    res = []
+    for dev, core in (("cuda", delta_rule_cuda), ("cpu", delta_rule_reference)):
+        wide = (lambda x: x.cuda()) if dev == "cuda" else (lambda x: x.double())
+        w = {k: wide(v) for k, v in t.items()}
+        m = SimpleNamespace(cfg=cfg, off=dict(q=0, k=H * d, v=2 * H * d, b=C), conv_w=w["conv_w"], A_log=w["A_log"], dt_bias=w["dt_bias"], norm=w["norm"])
+        out = torch.zeros(T, H * dv, device=dev, dtype=torch.bfloat16)
+        old = torch.get_default_dtype()
+        torch.set_default_dtype(torch.float64 if dev == "cpu" else old)
+        try:
+            some = meta[2] > 0 if dev == "cpu" else slice(None)          # the token loop takes no empty sequences
+            core(m, w["px"], w["z"], w["gate"], out, w["state"], w["conv"], *(v[some].to(dev) for v in meta), False)
+        finally:
+            torch.set_default_dtype(old)
+        res.append((out.double().cpu(), w["state"][..., :d].double().cpu()))
+    return res
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens,H,d,dv,taps,resume", [([16, 81, 47, 96], 2, 128, 128, 4, 1), ([111], 3, 100, 72, 3, 0), ([64, 0, 160, 17], 1, 128, 200, 2, 1),
+                                                     ([40], 1, 97, 4, 4, 1)])
+@pytest.mark.parametrize("decay", ["usual", "fast", "mixed", "none"])
+def test_delta_rule_in_chunks(lens, H, d, dv, taps, resume, decay):
+    """Prompts in chunks of sixteen: whole chunks, remainders, one token, no tokens; decays that fade within a chunk (pairs by products of decays),
+    channels of both kinds, zeros, no decay at all."""
+    def change(t, H, d):
+        if decay == "fast":
+            t["dt_bias"] += 8
+        if decay == "mixed":
+            t["dt_bias"][::3] += 12
+            t["z"][5::7, ::5] = 1e4
+        if decay == "none":
+            t["dt_bias"] -= 30
+    (out, state), (want, wstate) = delta_step(lens, H, d, dv, taps, resume, change=change)
+    assert rel(out, want) < 4e-3                              # both sides are rounded to bf16 (2^-9 each at most)
+    # fp32 sums of 128 and 16 terms and products of up to sixteen decays: some 20 roundings of 2^-24, ten times that at most
+    assert rel(state, wstate) < 1.2e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what,at", [("k", float("nan")), ("v", float("inf")), ("q", float("nan")), ("z", float("nan")), ("state", float("inf")), ("scale", 0.0)])
+def test_delta_rule_chunks_keep_odd_values_from_earlier_tokens(what, at):
+    """A NaN or an infinity reaches what the token-by-token equations let it reach, not the tokens of its chunk before it; columns of the state
+    may be of any size."""
+    def change(t, H, d):
+        if what in "kvq":
+            t["px"][107, {"q": 0, "k": H * d, "v": 2 * H * d}[what] + 3] = at
+        elif what == "z":
+            t["z"][107, 3] = at
+        elif what == "state":
+            t["state"][2, 0, 5, 7] = at
+        else:
+            t["state"] *= torch.logspace(-12, 12, t["state"].shape[2]).view(1, 1, -1, 1)
+            t["dt_bias"] += 4
+    (out, state), (want, wstate) = delta_step([90, 70], 2, 128, 64, 4, 1, change=change)
+    # an infinite state cancels to NaN or not by the order of a sum: those tokens alone are left to either
+    seen = torch.ones_like(out, dtype=torch.bool)
+    if what == "state":
+        seen[:90, :64] = False
+    assert torch.equal(torch.isfinite(out)[seen], torch.isfinite(want)[seen]) and torch.equal(torch.isfinite(state), torch.isfinite(wstate))
+    both = torch.isfinite(out) & torch.isfinite(want)
+    assert rel(out[both], want[both]) < 4e-3
+    for s in range(3):                                        # column by column
+        for h in range(2):
+            for c in range(64):
+                a, b = state[s, h, c], wstate[s, h, c]
+                if torch.isfinite(b).all():
+                    assert rel(a, b) < 1.2e-5 or b.norm() == 0
+
+
 @pytest.mark.parametrize("device,dtype", RUNS)
 def test_delta_rule_without_a_slot(device, dtype):
     """Sequences with slot -1 start from zero and keep nothing (the dummies of a padded decode batch)."""
