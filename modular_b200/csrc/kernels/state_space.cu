@@ -26,7 +26,7 @@
 namespace mb {
 namespace ssm {
 
-__device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
+__device__ __forceinline__ float silu(float x) { return __fdividef(x, 1.f + __expf(-x)); }
 __device__ __forceinline__ float softplus(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -83,7 +83,8 @@ __device__ __forceinline__ void store_bf16(__nv_bfloat16* p, const float (&v)[VE
 // channels and the tokens of one tile, so all tiles run at once; blocks whose row is below n_seqs take the
 // sequences' first W - 1 tokens instead, the only ones that need the state, and the same thread that reads
 // the state writes the new one (one reader, one writer, in order).
-// 4099 tokens x 4096 channels, width 4: 1104 us with one thread per channel walking a sequence, 30 us so. A decode step is bound
+// 4099 tokens x 4096 channels, width 4: 1104 us with one thread per channel walking a sequence, 30 with tiles whose rows were loaded
+// four at a time, 21 us with all rows of a tile on their way at once and the fast division in silu (10 at the copy rate). A decode step is bound
 // by the state, which is read and written in 16-byte pieces: 256 tokens of as many sequences x 4096 channels 11 us (19 with one
 // 4-byte access per value, 12 with one thread per channel).
 constexpr int kConvTile = 16;
@@ -191,6 +192,20 @@ __global__ void __launch_bounds__(128) causal_conv1d_kernel(const __nv_bfloat16*
     if (t0 >= hi) break;
     const int first = max(lo, t0 + W - 1), last = min(hi, cu_seqlens[s + 1]);
     if (first >= last) continue;
+    if (VEC == 4 && last - first == kConvTile) {     // a whole tile: all of its rows are on their way before the first is used
+      uint2 raw[kConvTile + W - 1];
+      const __nv_bfloat16* from = x + static_cast<size_t>(first - W + 1) * ldx + d;
+#pragma unroll
+      for (int k = 0; k < kConvTile + W - 1; ++k) raw[k] = *reinterpret_cast<const uint2*>(from + static_cast<size_t>(k) * ldx);
+#pragma unroll
+      for (int k = 0; k < kConvTile + W - 1; ++k) {
+        shift();
+        win[W - 1][0] = __uint_as_float(raw[k].x << 16); win[W - 1][1 % VEC] = __uint_as_float(raw[k].x & 0xffff0000u);
+        win[W - 1][2 % VEC] = __uint_as_float(raw[k].y << 16); win[W - 1][3 % VEC] = __uint_as_float(raw[k].y & 0xffff0000u);
+        if (k >= W - 1) emit(first + k - (W - 1));
+      }
+      continue;
+    }
 #pragma unroll
     for (int k = 1; k < W; ++k) load_bf16<VEC>(win[k], x + static_cast<size_t>(first - W + k) * ldx + d);
 #pragma unroll 4
@@ -207,17 +222,32 @@ __global__ void __launch_bounds__(128) causal_conv1d_kernel(const __nv_bfloat16*
 //   y[t, d] = sum_n C[t, n] * h + Dskip[d] * u[t, d];   y *= silu(z[t, d]) when z is given
 // The recurrence needs one exponential per state and token (all fp32): 268 M of them for 4099 tokens x 4096
 // channels x 16 states are 60 us of the special-function units, which is the floor for prompts that fill the chip.
-// Eight lanes share a channel (N / 8 states each, in registers), so that a few long sequences still give every SM
-// several warps (with four lanes the longest of three sequences had 1.8 per scheduler and took 285 us); a CTA walks one sequence for 32 channels. Inputs arrive kScanTile tokens at a time through cp.async,
+// Eight or four lanes (LPC) share a channel, N / LPC states each in registers, so that a few long sequences still give every SM
+// several warps; a CTA walks one sequence for 32 channels. Inputs arrive kScanTile tokens at a time through cp.async,
 // one tile ahead; step sizes (softplus) are made once per token and channel by all threads before the walk, and
-// the lanes' partial outputs of eight tokens meet in seven shuffles. Rows that are not 16-byte aligned are fetched
-// with plain loads, into the same tiles.
-// That prompt (three sequences): 3475 us with one thread per channel and two barriers per token, 233 us so. Short sequences fetch and
-// convert no more than their tokens (in eights): a decode step of 256 sequences x 4096 channels 130 us (167 with whole tiles of 32,
-// 132 with one thread per channel).
-constexpr int kScanTile = 32, kScanCh = 32, kScanThreads = 256;
-template <int N>
-__global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16* __restrict__ delta,
+// the lanes' partial outputs of eight tokens meet in seven or six shuffles (through shared memory, for a pass of their own, they
+// took 258 us where these take 218). Rows that are not 16-byte aligned are fetched with plain loads, into the same tiles.
+// That prompt (three sequences): 3475 us with one thread per channel and two barriers per token, 218 us so: some 30 instructions a
+// token and eight lanes, and the longest sequence alone at the end. Short sequences fetch and convert no more than their tokens
+// (in eights): a decode step of 256 sequences x 4096 channels 95 us (137 with eight lanes, 167 with whole tiles of 32).
+constexpr int kScanTile = 32, kScanCh = 32;
+template <int NS>
+__device__ __forceinline__ void load_states(float (&v)[NS], const float* p) {
+  if constexpr (NS % 4 == 0) {
+#pragma unroll
+    for (int i = 0; i < NS; i += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(p + i);
+      v[i] = f.x; v[i + 1] = f.y; v[i + 2] = f.z; v[i + 3] = f.w;
+    }
+  } else if constexpr (NS == 2) {
+    const float2 f = *reinterpret_cast<const float2*>(p);
+    v[0] = f.x; v[1] = f.y;
+  } else {
+    v[0] = p[0];
+  }
+}
+template <int N, int LPC>
+__global__ void __launch_bounds__(kScanCh * LPC) selective_scan_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16* __restrict__ delta,
                                       const float* __restrict__ A, const __nv_bfloat16* __restrict__ B,
                                       const __nv_bfloat16* __restrict__ C, const float* __restrict__ Dskip,
                                       const __nv_bfloat16* __restrict__ z, const float* __restrict__ dt_bias,
@@ -225,13 +255,13 @@ __global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(const __nv
                                       const int* __restrict__ cu_seqlens, const int* __restrict__ state_idx,
                                       const int* __restrict__ has_init, int D, int ld_u, int ld_z, int ld_b, int ld_c,
                                       int dt_softplus, int vec) {
-  constexpr int NS = N / 8, TT = kScanTile, CH = kScanCh;
+  constexpr int NS = N / LPC, TT = kScanTile, CH = kScanCh, NT = CH * LPC;
   struct Stage { __nv_bfloat16 u[TT][CH], dl[TT][CH], z[TT][CH], B[TT][N], C[TT][N]; };
   __shared__ __align__(16) Stage stages[2];
   __shared__ __align__(16) float sB[TT][N], sC[TT][N];
   __shared__ float2 sdt[TT][CH];                     // step size, step size * input
   __shared__ __align__(16) __nv_bfloat16 sy[TT][CH];
-  const int s = blockIdx.y, tid = threadIdx.x, lane = tid & 31, q = lane & 7, c = (tid >> 5) * 4 + (lane >> 3);
+  const int s = blockIdx.y, tid = threadIdx.x, lane = tid & 31, q = lane % LPC, c = tid / LPC;
   const int d0 = blockIdx.x * CH, d = d0 + c;
   const int t0 = cu_seqlens[s], n = cu_seqlens[s + 1] - t0;
   const int slot = state_idx && ssm_state ? state_idx[s] : -1;
@@ -248,18 +278,15 @@ __global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(const __nv
   auto fetch = [&](int c0, Stage& g) {
     const int mm = eights(c0);
     if (vec) {
-      const int j = (tid >> 2) & 31, k = (tid & 3) * 8;      // the first half of the threads fetches u and z, the other delta
+      const int j = (tid >> 2) & 31, k = (tid & 3) * 8;      // 128 threads a row set; with 256 the other half fetches delta
       const bool ok = c0 + j < n && d0 + k < D;
       const size_t row = static_cast<size_t>(t0 + (c0 + j < n ? c0 + j : 0)), col = d0 + k < D ? d0 + k : 0;
-      if (j >= mm) {
-        // no such token
-      } else if (tid < 128) {
+      if (j < mm && tid < 128) {
         cp_async16(&g.u[j][k], u + row * ld_u + col, ok);
         if (z) cp_async16(&g.z[j][k], z + row * ld_z + col, ok);
-      } else {
-        cp_async16(&g.dl[j][k], delta + row * ld_u + col, ok);
       }
-      for (int i = kScanThreads - 1 - tid; i < mm * (N / 8); i += kScanThreads) {
+      if (j < mm && (NT == 128 || tid >= 128)) cp_async16(&g.dl[j][k], delta + row * ld_u + col, ok);
+      for (int i = NT - 1 - tid; i < mm * (N / 8); i += NT) {
         const int jj = i / (N / 8), kk = (i % (N / 8)) * 8;
         const bool in = c0 + jj < n;
         const size_t r = static_cast<size_t>(t0 + (in ? c0 + jj : 0));
@@ -268,7 +295,7 @@ __global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(const __nv
       }
     } else {
       const __nv_bfloat16 zero = __float2bfloat16(0.f);
-      for (int i = tid; i < mm * CH; i += kScanThreads) {
+      for (int i = tid; i < mm * CH; i += NT) {
         const int j = i / CH, k = i % CH;
         const bool ok = c0 + j < n && d0 + k < D;
         const size_t row = static_cast<size_t>(t0 + c0 + j);
@@ -276,7 +303,7 @@ __global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(const __nv
         g.dl[j][k] = ok ? delta[row * ld_u + d0 + k] : zero;
         if (z) g.z[j][k] = ok ? z[row * ld_z + d0 + k] : zero;
       }
-      for (int i = tid; i < mm * N; i += kScanThreads) {
+      for (int i = tid; i < mm * N; i += NT) {
         const int j = i / N, k = i % N;
         const bool ok = c0 + j < n;
         const size_t row = static_cast<size_t>(t0 + c0 + j);
@@ -307,12 +334,12 @@ __global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(const __nv
     };
     if (m == TT) {
 #pragma unroll
-      for (int j = 0; j < TT; j += kScanThreads / 32) step(j + (tid >> 5));
+      for (int j = 0; j < TT; j += NT / 32) step(j + (tid >> 5));
 #pragma unroll
-      for (int i = 0; i < TT * N; i += kScanThreads) widen(i + tid);
+      for (int i = 0; i < TT * N; i += NT) widen(i + tid);
     } else {
-      for (int j = tid >> 5; j < mm; j += kScanThreads / 32) step(j);
-      for (int i = tid; i < mm * N; i += kScanThreads) widen(i);
+      for (int j = tid >> 5; j < mm; j += NT / 32) step(j);
+      for (int i = tid; i < mm * N; i += NT) widen(i);
     }
     __syncthreads();
     for (int j0 = 0; j0 < m; j0 += 8) {
@@ -320,27 +347,33 @@ __global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(const __nv
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
         const float2 e = sdt[j0 + r][c];
-        float acc = 0.f;
+        float acc = 0.f, vb[NS], vc[NS];
+        load_states<NS>(vb, &sB[j0 + r][q * NS]);
+        load_states<NS>(vc, &sC[j0 + r][q * NS]);
 #pragma unroll
         for (int i = 0; i < NS; ++i) {
-          h[i] = fmaf(ex2(e.x * a2[i]), h[i], e.y * sB[j0 + r][q * NS + i]);
-          acc = fmaf(sC[j0 + r][q * NS + i], h[i], acc);
+          h[i] = fmaf(ex2(e.x * a2[i]), h[i], e.y * vb[i]);
+          acc = fmaf(vc[i], h[i], acc);
         }
         part[r] = acc;
       }
-      // lane q of the channel ends up with token j0 + q
+      // lane q of the channel ends up with tokens j0 + q, j0 + q + LPC, ..
 #pragma unroll
-      for (int o = 4; o > 0; o >>= 1)
+      for (int o = LPC / 2; o > 0; o >>= 1)
 #pragma unroll
-        for (int r = 0; r < o; ++r) {
-          const float send = (q & o) ? part[r] : part[r + o], keep = (q & o) ? part[r + o] : part[r];
-          part[r] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        for (int r = 0; r < 8 / LPC * o; ++r) {
+          const int lo = (r / o) * LPC + r % o;
+          const float send = (q & o) ? part[lo] : part[lo + o], keep = (q & o) ? part[lo + o] : part[lo];
+          part[lo] = keep + __shfl_xor_sync(0xffffffffu, send, o);
         }
-      float v = part[0];
-      const int j = j0 + q;
-      v = fmaf(dsk, __bfloat162float(g.u[j][c]), v);
-      if (z) v *= silu(__bfloat162float(g.z[j][c]));
-      sy[j][c] = __float2bfloat16(v);
+#pragma unroll
+      for (int r = 0; r < 8 / LPC; ++r) {
+        float v = part[r * LPC];
+        const int j = j0 + r * LPC + q;
+        v = fmaf(dsk, __bfloat162float(g.u[j][c]), v);
+        if (z) v *= silu(__bfloat162float(g.z[j][c]));
+        sy[j][c] = __float2bfloat16(v);
+      }
     }
     __syncthreads();
     if (vec) {
@@ -348,7 +381,7 @@ __global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(const __nv
       if (tid < 128 && j < m && d0 + k < D)
         *reinterpret_cast<uint4*>(y + static_cast<size_t>(t0 + c0 + j) * ld_u + d0 + k) = *reinterpret_cast<const uint4*>(&sy[j][k]);
     } else {
-      for (int i = tid; i < m * CH; i += kScanThreads)
+      for (int i = tid; i < m * CH; i += NT)
         if (d0 + i % CH < D) y[static_cast<size_t>(t0 + c0 + i / CH) * ld_u + d0 + i % CH] = sy[i / CH][i % CH];
     }
   }
@@ -872,8 +905,14 @@ extern "C" int mb_selective_scan_varlen(const void* u, const void* delta, const 
   const int vec = D % 8 == 0 && ld_u % 8 == 0 && ld_b % 8 == 0 && ld_c % 8 == 0 && aligned16(u) && aligned16(delta) &&
                   aligned16(B) && aligned16(C) && aligned16(y) && (z == nullptr || (ld_z % 8 == 0 && aligned16(z)));
   dim3 grid((D + kScanCh - 1) / kScanCh, n_seqs);
+  // Four lanes a channel take 40 % fewer instructions per token than eight (wider reads of B and C, one exchange less) but give
+  // half the warps; from 2048 warps on they win: 4096 channels, 4099 tokens in 3, 4 and 8 sequences 239, 187 and 145 us against 218,
+  // 203 and 184; 2000 tokens in 32 72 against 86, one token of 256 each 95 against 125, 200 in two 14.1 against 13.3.
+  const bool many = static_cast<long long>(D) * n_seqs >= 16384;
 #define MB_SCAN(Nv)                                                                                             \
-  selective_scan_kernel<Nv><<<grid, kScanThreads, 0, stream>>>(                                                          \
+  if (many) MB_SCAN_L(Nv, 4); else MB_SCAN_L(Nv, 8)
+#define MB_SCAN_L(Nv, Lv)                                                                                                \
+  selective_scan_kernel<Nv, Lv><<<grid, kScanCh * Lv, 0, stream>>>(                                                      \
       static_cast<const __nv_bfloat16*>(u), static_cast<const __nv_bfloat16*>(delta), A,                        \
       static_cast<const __nv_bfloat16*>(B), static_cast<const __nv_bfloat16*>(C), Dskip,                        \
       static_cast<const __nv_bfloat16*>(z), dt_bias, static_cast<__nv_bfloat16*>(y), ssm_state, cu_seqlens,     \
@@ -884,6 +923,7 @@ extern "C" int mb_selective_scan_varlen(const void* u, const void* delta, const 
     case 32: MB_SCAN(32); break;
     default: return MB_ERR_SHAPE;
   }
+#undef MB_SCAN_L
 #undef MB_SCAN
   return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ERR_LAUNCH;
 }

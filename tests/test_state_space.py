@@ -176,6 +176,29 @@ def test_selective_scan_tiles(N, D, lead):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("N,D,lead", [(16, 2048, 8), (8, 2056, 8), (32, 2048, 8), (16, 2051, 1)])
+def test_selective_scan_is_the_same_in_any_batch(N, D, lead):
+    """Batches of many channels give a channel four lanes, single sequences eight: the states are the same, bit for bit, and
+    outputs differ by the order of a sum over N states (a rounding to bf16 apart)."""
+    torch.manual_seed(16)
+    dev, lens = "cuda", [1, 7, 8, 9, 31, 32, 33, 70]
+    T, cu = sum(lens), _cu(lens, dev)
+    bf = lambda *s, k=1.0: (torch.randn(*s, device=dev) * k).to(torch.bfloat16)
+    u, delta, z, B, C = bf(T, D), bf(T, D, k=0.5), _strided(bf(T, D), lead), _strided(bf(T, N), lead), _strided(bf(T, N), lead)
+    A, Dk, bias = -torch.rand(D, N, device=dev) * 4 - 0.1, torch.randn(D, device=dev), torch.randn(D, device=dev) * 0.1
+    idx = torch.tensor([5, 0, -1, 3, 1, 6, 2, 7], dtype=torch.int32, device=dev)
+    init = torch.tensor([1, 0, 0, 1, 0, 1, 0, 1], dtype=torch.int32, device=dev)
+    st = torch.randn(8, D, N, device=dev)
+    one = st.clone()
+    y = ss.selective_scan_varlen(u, delta, A, B, C, Dk, z, bias, cu, st, idx, init, True)
+    for i, n in enumerate(lens):
+        r = slice(sum(lens[:i]), sum(lens[:i]) + n)
+        w = ss.selective_scan_varlen(u[r], delta[r], A, B[r], C[r], Dk, z[r], bias, _cu([n], dev), one, idx[i: i + 1], init[i: i + 1], True)
+        assert _rel(y[r], w) < 2 ** -9
+    assert torch.equal(st, one)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("H,P,N,G,A0", [(4, 64, 128, 1, 1.0), (6, 32, 64, 2, 16.0), (2, 128, 16, 2, 0.1), (3, 8, 24, 1, 1.0), (2, 16, 40, 2, 4.0),
                                         (2, 4, 16, 1, 1.0), (2, 64, 136, 1, 1.0)])
 def test_ssd_chunks(H, P, N, G, A0):
