@@ -535,7 +535,11 @@ int mb_selective_scan_varlen(const void* u, const void* delta, const float* A, c
 int mb_ssd_scan_varlen(const void* x, const void* dt, const float* A, const void* B, const void* C,
                        const float* Dskip, const float* dt_bias, void* y, float* ssm_state,
                        const int* cu_seqlens, const int* state_idx, const int* has_init, int n_seqs, int tokens,
-                       int H, int P, int N, int G, int ldx, int ld_dt, int ldb, int ldc, int dt_softplus, cudaStream_t stream);
+                       int H, int P, int N, int G, int ldx, int ld_dt, int ldb, int ldc, int dt_softplus, float* scratch,
+                       long long scratch_floats, cudaStream_t stream);
+// Tokens of the segments that long prompts are cut into (0: none). They take (tokens / segment + n_seqs) * H * (P * N + 1) floats of scratch;
+// with less, sequences are walked whole.
+int mb_ssd_segment(int tokens, int n_seqs, int H, int P);
 int mb_gated_rms_norm(const void* y, const void* z, const void* w, void* out, int T, int D, int ldz, float eps, cudaStream_t stream);
 int mb_apply_token_bitmask(float* logits, const int32_t* bitmask, int rows, int vocab, int ld,
                            cudaStream_t stream);

@@ -508,7 +508,13 @@ struct SsdChunk {
   float* state;
   const int *cu_seqlens, *state_idx, *has_init;
   int H, P, N, G, ldx, ld_dt, ldb, ldc, dt_softplus, col_blocks;
+  // Long prompts in segments of `seg` tokens (0: whole sequences), each with its own CTA. parts [segments, H, P, N] holds the state that a
+  // segment makes of nothing, decays [segments, H] its decay.
+  int seg, n_seqs;
+  float *parts, *decays;
 };
+// Segments of a step: sequence s has numbers (cu_seqlens[s] / seg) + s + i, which never meet another sequence's.
+__device__ __forceinline__ int segment_base(const SsdChunk& p, int s) { return p.cu_seqlens[s] / p.seg + s; }
 // per chunk: c_i (and what its rounding left), 2^(sum beyond j) dt_j, dt_j, 2^c_i. With c_i alone a difference c_i - c_j would
 // carry the rounding of sums that may be thousands of times larger than it: after a token that decays by 2^-50000 the next ones'
 // weights were off by 2 in 1000.
@@ -554,7 +560,8 @@ __device__ __forceinline__ void ssd_products(const __nv_bfloat16* sC, const __nv
   }
 }
 
-template <int DK>
+// LOCAL: only the state that a segment makes of nothing, for all segments but a sequence's last one.
+template <int DK, bool LOCAL>
 __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_kernel(const SsdChunk p) {
   typedef __nv_bfloat16 bf16;
   constexpr int LDK = DK + 8, KB = DK / 16, kStage = kChunk * (2 * LDK + kLdV);
@@ -563,8 +570,28 @@ __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_ker
   bf16* sP = stages + 2 * kStage;                    // [hi | lo][chunk][kLdP]
   __shared__ SsdTimes times[2];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, mi = lane >> 3, r8 = lane & 7, row4 = lane >> 2, col2 = 2 * (lane & 3);
-  const int h = blockIdx.x / p.col_blocks, v0 = (blockIdx.x % p.col_blocks) * kNV, s = blockIdx.y, P = p.P, N = p.N;
-  const int t0 = p.cu_seqlens[s], n = p.cu_seqlens[s + 1] - t0, slot = p.state_idx && p.state ? p.state_idx[s] : -1;
+  const int h = blockIdx.x / p.col_blocks, v0 = (blockIdx.x % p.col_blocks) * kNV, P = p.P, N = p.N;
+  int s = blockIdx.y, part = 0;
+  if (p.seg > 0) {
+    int lo = 0, hi = p.n_seqs - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (segment_base(p, mid) <= static_cast<int>(blockIdx.y)) lo = mid; else hi = mid - 1;
+    }
+    s = lo;
+    part = blockIdx.y - segment_base(p, s);
+  }
+  const int slot = p.state_idx && p.state ? p.state_idx[s] : -1;
+  int t0 = p.cu_seqlens[s], n = p.cu_seqlens[s + 1] - t0;
+  bool last = true;
+  if (p.seg > 0) {
+    const int from = part * p.seg;
+    if (part > 0 && from >= n) return;
+    last = from + p.seg >= n;
+    t0 += from;
+    n = min(n - from, p.seg);
+    if (LOCAL && last) return;
+  }
   const bool resume = slot >= 0 && p.has_init && p.has_init[s];
   const int group = h / (p.H / p.G);
   const bf16 *xh = p.x + static_cast<size_t>(t0) * p.ldx + h * P, *Bh = p.B + static_cast<size_t>(t0) * p.ldb + group * N,
@@ -645,10 +672,28 @@ __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_ker
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       float2 f = make_float2(0.f, 0.f);
-      if (resume && vr + 8 * e < P && 8 * t < N) f = *reinterpret_cast<const float2*>(st + static_cast<size_t>(vr + 8 * e) * N + 8 * t + col2);
+      if (!LOCAL && resume && vr + 8 * e < P && 8 * t < N) f = *reinterpret_cast<const float2*>(st + static_cast<size_t>(vr + 8 * e) * N + 8 * t + col2);
       S[t][2 * e] = f.x; S[t][2 * e + 1] = f.y;
     }
-  bool have_state = resume;
+  bool have_state = !LOCAL && resume;
+  float decay = 1.f;
+  if (!LOCAL && part > 0) {                          // through the segments before
+    for (int i = 0; i < part; ++i) {
+      const size_t at = static_cast<size_t>(blockIdx.y - part + i) * p.H + h;
+      const float f = p.decays[at];
+      const float* from = p.parts + at * P * N;
+#pragma unroll
+      for (int t = 0; t < 2 * KB; ++t)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          if (vr + 8 * e >= P || 8 * t >= N) continue;
+          const float2 x = *reinterpret_cast<const float2*>(from + static_cast<size_t>(vr + 8 * e) * N + 8 * t + col2);
+          S[t][2 * e] = have_state ? fmaf(S[t][2 * e], f, x.x) : x.x;
+          S[t][2 * e + 1] = have_state ? fmaf(S[t][2 * e + 1], f, x.y) : x.y;
+        }
+      have_state = true;
+    }
+  }
   for (int c0 = 0, it = 0; c0 < n; c0 += kChunk, ++it) {
     const int m = min(kChunk, n - c0);
     const bf16 *sC = stages + (it & 1) * kStage, *sB = sC + kChunk * LDK, *sV = sB + kChunk * LDK;
@@ -659,6 +704,13 @@ __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_ker
     // NB: blocks of 16 tokens that have any
     auto chunk = [&](auto blocks) {
       constexpr int NB = decltype(blocks)::value;
+      if constexpr (LOCAL) {
+        if (warp == 0 && c0 + kChunk < n) {
+          make_times(c0 + kChunk, times[(it + 1) & 1]);
+          read_dt(c0 + 2 * kChunk);
+        }
+        decay *= tm.total;
+      } else {
       switch (warp) {
         case 0:                                        // the fewest products: this warp also prepares the next chunk's times
           ssd_products<0, DK>(sC, sB, sP, tm, lane);
@@ -757,6 +809,7 @@ __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_ker
                 __floats2bfloat162_rn(fmaf(dsk, xv.x, o[i][j][2 * e]), fmaf(dsk, xv.y, o[i][j][2 * e + 1]));
           }
         }
+      }
       // the state after the chunk
       if (have_state) {
         const float f = tm.total;
@@ -794,7 +847,12 @@ __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_ker
     if (m > 16) chunk(std::integral_constant<int, 4>());
     else chunk(std::integral_constant<int, 1>());      // a short prompt, or a prompt's end
   }
-  if (slot >= 0) {
+  if (LOCAL) {
+    const size_t at = static_cast<size_t>(blockIdx.y) * p.H + h;
+    st = p.parts + at * P * N;
+    if (tid == 0 && v0 == 0) p.decays[at] = decay;
+  }
+  if (LOCAL || (slot >= 0 && last)) {
 #pragma unroll
     for (int t = 0; t < 2 * KB; ++t)
 #pragma unroll
@@ -805,15 +863,18 @@ __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_ker
 }
 
 template <int DK>
-static int launch_ssd_chunk(const SsdChunk& p, int n_seqs, cudaStream_t stream) {
+static int launch_ssd_chunk(const SsdChunk& p, int n_seqs, int tokens, cudaStream_t stream) {
   constexpr int smem = (2 * kChunk * (2 * (DK + 8) + kLdV) + 2 * kChunk * kLdP) * 2;
   static PerDeviceOnce configured;
   if (configured.needed()) {
-    if (cudaFuncSetAttribute(ssd_chunk_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(ssd_chunk_kernel<DK, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaFuncSetAttribute(ssd_chunk_kernel<DK, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return MB_ERR_LAUNCH;
     configured.done();
   }
-  ssd_chunk_kernel<DK><<<dim3(p.H * p.col_blocks, n_seqs), kChunkThreads, smem, stream>>>(p);
+  const dim3 grid(p.H * p.col_blocks, p.seg > 0 ? tokens / p.seg + n_seqs : n_seqs);
+  if (p.seg > 0) ssd_chunk_kernel<DK, true><<<grid, kChunkThreads, smem, stream>>>(p);
+  ssd_chunk_kernel<DK, false><<<grid, kChunkThreads, smem, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ERR_LAUNCH;
 }
 
@@ -928,11 +989,29 @@ extern "C" int mb_selective_scan_varlen(const void* u, const void* delta, const 
   return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ERR_LAUNCH;
 }
 
+// Long prompts whose chains do not fill the chip are walked in segments of 512 tokens, or a sixteenth of the step if that is more (the states
+// of all segments lie in scratch): one launch makes every segment's state out of
+// nothing, another walks all segments at once from the states before them. Half of the products are done twice, so it pays where there is about
+// one CTA per SM at most, and sequences are long (80 heads x 64 x 128, us whole and in segments: 4096 tokens in one sequence 355 and 258, in two
+// 245 and 233, in four 192 and 225; 1000 tokens in two 74 and 76).
+extern "C" int mb_ssd_segment(int tokens, int n_seqs, int H, int P) {
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+  }
+  const long long chains = static_cast<long long>(n_seqs) * H * ((P + kNV - 1) / kNV);
+  if (chains * 4 > sms * 5LL || tokens < 1536LL * n_seqs) return 0;
+  const int sixteenth = (tokens / 16 + kChunk - 1) / kChunk * kChunk;
+  return sixteenth > 512 ? sixteenth : 512;
+}
+
 extern "C" int mb_ssd_scan_varlen(const void* x, const void* dt, const float* A, const void* B, const void* C,
                                   const float* Dskip, const float* dt_bias, void* y, float* ssm_state,
                                   const int* cu_seqlens, const int* state_idx, const int* has_init, int n_seqs,
                                   int tokens, int H, int P, int N, int G, int ldx, int ld_dt, int ldb, int ldc,
-                                  int dt_softplus, cudaStream_t stream) {
+                                  int dt_softplus, float* scratch, long long scratch_floats, cudaStream_t stream) {
   if (n_seqs <= 0 || H <= 0) return MB_OK;
   if (P <= 0 || P > 256 || (P & (P - 1)) || G <= 0 || H % G || N <= 0 || N > 256) return MB_ERR_SHAPE;
   // From four tokens per sequence on, the chunks win (64 sequences of 4 tokens: 80 heads x 64 x 128 563 against 111 us, 24 heads x 64 x
@@ -942,10 +1021,17 @@ extern "C" int mb_ssd_scan_varlen(const void* x, const void* dt, const float* A,
       aligned16(x) && aligned16(B) && aligned16(C) && (reinterpret_cast<uintptr_t>(ssm_state) & 7) == 0) {
     SsdChunk p{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dt), static_cast<const __nv_bfloat16*>(B),
                static_cast<const __nv_bfloat16*>(C), A, Dskip, dt_bias, static_cast<__nv_bfloat16*>(y), ssm_state, cu_seqlens,
-               state_idx, has_init, H, P, N, G, ldx, ld_dt, ldb, ldc, dt_softplus, (P + kNV - 1) / kNV};
-    if (N <= 32) return launch_ssd_chunk<32>(p, n_seqs, stream);
-    if (N <= 64) return launch_ssd_chunk<64>(p, n_seqs, stream);
-    return launch_ssd_chunk<128>(p, n_seqs, stream);
+               state_idx, has_init, H, P, N, G, ldx, ld_dt, ldb, ldc, dt_softplus, (P + kNV - 1) / kNV, 0, n_seqs, nullptr, nullptr};
+    const int seg = mb_ssd_segment(tokens, n_seqs, H, P);
+    const long long segments = seg > 0 ? static_cast<long long>(tokens) / seg + n_seqs : 0;
+    if (seg > 0 && scratch != nullptr && scratch_floats >= segments * H * (static_cast<long long>(P) * N + 1) && segments <= 65535) {
+      p.seg = seg;
+      p.parts = scratch;
+      p.decays = scratch + segments * H * P * N;
+    }
+    if (N <= 32) return launch_ssd_chunk<32>(p, n_seqs, tokens, stream);
+    if (N <= 64) return launch_ssd_chunk<64>(p, n_seqs, tokens, stream);
+    return launch_ssd_chunk<128>(p, n_seqs, tokens, stream);
   }
   int J = 256 / P;            // threads per state row
   if (J > 32) J = 32;

@@ -251,6 +251,37 @@ def test_strides_of_single_elements(H, P, N):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("lens,H,P,N,A0", [([4000, 1, 800], 4, 64, 128, 1.0), ([1537], 3, 72, 64, 0.05), ([512, 0, 4608, 1025], 2, 32, 24, 0.01),
+                                             ([10000], 1, 16, 8, 0.003)])
+def test_ssd_segments(lens, H, P, N, A0):
+    """Long prompts in segments of 512 tokens and more, ragged, beside short ones: the same as in portions of 500 tokens that are walked whole."""
+    torch.manual_seed(17)
+    dev, T, B_ = "cuda", sum(lens), len(lens)
+    bf = lambda *s, k=1.0: (torch.randn(*s, device=dev) * k).to(torch.bfloat16)
+    x, dt, B, C = bf(T, H, P), bf(T, H, k=0.5), bf(T, 1, N), bf(T, 1, N)
+    A, Dk, bias = -torch.rand(H, device=dev) * A0 - 1e-3, torch.randn(H, device=dev), torch.randn(H, device=dev) * 0.1
+    idx = torch.tensor([3, -1, 0, 2][:B_], dtype=torch.int32, device=dev)
+    init = torch.tensor([1, 0, 0, 1][:B_], dtype=torch.int32, device=dev)
+    start = torch.randn(5, H, P, N, device=dev)
+    st = start.clone()
+    y = ss.ssd_scan_varlen(x, dt, A, B, C, Dk, bias, _cu(lens, dev), st, idx, init, True)
+    for i, n in enumerate(lens):
+        if n == 0:
+            continue
+        one, slot = start.clone(), max(int(idx[i]), 0)
+        keep = torch.tensor([slot if int(idx[i]) >= 0 else 4], dtype=torch.int32, device=dev)      # a slot of its own for the one without
+        want = []
+        for c in range(0, n, 500):
+            r = slice(sum(lens[:i]) + c, sum(lens[:i]) + min(c + 500, n))
+            want.append(ss.ssd_scan_varlen(x[r], dt[r], A, B[r], C[r], Dk, bias, _cu([r.stop - r.start], dev), one, keep,
+                                           init[i: i + 1] if c == 0 else torch.ones(1, dtype=torch.int32, device=dev), True))
+        assert _rel(y[sum(lens[:i]): sum(lens[:i]) + n], torch.cat(want)) < 2 ** -8          # a rounding to bf16 on either side
+        if int(idx[i]) >= 0:
+            assert _rel(st[slot], one[slot]) < 1e-5        # fp32 sums over the state's memory, cut at other tokens
+    assert torch.equal(st[1], start[1]) and torch.equal(st[4], start[4])
+
+
+@pytest.mark.gpu
 def test_ssd_special_inputs_stay_causal():
     """An infinite or NaN input of a prompt changes its own row of the state from its token on, and nothing before it."""
     torch.manual_seed(10)
