@@ -319,7 +319,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 // multiplied into the other of two 256-column TMEM buffers meanwhile. The sums run over K in the same order as above.
 // CTAs are persistent, so one tile's stores run under the next one's first loads.
 //   PAIR    dense: two CTAs share the tile (256 tokens x 256 weight rows, each loads half of either operand), which halves
-//           the bytes per operation that come from L2: 2050 x 57344 x 8192 in 1140 us (2094 with weights on M).
+//           the bytes per operation that come from L2: 2050 x 57344 x 8192 in 1080 us (2094 with weights on M). A K group
+//           takes a promotion warp about 1100 cycles at two of them a scheduler (wait, four TMEM reads of 150 cycles, 64 packed FMAs,
+//           release), while its MMAs take 512: that chain is the bound, not a unit.
 //   !PAIR   experts: the tiles of one expert's tokens after another; weights are read from memory once and are the bound:
 //           16800 rows, 256 experts of 4096 x 7168: 1400 us (2998 with weights on M).
 constexpr int kRowStages = 6, kRowTileN = 256, kMaxRowTiles = 1024;
@@ -337,7 +339,7 @@ struct RowTail {
   int abort_word;
   int n_tiles;                        // grouped: token tiles
   int2 tile[kMaxRowTiles];            // grouped: expert, first row
-  float factor[8][kAhead][64];        // per promotion warp and K group: sx of its 32 rows, then sw 32 times
+  float factor[8][kAhead][64];        // grouped: per promotion warp and K group: sx of its 32 rows, then sw 32 times
 };
 
 __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
@@ -505,7 +507,10 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
       uint64_t acc[64];
 #pragma unroll
       for (int i = 0; i < 64; ++i) acc[i] = 0;
-      // a lane fetches its own factors, kAhead K groups ahead (one commit per K group, empty beyond the last one)
+      // A lane reads its own factors kAhead K groups ahead: into registers (through shared memory the two copies and their wait were 150
+      // of a group's thousand cycles; 2050 x 57344 x 8192 1147 -> 1082 us), experts through shared memory (one commit per K group, empty
+      // beyond the last one), because they have no registers left: with the factors in them the kernel spills and takes 2 % longer.
+      float px[kAhead], pw[kAhead];
       float* mine = &tail->factor[warp - 4][0][lane];
       auto fetch = [&](int kb) {
         if (kb < kb_total) {
@@ -515,16 +520,37 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         asm volatile("cp.async.commit_group;" ::: "memory");
       };
 #pragma unroll
-      for (int j = 0; j < kAhead; ++j) fetch(j);
+      for (int j = 0; j < kAhead; ++j) {
+        if constexpr (PAIR) {
+          px[j] = live && j < kb_total ? sx[static_cast<size_t>(j) * p.M] : 0.f;
+          pw[j] = j < kb_total ? sw[j] : 0.f;
+        } else {
+          fetch(j);
+        }
+      }
       for (int kb = 0; kb < kb_total; ++kb) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
-        const float* at = mine + (kb % kAhead) * 64;
-        const float f = live ? at[0] * at[32] : 0.f;
-        fetch(kb + kAhead);
+        float f;
+        if constexpr (PAIR) {
+          f = px[0] * pw[0];
+#pragma unroll
+          for (int j = 0; j < kAhead - 1; ++j) { px[j] = px[j + 1]; pw[j] = pw[j + 1]; }
+          const int next = kb + kAhead;
+          if (next < kb_total) {
+            px[kAhead - 1] = live ? sx[static_cast<size_t>(next) * p.M] : 0.f;
+            pw[kAhead - 1] = sw[next];
+          }
+        } else {
+          asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
+          const float* at = mine + (kb % kAhead) * 64;
+          f = live ? at[0] * at[32] : 0.f;
+          fetch(kb + kAhead);
+        }
         uint64_t f2;
         asm("mov.b64 %0, {%1, %1};" : "=l"(f2) : "r"(__float_as_uint(f)));
         const uint32_t buf = g & 1;
-        ok = mbar_wait(&tail->acc_full[buf], (g >> 1) & 1, abort_word, p.err, 514);
+        // one lane asks: 32 of them are served one after the other
+        ok = (PAIR && lane != 0) || mbar_wait(&tail->acc_full[buf], (g >> 1) & 1, abort_word, p.err, 514);
+        if (PAIR) ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) break;
         ++g;
         tc_fence_after();
@@ -546,7 +572,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
           for (int i = 0; i < W / 2; ++i) acc[c * (W / 2) + i] = fma2(v[c & 1][2 * i], v[c & 1][2 * i + 1], f2, acc[c * (W / 2) + i]);
         }
       }
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      if (!PAIR) asm volatile("cp.async.wait_group 0;" ::: "memory");
       if (!ok) break;
       // 64 features (one 128-byte line) at a time; a residual line is read before the line before it is written
       __nv_bfloat16* y = p.Y + static_cast<size_t>(live ? row : 0) * p.ldy + col0;
