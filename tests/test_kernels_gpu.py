@@ -93,6 +93,24 @@ def test_gemm_pair_token_major(M, N, K):
     ops.check_device_error()
 
 
+@pytest.mark.parametrize("M", [3073, 3328, 6401, 9300])           # token tiles of 256: one more than a band holds, two bands, three, four
+def test_gemm_pair_bands_of_token_tiles(M):
+    """Tiles walked in bands: every tile once, whatever the last band's height; the same sums as the one-CTA kernel."""
+    torch.manual_seed(9)
+    N, K = 2312, 192                                              # ten feature blocks, the last one 8 wide
+    x = torch.randn(M, K, device=DEV, dtype=torch.bfloat16)
+    w = (torch.randn(N, K, device=DEV) * 0.05).to(torch.bfloat16)
+    r = torch.randn(M, N, device=DEV, dtype=torch.bfloat16)
+    y, yr, ys = (torch.full((M, n), float("nan"), device=DEV, dtype=torch.bfloat16) for n in (N, N, 1152))
+    ops.linear(x, w, out=y, impl="pair")
+    ops.linear(x, w, residual=r, out=yr, impl="pair")
+    ops.linear_swiglu(x, w[:2304], out=ys, impl="pair")
+    assert torch.equal(y, ops.linear(x, w, impl="tiled"))
+    assert torch.equal(yr, ops.linear(x, w, residual=r, impl="tiled"))
+    assert torch.equal(ys, ops.linear_swiglu(x, w[:2304], impl="tiled"))
+    ops.check_device_error()
+
+
 def test_gemm_pair_persistent_swiglu():
     torch.manual_seed(6)
     M, K, I = 2176, 1024, 1536                    # 17 token tiles x 6 row pairs: more tiles than pairs of SMs
