@@ -325,6 +325,70 @@ void rope_kv_store(Tensor& qkv, const Tensor& positions, const Tensor& slots, co
            "rope_kv_store");
 }
 
+// The pieces of a step of few tokens (norms and rope inside the split-K reductions). `part` is fp32 scratch that
+// gemm_partials fills with [splits][M][N].
+int gemm_partials(const Tensor& x, const Tensor& w, Tensor& part) {
+  need_cuda(x, "x");
+  TORCH_CHECK(x.is_contiguous() && w.is_contiguous() && x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) &&
+                  x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
+                  part.scalar_type() == at::kFloat && part.is_contiguous(),
+              "gemm_partials: x [M, K], w [N, K] bf16, part fp32");
+  int splits = 1;
+  check_rc(mb_gemm_bf16_partials(x.data_ptr(), w.data_ptr(), x.size(0), w.size(0), x.size(1), 0, part.data_ptr(),
+                                 part.nbytes(), &splits, error_flag(), num_sms(), cur_stream()),
+           "gemm_partials");
+  return splits;
+}
+
+void reduce_residual(const Tensor& part, int splits, Tensor& h, const Tensor& w, double offset, Tensor& xw, Tensor& ssq) {
+  need_cuda(h, "h");
+  TORCH_CHECK(h.dim() == 2 && h.is_contiguous() && xw.is_contiguous() && xw.sizes() == h.sizes() && w.is_contiguous() &&
+                  w.numel() == h.size(1) && h.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
+                  xw.scalar_type() == at::kBFloat16 && ssq.scalar_type() == at::kFloat && ssq.is_contiguous() &&
+                  ssq.numel() >= h.size(0) * mb_ssq_blocks(h.size(1)) && splits > 0 &&
+                  part.scalar_type() == at::kFloat && part.is_contiguous() && part.numel() >= splits * h.numel(),
+              "reduce_residual: shapes");
+  check_rc(mb_reduce_residual(part.data_ptr<float>(), splits, h.data_ptr(), w.data_ptr(), offset, xw.data_ptr(),
+                              ssq.data_ptr<float>(), h.size(0), h.size(1), cur_stream()),
+           "reduce_residual");
+}
+
+void reduce_rope_store(const Tensor& part, int splits, const c10::optional<Tensor>& ssq, int hidden, double eps,
+                       Tensor& qkv, const Tensor& positions, const Tensor& slots, const Tensor& cos_sin,
+                       Tensor& k_cache, Tensor& v_cache, int n_q, int n_kv, int head_dim, bool interleaved) {
+  need_cuda(qkv, "qkv");
+  TORCH_CHECK(qkv.is_contiguous() && qkv.dim() == 2 && qkv.size(1) == (n_q + 2 * n_kv) * head_dim &&
+                  positions.scalar_type() == at::kInt && slots.scalar_type() == at::kLong &&
+                  cos_sin.scalar_type() == at::kFloat && splits > 0 && part.scalar_type() == at::kFloat &&
+                  part.is_contiguous() && part.numel() >= splits * qkv.numel(),
+              "reduce_rope_store: shapes");
+  TORCH_CHECK(k_cache.dim() == 4 && k_cache.stride(3) == 1 && k_cache.stride(2) == head_dim, "cache layout");
+  TORCH_CHECK(v_cache.stride(0) == k_cache.stride(0) && v_cache.stride(1) == k_cache.stride(1), "k/v strides");
+  const bool normed = ssq.has_value() && ssq->defined();
+  TORCH_CHECK(!normed || (ssq->scalar_type() == at::kFloat && ssq->is_contiguous() &&
+                          ssq->numel() >= qkv.size(0) * mb_ssq_blocks(hidden)), "ssq");
+  check_rc(mb_reduce_rope_store(part.data_ptr<float>(), splits, normed ? ssq->data_ptr<float>() : nullptr, hidden, eps,
+                                qkv.data_ptr(), positions.data_ptr<int32_t>(), slots.data_ptr<int64_t>(),
+                                cos_sin.data_ptr<float>(), k_cache.data_ptr(), v_cache.data_ptr(), qkv.size(0), n_q,
+                                n_kv, head_dim, k_cache.size(2), k_cache.stride(0), k_cache.stride(1), interleaved,
+                                cur_stream()),
+           "reduce_rope_store");
+}
+
+void swiglu_normed(const Tensor& x, const Tensor& w, Tensor& y, const Tensor& ssq, double eps) {
+  need_cuda(x, "x");
+  TORCH_CHECK(x.is_contiguous() && w.is_contiguous() && y.is_contiguous() && x.dim() == 2 && w.dim() == 2 &&
+                  y.dim() == 2 && w.size(1) == x.size(1) && y.size(0) == x.size(0) && w.size(0) == 2 * y.size(1) &&
+                  x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
+                  y.scalar_type() == at::kBFloat16 && ssq.scalar_type() == at::kFloat && ssq.is_contiguous() &&
+                  ssq.numel() >= x.size(0) * mb_ssq_blocks(x.size(1)),
+              "swiglu_normed: x [M, K], w [2 N, K], y [M, N] bf16");
+  check_rc(mb_gemm_bf16_swiglu_normed(x.data_ptr(), w.data_ptr(), y.data_ptr(), x.size(0), y.size(1), x.size(1), 0,
+                                      ssq.data_ptr<float>(), mb_ssq_blocks(x.size(1)), eps, error_flag(), num_sms(),
+                                      cur_stream()),
+           "swiglu_normed");
+}
+
 void paged_attention(const Tensor& q, Tensor& out, const Tensor& k_cache, const Tensor& v_cache,
                      const Tensor& block_table, const Tensor& q_start, const Tensor& q_len,
                      const Tensor& kv_len, const c10::optional<Tensor>& tile_seq,
@@ -600,6 +664,7 @@ class PyDecoderExecutor {
     ex.tp.lam_rows = lam_rows;
   }
   bool dec_usable(int T) const { return ex.dec_usable(T); }
+  bool lean_usable(int T) const { return ex.lean_usable(T); }
   long launches() const { return ex.launches; }
   void set_profiling(bool on) { ex.profiling = on; }
   py::list profile() {
@@ -778,6 +843,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embedding", &embedding);
   m.def("gather_rows", &gather_rows);
   m.def("rope_kv_store", &rope_kv_store);
+  m.def("gemm_partials", &gemm_partials);
+  m.def("reduce_residual", &reduce_residual);
+  m.def("reduce_rope_store", &reduce_rope_store);
+  m.def("swiglu_normed", &swiglu_normed);
   m.def("paged_attention", &paged_attention);
   m.def("paged_attention_tma", &paged_attention_tma);
   m.def("argmax", &argmax);
@@ -1297,6 +1366,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("set_dec", &PyDecoderExecutor::set_dec)
       .def("set_tp_lamport", &PyDecoderExecutor::set_tp_lamport)
       .def("dec_usable", &PyDecoderExecutor::dec_usable)
+      .def("lean_usable", &PyDecoderExecutor::lean_usable)
       .def("forward", &PyDecoderExecutor::forward)
       .def("launches", &PyDecoderExecutor::launches)
       .def("set_profiling", &PyDecoderExecutor::set_profiling)

@@ -62,6 +62,23 @@ int mb_gemm_bf16_persistent(const void* X, const void* W, void* Y, const void* R
                             int force_mode, void* ws, int* counters, int* err, int num_sms,
                             cudaStream_t stream);
 
+// Steps of few tokens: the norm's factor is applied behind the products, so that the split-K reductions do the work of
+// the norm and rope launches. `ssq` holds one sum of squares per row and 1024 columns, mb_ssq_blocks(hidden) of them.
+//   mb_gemm_bf16_partials: fp32 K splits of X · W^T in `ws` ([*splits][M][N]; MB_ERR_TOO_LARGE if one does not fit)
+//   mb_reduce_residual:    H += sum of splits, XW = H * (w + offset), ssq of H
+//   mb_reduce_rope_store:  QKV = sum of splits * factor, rotated, keys and values to the cache (ssq nullptr: factor 1)
+int mb_ssq_blocks(int hidden);
+int mb_gemm_bf16_partials(const void* X, const void* W, int M, int N, int K, int flags, void* ws, size_t ws_bytes,
+                          int* splits, int* err, int num_sms, cudaStream_t stream);
+int mb_reduce_residual(const float* part, int splits, void* H, const void* w, float offset, void* XW, float* ssq,
+                       int M, int N, cudaStream_t stream);
+int mb_reduce_rope_store(const float* part, int splits, const float* ssq, int hidden, float eps, void* qkv,
+                         const int32_t* positions, const int64_t* slots, const float* cos_sin, void* k_cache,
+                         void* v_cache, int T, int n_q, int n_kv, int head_dim, int page_size, int64_t page_stride,
+                         int64_t head_stride, int interleaved, cudaStream_t stream);
+int mb_gemm_bf16_swiglu_normed(const void* X, const void* W, void* Y, int M, int N, int K, int flags, const float* ssq,
+                               int ssq_blocks, float eps, int* err, int num_sms, cudaStream_t stream);
+
 // Decode-step GEMM (gemm_decode.cu): M <= 256 tokens, equal K-block shares on every SM, epilogue over the
 // whole output after one grid-wide meeting point. mode 0 bf16 store, 1 SwiGLU over W = [gate; up],
 // 2 all-reduce over `world` ranks (sentinel-polled receive buffers `lam`) + residual `h` + RMSNorm -> `xn`.

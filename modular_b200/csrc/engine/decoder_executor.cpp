@@ -192,6 +192,25 @@ int DecoderExecutor::forward_dec(const StepInputs& in, cudaStream_t stream) {
   return MB_OK;
 }
 
+// Steps of few tokens with bf16 weights: norms and rope ride on the split-K reductions. The bound is the rows whose
+// factors the SwiGLU kernel's epilogue holds; it also lies below the first token count of the pair kernels.
+bool DecoderExecutor::lean_usable(int T) const {
+  const DecoderConfig& c = cfg;
+  constexpr int kMaxRows = 128;
+  if (T <= 0 || T > kMaxRows || c.gemm_impl != 2 || !c.fuse_swiglu || buf.p_ws == nullptr || c.head_dim % 16)
+    return false;
+  const int qkv_dim = (c.n_q + 2 * c.n_kv) * c.head_dim;
+  const size_t rows = static_cast<size_t>(T) * sizeof(float);
+  if (rows * (qkv_dim > c.hidden ? qkv_dim : c.hidden) + rows * mb_ssq_blocks(c.hidden) + 16 > buf.workspace_bytes)
+    return false;
+  for (const DecoderLayerWeights& w : layers)
+    if (w.wqkv_s || w.wo_s || w.wgu_s || w.wd_s || w.qkv_bias || w.q_norm) return false;
+  for (const int n : {qkv_dim, c.hidden}) {
+    if ((n + 127) / 128 >= 4 * c.num_sms || mb_gemm_pair_choice(T, n, 0, c.num_sms)) return false;
+  }
+  return !mb_gemm_pair_choice(T, c.inter, 1, c.num_sms);
+}
+
 int DecoderExecutor::forward(const StepInputs& in, cudaStream_t stream) {
   if (dec_usable(in.T)) return forward_dec(in, stream);
   if (tp.world > 1) return forward_tp(in, stream);
@@ -237,6 +256,24 @@ int DecoderExecutor::forward(const StepInputs& in, cudaStream_t stream) {
                         stages, buf.workspace, buf.err, c.num_sms, stream);
   };
 
+  const bool lean = lean_usable(T);
+  // the sums of squares stand behind the partial products
+  const size_t ssq_bytes = lean ? (static_cast<size_t>(T) * mb_ssq_blocks(c.hidden) * sizeof(float) + 15) / 16 * 16 : 0;
+  const size_t part_bytes = (buf.workspace_bytes - ssq_bytes) / 16 * 16;
+  float* part = static_cast<float*>(buf.workspace);
+  float* ssq = reinterpret_cast<float*>(static_cast<char*>(buf.workspace) + part_bytes);
+  int splits = 1;
+  auto partials = [&](const void* X, const void* W, int N, int K) {
+    launches += 2;   // the product and the reduction that follows it
+    return mb_gemm_bf16_partials(X, W, T, N, K, c.prefetch_weights ? 128 : 0, part, part_bytes, &splits, buf.err,
+                                 c.num_sms, stream);
+  };
+  // buf.h += X · W^T; buf.xn = buf.h * norm weight, its factor left to the next product
+  auto residual = [&](const void* X, const void* W, int K, const void* norm) {
+    MB_TRY(partials(X, W, c.hidden, K));
+    return mb_reduce_residual(part, splits, buf.h, norm, c.norm_weight_offset, buf.xn, ssq, T, c.hidden, stream);
+  };
+
   mark("begin", stream);
   if (in.future_src != nullptr) {
     MB_TRY(mb_realize_future_tokens(const_cast<int64_t*>(in.tokens), in.future_src, buf.sampled, T,
@@ -251,10 +288,19 @@ int DecoderExecutor::forward(const StepInputs& in, cudaStream_t stream) {
     char* kbase = static_cast<char*>(kv.base) + 2 * (static_cast<int64_t>(l) * kv.layer_stride);
     void* kc = kbase;
     void* vc = kbase + 2 * kv.kv_stride;
-    MB_TRY(mb_rmsnorm(buf.h, w.attn_norm, buf.xn, T, c.hidden, c.hidden, c.hidden, c.eps,
-                      c.norm_weight_offset, c.multiply_before_cast, stream));
-    mark("rmsnorm", stream);
-    if (w.wqkv_s != nullptr) {
+    if (!lean || l == 0) {
+      MB_TRY(mb_rmsnorm(buf.h, w.attn_norm, buf.xn, T, c.hidden, c.hidden, c.hidden, c.eps,
+                        c.norm_weight_offset, c.multiply_before_cast, stream));
+      launches += 1;
+      mark("rmsnorm", stream);
+    }
+    if (lean) {
+      MB_TRY(partials(buf.xn, w.wqkv, qkv_dim, c.hidden));
+      mark("gemm_qkv", stream);
+      MB_TRY(mb_reduce_rope_store(part, splits, l == 0 ? nullptr : ssq, c.hidden, c.eps, buf.qkv, in.positions,
+                                  in.slots, cos_sin, kc, vc, T, c.n_q, c.n_kv, c.head_dim, c.page_size,
+                                  kv.page_stride, kv.head_stride, c.rope_interleaved, stream));
+    } else if (w.wqkv_s != nullptr) {
       MB_TRY(linear_fp8(buf, c, buf.xn, c.hidden, w.wqkv, w.wqkv_s, buf.qkv, nullptr, T, qkv_dim, c.hidden,
                         &launches, stream));
     } else {
@@ -268,10 +314,13 @@ int DecoderExecutor::forward(const StepInputs& in, cudaStream_t stream) {
       MB_TRY(mb_qk_norm(buf.qkv, w.q_norm, w.k_norm, T, c.n_q, c.n_kv, c.head_dim, qkv_dim, c.eps, stream));
       launches += 1;
     }
-    mark("gemm_qkv", stream);
-    MB_TRY(mb_rope_kv_store(buf.qkv, in.positions, in.slots, cos_sin, kc, vc, T, c.n_q, c.n_kv,
-                            c.head_dim, c.page_size, kv.page_stride, kv.head_stride,
-                            c.rope_interleaved, stream));
+    if (!lean) {
+      mark("gemm_qkv", stream);
+      MB_TRY(mb_rope_kv_store(buf.qkv, in.positions, in.slots, cos_sin, kc, vc, T, c.n_q, c.n_kv,
+                              c.head_dim, c.page_size, kv.page_stride, kv.head_stride,
+                              c.rope_interleaved, stream));
+      launches += 1;
+    }
     mark("rope_kv_store", stream);
     if (c.attn_impl == 1 && c.page_size % 64 == 0) {
       const long long hd = c.head_dim;
@@ -282,27 +331,36 @@ int DecoderExecutor::forward(const StepInputs& in, cudaStream_t stream) {
           in.block_table, in.bt_stride, in.q_start, in.q_len, in.kv_len, in.tile_seq, in.tile_q0,
           in.n_tiles, in.n_decode, in.decode_seq, c.n_q, c.n_kv, c.head_dim, c.page_size,
           c.attn_scale, buf.err, stream));
-      launches += 3;   // rmsnorm, rope+store, attention
+      launches += 1;
     } else {
       MB_TRY(mb_paged_attention(buf.qkv, qkv_dim, buf.attn, q_dim, kc, vc, in.block_table,
                                 in.bt_stride, in.q_start, in.q_len, in.kv_len, in.tile_seq,
                                 in.tile_q0, in.n_tiles, in.n_decode, in.decode_seq, c.n_q, c.n_kv,
                                 c.head_dim, c.page_size, kv.page_stride, kv.head_stride,
                                 c.attn_scale, stream));
-      launches += 2 + (in.n_tiles > 0) + (in.n_decode > 0);
+      launches += (in.n_tiles > 0) + (in.n_decode > 0);
     }
     mark("attention", stream);
-    if (w.wo_s != nullptr) {
+    if (lean) {
+      MB_TRY(residual(buf.attn, w.wo, q_dim, w.mlp_norm));
+    } else if (w.wo_s != nullptr) {
       MB_TRY(linear_fp8(buf, c, buf.attn, q_dim, w.wo, w.wo_s, buf.h, buf.h, T, c.hidden, q_dim, &launches, stream));
     } else {
       MB_TRY(gemm(buf.attn, w.wo, buf.h, buf.h, T, c.hidden, q_dim, q_dim, c.hidden, 2));
     }
     mark("gemm_o", stream);
-    MB_TRY(mb_rmsnorm(buf.h, w.mlp_norm, buf.xn, T, c.hidden, c.hidden, c.hidden, c.eps,
-                      c.norm_weight_offset, c.multiply_before_cast, stream));
-    launches += 1;
-    mark("rmsnorm", stream);
-    if (w.wgu_s != nullptr) {
+    if (!lean) {
+      MB_TRY(mb_rmsnorm(buf.h, w.mlp_norm, buf.xn, T, c.hidden, c.hidden, c.hidden, c.eps,
+                        c.norm_weight_offset, c.multiply_before_cast, stream));
+      launches += 1;
+      mark("rmsnorm", stream);
+    }
+    if (lean) {
+      MB_TRY(mb_gemm_bf16_swiglu_normed(buf.xn, w.wgu, buf.act, T, c.inter, c.hidden,
+                                        (c.use_pdl ? 8 : 0) | (c.prefetch_weights ? 128 : 0), ssq,
+                                        mb_ssq_blocks(c.hidden), c.eps, buf.err, c.num_sms, stream));
+      launches += 1;
+    } else if (w.wgu_s != nullptr) {
       if (buf.gu == nullptr) return MB_ERR_SHAPE;
       MB_TRY(linear_fp8(buf, c, buf.xn, c.hidden, w.wgu, w.wgu_s, buf.gu, nullptr, T, 2 * c.inter, c.hidden,
                         &launches, stream));
@@ -317,7 +375,9 @@ int DecoderExecutor::forward(const StepInputs& in, cudaStream_t stream) {
       launches += 1;
     }
     mark("gemm_gate_up", stream);
-    if (w.wd_s != nullptr) {
+    if (lean && l + 1 < c.n_layers) {
+      MB_TRY(residual(buf.act, w.wd, c.inter, layers[l + 1].attn_norm));
+    } else if (w.wd_s != nullptr) {
       MB_TRY(linear_fp8(buf, c, buf.act, c.inter, w.wd, w.wd_s, buf.h, buf.h, T, c.hidden, c.inter, &launches, stream));
     } else {
       MB_TRY(gemm(buf.act, w.wd, buf.h, buf.h, T, c.hidden, c.inter, c.inter, c.hidden, 2));

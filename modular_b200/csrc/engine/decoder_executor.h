@@ -152,6 +152,9 @@ class DecoderExecutor {
   // True when a step of T tokens takes the decode-step path (forward_dec).
   bool dec_usable(int T) const;
 
+  // True when forward() lets a step of T tokens do its norms and rope inside the split-K reductions.
+  bool lean_usable(int T) const;
+
   // Per-kernel timing of eager (not graph-captured) steps: when `profiling` is set, an event is
   // recorded after every launch group; profile_ms() synchronises and returns, per label, the
   // number of intervals and their summed duration since the last call.

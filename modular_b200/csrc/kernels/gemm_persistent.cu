@@ -72,7 +72,14 @@ struct Params {
   int gate_rpr, gate_world;
   int packed_kb;     // > 0: W is pre-tiled [rows/128][K/64][128][64]; value = K/64
   int w_static;      // W is written by no kernel of the stream: its first tiles are requested before the dependency wait
+  // Rows of X that still lack their RMSNorm factor (nullptr = none; SwiGLU, whole tiles, M <= kNormRows only): row t
+  // has the sum of squares ssq[t * ssq_blocks ..], and both products of a token are scaled by
+  // rsqrt(sum * inv_cols + eps) before the activation.
+  const float* ssq;
+  int ssq_blocks;
+  float inv_cols, eps;
 };
+constexpr int kNormRows = 128;
 
 struct Tail {
   uint64_t full[8];
@@ -325,6 +332,18 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW,
     const size_t slot_floats = static_cast<size_t>(p.acc_cols) * kBM;
     SegIter it(p, g, G);
     Seg s;
+    // every lane keeps the factors of the tokens lane, lane + 32, ...; a chunk of 16 tokens fetches its own by shuffle
+    float factor[kNormRows / 32];
+    if (DUAL && p.ssq != nullptr) {
+#pragma unroll
+      for (int i = 0; i < kNormRows / 32; ++i) {
+        const int t = i * 32 + lane;
+        float sum = 0.f;
+        if (t < p.M)
+          for (int b = 0; b < p.ssq_blocks; ++b) sum += p.ssq[t * p.ssq_blocks + b];
+        factor[i] = rsqrtf(sum * p.inv_cols + p.eps);
+      }
+    }
     while (it.next(s)) {
       const int buf = s.idx % p.nbufs;
       const uint32_t bph = (s.idx / p.nbufs) & 1;
@@ -345,6 +364,16 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmW,
             uint32_t b[16];
             tmem_ld_32x16(acc + p.BN + c0, b);
             tc_wait_ld();
+            if (p.ssq != nullptr) {
+              const int tg = (t0 + c0) >> 5;
+              const float f = tg == 0 ? factor[0] : tg == 1 ? factor[1] : tg == 2 ? factor[2] : factor[3];
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const float fj = __shfl_sync(0xffffffffu, f, ((t0 + c0) & 16) + j);
+                a[j] = __float_as_uint(__uint_as_float(a[j]) * fj);
+                b[j] = __float_as_uint(__uint_as_float(b[j]) * fj);
+              }
+            }
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = silu_f(__uint_as_float(a[j])) * __uint_as_float(b[j]);
           } else {
@@ -545,12 +574,10 @@ extern "C" int mb_gemm_bf16_persistent(const void* X, const void* W, void* Y, co
                                        ws, counters, err, num_sms, nullptr, 1, 0, stream);
 }
 
-// Same kernel with tensor-parallel gating of the token tiles (see Params::gate_flags).
-extern "C" int mb_gemm_bf16_persistent_gated(const void* X, const void* W, void* Y, const void* R, int M,
-                                             int N, int K, int ldx, int ldw, int ldy, int ldr, int flags,
-                                             int bn, int stages, int force_mode, void* ws, int* counters,
-                                             int* err, int num_sms, const int* gate_flags, int gate_rpr,
-                                             int gate_world, cudaStream_t stream) {
+static int run_persistent(const void* X, const void* W, void* Y, const void* R, int M, int N, int K, int ldx, int ldw,
+                          int ldy, int ldr, int flags, int bn, int stages, int force_mode, void* ws, int* counters,
+                          int* err, int num_sms, const int* gate_flags, int gate_rpr, int gate_world,
+                          const float* ssq, int ssq_blocks, float eps, cudaStream_t stream) {
   using namespace mb::pg;
   if (gate_flags != nullptr && (gate_rpr < 1 || gate_world < 1 || gate_world > mb::kMaxRanks)) return MB_ERR_SHAPE;
   if (M <= 0 || N <= 0) return MB_OK;
@@ -586,6 +613,7 @@ extern "C" int mb_gemm_bf16_persistent_gated(const void* X, const void* W, void*
   if (bn % 16 || bn < 16 || bn > max_bn) return MB_ERR_SHAPE;
   Params p;
   p.gate_flags = gate_flags; p.gate_rpr = gate_rpr; p.gate_world = gate_world;
+  p.ssq = ssq; p.ssq_blocks = ssq_blocks; p.inv_cols = 1.0f / static_cast<float>(K); p.eps = eps;
   p.packed_kb = packed ? K / kBK : 0;
   p.w_static = (flags & 128) ? 1 : 0;
   p.Y = Y; p.R = static_cast<const __nv_bfloat16*>(R);
@@ -644,4 +672,24 @@ extern "C" int mb_gemm_bf16_persistent_gated(const void* X, const void* W, void*
   if (f32) return launch<false, EPI_F32>(tw, tx, p, grid, pdl, stream);
   if (resid) return launch<false, EPI_RESID>(tw, tx, p, grid, pdl, stream);
   return launch<false, EPI_BF16>(tw, tx, p, grid, pdl, stream);
+}
+
+// Same kernel with tensor-parallel gating of the token tiles (see Params::gate_flags).
+extern "C" int mb_gemm_bf16_persistent_gated(const void* X, const void* W, void* Y, const void* R, int M,
+                                             int N, int K, int ldx, int ldw, int ldy, int ldr, int flags,
+                                             int bn, int stages, int force_mode, void* ws, int* counters,
+                                             int* err, int num_sms, const int* gate_flags, int gate_rpr,
+                                             int gate_world, cudaStream_t stream) {
+  return run_persistent(X, W, Y, R, M, N, K, ldx, ldw, ldy, ldr, flags, bn, stages, force_mode, ws, counters, err,
+                        num_sms, gate_flags, gate_rpr, gate_world, nullptr, 0, 0.f, stream);
+}
+
+// Y[M, N] = SwiGLU(rmsnorm-scaled X · [gate; up]^T) for at most 128 rows X = h * weight whose factor
+// rsqrt(sum of squares of h / K + eps) is applied to the products (see Params::ssq). flags: bits 3 and 7 of the others.
+extern "C" int mb_gemm_bf16_swiglu_normed(const void* X, const void* W, void* Y, int M, int N, int K, int flags,
+                                          const float* ssq, int ssq_blocks, float eps, int* err, int num_sms,
+                                          cudaStream_t stream) {
+  if (M > mb::pg::kNormRows || ssq == nullptr || ssq_blocks < 1) return MB_ERR_SHAPE;
+  return run_persistent(X, W, Y, nullptr, M, N, K, K, K, N, N, 1 | (flags & (8 | 128)), 0, 0, 0, nullptr, nullptr, err,
+                        num_sms, nullptr, 1, 0, ssq, ssq_blocks, eps, stream);
 }

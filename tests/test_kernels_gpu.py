@@ -1211,3 +1211,56 @@ def test_paged_attention_decode_split(n_q, n_kv, hd, ps, case, split):
         assert _rel_err(o, o_ref) < 1e-2
         assert (o.float() - o_ref.float()).abs().max() < 3e-2
     assert torch.equal(outs[0], outs[1]), "the combine order must not depend on arrival order"
+
+
+@pytest.mark.parametrize("M,hidden,inter,n_q,n_kv,hd,interleaved", [
+    (1, 4096, 1024, 8, 2, 128, False), (7, 1032, 520, 3, 1, 16, True), (33, 2048, 136, 4, 4, 64, False),
+    (128, 1024, 8200, 2, 1, 128, True)])
+def test_norm_and_rope_inside_the_split_reductions(M, hidden, inter, n_q, n_kv, hd, interleaved):
+    """A step's pieces against float64 on the stored operands of each: half a unit of bf16 (2^-9) for the value stored,
+    as much again for the rounded operand where one result feeds the next check, and 2^-10 for fp32 sums of order one."""
+    from modular_b200._native import lib
+    from modular_b200.nn.rotary_embedding import cos_sin_table
+
+    torch.manual_seed(41)
+    mk = lambda *s, scale=1.0: (torch.randn(*s, device=DEV) * scale).to(torch.bfloat16)
+    close = lambda a, b: torch.allclose(a.double(), b.double(), rtol=2 ** -8, atol=2 ** -10)
+    eps, offset, nblk = 1e-5, 1.0, (hidden + 1023) // 1024
+    part = torch.empty(8 * M * max(hidden, (n_q + 2 * n_kv) * hd), device=DEV)
+    x, wo, h, g = mk(M, 512), mk(hidden, 512, scale=512 ** -0.5), mk(M, hidden), mk(hidden, scale=0.2)
+    want = h.double() + x.double() @ wo.double().T
+    xw, ssq = torch.full_like(h, float("nan")), torch.full((M, nblk), float("nan"), device=DEV)
+    lib().reduce_residual(part, lib().gemm_partials(x, wo, part), h, g, offset, xw, ssq)
+    assert close(h, want)
+    assert torch.equal(xw, (h.float() * (g.float() + offset)).to(torch.bfloat16))
+    assert torch.allclose(ssq.double().sum(1), h.double().square().sum(1), rtol=1e-5)
+    f = (h.double().square().mean(1, keepdim=True) + eps).rsqrt()
+
+    wgu, act = mk(2 * inter, hidden, scale=hidden ** -0.5), torch.full((M, inter), float("nan"), device=DEV, dtype=torch.bfloat16)
+    lib().swiglu_normed(xw, wgu, act, ssq, eps)
+    gate, up = ((xw.double() @ wgu.double().T) * f).chunk(2, 1)
+    assert close(act, torch.nn.functional.silu(gate) * up)
+
+    page, pages, N = 16, 20, (n_q + 2 * n_kv) * hd
+    w = mk(N, hidden, scale=hidden ** -0.5)
+    cs = cos_sin_table(hd, 2048, 500000.0, None, DEV)
+    pos = torch.randint(0, 2048, (M,), device=DEV, dtype=torch.int32)
+    slots = torch.randperm(page * pages, device=DEV)[:M].long()
+    slots[M // 2:M // 2 + (M > 1)] = -1
+    for scale in (None, ssq):
+        kv, kv_want = (torch.zeros(pages, 2, n_kv, page, hd, device=DEV, dtype=t) for t in (torch.bfloat16, torch.double))
+        qkv = torch.zeros(M, N, device=DEV, dtype=torch.bfloat16)
+        lib().reduce_rope_store(part, lib().gemm_partials(xw, w, part), scale, hidden, eps, qkv, pos, slots, cs, kv[:, 0],
+                                kv[:, 1], n_q, n_kv, hd, interleaved)
+        exact = (xw.double() @ w.double().T) * (1.0 if scale is None else f)
+        heads = exact.view(M, n_q + 2 * n_kv, hd).clone()
+        c, s = cs.double()[pos.long()][:, None].chunk(2, -1)
+        rot = heads[:, : n_q + n_kv]
+        a, b = (rot[..., 0::2], rot[..., 1::2]) if interleaved else rot.chunk(2, -1)
+        ra, rb = a * c - b * s, b * c + a * s
+        rot = torch.stack([ra, rb], -1).flatten(-2) if interleaved else torch.cat([ra, rb], -1)
+        keep = slots >= 0
+        kv_want[slots[keep] // page, 0, :, slots[keep] % page] = rot[keep, n_q:]
+        kv_want[slots[keep] // page, 1, :, slots[keep] % page] = heads[keep, n_q + n_kv:]
+        assert close(qkv.view(M, -1, hd)[:, :n_q], rot[:, :n_q]) and close(kv, kv_want)
+    ops.check_device_error()
