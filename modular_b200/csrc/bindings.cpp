@@ -411,6 +411,8 @@ void paged_attention(const Tensor& q, Tensor& out, const Tensor& k_cache, const 
 }
 
 // TMA-fed attention over the whole cache tensor kv: [pages, 2, layers, n_kv, page_size, head_dim].
+// STEP: the launch before on the stream wrote the queries and new cache rows only (mb_paged_attention_tma_step)
+template <bool STEP>
 void paged_attention_tma(const Tensor& q, Tensor& out, const Tensor& kv, int layer,
                          const Tensor& block_table, const Tensor& q_start, const Tensor& q_len,
                          const Tensor& kv_len, const c10::optional<Tensor>& tile_seq,
@@ -423,7 +425,7 @@ void paged_attention_tma(const Tensor& q, Tensor& out, const Tensor& kv, int lay
   const int n_tiles = tile_seq.has_value() && tile_seq->defined() ? tile_seq->numel() : 0;
   const int n_dec = decode_seq.has_value() && decode_seq->defined() ? decode_seq->numel() : 0;
   const long long hd = head_dim;
-  check_rc(mb_paged_attention_tma(
+  check_rc((STEP ? mb_paged_attention_tma_step : mb_paged_attention_tma)(
                q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), kv.data_ptr(), kv.numel() / hd,
                layer * kv.stride(2) / hd, (layer * kv.stride(2) + kv.stride(1)) / hd, kv.stride(0) / hd,
                block_table.data_ptr<int32_t>(), block_table.stride(0), q_start.data_ptr<int32_t>(),
@@ -848,7 +850,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("reduce_rope_store", &reduce_rope_store);
   m.def("swiglu_normed", &swiglu_normed);
   m.def("paged_attention", &paged_attention);
-  m.def("paged_attention_tma", &paged_attention_tma);
+  m.def("paged_attention_tma", &paged_attention_tma<false>);
+  m.def("paged_attention_tma_step", &paged_attention_tma<true>);
   m.def("argmax", &argmax);
   m.def("sample", &sample);
   m.def("apply_penalties", &apply_penalties);

@@ -197,6 +197,14 @@ int mb_paged_attention_tma(const void* q, int ldq, void* out, int ldo, const voi
                            const int32_t* tile_seq, const int32_t* tile_q0, int n_tiles, int n_decode,
                            const int32_t* decode_seq, int n_q, int n_kv, int head_dim, int page_size,
                            float scale, int* err, cudaStream_t stream);
+// ... whose previous launch wrote the step's queries and cache rows only: may start reading older rows under it
+int mb_paged_attention_tma_step(const void* q, int ldq, void* out, int ldo, const void* kv_base,
+                                long long total_rows, long long k_off_rows, long long v_off_rows,
+                                long long page_rows, const int32_t* block_table, int bt_stride,
+                                const int32_t* q_start, const int32_t* q_len, const int32_t* kv_len,
+                                const int32_t* tile_seq, const int32_t* tile_q0, int n_tiles, int n_decode,
+                                const int32_t* decode_seq, int n_q, int n_kv, int head_dim, int page_size,
+                                float scale, int* err, cudaStream_t stream);
 // ... with a sliding window and a sink score per query head; prompt tiles (128 / G tokens for head_dim 128, 64 / G for
 // 64) or one-token rows
 int mb_paged_attention_window(const void* q, int ldq, void* out, int ldo, const void* kv_base, long long total_rows,

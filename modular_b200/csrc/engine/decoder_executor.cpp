@@ -324,7 +324,7 @@ int DecoderExecutor::forward(const StepInputs& in, cudaStream_t stream) {
     mark("rope_kv_store", stream);
     if (c.attn_impl == 1 && c.page_size % 64 == 0) {
       const long long hd = c.head_dim;
-      MB_TRY(mb_paged_attention_tma(
+      MB_TRY(mb_paged_attention_tma_step(
           buf.qkv, qkv_dim, buf.attn, q_dim, kv.base, kv.total_elems / hd,
           static_cast<long long>(l) * kv.layer_stride / hd,
           (static_cast<long long>(l) * kv.layer_stride + kv.kv_stride) / hd, kv.page_stride / hd,

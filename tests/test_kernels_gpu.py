@@ -1264,3 +1264,41 @@ def test_norm_and_rope_inside_the_split_reductions(M, hidden, inter, n_q, n_kv, 
         kv_want[slots[keep] // page, 1, :, slots[keep] % page] = heads[keep, n_q + n_kv:]
         assert close(qkv.view(M, -1, hd)[:, :n_q], rot[:, :n_q]) and close(kv, kv_want)
     ops.check_device_error()
+
+
+@pytest.mark.parametrize("n_kv,hd,lens", [
+    (8, 128, (1, 2, 64, 65, 128, 129, 700)),                # tiles shared out over CTAs
+    (2, 64, (64, 1, 1000)),
+    (8, 128, tuple(1 + 37 * i % 300 for i in range(40))),   # one CTA per sequence and head
+    (4, 128, (64, 65, 192, 193, 1) * 12)])
+def test_decode_attention_started_under_the_cache_store(n_kv, hd, lens):
+    """Older tiles are requested before the launch that stores the step's own rows has ended: the same bits."""
+    from modular_b200._native import lib
+    from modular_b200.nn.rotary_embedding import cos_sin_table
+
+    torch.manual_seed(42)
+    B, n_q, ps = len(lens), 4 * n_kv, 64
+    per = [-(-n // ps) for n in lens]
+    order = torch.randperm(sum(per)).tolist()
+    bt = torch.zeros(B, max(per), dtype=torch.int32)
+    for b, n in enumerate(per):
+        bt[b, :n] = torch.tensor([order.pop() for _ in range(n)])
+    kv_len = torch.tensor(lens, dtype=torch.int32)
+    pos = kv_len - 1
+    slots = (bt[torch.arange(B), (pos // ps).long()].long() * ps + pos % ps).to(DEV)
+    ones, start = torch.ones(B, dtype=torch.int32, device=DEV), torch.arange(B, dtype=torch.int32, device=DEV)
+    bt, kv_len, pos = bt.to(DEV), kv_len.to(DEV), pos.to(DEV)
+    kv0 = torch.randn(sum(per), 2, 2, n_kv, ps, hd, device=DEV).to(torch.bfloat16)
+    qkv0 = torch.randn(B, (n_q + 2 * n_kv) * hd, device=DEV).to(torch.bfloat16)
+    cs = cos_sin_table(hd, 2048, 500000.0, None, DEV)
+    ops.ensure_attention_split_workspace(torch.device(DEV))
+    got = []
+    for fn in (lib().paged_attention_tma, lib().paged_attention_tma_step, lib().paged_attention_tma_step):
+        kv, qkv = kv0.clone(), qkv0.clone()
+        out = torch.full((B, n_q * hd), float("nan"), device=DEV, dtype=torch.bfloat16)
+        torch.cuda.synchronize()
+        ops.rope_kv_store(qkv, pos, slots, cs, kv[:, 0, 1], kv[:, 1, 1], n_q, n_kv, hd, False)
+        fn(qkv, out, kv, 1, bt, start, ones, kv_len, None, None, start, n_q, n_kv, hd, hd ** -0.5)
+        got.append(out)
+    assert got[0].isfinite().all() and torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    ops.check_device_error()
