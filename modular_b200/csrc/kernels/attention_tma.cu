@@ -61,8 +61,8 @@ struct Params {
   // Decode steps whose launch before this one writes q and the cache rows of the step's own tokens and nothing else: the
   // metadata and the tiles of older tokens are requested before the programmatic-dependency wait. A CTA of a short
   // context spends most of its time on that chain of latencies (lengths, block table, first tiles), which then runs
-  // under the launch before: generating with 8 sequences of about 1000 tokens 83.6 -> 82.0 ms (2.2 us a layer), with 13
-  // sampled ones 82.4 -> 81.4 ms.
+  // under the launch before: generating with one sequence of 340 tokens 83.6 -> 82.0 ms (2.2 us a layer), with 13 sampled
+  // ones 82.4 -> 81.4 ms.
   bool early;
 };
 
@@ -568,15 +568,18 @@ attn_decode_split_kernel(const __grid_constant__ CUtensorMap tmKV, const Params 
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
       }
+      // The product that follows requests up to 27 MB of its weights as it starts. Tiles requested behind them waited
+      // 3 us longer (one sequence of 340 tokens), so it starts when the last tile is on its way.
+      if (p.early) {
+        pdl_wait();
+        pdl_trigger();
+      }
     }
     return;
   }
 
   // ------------------------------------------------------------ compute warps
-  if (p.early) {
-    pdl_wait();
-    pdl_trigger();
-  }
+  if (p.early) pdl_wait();
   int s = 0;
   uint32_t ph = 0;
   bool ok = true;

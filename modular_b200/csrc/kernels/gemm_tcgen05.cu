@@ -977,11 +977,13 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, const __nv_
   *reinterpret_cast<uint2*>(Y + static_cast<size_t>(t) * ldy + n) = out;
 }
 
-// Reductions of a step of few tokens. Such a layer is bound by its chain of launches (a norm of 8 rows of 4096 took
+// Reductions of a step of few tokens. Such a layer is bound by its chain of launches (a norm of one row of 4096 took
 // 4.2 us, rope 2.6 us, each plain reduction 1.4 to 2 us, next to 67 us of weights), and an RMSNorm's factor is one number
 // a row, which commutes with the product: the reduction of one product stores h * weight unscaled with its sums of
 // squares, and whoever finishes the next product applies the factor. That takes the norm and rope launches away: a layer
-// of hidden 4096, 32 / 8 heads and 14336 wide went from 102 to 96 us at 8 rows, from 126 to 123 us at 64.
+// of hidden 4096, 32 / 8 heads and 14336 wide went from 102 to 96 us at one row, from 126 to 121 us at 64.
+// The launch before either kernel is the product, which itself waited for all that came earlier: only the partial sums are
+// read after the dependency wait.
 constexpr int kSsqCols = 1024;   // columns of a block of reduce_residual_kernel: one sum of squares each
 constexpr int kMaxSplits = 8;
 
@@ -1013,14 +1015,18 @@ __global__ void __launch_bounds__(kSsqCols / 4)
 reduce_residual_kernel(const float* __restrict__ part, int splits, __nv_bfloat16* __restrict__ H,
                        const __nv_bfloat16* __restrict__ w, float offset, __nv_bfloat16* __restrict__ XW,
                        float* __restrict__ ssq, int M, int N) {
-  pdl_wait();
-  pdl_trigger();
   __shared__ float red[kSsqCols / 4 / 32];
   const int n = blockIdx.x * kSsqCols + threadIdx.x * 4, t = blockIdx.y;
+  const size_t at = static_cast<size_t>(t) * N + n;
+  uint2 hv, wv;
+  if (n < N) {
+    hv = *reinterpret_cast<const uint2*>(H + at);
+    wv = *reinterpret_cast<const uint2*>(w + n);
+  }
+  pdl_wait();
+  pdl_trigger();
   float sq = 0.f;
   if (n < N) {
-    const size_t at = static_cast<size_t>(t) * N + n;
-    const uint2 hv = *reinterpret_cast<const uint2*>(H + at), wv = *reinterpret_cast<const uint2*>(w + n);
     const float4 a = sum_splits(part + at, static_cast<size_t>(M) * N, splits);
     const float4 r = unpack4(hv), g = unpack4(wv);
     const uint2 out = pack4(a.x + r.x, a.y + r.y, a.z + r.z, a.w + r.w);
@@ -1051,13 +1057,11 @@ reduce_rope_store_kernel(const float* __restrict__ part, int splits, const float
                          const float* __restrict__ cos_sin, __nv_bfloat16* __restrict__ k_cache,
                          __nv_bfloat16* __restrict__ v_cache, int T, int n_q, int n_kv, int head_dim, int page_size,
                          int64_t page_stride, int64_t head_stride, int interleaved) {
-  pdl_wait();
-  pdl_trigger();
   const int half = head_dim >> 1, per_rot = half >> 2, per_v = head_dim >> 2;
   const int n_rot = (n_q + n_kv) * per_rot;
   const int t = blockIdx.y;
   int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= n_rot + n_kv * per_v) return;
+  if (w >= n_rot + n_kv * per_v) return;   // not the whole block: its other threads wait and trigger
   const int64_t slot = slots[t];
   const int row = (n_q + 2 * n_kv) * head_dim;
   const size_t stride = static_cast<size_t>(T) * row;
@@ -1070,19 +1074,23 @@ reduce_rope_store_kernel(const float* __restrict__ part, int splits, const float
   }
   const int64_t page = slot / page_size;
   const int64_t at = page * page_stride + (slot % page_size) * head_dim;
-  if (w >= n_rot) {
-    w -= n_rot;
-    const int h = w / per_v, d = (w % per_v) * 4;
+  const bool rot = w < n_rot;
+  const int h = rot ? w / per_rot : (w - n_rot) / per_v, d = (rot ? w % per_rot : (w - n_rot) % per_v) * 4;
+  float4 c = {}, s = {};
+  if (rot) {
+    const float* cs = cos_sin + static_cast<size_t>(positions[t]) * head_dim + d;
+    c = make_float4(cs[0], cs[1], cs[2], cs[3]);
+    s = make_float4(cs[half], cs[half + 1], cs[half + 2], cs[half + 3]);
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (!rot) {
     const float4 v = sum_splits(src + (n_q + n_kv + h) * head_dim + d, stride, splits);
     if (slot >= 0)
       *reinterpret_cast<uint2*>(v_cache + at + h * head_stride + d) = pack4(v.x * f, v.y * f, v.z * f, v.w * f);
     return;
   }
-  const int h = w / per_rot, d = (w % per_rot) * 4;
   const int d0 = interleaved ? 2 * d : d, d1 = interleaved ? 2 * d + 4 : half + d;
-  const float* cs = cos_sin + static_cast<size_t>(positions[t]) * head_dim + d;
-  const float4 c = make_float4(cs[0], cs[1], cs[2], cs[3]);
-  const float4 s = make_float4(cs[half], cs[half + 1], cs[half + 2], cs[half + 3]);
   float4 a = sum_splits(src + h * head_dim + d0, stride, splits), b = sum_splits(src + h * head_dim + d1, stride, splits);
   a.x *= f; a.y *= f; a.z *= f; a.w *= f;
   b.x *= f; b.y *= f; b.z *= f; b.w *= f;
@@ -1408,6 +1416,8 @@ extern "C" void mb_gemm_bf16_plan(int M, int N, int K, int dual, int num_sms, in
   const bool one_wave = ctas * splits <= num_sms;
   int budget = (!one_wave && tmem_need <= 256 && stage_bytes * 4 + 12 * 1024 <= 112 * 1024) ? 100 * 1024
                                                                                            : 212 * 1024;
+  // Not more than eight: twelve stages of 18 KiB request more weights before the dependency wait, but a step of one row
+  // took 0.5 % longer, its attention's tiles waiting behind them.
   int stages = budget / stage_bytes;
   if (stages > 8) stages = 8;
   if (stages < 2) stages = 2;
