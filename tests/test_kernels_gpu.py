@@ -1217,8 +1217,8 @@ def test_paged_attention_decode_split(n_q, n_kv, hd, ps, case, split):
     (1, 4096, 1024, 8, 2, 128, False), (7, 1032, 520, 3, 1, 16, True), (33, 2048, 136, 4, 4, 64, False),
     (128, 1024, 8200, 2, 1, 128, True)])
 def test_norm_and_rope_inside_the_split_reductions(M, hidden, inter, n_q, n_kv, hd, interleaved):
-    """A step's pieces against float64 on the stored operands of each: half a unit of bf16 (2^-9) for the value stored,
-    as much again for the rounded operand where one result feeds the next check, and 2^-10 for fp32 sums of order one."""
+    """A step's pieces against float64 on the stored operands of each: one rounding to bf16 (2^-8 of the value, which has 8
+    significant bits) and 2^-10 for fp32 sums of order one."""
     from modular_b200._native import lib
     from modular_b200.nn.rotary_embedding import cos_sin_table
 
@@ -1302,3 +1302,40 @@ def test_decode_attention_started_under_the_cache_store(n_kv, hd, lens):
         got.append(out)
     assert got[0].isfinite().all() and torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
     ops.check_device_error()
+
+
+@pytest.mark.parametrize("cols", [8, 1024, 1032, 2048, 2056, 8192, 8200, 32768])
+def test_rmsnorm_widths(cols):
+    """Every split of a row over threads, with a residual too: two roundings to bf16, 2^-8 each (8 significant bits)."""
+    torch.manual_seed(43)
+    x, r = (torch.randn(5, cols, device=DEV).to(torch.bfloat16) for _ in range(2))
+    w = (torch.randn(cols, device=DEV) * 0.3 + 1).to(torch.bfloat16)
+    exact = lambda v: v.double() * (v.double().square().mean(1, keepdim=True) + 1e-5).rsqrt() * w.double()
+    close = lambda a, b: torch.allclose(a.double(), b, rtol=2 ** -7, atol=1e-6)
+    assert close(ops.rms_norm(x, w, 1e-5), exact(x))
+    total = (x.float() + r.float()).to(torch.bfloat16)
+    res = r.clone()
+    y, _ = ops.add_rms_norm(x, res, w, 1e-5)
+    assert torch.equal(res, total) and close(y, exact(total))
+
+
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("n_q,n_kv,hd", [(1, 1, 16), (40, 8, 128), (5, 3, 80), (6, 2, 256), (70, 1, 64), (1, 1, 4096)])
+def test_rope_heads_of_a_thread(n_q, n_kv, hd, interleaved):
+    """Head counts and widths that leave threads without a head, or take several rounds; a skipped row keeps its cache."""
+    torch.manual_seed(44)
+    T, ps = 9, 16
+    kv = torch.zeros(2, 2, 1, n_kv, ps, hd, device=DEV, dtype=torch.bfloat16)
+    qkv = torch.randn(T, (n_q + 2 * n_kv) * hd, device=DEV).to(torch.bfloat16)
+    pos = torch.randint(0, 500, (T,), device=DEV, dtype=torch.int32)
+    slots = torch.randperm(2 * ps, device=DEV)[:T].long()
+    slots[3] = -1
+    ang = torch.rand(512, hd // 2, device=DEV) * 6.28
+    cos_sin = torch.cat([ang.cos(), ang.sin()], dim=1).contiguous()
+    kv_ref, qkv_ref = kv.clone(), qkv.clone()
+    ops.rope_kv_store(qkv, pos, slots, cos_sin, kv[:, 0, 0], kv[:, 1, 0], n_q, n_kv, hd, interleaved)
+    ref.rope_kv_store(qkv_ref, pos, slots, cos_sin, kv_ref[:, 0, 0], kv_ref[:, 1, 0], n_q, n_kv, hd, interleaved)
+    # one rounding to bf16 each, of sums whose fp32 terms are of order one
+    assert torch.allclose(qkv[:, : n_q * hd].float(), qkv_ref[:, : n_q * hd].float(), rtol=2 ** -7, atol=1e-5)
+    assert torch.allclose(kv.float(), kv_ref.float(), rtol=2 ** -7, atol=1e-5)
+    assert torch.equal(kv[:, 1], kv_ref[:, 1])
