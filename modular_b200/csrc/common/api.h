@@ -76,6 +76,8 @@ int mb_reduce_rope_store(const float* part, int splits, const float* ssq, int hi
                          const int32_t* positions, const int64_t* slots, const float* cos_sin, void* k_cache,
                          void* v_cache, int T, int n_q, int n_kv, int head_dim, int page_size, int64_t page_stride,
                          int64_t head_stride, int interleaved, cudaStream_t stream);
+int mb_gemm_bf16_swiglu_half(const void* X, const void* W, void* Y, int M, int N, int K, int flags, const float* ssq,
+                             int ssq_blocks, float eps, int* err, cudaStream_t stream);
 int mb_gemm_bf16_swiglu_normed(const void* X, const void* W, void* Y, int M, int N, int K, int flags, const float* ssq,
                                int ssq_blocks, float eps, int* err, int num_sms, cudaStream_t stream);
 

@@ -43,7 +43,16 @@ constexpr int kATileBytes = kBM * kBK * 2;  // 16 KiB
 constexpr int kStageWarpBytes = 32 * 32 * 2;  // per-epilogue-warp transpose buffer
 constexpr int kGemmThreads = 192;
 
-enum GemmEpi { EPI_BF16 = 0, EPI_BF16_RESIDUAL = 1, EPI_F32 = 2 };
+// EPI_SWIGLU_HALF: a tile is 64 gate rows over their 64 up rows (SwiGLU of few rows, see mb_gemm_bf16_swiglu_half)
+enum GemmEpi { EPI_BF16 = 0, EPI_BF16_RESIDUAL = 1, EPI_F32 = 2, EPI_SWIGLU_HALF = 3 };
+
+// Rows of X that still lack their RMSNorm factor rsqrt(sum of squares * inv_cols + eps) (EPI_SWIGLU_HALF)
+struct RowNorm {
+  const float* ssq;
+  int blocks;
+  float inv_cols, eps;
+};
+constexpr int kHalfRows = 64;   // most token rows of EPI_SWIGLU_HALF
 
 struct GemmSmemTail {
   uint64_t full[8];
@@ -144,6 +153,51 @@ __device__ __forceinline__ void epilogue_tile(uint32_t tmem_base, uint8_t* stage
     }
 }
 
+// Epilogue of EPI_SWIGLU_HALF by four warps: quads 0 and 1 hold 64 gate rows, 2 and 3 their up rows. Of every chunk of 16
+// tokens the gate warp finishes the first eight and the up warp the others; they swap what they lack through the ring's
+// shared memory (all its loads and MMAs are over). `ok` false (a wait ran out): the warp still meets the others.
+__device__ __forceinline__ void epilogue_half(uint32_t tmem_base, float* swap, uint8_t* stage_buf, int quad, int lane,
+                                              __nv_bfloat16* __restrict__ Y, int M, int N, int BN, int n0,
+                                              const float (&factor)[kHalfRows / 32], bool ok) {
+  const int pair = quad & 1, up = quad >> 1, chunks = (min(BN, M) + 15) >> 4;
+  const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+  float* mine = swap + quad * chunks * 256 + lane;               // [quad][chunk][token][row]
+  const float* other = swap + (quad ^ 2) * chunks * 256 + lane;
+  uint32_t a[16];
+  if (ok) {
+    for (int c = 0; c < chunks; ++c) {
+      tmem_ld_32x16(lane_addr + c * 16, a);
+      tc_wait_ld();
+#pragma unroll
+      for (int j = 0; j < 8; ++j) mine[(c * 8 + j) * 32] = __uint_as_float(up ? a[j] : a[8 + j]);
+    }
+  }
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  if (!ok) return;
+  __nv_bfloat16* stg = reinterpret_cast<__nv_bfloat16*>(stage_buf + quad * kStageWarpBytes);
+  for (int c = 0; c < chunks; ++c) {
+    const int first = c * 16 + up * 8;
+    if (first >= M) break;   // warp-uniform
+    if (chunks > 1) {        // a single chunk is still in the registers
+      tmem_ld_32x16(lane_addr + c * 16, a);
+      tc_wait_ld();
+    }
+    const float f = c < 2 ? factor[0] : factor[1];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (first + j >= M) break;
+      const float fj = __shfl_sync(0xffffffffu, f, (c & 1) * 16 + up * 8 + j);
+      const float x = __uint_as_float(up ? a[8 + j] : a[j]) * fj, y = other[(c * 8 + j) * 32] * fj;
+      stg[j * 32 + lane] = __float2bfloat16(up ? silu_f(y) * x : silu_f(x) * y);
+    }
+    __syncwarp();
+    const int j = lane >> 2, seg = lane & 3, t = first + j, n = n0 + pair * 32 + seg * 8;
+    if (t < M && n < N)
+      *reinterpret_cast<uint4*>(Y + static_cast<size_t>(t) * N + n) = *reinterpret_cast<const uint4*>(stg + j * 32 + seg * 8);
+    __syncwarp();
+  }
+}
+
 template <bool DUAL, int EPI>
 __global__ void __launch_bounds__(kGemmThreads)
 gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
@@ -151,7 +205,7 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
                int ldy, int ldr, int dual_rows, int k_per_split, int BN, int stages,
                uint32_t tmem_cols, int* err, const int32_t* __restrict__ expert_offsets,
                int w_rows_per_expert, const int* gate_flags, int gate_rpr, int gate_world,
-               int packed_kb, int x_batch_off, int y_batch_off, int w_static) {
+               int packed_kb, int x_batch_off, int y_batch_off, int w_static, const RowNorm rn) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -169,7 +223,8 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   // [expert_offsets[e], expert_offsets[e+1]) of X / Y and its weights start at row
   // e * w_rows_per_expert of W. CTAs beyond an expert's rows leave before touching TMEM.
   int split = blockIdx.z;
-  const int n0 = n_tile * kBM;
+  constexpr bool kHalf = EPI == EPI_SWIGLU_HALF;
+  const int n0 = n_tile * (kHalf ? kBM / 2 : kBM);
   int t0 = m_tile * BN;
   int Mlim = M, w_row0 = 0;
   if (expert_offsets != nullptr) {
@@ -234,6 +289,7 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         if (DUAL) tma_load_2d(sa + kATileBytes, &tmW, full_s, 0, (((w_row0 + dual_rows + n0) >> 7) * packed_kb + kb) << 7);
       } else {
         tma_load_2d(sa, &tmW, full_s, kc, w_row0 + n0);
+        if (kHalf) tma_load_2d(sa + kATileBytes / 2, &tmW, full_s, kc, dual_rows + n0);
         if (DUAL) tma_load_2d(sa + kATileBytes, &tmW, full_s, kc, w_row0 + dual_rows + n0);
       }
     }
@@ -288,6 +344,7 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
                         (((w_row0 + dual_rows + n0) >> 7) * packed_kb + kb) << 7);
         } else {
           tma_load_2d(sa, &tmW, full_s, kc, w_row0 + n0);
+          if (kHalf) tma_load_2d(sa + kATileBytes / 2, &tmW, full_s, kc, dual_rows + n0);
           if (DUAL) tma_load_2d(sa + kATileBytes, &tmW, full_s, kc, w_row0 + dual_rows + n0);
         }
         tma_load_2d(sb, &tmX, full_s, xk0 + kc, t0);
@@ -324,9 +381,23 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)
     const int quad = warp & 3;  // TMEM lane quadrant this warp may read
+    float factor[kHalfRows / 32];   // of the tokens lane, lane + 32, ...
+    if constexpr (kHalf) {
+#pragma unroll
+      for (int i = 0; i < kHalfRows / 32; ++i) {
+        const int t = i * 32 + lane;
+        float sum = 0.f;
+        if (t < M)
+          for (int b = 0; b < rn.blocks; ++b) sum += rn.ssq[t * rn.blocks + b];
+        factor[i] = rsqrtf(sum * rn.inv_cols + rn.eps);
+      }
+    }
     const bool ok = mbar_wait(&tail->tmem_full, 0, abort_word, err, 103);
     tc_fence_after();
-    if (ok && k_iters > 0)
+    if constexpr (kHalf)
+      epilogue_half(tmem_base, reinterpret_cast<float*>(smem), stage_buf, quad, lane, static_cast<__nv_bfloat16*>(Yv), M, N,
+                    BN, n0, factor, ok && k_iters > 0);
+    else if (ok && k_iters > 0)
       epilogue_tile<DUAL, EPI>(tmem_base, stage_buf, quad, lane, Yv, R, M, N, ldy, ldr, BN, n0, t0, Mlim, split);
   }
 
@@ -1230,7 +1301,7 @@ static int launch_cfg(const CUtensorMap& tw, const CUtensorMap& tx, void* Y, con
                       const int32_t* expert_offsets = nullptr, int n_experts = 0,
                       int w_rows_per_expert = 0, const int* gate_flags = nullptr, int gate_rpr = 1,
                       int gate_world = 0, int packed_kb = 0, int batch = 0, int x_batch_off = 0,
-                      int y_batch_off = 0, int w_static = 0) {
+                      int y_batch_off = 0, int w_static = 0, RowNorm rn = RowNorm{}) {
   const int stage_bytes = kATileBytes * (DUAL ? 2 : 1) + BN * kBK * 2;
   const size_t smem = static_cast<size_t>(stages) * stage_bytes + 4 * kStageWarpBytes +
                       sizeof(GemmSmemTail) + 1024;
@@ -1242,12 +1313,13 @@ static int launch_cfg(const CUtensorMap& tw, const CUtensorMap& tx, void* Y, con
       return MB_ERR_LAUNCH;
     configured.done();
   }
-  dim3 grid((M + BN - 1) / BN, (N + kBM - 1) / kBM, expert_offsets ? n_experts : (batch > 0 ? batch : splits));
+  const int tile_rows = EPI == EPI_SWIGLU_HALF ? kBM / 2 : kBM;
+  dim3 grid((M + BN - 1) / BN, (N + tile_rows - 1) / tile_rows, expert_offsets ? n_experts : (batch > 0 ? batch : splits));
   const uint32_t tmem_cols = pow2_cols(DUAL ? 2 * BN : BN);
   const cudaError_t e = launch_k(kern, grid, dim3(kGemmThreads), smem, stream, tw, tx, Y,
                                  static_cast<const __nv_bfloat16*>(R), M, N, K, ldy, ldr, dual_rows, k_per_split,
                                  BN, stages, tmem_cols, err, expert_offsets, w_rows_per_expert, gate_flags,
-                                 gate_rpr, gate_world, packed_kb, x_batch_off, y_batch_off, w_static);
+                                 gate_rpr, gate_world, packed_kb, x_batch_off, y_batch_off, w_static, rn);
   return e == cudaSuccess ? MB_OK : MB_ERR_LAUNCH;
 }
 
@@ -1538,6 +1610,26 @@ extern "C" int mb_gemm_bf16_partials(const void* X, const void* W, int M, int N,
   return launch_cfg<false, EPI_F32>(tw, tx, ws, nullptr, M, N, K, N, 0, 0, splits > 1 ? k_per_split : K, splits, bn,
                                     stages, err, stream, nullptr, 0, 0, nullptr, 1, 0, 0, 0, 0, 0,
                                     (flags & 128) ? 1 : 0);
+}
+
+// SwiGLU of at most 64 normalised rows in tiles of 64 gate rows and their 64 up rows, two CTAs an SM: twice as many
+// tiles as mb_gemm_bf16_swiglu_normed, which calls it where its own would leave SMs idle.
+extern "C" int mb_gemm_bf16_swiglu_half(const void* X, const void* W, void* Y, int M, int N, int K, int flags,
+                                        const float* ssq, int ssq_blocks, float eps, int* err, cudaStream_t stream) {
+  if (M <= 0 || M > kHalfRows || N <= 0 || K % 8 || N % 8 || ssq == nullptr || ssq_blocks < 1) return MB_ERR_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(Y)) & 15)
+    return MB_ERR_ALIGN;
+  const int bn = (M + 15) / 16 * 16;
+  int stages = 100 * 1024 / (kATileBytes + bn * kBK * 2);   // two CTAs per SM; the swapped chunks need 256 bytes a token
+  if (stages > 8) stages = 8;
+  CUtensorMap tw, tx;
+  int rc = cached_tmap(&tw, W, 2ull * N, K, K, kBM / 2, 2);
+  if (rc != MB_OK) return rc;
+  rc = cached_tmap(&tx, X, M, K, K, bn, 2);
+  if (rc != MB_OK) return rc;
+  return launch_cfg<false, EPI_SWIGLU_HALF>(tw, tx, Y, nullptr, M, N, K, N, 0, N, K, 1, bn, stages, err, stream, nullptr, 0,
+                                            0, nullptr, 1, 0, 0, 0, 0, 0, (flags & 128) ? 1 : 0,
+                                            RowNorm{ssq, ssq_blocks, 1.0f / static_cast<float>(K), eps});
 }
 
 extern "C" int mb_reduce_residual(const float* part, int splits, void* H, const void* w, float offset, void* XW,

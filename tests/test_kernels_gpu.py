@@ -1214,8 +1214,9 @@ def test_paged_attention_decode_split(n_q, n_kv, hd, ps, case, split):
 
 
 @pytest.mark.parametrize("M,hidden,inter,n_q,n_kv,hd,interleaved", [
-    (1, 4096, 1024, 8, 2, 128, False), (7, 1032, 520, 3, 1, 16, True), (33, 2048, 136, 4, 4, 64, False),
-    (128, 1024, 8200, 2, 1, 128, True)])
+    (1, 4096, 1024, 8, 2, 128, False), (7, 1032, 520, 3, 1, 16, True), (25, 512, 72, 1, 1, 16, False),
+    (33, 2048, 136, 4, 4, 64, False), (64, 256, 200, 2, 1, 16, True), (65, 256, 200, 2, 1, 16, True),
+    (128, 1024, 8200, 2, 1, 128, True), (70, 256, 19008, 1, 1, 16, False)])
 def test_norm_and_rope_inside_the_split_reductions(M, hidden, inter, n_q, n_kv, hd, interleaved):
     """A step's pieces against float64 on the stored operands of each: one rounding to bf16 (2^-8 of the value, which has 8
     significant bits) and 2^-10 for fp32 sums of order one."""
