@@ -509,7 +509,8 @@ struct SsdChunk {
   const int *cu_seqlens, *state_idx, *has_init;
   int H, P, N, G, ldx, ld_dt, ldb, ldc, dt_softplus, col_blocks;
   // Long prompts in segments of `seg` tokens (0: whole sequences), each with its own CTA. parts [segments, H, P, N] holds the state that a
-  // segment makes of nothing, decays [segments, H] its decay.
+  // segment makes of nothing, decays [segments, H] its decay. Nobody needs that of a sequence's last segment: its entry holds a copy of the
+  // kept state instead, because the CTA that walks the last segment replaces the kept one while others of its launch may not have begun.
   int seg, n_seqs;
   float *parts, *decays;
 };
@@ -560,7 +561,7 @@ __device__ __forceinline__ void ssd_products(const __nv_bfloat16* sC, const __nv
   }
 }
 
-// LOCAL: only the state that a segment makes of nothing, for all segments but a sequence's last one.
+// LOCAL: only the state that a segment makes of nothing, for all segments but a sequence's last one, and the copy of the kept state.
 template <int DK, bool LOCAL>
 __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_kernel(const SsdChunk p) {
   typedef __nv_bfloat16 bf16;
@@ -582,17 +583,26 @@ __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_ker
     part = blockIdx.y - segment_base(p, s);
   }
   const int slot = p.state_idx && p.state ? p.state_idx[s] : -1;
+  const bool resume = slot >= 0 && p.has_init && p.has_init[s];
+  float* st = p.state + (static_cast<size_t>(slot >= 0 ? slot : 0) * p.H + h) * P * N;
+  const float* kept = st;
   int t0 = p.cu_seqlens[s], n = p.cu_seqlens[s + 1] - t0;
   bool last = true;
   if (p.seg > 0) {
     const int from = part * p.seg;
     if (part > 0 && from >= n) return;
     last = from + p.seg >= n;
+    if (part > 0 || !last) {
+      float* copy = p.parts + (static_cast<size_t>(blockIdx.y - part + (n - 1) / p.seg) * p.H + h) * P * N;
+      kept = copy;
+      if (LOCAL && last && resume)
+        for (int i = v0 * N + 2 * tid; i < min(v0 + kNV, P) * N; i += 2 * kChunkThreads)
+          *reinterpret_cast<float2*>(copy + i) = *reinterpret_cast<const float2*>(st + i);
+    }
+    if (LOCAL && last) return;
     t0 += from;
     n = min(n - from, p.seg);
-    if (LOCAL && last) return;
   }
-  const bool resume = slot >= 0 && p.has_init && p.has_init[s];
   const int group = h / (p.H / p.G);
   const bf16 *xh = p.x + static_cast<size_t>(t0) * p.ldx + h * P, *Bh = p.B + static_cast<size_t>(t0) * p.ldb + group * N,
              *Ch = p.C + static_cast<size_t>(t0) * p.ldc + group * N, *dth = p.dt + static_cast<size_t>(t0) * p.ld_dt + h;
@@ -665,14 +675,13 @@ __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_ker
   const float dsk = p.Dskip ? p.Dskip[h] : 0.f;
   // S^T: 16 rows p of this warp as accumulator tiles of 8 columns n: [0], [1] row row4, [2], [3] row row4 + 8
   float S[2 * KB][4];
-  float* st = p.state + (static_cast<size_t>(slot >= 0 ? slot : 0) * p.H + h) * P * N;
   const int vr = v0 + warp * 16 + row4;
 #pragma unroll
   for (int t = 0; t < 2 * KB; ++t)
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       float2 f = make_float2(0.f, 0.f);
-      if (!LOCAL && resume && vr + 8 * e < P && 8 * t < N) f = *reinterpret_cast<const float2*>(st + static_cast<size_t>(vr + 8 * e) * N + 8 * t + col2);
+      if (!LOCAL && resume && vr + 8 * e < P && 8 * t < N) f = *reinterpret_cast<const float2*>(kept + static_cast<size_t>(vr + 8 * e) * N + 8 * t + col2);
       S[t][2 * e] = f.x; S[t][2 * e + 1] = f.y;
     }
   bool have_state = !LOCAL && resume;

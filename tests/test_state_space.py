@@ -282,6 +282,31 @@ def test_ssd_segments(lens, H, P, N, A0):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("lens,H,N", [([4097, 4097], 80, 128), ([513, 3585], 20, 24), ([4097], 3, 64)])
+def test_ssd_segments_continue_kept_states(lens, H, N):
+    """Every sequence goes on from a kept state that decays slowly and is far from the new one, its last segment is one token (the first to
+    end), and the first case has more CTAs than the chip holds at once: all segments start from the kept state, none from the new one."""
+    torch.manual_seed(18)
+    dev, T, P = "cuda", sum(lens), 64
+    bf = lambda *s, k=1.0: (torch.randn(*s, device=dev) * k).to(torch.bfloat16)
+    x, dt, B, C = bf(T, H, P), bf(T, H, k=0.5), bf(T, 1, N), bf(T, 1, N)
+    A, bias = -torch.rand(H, device=dev) * 1e-3 - 1e-3, torch.randn(H, device=dev) * 0.1
+    idx = torch.tensor([2, 0][: len(lens)], dtype=torch.int32, device=dev)
+    one = torch.ones(len(lens), dtype=torch.int32, device=dev)
+    st = torch.randn(3, H, P, N, device=dev) * 10
+    want_st, want = st.clone(), []
+    y = ss.ssd_scan_varlen(x, dt, A, B, C, None, bias, _cu(lens, dev), st, idx, one, True)
+    for i, n in enumerate(lens):
+        for c in range(0, n, 500):                     # portions that are walked whole
+            r = slice(sum(lens[:i]) + c, sum(lens[:i]) + min(c + 500, n))
+            want.append(ss.ssd_scan_varlen(x[r], dt[r], A, B[r], C[r], None, bias, _cu([r.stop - r.start], dev), want_st, idx[i: i + 1], one[:1], True))
+    want = torch.cat(want)
+    for r in range(0, T, 256):                         # a stretch by itself: one wrong segment is a small part of the whole
+        assert _rel(y[r: r + 256], want[r: r + 256]) < 2 ** -8          # a rounding to bf16 on either side
+    assert _rel(st, want_st) < 1e-5                    # fp32 sums over the state's memory, cut at other tokens
+
+
+@pytest.mark.gpu
 def test_ssd_special_inputs_stay_causal():
     """An infinite or NaN input of a prompt changes its own row of the state from its token on, and nothing before it."""
     torch.manual_seed(10)
