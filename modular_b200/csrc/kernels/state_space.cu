@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(kChunkThreads, DK == 32 ? 3 : 2) ssd_chunk_ker
   bool last = true;
   if (p.seg > 0) {
     const int from = part * p.seg;
-    if (part > 0 && from >= n) return;
+    if (part < 0 || (part > 0 && from >= n)) return;     // before the first sequence, or behind the end of this one
     last = from + p.seg >= n;
     if (part > 0 || !last) {
       float* copy = p.parts + (static_cast<size_t>(blockIdx.y - part + (n - 1) / p.seg) * p.H + h) * P * N;

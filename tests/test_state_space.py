@@ -307,6 +307,29 @@ def test_ssd_segments_continue_kept_states(lens, H, N):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("lens", [[0, 2000, 1700], [1700, 3000]])
+def test_ssd_segments_leave_rows_before_the_first_sequence(lens):
+    """Sequences that begin some segments into the rows: nobody walks the rows before them, and an empty one keeps its state."""
+    torch.manual_seed(19)
+    dev, lead, H, P, N = "cuda", 1300, 3, 64, 64
+    T = lead + sum(lens)
+    bf = lambda *s, k=1.0: (torch.randn(*s, device=dev) * k).to(torch.bfloat16)
+    x, dt, B, C = bf(T, H, P), bf(T, H, k=0.5), bf(T, 1, N), bf(T, 1, N)
+    A = -torch.rand(H, device=dev) * 1e-2 - 1e-3
+    idx, one = torch.arange(len(lens), dtype=torch.int32, device=dev), torch.ones(len(lens), dtype=torch.int32, device=dev)
+    st = torch.randn(len(lens), H, P, N, device=dev)
+    start, want = st.clone(), st.clone()
+    y = torch.full_like(x, 7.0)
+    from modular_b200._native import lib
+    lib().ssd_scan_varlen(x, dt, A, B, C, None, None, y, st, _cu([lead, *lens], dev)[1:].contiguous(), idx, one, True)
+    w = ss.ssd_scan_varlen(x[lead:], dt[lead:], A, B[lead:], C[lead:], None, None, _cu(lens, dev), want, idx, one, True)
+    assert (y[:lead] == 7.0).all()
+    assert _rel(y[lead:], w) < 2 ** -8 and _rel(st, want) < 1e-5          # segments begin at other tokens
+    for i, n in enumerate(lens):
+        assert n > 0 or torch.equal(st[i], start[i])
+
+
+@pytest.mark.gpu
 def test_ssd_special_inputs_stay_causal():
     """An infinite or NaN input of a prompt changes its own row of the state from its token on, and nothing before it."""
     torch.manual_seed(10)
