@@ -548,9 +548,13 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         uint64_t f2;
         asm("mov.b64 %0, {%1, %1};" : "=l"(f2) : "r"(__float_as_uint(f)));
         const uint32_t buf = g & 1;
-        // one lane asks: 32 of them are served one after the other
+        // One lane asks: 32 of them are served one after the other. The others learn of it by a shuffle, which orders no memory: the
+        // barrier of the warp makes what lane 0 saw complete hold for them as well.
         ok = (PAIR && lane != 0) || mbar_wait(&tail->acc_full[buf], (g >> 1) & 1, abort_word, p.err, 514);
-        if (PAIR) ok = __shfl_sync(0xffffffffu, ok, 0);
+        if (PAIR) {
+          __syncwarp();
+          ok = __shfl_sync(0xffffffffu, ok, 0);
+        }
         if (!ok) break;
         ++g;
         tc_fence_after();
