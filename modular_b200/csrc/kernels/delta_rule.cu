@@ -19,7 +19,6 @@
 //
 // Steps of few tokens, fp32 runs, one decay per head and other widths go token by token. What bounds that is the chain of a token, 650 cycles of
 // shared-memory reads, two dot products and three shuffles; bf16 prompts with 128 rows run in chunks (below).
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include "../common/api.h"
@@ -575,20 +574,19 @@ static int scan(const MbDelta& p, int num_sms, cudaStream_t stream) {
 // zeros. delta_chunk_prep_kernel does what needs no state for all chunks at once, two warps a (chunk, head): convolution, norms and
 // decays as above, the products of pairs, the inverse by substitution. delta_chunk_scan_kernel walks a sequence's chunks with S in accumulator fragments: a warp owns 16 columns
 // of one head, which are the M side of every product; the fragments of one product are the operands of the next.
-// Every operand stays 32 bits wide and enters a product as two numbers of 11 bits (three products of halves): keys, queries and state as
-// fp16 with a power of two ahead (per token for keys and queries, per column for the state and u, so that the largest value of a
-// row lies near 2^8 or 2^11 and what the halves drop is 2^-33 of it, however far decays or columns reach), the small matrices as tf32. Keys and queries are taken apart once, where they
-// are made, and travel as rows of halves of the same size.
-// 8192 tokens in four prompts of at most 3076, 16 heads of 128 x 128: the scan took 1065 us token by token, takes 875 in chunks with tf32
-// operands and one warp per 16 columns, 521 with the rows of a column over four warps and the longest sequences first, 420 with
-// fp16 halves: 3300 cycles a chunk where a CTA has its SM, half of them products (8.2 cycles a scheduler, tf32 or fp16), half
-// barriers, the exchange between the four warps and making fragments. The preparation takes 270 us with the products of pairs, as
-// much as it took without: 14 thousand instructions a chunk and head on the 16 warps an SM that rows in shared memory leave.
-// Error of the state against 64 bits: 4.4e-7 after 300 tokens, 2.3e-7 where nothing decays (4.5e-7 and 3.4e-7 token by token).
+// An operand x enters a product as two tf32 numbers, x rounded to 11 bits and what is left, of which the unit reads 11 more: together they
+// are within 2^-23 of x, whatever lies beside it, and the product of two such pairs leaves out 2^-22 of itself. (Two fp16 numbers under a
+// power of two per row hold that for the row's largest entries only: where channels of keys and state reached 2^20, entries of the state were
+// off by 8e-5 of their channel, with fast decays by 4e-3; here and token by token by 8e-6 at most.) Keys and queries travel as fp32 rows and are taken apart in registers.
+// 8192 tokens in four prompts of at most 3076, 16 heads of 128 x 128: the scan took 1065 us token by token, 875 in chunks with one warp
+// per 16 columns, 508 with the rows of a column over four warps and the longest sequences first (fp16 halves, half the products: 435): two
+// thirds of a chunk are products (8.2 cycles a scheduler), the rest barriers, the exchange between the four warps and making fragments. The
+// preparation takes 229 us with the products of pairs (270 token by token, without them): its instructions on the 16 warps an SM that rows in
+// shared memory leave.
+// Error of the state against 64 bits, root mean square over its channels, after 300 tokens: 1.2e-6 with decays near one (token by token 1.2e-6),
+// 1.7e-7 without decay (2.2e-7), 1.6e-7 where little outlasts ten tokens (1.3e-7).
 constexpr int kCh = 16;
-// floats of a chunk's record: b_last [128], a flag (something in the chunk is not finite), powers of two that give back the rows of
-// b k and b q, and those of the keys that enter the state, [16] each at kBack
-constexpr int kBack = 132, kRec = kBack + 3 * kCh;
+constexpr int kRec = 132;          // floats of a chunk's record: b_last [128] and a flag (something in the chunk is not finite)
 constexpr int kRowFloats = 4 * kCh;
 constexpr int kChunkCols = 32;     // columns of a scan CTA
 
@@ -609,57 +607,12 @@ __device__ __forceinline__ float lanes_reduce(float (&v)[N]) {
   return v[0];
 }
 
-// maxima of 16 values over all lanes: lane l ends with that of value l / 2
-__device__ __forceinline__ float lanes_max(float (&v)[16]) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int n = 8, o = 16; n >= 1; n >>= 1, o >>= 1) {
-    const bool up = (lane & o) != 0;
-#pragma unroll
-    for (int i = 0; i < n; ++i) v[i] = fmaxf(up ? v[i + n] : v[i], __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + n], o));
-  }
-  return fmaxf(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1));
-}
-__device__ __forceinline__ float top4(float4 a) { return fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))); }
 __device__ __forceinline__ float4 mul4(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
 __device__ __forceinline__ float zero_times(float4 a, float acc) { return fmaf(a.x, 0.f, fmaf(a.y, 0.f, fmaf(a.z, 0.f, fmaf(a.w, 0.f, acc)))); }
 
-// 2^n that takes `top` to [2^want, 2^(want + 1)), and 2^-n; 1 where it is zero. Values beyond what the exponents reach stay at
-// their ends; infinities and NaN are found elsewhere.
-__device__ __forceinline__ float scale_to(float top, int want, float& back) {
-  int e = (__float_as_int(top) >> 23) - 127;       // top >= 0
-  e = top == 0.f ? want : max(-100, min(e, 120));
-  back = __int_as_float((127 + e - want) << 23);
-  return __int_as_float((127 + want - e) << 23);
-}
-constexpr int kKeyExp = 7;
-// two numbers as fp16 and what is left of them as fp16
-__device__ __forceinline__ void split_h2(float x, float y, uint32_t& hi, uint32_t& lo) {
-  const __half2 h = __floats2half2_rn(x, y);
-  const float2 f = __half22float2(h);
-  const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
-}
-__device__ __forceinline__ float2 join_h2(uint32_t hi, uint32_t lo) {
-  const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&hi)), b = __half22float2(*reinterpret_cast<const __half2*>(&lo));
-  return make_float2(a.x + b.x, a.y + b.y);
-}
-// A row of keys or queries in halves, 16 bytes per four channels: high parts, low parts.
-__device__ __forceinline__ uint4 row_halves(float4 v, float scale) {
-  uint4 r;
-  split_h2(v.x * scale, v.y * scale, r.x, r.z);
-  split_h2(v.z * scale, v.w * scale, r.y, r.w);
-  return r;
-}
-// A row of the keys that enter the state: high parts of all channels, then low parts; of sixteen channels first 4 t and 4 t + 1
-// (t = 0 .. 3), then 4 t + 2 and 4 t + 3, as the accumulator tiles of the state hold them. `c` is a multiple of four.
-__device__ __forceinline__ int state_key_word(int c) { return (c >> 4) * 8 + ((c >> 2) & 3); }
-__device__ __forceinline__ void store_state_key(float* row, int c, float4 v, float scale) {
-  uint32_t* w = reinterpret_cast<uint32_t*>(row) + state_key_word(c);
-  split_h2(v.x * scale, v.y * scale, w[0], w[64]);
-  split_h2(v.z * scale, v.w * scale, w[4], w[68]);
-}
+// A row of the keys that enter the state: of every four channels first 0 and 2, then 1 and 3, which are the neighbours in the
+// accumulator tiles of the state.
+__device__ __forceinline__ float4 state_key(float4 v) { return make_float4(v.x, v.z, v.y, v.w); }
 
 struct ChunkPrepPair {
   float4 q[kCh][32], k[kCh][32], g[kCh][32];       // rows of 128; a lane works on its four channels
@@ -801,67 +754,36 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const __grid_c
     if (lane == 0) sm.bad[role] = odd;
   }
   pair_sync();                     // decays are there
-  const bool bad = sm.bad[0] || sm.bad[1];         // something is not finite: rows stay as they are, fp32
+  const bool bad = sm.bad[0] || sm.bad[1];         // something is not finite
   // Decays relative to the chunk's start are enough as long as no channel fades below 1e-15 in it (their inverses stay far from
   // the largest number, products keep their relative error); otherwise pairs take the product of the decays between them.
   const float4 ones = make_float4(1.f, 1.f, 1.f, 1.f);
   float4 run = ones;
-  float tops[kCh], to, back;         // of token lane / 2
-  // exponents of the rows b_t x_t
-  auto forward_tops = [&](const float4 (*x)[32], bool products, float* keep) {
-    run = ones;
-#pragma unroll
-    for (int j = 0; j < kCh; ++j) {
-      run = products ? sm.g[j][lane] : mul4(run, sm.g[j][lane]);
-      tops[j] = top4(mul4(run, x[j][lane]));
-    }
-    to = scale_to(lanes_max(tops), kKeyExp, back);
-    if ((lane & 1) == 0) keep[lane >> 1] = back;
-    run = ones;
-  };
   if (role == 0) {
-#pragma unroll
-    for (int j = kCh - 1; j >= 0; --j) {
-      tops[j] = top4(mul4(run, sm.k[j][lane]));
-      run = mul4(run, sm.g[j][lane]);
-    }
-    to = scale_to(lanes_max(tops), kKeyExp, back);
-    if ((lane & 1) == 0) rec[kBack + 2 * kCh + (lane >> 1)] = back;
-    run = ones;
 #pragma unroll 4
     for (int j = kCh - 1; j >= 0; --j) {
-      const float4 a = mul4(run, sm.k[j][lane]);
-      const float scale = __shfl_sync(0xffffffffu, to, 2 * j);
-      float* row = p.g + first - c + j * step;
-      if (j < m) {
-        if (bad) *reinterpret_cast<float4*>(row + c) = a; else store_state_key(row, c, a, scale);
-      }
+      if (j < m) *reinterpret_cast<float4*>(p.g + first + j * step) = state_key(mul4(run, sm.k[j][lane]));
       run = mul4(run, sm.g[j][lane]);
     }
     *reinterpret_cast<float4*>(rec + c) = run;
     const float fade = fminf(fminf(run.x, run.y), fminf(run.z, run.w));
     const bool ok = __all_sync(0xffffffffu, !on || fade >= 1e-15f);
     if (lane == 0) sm.near = ok;
-    forward_tops(sm.k, false, rec + kBack);
+    run = ones;
 #pragma unroll 4
     for (int j = 0; j < kCh; ++j) {
       run = mul4(run, sm.g[j][lane]);
-      const float4 a = mul4(run, sm.k[j][lane]);
-      const float scale = __shfl_sync(0xffffffffu, to, 2 * j);
-      if (j < m) *reinterpret_cast<uint4*>(p.k + first + j * step) = bad ? *reinterpret_cast<const uint4*>(&a) : row_halves(a, scale);
+      if (j < m) *reinterpret_cast<float4*>(p.k + first + j * step) = mul4(run, sm.k[j][lane]);
       if (ok) sm.g[j][lane] = run;                 // from here on the running product
     }
   }
   pair_sync();                     // queries and running products are there
   const bool near = sm.near;
   if (role == 1) {
-    forward_tops(sm.q, near, rec + kBack + kCh);
 #pragma unroll 4
     for (int j = 0; j < kCh; ++j) {
       run = near ? sm.g[j][lane] : mul4(run, sm.g[j][lane]);
-      const float4 b = mul4(run, sm.q[j][lane]);
-      const float scale = __shfl_sync(0xffffffffu, to, 2 * j);
-      if (j < m) *reinterpret_cast<uint4*>(p.q + first + j * step) = bad ? *reinterpret_cast<const uint4*>(&b) : row_halves(b, scale);
+      if (j < m) *reinterpret_cast<float4*>(p.q + first + j * step) = mul4(run, sm.q[j][lane]);
     }
   }
   if (near) {
@@ -981,16 +903,10 @@ __device__ __noinline__ void delta_chunk_plain(const MbDelta& p, ChunkScanSmem& 
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, H = p.heads, V = p.vdim;
   // rows r and u of this warp's columns take the place of its products: nobody reads those once the group has met below
   float *r = reinterpret_cast<float*>(sm.part[warp]), *u = r + kCh * 16;
-  const bool raw = rec[128] != 0.f;
-  auto with_state = [&](const float* x, float back, float (&y)[2]) {         // x . S over this warp's rows
+  auto with_state = [&](const float* x, float (&y)[2]) {         // x . S over this warp's rows
     y[0] = y[1] = 0.f;
     for (int i = 0; i < 2; ++i) {
-      float4 a = *reinterpret_cast<const float4*>(x + 32 * ks + 16 * i + 4 * t);
-      if (!raw) {
-        const uint4 w = *reinterpret_cast<const uint4*>(&a);
-        const float2 lo = join_h2(w.x, w.z), hi = join_h2(w.y, w.w);
-        a = make_float4(lo.x * back, lo.y * back, hi.x * back, hi.y * back);
-      }
+      const float4 a = *reinterpret_cast<const float4*>(x + 32 * ks + 16 * i + 4 * t);
 #pragma unroll
       for (int e = 0; e < 2; ++e)
         y[e] = fmaf(a.x, S[2 * i][2 * e], fmaf(a.y, S[2 * i][2 * e + 1], fmaf(a.z, S[2 * i + 1][2 * e], fmaf(a.w, S[2 * i + 1][2 * e + 1], y[e]))));
@@ -1004,8 +920,8 @@ __device__ __noinline__ void delta_chunk_plain(const MbDelta& p, ChunkScanSmem& 
   for (int i = 0; i < m; ++i) {
     const size_t at = row + static_cast<size_t>(i) * H;
     float a[2], b[2];
-    with_state(p.k + at * DP, rec[kBack + i], a);
-    with_state(p.q + at * DP, rec[kBack + kCh + i], b);
+    with_state(p.k + at * DP, a);
+    with_state(p.q + at * DP, b);
     if (t < 2) sm.y[i & 1][warp][t][g] = t ? make_float2(b[0], b[1]) : make_float2(a[0], a[1]);
     group_sync(group);
     if (t < 2) {                   // column g + 8 t, by all four warps
@@ -1039,16 +955,7 @@ __device__ __noinline__ void delta_chunk_plain(const MbDelta& p, ChunkScanSmem& 
       S[2 * i][2 * e] *= d.x; S[2 * i][2 * e + 1] *= d.y; S[2 * i + 1][2 * e] *= d.z; S[2 * i + 1][2 * e + 1] *= d.w;
     }
     for (int j = 0; j < m; ++j) {
-      const float* at = p.g + (row + static_cast<size_t>(j) * H) * DP;
-      float4 k;
-      if (raw) {
-        k = *reinterpret_cast<const float4*>(at + c);
-      } else {
-        const uint32_t* w = reinterpret_cast<const uint32_t*>(at) + state_key_word(c);
-        const float2 lo = join_h2(w[0], w[64]), hi = join_h2(w[4], w[68]);
-        const float back = rec[kBack + 2 * kCh + j];
-        k = make_float4(lo.x * back, lo.y * back, hi.x * back, hi.y * back);
-      }
+      const float4 k = state_key(*reinterpret_cast<const float4*>(p.g + (row + static_cast<size_t>(j) * H) * DP + c));
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const float x = u[j * 16 + g + 8 * e];
@@ -1064,23 +971,6 @@ __device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, boo
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src), "r"(on ? 16 : 0)
                : "memory");
 }
-__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint4 ldsm_x4_trans(const void* p) {
-  uint4 r;
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))) : "memory");
-  return r;
-}
-// the same for a fragment row, whose values lie in four lanes
-__device__ __forceinline__ float row_scale(float top, float& back) {
-  top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
-  top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
-  return scale_to(top, 10, back);
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(const __grid_constant__ MbDelta p, int col_blocks, int num_sms) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -1159,17 +1049,9 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(co
       if (c0 + kCh < n) fetch(c0 + kCh);           // travels while this chunk is worked on
       const ChunkStage& in = sm.stage[(c0 / kCh) & 1];
       bool plain = in.rec[128] != 0.f;             // something is not finite
-      float U[2][4];
+      uint32_t uh[2][4], ul[2][4];
       if (!plain) {
         // what the state says about keys and queries: tiles 0, 1 keys of tokens 0-7, 8-15, tiles 2, 3 queries
-        float back[2], to[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          float top = 0.f;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) top = fmaxf(top, fmaxf(fabsf(S[i][2 * e]), fabsf(S[i][2 * e + 1])));
-          to[e] = row_scale(top, back[e]);
-        }
         float Wm[4][4], Wl[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -1177,30 +1059,33 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(co
           for (int e = 0; e < 4; ++e) Wm[i][e] = Wl[i][e] = 0.f;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          // (a0, a1, a2, a3): row g and row g + 8 of the first tile, then of the second
-          uint32_t ah[4], al[4];
-#pragma unroll
-          for (int u = 0; u < 2; ++u)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) split_h2(S[2 * i + u][2 * e] * to[e], S[2 * i + u][2 * e + 1] * to[e], ah[2 * u + e], al[2 * u + e]);
-          uint4 b[4];
+          float4 x[4];
 #pragma unroll
           for (int w = 0; w < 4; ++w)
-            b[w] = *reinterpret_cast<const uint4*>((w < 2 ? in.k : in.q) + ((w & 1) * 8 + g) * kKeyRow + (r0 + 16 * i + 4 * t) * 4);
-          // products that follow one another go to different accumulators
+            x[w] = *reinterpret_cast<const float4*>((w < 2 ? in.k : in.q) + ((w & 1) * 8 + g) * kKeyRow + (r0 + 16 * i + 4 * t) * 4);
 #pragma unroll
-          for (int w = 0; w < 4; ++w) mma_f16(Wm[w], ah, b[w].x, b[w].y);
+          for (int u = 0; u < 2; ++u) {
+            // k index t of these products is row 16 i + 4 t + 2 u, k index t + 4 the next row
+            uint32_t ah[4], al[4], bh[4][2], bl[4][2];
 #pragma unroll
-          for (int w = 0; w < 4; ++w) mma_f16(Wl[w], al, b[w].x, b[w].y);
+            for (int e = 0; e < 4; ++e) split_tf32(S[2 * i + u][e], ah[e], al[e]);
 #pragma unroll
-          for (int w = 0; w < 4; ++w) mma_f16(Wl[w], ah, b[w].z, b[w].w);
+            for (int w = 0; w < 4; ++w) {
+              split_tf32(u ? x[w].z : x[w].x, bh[w][0], bl[w][0]);
+              split_tf32(u ? x[w].w : x[w].y, bh[w][1], bl[w][1]);
+            }
+            // products that follow one another go to different accumulators
+#pragma unroll
+            for (int w = 0; w < 4; ++w) mma_tf32(Wm[w], ah[0], ah[2], ah[1], ah[3], bh[w][0], bh[w][1]);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) mma_tf32(Wl[w], al[0], al[2], al[1], al[3], bh[w][0], bh[w][1]);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) mma_tf32(Wl[w], ah[0], ah[2], ah[1], ah[3], bl[w][0], bl[w][1]);
+          }
         }
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          const float2 f = *reinterpret_cast<const float2*>(in.rec + kBack + 8 * w + 2 * t);      // of tokens 2 t and 2 t + 1
-          sm.part[warp][w][lane] = make_float4((Wm[w][0] + Wl[w][0]) * (f.x * back[0]), (Wm[w][1] + Wl[w][1]) * (f.y * back[0]),
-                                               (Wm[w][2] + Wl[w][2]) * (f.x * back[1]), (Wm[w][3] + Wl[w][3]) * (f.y * back[1]));
-        }
+        for (int w = 0; w < 4; ++w)
+          sm.part[warp][w][lane] = make_float4(Wm[w][0] + Wl[w][0], Wm[w][1] + Wl[w][1], Wm[w][2] + Wl[w][2], Wm[w][3] + Wl[w][3]);
         group_sync(group);
         auto whole = [&](int w) {  // the four warps' parts, always in one order
           const float4 a = sm.part[4 * group][w][lane], b = sm.part[4 * group + 1][w][lane], c = sm.part[4 * group + 2][w][lane],
@@ -1208,7 +1093,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(co
           return make_float4((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y), (a.z + b.z) + (c.z + d.z), (a.w + b.w) + (c.w + d.w));
         };
         // u = M r in all four warps: each needs it for its rows of the state
-        float Ul[2][4];
+        float U[2][4], Ul[2][4];
         float finite = 0.f;
 #pragma unroll
         for (int i = 0; i < 2; ++i)
@@ -1240,7 +1125,8 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(co
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             U[j][e] += Ul[j][e];
-            finite = fmaf(U[j][e], 0.f, finite);
+            split_tf32(U[j][e], uh[j][e], ul[j][e]);
+            finite = fmaf(__uint_as_float(ul[j][e]), 0.f, fmaf(__uint_as_float(uh[j][e]), 0.f, finite));      // NaN may have lost its upper half
           }
         plain = __any_sync(0xffffffffu, finite != 0.f);          // the same in the four warps
         if (!plain && ks < 2) {
@@ -1250,14 +1136,11 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(co
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
             if (j > ks) continue;
-            uint32_t uh[4], ul[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) split_tf32(U[j][e], uh[e], ul[e]);
             const float* base = in.mat + (8 * ks + g) * kMatRow + 2 * kCh + 8 * j + 2 * t;
             const uint2 bh = *reinterpret_cast<const uint2*>(base), bl = *reinterpret_cast<const uint2*>(base + kCh);
-            mma_tf32(Ol, ul[0], ul[2], ul[1], ul[3], bh.x, bh.y);
-            mma_tf32(O, uh[0], uh[2], uh[1], uh[3], bh.x, bh.y);
-            mma_tf32(Ol, uh[0], uh[2], uh[1], uh[3], bl.x, bl.y);
+            mma_tf32(Ol, ul[j][0], ul[j][2], ul[j][1], ul[j][3], bh.x, bh.y);
+            mma_tf32(O, uh[j][0], uh[j][2], uh[j][1], uh[j][3], bh.x, bh.y);
+            mma_tf32(Ol, uh[j][0], uh[j][2], uh[j][1], uh[j][3], bl.x, bl.y);
           }
           const float w[4] = {y.x, y.y, y.z, y.w};
           float* o = p.o + (static_cast<size_t>(t0 + c0 + 8 * ks + 2 * t) * H + h) * V + col0 + g;
@@ -1268,46 +1151,39 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(co
       }
       if (!plain) {
         // S <- diag(b_last) S + sum_j k_j u_j; the sum has its own accumulators, so that S itself is rounded once a chunk
-        float back[2], to[2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const float2 f = *reinterpret_cast<const float2*>(in.rec + kBack + 2 * kCh + 8 * j + 2 * t);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) U[j][e] *= e & 1 ? f.y : f.x;
-        }
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-          to[e] = row_scale(fmaxf(fmaxf(fabsf(U[0][2 * e]), fabsf(U[0][2 * e + 1])), fmaxf(fabsf(U[1][2 * e]), fabsf(U[1][2 * e + 1]))), back[e]);
-        uint32_t uh[4], ul[4];
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) split_h2(U[j][2 * e] * to[e], U[j][2 * e + 1] * to[e], uh[2 * j + e], ul[2 * j + e]);
         float d[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
           for (int e = 0; e < 4; ++e) d[i][e] = 0.f;
-        // four 8 x 8 tiles for one accumulator tile: tokens 0-7 and 8-15, high halves, then low ones
-        uint4 b[4];
-        const uint8_t* rows = in.g + ((lane >> 3 & 1) * 8 + (lane & 7)) * kStateRow + (lane >> 4) * 256 + r0 * 2;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) b[i] = ldsm_x4_trans(rows + i * 16);
+        for (int j = 0; j < 2; ++j) {
+          // rows of the tiles 2 i and 2 i + 1 side by side, of tokens 8 j + 2 t and the next
+          uint32_t bh[4][2], bl[4][2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) mma_f16(d[i], ul, b[i].x, b[i].y);
+          for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) mma_f16(d[i], uh, b[i].z, b[i].w);
+            for (int o = 0; o < 2; ++o) {
+              const float2 x = *reinterpret_cast<const float2*>(in.g + (8 * j + 2 * t + o) * kStateRow + (r0 + 16 * i + 2 * g) * 4);
+              split_tf32(x.x, bh[2 * i][o], bl[2 * i][o]);
+              split_tf32(x.y, bh[2 * i + 1][o], bl[2 * i + 1][o]);
+            }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) mma_f16(d[i], uh, b[i].x, b[i].y);
+          for (int i = 0; i < 4; ++i) mma_tf32(d[i], ul[j][0], ul[j][2], ul[j][1], ul[j][3], bh[i][0], bh[i][1]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) mma_tf32(d[i], uh[j][0], uh[j][2], uh[j][1], uh[j][3], bl[i][0], bl[i][1]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) mma_tf32(d[i], uh[j][0], uh[j][2], uh[j][1], uh[j][3], bh[i][0], bh[i][1]);
+        }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const float4 f = *reinterpret_cast<const float4*>(in.rec + r0 + 16 * i + 4 * t);
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            S[2 * i][2 * e] = fmaf(S[2 * i][2 * e], f.x, d[2 * i][2 * e] * back[e]);
-            S[2 * i][2 * e + 1] = fmaf(S[2 * i][2 * e + 1], f.y, d[2 * i][2 * e + 1] * back[e]);
-            S[2 * i + 1][2 * e] = fmaf(S[2 * i + 1][2 * e], f.z, d[2 * i + 1][2 * e] * back[e]);
-            S[2 * i + 1][2 * e + 1] = fmaf(S[2 * i + 1][2 * e + 1], f.w, d[2 * i + 1][2 * e + 1] * back[e]);
+            S[2 * i][2 * e] = fmaf(S[2 * i][2 * e], f.x, d[2 * i][2 * e]);
+            S[2 * i][2 * e + 1] = fmaf(S[2 * i][2 * e + 1], f.y, d[2 * i][2 * e + 1]);
+            S[2 * i + 1][2 * e] = fmaf(S[2 * i + 1][2 * e], f.z, d[2 * i + 1][2 * e]);
+            S[2 * i + 1][2 * e + 1] = fmaf(S[2 * i + 1][2 * e + 1], f.w, d[2 * i + 1][2 * e + 1]);
           }
         }
       } else {
@@ -1408,8 +1284,9 @@ extern "C" int mb_delta_dim_pad(int dim) {
 }
 
 // Floats of scratch for a step in chunks (records, then rows of pairs); 0 where steps run token by token: fp32 runs, decays per head, shared keys,
-// wider heads, and steps of few tokens a sequence, where most of a chunk would be padding: a layer of 16 heads of 128 x 128 takes 169 us in
-// chunks and 116 token by token for 64 sequences of 17 tokens, 358 and 446 for 64 of 62, 39 and 43 for four of 25.
+// wider heads, and steps of few tokens a sequence, where most of a chunk would be padding: a layer of 16 heads of 128 x 128 takes 359 us in
+// chunks and 381 token by token for 64 sequences of 62 tokens (heads of 100 x 64: 275 and 267), 34 and 40 for one of 40; with 64 of 17 it
+// was 169 and 116 when the operands were fp16 halves.
 extern "C" long long mb_delta_chunk_floats(int T, int B, int heads, int kv_heads, int dim, int vdim, int head_decay, int dtype) {
   if (dtype != kBf16 || head_decay || heads != kv_heads || mb_delta_dim_pad(dim) != 128 || vdim % 4 || T < 40LL * B) return 0;
   return (static_cast<long long>(T) / delta::kCh + B + 1) * heads * delta::kRec + static_cast<long long>(T) * heads * delta::kRowFloats;
