@@ -330,6 +330,24 @@ def test_ssd_segments_leave_rows_before_the_first_sequence(lens):
 
 
 @pytest.mark.gpu
+def test_silu_of_large_negative_inputs():
+    """silu(x) down to where it leaves bf16's normal numbers: 1 + exp(-x) is above 2^126 from -87.4 on, where a fast division gives zero."""
+    dev = "cuda"
+    v = torch.tensor([-88.5, -88.0, -87.5, -87.0, -60.0, -20.0, -1.0, 0.5], device=dev).bfloat16().repeat(20, 1).contiguous()
+    want = (v.double() * torch.sigmoid(v.double()))
+    close = lambda a, b: torch.allclose(a.double(), b, rtol=2 ** -7, atol=0)          # __expf of 88 is good to 2^-15, then a rounding to bf16
+    w = torch.zeros(8, 4, device=dev, dtype=torch.bfloat16)
+    w[:, 3] = 1
+    assert close(ss.causal_conv1d_varlen(v, w, None, _cu([20], dev)), want)
+    y, one = torch.full_like(v, 2.0), torch.ones(8, device=dev, dtype=torch.bfloat16)
+    g = 2 * want
+    assert close(ss.gated_rms_norm(y, v, one, 1e-6), g * (g.square().mean(1, keepdim=True) + 1e-6).rsqrt())
+    zero = torch.zeros_like(v)
+    scan = ss.selective_scan_varlen(one.expand(20, 8).contiguous(), zero, -torch.ones(8, 8, device=dev), zero, zero, torch.ones(8, device=dev), v, None, _cu([20], dev))
+    assert close(scan, want)
+
+
+@pytest.mark.gpu
 def test_ssd_special_inputs_stay_causal():
     """An infinite or NaN input of a prompt changes its own row of the state from its token on, and nothing before it."""
     torch.manual_seed(10)
