@@ -55,6 +55,33 @@ def test_executor_logits_match_fp32_reference(small):
     assert int(got.argmax()) == int(ref.argmax()) or ref.topk(2).values.diff().abs().item() < 0.05
 
 
+@pytest.mark.parametrize("T", [1, 17, 33, 64, 65, 128, 129])
+def test_small_steps_with_norms_in_their_reductions(small, T):
+    """Steps of up to 128 rows hand the norm's factor from layer to layer; a prompt of T tokens and the decode steps after it are as near to
+    the fp32 model as steps that run op by op, up to half as much again (single rows, rounded in other places)."""
+    from tests.test_engine_cpu import eager_logits
+
+    cfg, w = small
+    wc, errs = _cpu_copy(cfg, w), []
+    prompt = np.random.default_rng(T).integers(0, cfg.vocab_size, size=T).tolist()
+    for native in (True, False):
+        llm = _mk(cfg, w, enable_overlap_scheduler=False, device_graph_capture=False, enable_prefix_caching=False)
+        if native:
+            assert llm.model.executor.lean_usable(T) == (T <= 128)
+        llm.model.use_executor = native
+        seen, step = [], llm.model.forward_tensors
+        llm.model.forward_tensors = lambda *a, **kw: seen.append(step(*a, **kw)) or seen[-1]
+        per_step = []
+        for new in (1, 2, 5):
+            rec = llm.generate([prompt], SamplingParams(temperature=0.0, max_new_tokens=new, ignore_eos=True))[0]
+            logits = (llm.model.logits_buf if native else seen[-1])[0].float().cpu()
+            ref = eager_logits(cfg, wc, prompt + list(rec.tokens[: new - 1]))[-1]
+            per_step.append((logits - ref).norm().item() / ref.norm().item())
+        errs.append(per_step)
+    ops.check_device_error()
+    assert max(errs[0]) <= 1.5 * max(errs[1]) and max(errs[0]) < 0.06, errs
+
+
 def test_executor_matches_op_by_op(small):
     cfg, w = small
     rng = np.random.default_rng(1)

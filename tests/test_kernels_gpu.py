@@ -570,6 +570,40 @@ def test_sampler_lists_at_their_limits(rows):
             assert (a != b).sum().item() <= max(1, rows // 66), (crowd, list(kw), a.tolist(), b.tolist())
 
 
+@pytest.mark.parametrize("crowd", [0, 200, 513, 2046, 2047, 2048, 5000])
+def test_sampler_lists_of_single_rows(crowd):
+    """The same limits where a row has a cluster of eight CTAs to itself: 64 rows, one call each. Draws are those of the one-CTA kernel
+    and lie in the kept set in 64 bits."""
+    torch.manual_seed(87)
+    V, rows = 40000, 64
+    seeds, temp = torch.arange(rows, device=DEV, dtype=torch.int64) * 17 + 3, torch.full((rows,), 0.9, device=DEV)
+    lg = torch.randn(rows, V, device=DEV)
+    at = torch.arange(1000, 1000 + crowd, device=DEV) if crowd % 2 else torch.randperm(V, device=DEV)[:crowd]
+    lg[:, at] = 6.0 + (0.0 if crowd == 513 else 0.02) * torch.rand(rows, crowd, device=DEV)
+    x = lg * (1 / temp[:, None])                              # in fp32, as both kernels scale: equal values are one tie
+    mass = (x.double() - x.double().amax(1, keepdim=True)).exp()
+    order = x.argsort(1, descending=True)
+    for k, p, m in [(k, *f) for k in (255, 256, 257, 511, 513) for f in ((1.0, 0.0), (0.7, 1e-3))] + \
+                   [(0, p, 0.0) for p in (0.05, 0.6, 0.95, 0.9999)] + [(0, 1.0, 0.3), (0, 0.5, 0.01)]:
+        kw = dict(temperature=temp, seeds=seeds)
+        kw.update({n: torch.full((rows,), v, device=DEV, dtype=t) for n, v, t, on in (("top_k", k, torch.int32, k > 0),
+                  ("top_p", p, torch.float32, p < 1), ("min_p", m, torch.float32, m > 0)) if on})
+        got = torch.cat([ops.sample(lg[i: i + 1], step=i, **{n: v[i: i + 1] for n, v in kw.items()}) for i in range(rows)])
+        ops.set_sample_cluster(False)
+        want = torch.cat([ops.sample(lg[i: i + 1], step=i, **{n: v[i: i + 1] for n, v in kw.items()}) for i in range(rows)])
+        ops.set_sample_cluster(True)
+        assert (got != want).sum().item() <= 1, (k, p, m, got.tolist(), want.tolist())          # see above: about 1e-5 of a draw each
+        mine, w = x.gather(1, got[:, None]), mass.clone()
+        if k:
+            assert ((x > mine).sum(1) < k).all()
+            w[x < x.gather(1, order[:, k - 1: k])] = 0
+        if m:
+            assert (mass.gather(1, got[:, None]) >= m * (1 - 1e-5)).all()
+            w[mass < m] = 0
+        if p < 1:                                             # what lies above the token holds less than p
+            assert ((w * (x > mine)).sum(1) < (p + 1e-5) * w.sum(1)).all()
+
+
 def test_sampling_without_filters_is_the_same_in_any_batch():
     """Large batches take the kernel of one CTA a row, small ones clusters: a row's draw depends on neither."""
     torch.manual_seed(85)
@@ -1302,6 +1336,54 @@ def test_decode_attention_started_under_the_cache_store(n_kv, hd, lens):
         fn(qkv, out, kv, 1, bt, start, ones, kv_len, None, None, start, n_q, n_kv, hd, hd ** -0.5)
         got.append(out)
     assert got[0].isfinite().all() and torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    ops.check_device_error()
+
+
+@pytest.mark.parametrize("n_kv,hd,lens", [(8, 128, (1, 60, 64, 125, 700)), (2, 64, (1000, 61, 123)), (8, 128, tuple(1 + 37 * i % 300 for i in range(40)))])
+def test_decode_attention_under_the_cache_store_of_captured_steps(n_kv, hd, lens):
+    """Steps of a captured graph, store and attention back to back without a host between them, each reading the rows that the step before
+    it stored: the same bits as without the early start."""
+    from modular_b200._native import lib
+    from modular_b200.nn.rotary_embedding import cos_sin_table
+
+    torch.manual_seed(46)
+    B, n_q, ps, steps = len(lens), 4 * n_kv, 64, 6
+    per = [-(-(n + steps) // ps) for n in lens]
+    order = torch.randperm(sum(per)).tolist()
+    bt = torch.zeros(B, max(per), dtype=torch.int32)
+    for b, n in enumerate(per):
+        bt[b, :n] = torch.tensor([order.pop() for _ in range(n)])
+    ones, start = torch.ones(B, dtype=torch.int32, device=DEV), torch.arange(B, dtype=torch.int32, device=DEV)
+    kv_len = [torch.tensor(lens, dtype=torch.int32) + i for i in range(steps)]
+    slots = [(bt[torch.arange(B), ((n - 1) // ps).long()].long() * ps + (n - 1) % ps).to(DEV) for n in kv_len]
+    pos, kv_len, bt = [(n - 1).to(DEV) for n in kv_len], [n.to(DEV) for n in kv_len], bt.to(DEV)
+    kv0 = torch.randn(sum(per), 2, 1, n_kv, ps, hd, device=DEV).to(torch.bfloat16)
+    qkv0 = torch.randn(steps, B, (n_q + 2 * n_kv) * hd, device=DEV).to(torch.bfloat16)
+    cs = cos_sin_table(hd, 2048, 500000.0, None, DEV)
+    ops.ensure_attention_split_workspace(torch.device(DEV))
+
+    def outputs(fn):
+        kv, qkv = kv0.clone(), qkv0.clone()
+        out = torch.full((steps, B, n_q * hd), float("nan"), device=DEV, dtype=torch.bfloat16)
+
+        def run():
+            for i in range(steps):
+                ops.rope_kv_store(qkv[i], pos[i], slots[i], cs, kv[:, 0, 0], kv[:, 1, 0], n_q, n_kv, hd, False)
+                fn(qkv[i], out[i], kv, 0, bt, start, ones, kv_len[i], None, None, start, n_q, n_kv, hd, hd ** -0.5)
+        run()                                # configures the kernels before the capture
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            run()
+        seen = []
+        for _ in range(20):
+            kv.copy_(kv0), qkv.copy_(qkv0), out.fill_(float("nan"))
+            graph.replay()
+            seen.append(out.clone())
+        return seen
+
+    want = outputs(lib().paged_attention_tma)
+    got = outputs(lib().paged_attention_tma_step)
+    assert want[0].isfinite().all() and all(torch.equal(want[0], o) for o in want + got)
     ops.check_device_error()
 
 
