@@ -349,6 +349,7 @@ extern "C" int mb_rmsnorm(const void* x, const void* w, void* out, int rows, int
                           int ldo, float eps, float weight_offset, int mbc, cudaStream_t stream) {
   if (rows <= 0) return MB_OK;
   if (cols % 8 || ldx % 8 || ldo % 8 || cols > 32768) return MB_ERR_SHAPE;
+  if (cols <= 0) return MB_OK;
   launch_rmsnorm<false>(static_cast<const bf16*>(x), nullptr, static_cast<const bf16*>(w), static_cast<bf16*>(out), rows,
                         cols, ldx, ldo, eps, weight_offset, mbc, stream);
   return MB_LAUNCH_OK();
@@ -359,6 +360,7 @@ extern "C" int mb_add_rmsnorm(const void* x, void* residual, const void* w, void
                               cudaStream_t stream) {
   if (rows <= 0) return MB_OK;
   if (cols % 8 || cols > 32768) return MB_ERR_SHAPE;
+  if (cols <= 0) return MB_OK;
   launch_rmsnorm<true>(static_cast<const bf16*>(x), static_cast<bf16*>(residual), static_cast<const bf16*>(w),
                        static_cast<bf16*>(out), rows, cols, cols, cols, eps, weight_offset, mbc, stream);
   return MB_LAUNCH_OK();

@@ -1402,6 +1402,14 @@ def test_rmsnorm_widths(cols):
     assert torch.equal(res, total) and close(y, exact(total))
 
 
+def test_rmsnorm_of_no_columns():
+    """Rows without columns are no work and no error."""
+    x, w, wide = torch.empty(5, 0, device=DEV, dtype=torch.bfloat16), torch.empty(0, device=DEV, dtype=torch.bfloat16), torch.ones(5, 16, device=DEV, dtype=torch.bfloat16)
+    y, r = ops.add_rms_norm(x, x.clone(), w, 1e-5)
+    assert y.shape == r.shape == (5, 0)
+    assert ops.rms_norm(wide[:, :0], w, 1e-5, out=wide[:, 8:8]).shape == (5, 0) and (wide == 1).all()
+
+
 @pytest.mark.parametrize("interleaved", [False, True])
 @pytest.mark.parametrize("n_q,n_kv,hd", [(1, 1, 16), (40, 8, 128), (5, 3, 80), (6, 2, 256), (70, 1, 64), (1, 1, 4096)])
 def test_rope_heads_of_a_thread(n_q, n_kv, hd, interleaved):
