@@ -458,7 +458,7 @@ sample_kernel(const float* __restrict__ logits, int64_t* __restrict__ out, int v
 // passes), and the draw is a prefix sum over the warps' shares.
 // Masses are integers, so sums do not depend on their order: 42 fractional bits where few weights meet in registers, and
 // per bin the weights relative to the bin's upper edge as 26-bit numbers in two halves, because 32-bit atomics on shared
-// memory are native and 64-bit ones are not (with those 64 nucleus rows took 122 us, with these 101).
+// memory are native and 64-bit ones are not.
 // What bounds it: the chain of a nucleus row. Of its 51 thousand cycles (64 rows, two CTAs an SM) the histogram takes 20, nine
 // cycles an atomic and SM; the passes over the row 6 (from memory) and 9; the rest are barriers of the cluster and round trips
 // between its CTAs, each about one.
@@ -991,7 +991,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
     if (thr > hi_key) thr = hi_key;                        // a min_p above one keeps the maximum alone
     const int kept = __syncthreads_count(tid < n && mykey >= thr);
     if (use_p && kept > 0) {
-      const u64 target = nucleus ? ptarget : portion(tp, sm->sp[kept - 1]);
+      const u64 target = portion(tp, sm->sp[kept - 1]);
       if (tid < kept && incl >= target && incl - mine < target) sm->cut = tid;
       __syncthreads();
       const int r = sm->cut >= 0 ? sm->cut : kept - 1;
