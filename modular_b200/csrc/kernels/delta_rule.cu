@@ -570,24 +570,24 @@ static int scan(const MbDelta& p, int num_sms, cudaStream_t stream) {
 // With b_t the running product of a chunk's decays, S the state before it and L the strictly lower triangle:
 //   A = L(beta_t k_t diag(b_t / b_j) k_j),  u = (1 + A)^-1 beta (v - (b k) S),  o = (b q) S + (q diag(b_t / b_j) k_j, j <= t) u
 //   S <- diag(b_last) S + sum_j (b_last / b_j) k_j u_j
-// b_t / b_j is formed as the product of the decays between them, never as a quotient: nothing overflows, decays of zero stay
-// zeros. delta_chunk_prep_kernel does what needs no state for all chunks at once, two warps a (chunk, head): convolution, norms and
-// decays as above, the products of pairs, the inverse by substitution. delta_chunk_scan_kernel walks a sequence's chunks with S in accumulator fragments: a warp owns 16 columns
-// of one head, which are the M side of every product; the fragments of one product are the operands of the next.
-// An operand x enters a product as two tf32 numbers, x rounded to 11 bits and what is left, of which the unit reads 11 more: together they
-// are within 2^-23 of x, whatever lies beside it, and the product of two such pairs leaves out 2^-22 of itself. (Two fp16 numbers under a
-// power of two per row hold that for the row's largest entries only: where channels of keys and state reached 2^20, entries of the state were
-// off by 8e-5 of their channel, with fast decays by 4e-3; here and token by token by 8e-6 at most.) Keys and queries travel as fp32 rows and are taken apart in registers.
-// 8192 tokens in four prompts of at most 3076, 16 heads of 128 x 128: the scan took 1065 us token by token, 875 in chunks with one warp
-// per 16 columns, 508 with the rows of a column over four warps and the longest sequences first (fp16 halves, half the products: 435): two
-// thirds of a chunk are products (8.2 cycles a scheduler), the rest barriers, the exchange between the four warps and making fragments. The
-// preparation takes 229 us with the products of pairs (270 token by token, without them): its instructions on the 16 warps an SM that rows in
-// shared memory leave.
-// Error of the state against 64 bits, root mean square over its channels, after 300 tokens: 1.2e-6 with decays near one (token by token 1.2e-6),
-// 1.7e-7 without decay (2.2e-7), 1.6e-7 where little outlasts ten tokens (1.3e-7).
+// b_t / b_j is formed as the product of the decays between them where a channel fades far within a chunk: nothing overflows, decays of
+// zero stay zeros. delta_chunk_prep_kernel does what needs no state for all chunks at once, two warps a (chunk, head): convolution, norms and
+// decays as above, the products of pairs, the inverse by substitution. delta_chunk_scan_kernel walks a sequence's chunks with S in accumulator
+// fragments: a warp owns 32 rows of 16 columns of one head; the columns are the M side of every product.
+// Products with S and the sums of k_j u_j run on the tensor cores. Their operands enter as three bf16 numbers, which hold all 24 bits whatever lies beside
+// them, and six of the nine products of such parts are made: what is left out is below 2^-24 of the whole. Operands travel as fp32 and are taken apart in
+// registers. Products with the two small matrices are FMAs, a quarter of the tokens a warp.
+// 8192 tokens in four prompts of at most 3076, 16 heads of 128 x 128, prepared, walked and gated: 792 us, token by token 1381; four prompts of 1000 388
+// and 544, one of 4000 681 and 1265. (Two tf32 numbers and three products an operand hold 23 bits and leave out 2^-22: 373 and 636 us, but outputs 1.3 to
+// 1.5 times as far from their value as token by token. Two fp16 numbers under a power of two per row hold the row's largest entries only. The small matrices
+// on the tensor cores as well: 407 and 714.) What bounds it: the walk's products (8.2 cycles a scheduler), barriers, the exchange between the four warps of
+// a column; the preparation's instructions, on the 16 warps an SM that rows in shared memory leave.
+// Error against 64 bits, root mean square, in parts of that token by token: outputs 0.83 without decay, 0.77 to 0.92 with decays near one, 0.96 with usual
+// ones, 1.1 to 1.2 (1.5e-7 against 1.3e-7) where little outlasts a token, because the units cut sums off where FMAs round. States 0.64, 0.78 to 0.95, 0.94
+// and 0.93 to 1.1.
 constexpr int kCh = 16;
 constexpr int kRec = 132;          // floats of a chunk's record: b_last [128] and a flag (something in the chunk is not finite)
-constexpr int kRowFloats = 4 * kCh;
+constexpr int kRowFloats = 2 * kCh;
 constexpr int kChunkCols = 32;     // columns of a scan CTA
 
 // Chunk records of a step: sequence s has chunks (q_start[s] >> 4) + s + i, which never meet another sequence's.
@@ -620,15 +620,23 @@ struct ChunkPrepPair {
   int near, bad[2], fill;
 };
 
-__device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+__device__ __forceinline__ void mma16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// x as the sum of two tf32 numbers: x rounded to 11 bits, and the first 11 bits of what is left (of either sign; the unit reads no more)
-__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
-  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-  lo = __float_as_uint(x - __uint_as_float(hi));
+// Pair `i` of an operand: x and y as sums of three bf16 numbers each, the next one what the rounding before left. All 24 bits.
+template <int N>
+__device__ __forceinline__ void split(uint32_t (&p)[3][N], int i, float x, float y) {
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[q][i]) : "f"(y), "f"(x));
+    x -= __uint_as_float(p[q][i] << 16);
+    y -= __uint_as_float(p[q][i] & 0xffff0000u);
+  }
 }
+// the products of such parts that count, smallest first: the last one is the main part
+constexpr int kProducts = 6;
+__device__ constexpr int kPartA[kProducts] = {2, 0, 1, 1, 0, 0}, kPartB[kProducts] = {0, 2, 1, 0, 1, 0};
 
 // Loops stay rolled up: a warp runs through every instruction once a chunk, and code that does not fit the instruction cache
 // took 67 us for a single chunk.
@@ -732,15 +740,9 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const __grid_c
   }
   // what meets the state: k_j with the decays behind it, b_t k_t, b_t q_t
   float* rec = p.chunk + (static_cast<size_t>(id) * H + h) * kRec;
-  // a token's row of the inverse and of the query products, each as two halves
+  // a token's row of the inverse and of the query products
   float* rows = p.chunk_rows + (t0 * H + h) * kRowFloats;
   const size_t rstep = static_cast<size_t>(H) * kRowFloats;
-  auto put = [&](float* to, float v) {
-    uint32_t hi, lo;
-    split_tf32(v, hi, lo);
-    to[0] = __uint_as_float(hi);
-    to[kCh] = __uint_as_float(lo);
-  };
   const size_t step = static_cast<size_t>(H) * DP, first = (t0 * H + h) * DP + c;
   {
     bool odd = beta * 0.f != 0.f || finite != 0.f;               // true for NaN
@@ -797,26 +799,21 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const __grid_c
       for (int e = 0; e < 4; ++e) acc[n][e] = low[n][e] = 0.f;
 #pragma unroll 1
     for (int i = 0; i < 8; ++i) {
-      uint32_t bh[2][4], bl[2][4], ah[2][4], al[2][4];
+      uint32_t a[3][4], b[2][3][2];
+      // channels 4 t and 4 t + 1 of the sixteen are neighbours in the products, 4 t + 2 and 4 t + 3 the other two of a lane
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
-        const float4 b = sm.g[8 * n + g][4 * i + t], k = sm.k[8 * n + g][4 * i + t], x = left[8 * n + g][4 * i + t];
+        const float4 d = sm.g[8 * n + g][4 * i + t], k = sm.k[8 * n + g][4 * i + t], x = left[8 * n + g][4 * i + t];
         const bool in = 16 * i + 4 * t < D;
-        split_tf32(in ? __fdividef(k.x, b.x) : 0.f, bh[n][0], bl[n][0]); split_tf32(in ? __fdividef(k.y, b.y) : 0.f, bh[n][1], bl[n][1]);
-        split_tf32(in ? __fdividef(k.z, b.z) : 0.f, bh[n][2], bl[n][2]); split_tf32(in ? __fdividef(k.w, b.w) : 0.f, bh[n][3], bl[n][3]);
-        split_tf32(x.x * b.x, ah[n][0], al[n][0]); split_tf32(x.y * b.y, ah[n][1], al[n][1]);
-        split_tf32(x.z * b.z, ah[n][2], al[n][2]); split_tf32(x.w * b.w, ah[n][3], al[n][3]);
+        split(b[n], 0, in ? __fdividef(k.x, d.x) : 0.f, in ? __fdividef(k.y, d.y) : 0.f);
+        split(b[n], 1, in ? __fdividef(k.z, d.z) : 0.f, in ? __fdividef(k.w, d.w) : 0.f);
+        split(a, n, x.x * d.x, x.y * d.y);
+        split(a, 2 + n, x.z * d.z, x.w * d.w);
       }
-      // channels 4 t and 4 t + 1 of the sixteen in one step, 4 t + 2 and 4 t + 3 in the other
 #pragma unroll
-      for (int u = 0; u < 4; u += 2) {
+      for (int q = 0; q < kProducts; ++q)
 #pragma unroll
-        for (int n = 0; n < 2; ++n) mma_tf32(acc[n], ah[0][u], ah[1][u], ah[0][u + 1], ah[1][u + 1], bh[n][u], bh[n][u + 1]);
-#pragma unroll
-        for (int n = 0; n < 2; ++n) mma_tf32(low[n], al[0][u], al[1][u], al[0][u + 1], al[1][u + 1], bh[n][u], bh[n][u + 1]);
-#pragma unroll
-        for (int n = 0; n < 2; ++n) mma_tf32(low[n], ah[0][u], ah[1][u], ah[0][u + 1], ah[1][u + 1], bl[n][u], bl[n][u + 1]);
-      }
+        for (int n = 0; n < 2; ++n) mma16(q + 1 < kProducts ? low[n] : acc[n], a[kPartA[q]], b[n][kPartB[q]]);
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r)
@@ -829,13 +826,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const __grid_c
         } else {
           if (j > tt) y.x = 0.f;
           if (j + 1 > tt) y.y = 0.f;
-          if (tt < m) {
-            uint2 hi, lo;
-            split_tf32(y.x, hi.x, lo.x);
-            split_tf32(y.y, hi.y, lo.y);
-            *reinterpret_cast<uint2*>(rows + tt * rstep + 2 * kCh + j) = hi;
-            *reinterpret_cast<uint2*>(rows + tt * rstep + 3 * kCh + j) = lo;
-          }
+          if (tt < m) *reinterpret_cast<float2*>(rows + tt * rstep + kCh + j) = y;
         }
       }
   } else {
@@ -852,12 +843,12 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const __grid_c
           if (lane == 0) sm.A[t][j] = y;
         } else {
           if (lane == 0) {
-            put(rows + t * rstep + 2 * kCh + j, y);
-            if (t > j) put(rows + j * rstep + 2 * kCh + t, 0.f);
+            rows[t * rstep + kCh + j] = y;
+            if (t > j) rows[j * rstep + kCh + t] = 0.f;
           }
         }
       }
-      if (role == 1 && lane >= m && lane < kCh) put(rows + j * rstep + 2 * kCh + lane, 0.f);
+      if (role == 1 && lane >= m && lane < kCh) rows[j * rstep + kCh + lane] = 0.f;
     }
   }
   __syncwarp();
@@ -872,14 +863,14 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const __grid_c
         if (j >= lane) sum = fmaf(sm.A[i][j], xi[j], sum);
       const float bi = __shfl_sync(0xffffffffu, beta, i);
       xi[i] = i == lane ? 1.f : i > lane ? -bi * sum : 0.f;
-      if (lane < kCh && i < m) put(rows + i * rstep + lane, i >= lane ? xi[i] * beta : 0.f);
+      if (lane < kCh && i < m) rows[i * rstep + lane] = i >= lane ? xi[i] * beta : 0.f;
     }
   }
   if (lane == 0 && role == 0) rec[128] = bad ? 1.f : 0.f;
 }
 
 constexpr int kScanWarps = 8;      // two groups of 16 columns, four warps each: a warp has 32 of the 128 rows of its columns
-constexpr int kKeyRow = 576, kStateRow = 528, kMatRow = 72, kVRow = kChunkCols + 4;   // bytes, bytes, floats, floats: rows that are read together lie in other banks
+constexpr int kKeyRow = 576, kStateRow = 528, kMatRow = 40, kVRow = kChunkCols + 4, kURow = 24;   // bytes, bytes, then floats: rows that are read together lie in other banks
 struct ChunkStage {
   uint8_t k[kCh * kKeyRow], q[kCh * kKeyRow], g[kCh * kStateRow];
   float mat[kCh * kMatRow], v[kCh * kVRow], rec[kRec];
@@ -887,6 +878,7 @@ struct ChunkStage {
 struct ChunkScanSmem {
   ChunkStage stage[2];
   float4 part[kScanWarps][4][32];                                // what a warp's rows say about keys and queries
+  float u[2][16][kURow];                                         // u of a column group, a row a column
   float2 y[2][kScanWarps][2][8];                                 // delta_chunk_plain: the same for one token
   int seq, fill[3];
 };
@@ -926,10 +918,6 @@ __device__ __noinline__ void delta_chunk_plain(const MbDelta& p, ChunkScanSmem& 
     group_sync(group);
     if (t < 2) {                   // column g + 8 t, by all four warps
       const float* mi = p.chunk_rows + at * kRowFloats;
-      auto both = [&](int j) {     // a low half of an infinity is NaN
-        const float x = mi[j], y = mi[kCh + j];
-        return x * 0.f == 0.f ? x + y : x;
-      };
       const int c = g + 8 * t, col = col0 + c;
       float kx = 0.f, o = 0.f;
       for (int w = 0; w < 4; ++w) {
@@ -939,9 +927,9 @@ __device__ __noinline__ void delta_chunk_plain(const MbDelta& p, ChunkScanSmem& 
       }
       r[i * 16 + c] = (col < V ? p.v[at * V + col] : 0.f) - kx;
       float x = 0.f;
-      for (int j = 0; j <= i; ++j) x = fmaf(both(j), r[j * 16 + c], x);
+      for (int j = 0; j <= i; ++j) x = fmaf(mi[j], r[j * 16 + c], x);
       u[i * 16 + c] = x;
-      for (int j = 0; j <= i; ++j) o = fmaf(both(2 * kCh + j), u[j * 16 + c], o);
+      for (int j = 0; j <= i; ++j) o = fmaf(mi[kCh + j], u[j * 16 + c], o);
       if (ks == 0 && col < V) p.o[at * V + col] = o;
     }
   }
@@ -997,11 +985,11 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(co
   const int t0 = p.q_start[s], n = p.q_len[s], slot = p.state_idx[s];
   const bool resume = slot >= 0 && p.kv_len[s] > n;
   if (n > 0) {
-    // this thread's pieces of a chunk: rows tid / 32 and 8 more of keys and queries, one row of the small matrices and one of the values
-    const int fj = tid >> 5, fc = tid & 31, sj = tid >> 4, sc = (tid & 15) * 4, vj = (tid & 127) >> 3, vc = (tid & 7) * 4;
+    // this thread's pieces of a chunk: rows tid / 32 and 8 more of keys and queries, and one of the values or of the small matrices
+    const int fj = tid >> 5, fc = tid & 31, vj = (tid & 127) >> 3, vc = (tid & 7) * 4;
     const size_t head = static_cast<size_t>(t0) * H + h, half = static_cast<size_t>(8) * H * DP;
     size_t at = (head + static_cast<size_t>(fj) * H) * DP + fc * 4;
-    const float* mat = p.chunk_rows + (head + static_cast<size_t>(sj) * H) * kRowFloats + sc;
+    const float* mat = p.chunk_rows + (head + static_cast<size_t>(vj) * H) * kRowFloats + vc;
     const float* val = p.v + (head + static_cast<size_t>(vj) * H) * V + cbase + vc;
     const float* rec = p.chunk + (static_cast<size_t>(chunk_base(p, s)) * H + h) * kRec + tid * 4;
     auto fetch = [&](int c0) {
@@ -1015,13 +1003,13 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(co
       cp_async16_zfill(d.k + (fj + 8) * kKeyRow + fc * 16, p.k + a1, on8);
       cp_async16_zfill(d.q + (fj + 8) * kKeyRow + fc * 16, p.q + a1, on8);
       cp_async16_zfill(d.g + (fj + 8) * kStateRow + fc * 16, p.g + a1, on8);
-      cp_async16_zfill(d.mat + sj * kMatRow + sc, sj < m ? mat : p.chunk_rows, sj < m);
       if (tid < 128) {
         const bool von = vj < m && cbase + vc < V;
         cp_async16_zfill(d.v + vj * kVRow + vc, von ? val : p.v, von);
-      } else if (tid < 128 + kRec / 4) {
-        cp_async16(d.rec + (tid - 128) * 4, rec - 128 * 4);
+      } else {
+        cp_async16_zfill(d.mat + vj * kMatRow + vc, vj < m ? mat : p.chunk_rows, vj < m);
       }
+      if (tid < kRec / 4) cp_async16(d.rec + tid * 4, rec);
       cp_async_commit();
       at += 2 * half;
       mat += static_cast<size_t>(kCh) * H * kRowFloats;
@@ -1049,7 +1037,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(co
       if (c0 + kCh < n) fetch(c0 + kCh);           // travels while this chunk is worked on
       const ChunkStage& in = sm.stage[(c0 / kCh) & 1];
       bool plain = in.rec[128] != 0.f;             // something is not finite
-      uint32_t uh[2][4], ul[2][4];
+      uint32_t up[3][4];           // u of all sixteen tokens: the left side of two products
       if (!plain) {
         // what the state says about keys and queries: tiles 0, 1 keys of tokens 0-7, 8-15, tiles 2, 3 queries
         float Wm[4][4], Wl[4][4];
@@ -1059,29 +1047,24 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(co
           for (int e = 0; e < 4; ++e) Wm[i][e] = Wl[i][e] = 0.f;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          float4 x[4];
-#pragma unroll
-          for (int w = 0; w < 4; ++w)
-            x[w] = *reinterpret_cast<const float4*>((w < 2 ? in.k : in.q) + ((w & 1) * 8 + g) * kKeyRow + (r0 + 16 * i + 4 * t) * 4);
+          // rows 16 i + 4 t and the next one are neighbours in the products, the two behind them the other two of a lane
+          uint32_t a[3][4], b[4][3][2];
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
-            // k index t of these products is row 16 i + 4 t + 2 u, k index t + 4 the next row
-            uint32_t ah[4], al[4], bh[4][2], bl[4][2];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) split_tf32(S[2 * i + u][e], ah[e], al[e]);
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-              split_tf32(u ? x[w].z : x[w].x, bh[w][0], bl[w][0]);
-              split_tf32(u ? x[w].w : x[w].y, bh[w][1], bl[w][1]);
-            }
-            // products that follow one another go to different accumulators
-#pragma unroll
-            for (int w = 0; w < 4; ++w) mma_tf32(Wm[w], ah[0], ah[2], ah[1], ah[3], bh[w][0], bh[w][1]);
-#pragma unroll
-            for (int w = 0; w < 4; ++w) mma_tf32(Wl[w], al[0], al[2], al[1], al[3], bh[w][0], bh[w][1]);
-#pragma unroll
-            for (int w = 0; w < 4; ++w) mma_tf32(Wl[w], ah[0], ah[2], ah[1], ah[3], bl[w][0], bl[w][1]);
+            split(a, 2 * u, S[2 * i + u][0], S[2 * i + u][1]);
+            split(a, 2 * u + 1, S[2 * i + u][2], S[2 * i + u][3]);
           }
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            const float4 x = *reinterpret_cast<const float4*>((w < 2 ? in.k : in.q) + ((w & 1) * 8 + g) * kKeyRow + (r0 + 16 * i + 4 * t) * 4);
+            split(b[w], 0, x.x, x.y);
+            split(b[w], 1, x.z, x.w);
+          }
+          // products that follow one another go to different accumulators
+#pragma unroll
+          for (int q = 0; q < kProducts; ++q)
+#pragma unroll
+            for (int w = 0; w < 4; ++w) mma16(q + 1 < kProducts ? Wl[w] : Wm[w], a[kPartA[q]], b[w][kPartB[q]]);
         }
 #pragma unroll
         for (int w = 0; w < 4; ++w)
@@ -1092,61 +1075,60 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(co
                        d = sm.part[4 * group + 3][w][lane];
           return make_float4((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y), (a.z + b.z) + (c.z + d.z), (a.w + b.w) + (c.w + d.w));
         };
-        // u = M r in all four warps: each needs it for its rows of the state
-        float U[2][4], Ul[2][4];
-        float finite = 0.f;
+        // Products with the small matrices, in FMAs: warp ks makes tokens 8 (ks / 2) + 2 i + ks % 2, of which lane t ends with i = t, from sixteen
+        // tokens of columns g and g + 8 spread over the lanes of a column (8 j + 2 t and the next)
+        const int tok = 8 * (ks >> 1) + 2 * t + (ks & 1);
+        auto small = [&](const float* mat, const float (&x)[2][4], float (&y)[2]) {
+          float a[4][2], b[2][2];
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+          for (int i = 0; i < 4; ++i) {
+            const float* row = mat + (8 * (ks >> 1) + 2 * i + (ks & 1)) * kMatRow + 2 * t;
+            const float2 lo = *reinterpret_cast<const float2*>(row), hi = *reinterpret_cast<const float2*>(row + 8);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) U[i][e] = Ul[i][e] = 0.f;
+            for (int c = 0; c < 2; ++c) a[i][c] = fmaf(hi.y, x[1][2 * c + 1], fmaf(hi.x, x[1][2 * c], fmaf(lo.y, x[0][2 * c + 1], lo.x * x[0][2 * c])));
+          }
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {              // tokens 8 j + 2 t, + 1 of r
-          const float4 y = whole(j);
-          const float w[4] = {y.x, y.y, y.z, y.w};
-          uint32_t rh[4], rl[4];
+          for (int c = 0; c < 2; ++c) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) b[i][c] = ((t & 2) ? a[2 + i][c] : a[i][c]) + __shfl_xor_sync(0xffffffffu, (t & 2) ? a[i][c] : a[2 + i][c], 2);
+            y[c] = ((t & 1) ? b[1][c] : b[0][c]) + __shfl_xor_sync(0xffffffffu, (t & 1) ? b[0][c] : b[1][c], 1);
+          }
+        };
+        // u = M r, which all four warps need for their rows of the state
+        float U[2][4], y[2];
+        float finite = 0.f;        // 1.01: what would not be finite as a bf16 counts, too
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float4 w = whole(j);
+          const float wj[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const float r = in.v[(8 * j + 2 * t + (e & 1)) * kVRow + lc + g + 8 * (e >> 1)] - w[e];
-            finite = fmaf(r, 0.f, finite);
-            split_tf32(r, rh[e], rl[e]);
-          }
-          // k index t of these products is token 8 j + 2 t, k index t + 4 token 8 j + 2 t + 1
-#pragma unroll
-          for (int i = j; i < 2; ++i) {            // M is lower triangular
-            const float* base = in.mat + (8 * i + g) * kMatRow + 8 * j + 2 * t;
-            const uint2 bh = *reinterpret_cast<const uint2*>(base), bl = *reinterpret_cast<const uint2*>(base + kCh);
-            mma_tf32(Ul[i], rl[0], rl[2], rl[1], rl[3], bh.x, bh.y);
-            mma_tf32(U[i], rh[0], rh[2], rh[1], rh[3], bh.x, bh.y);
-            mma_tf32(Ul[i], rh[0], rh[2], rh[1], rh[3], bl.x, bl.y);
+            U[j][e] = in.v[(8 * j + 2 * t + (e & 1)) * kVRow + lc + g + 8 * (e >> 1)] - wj[e];
+            finite = fmaf(U[j][e] * 1.01f, 0.f, finite);
           }
         }
+        small(in.mat, U, y);
+        sm.u[group][g][tok] = y[0];
+        sm.u[group][g + 8][tok] = y[1];
+        group_sync(group);
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < 2; ++j) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            U[j][e] += Ul[j][e];
-            split_tf32(U[j][e], uh[j][e], ul[j][e]);
-            finite = fmaf(__uint_as_float(ul[j][e]), 0.f, fmaf(__uint_as_float(uh[j][e]), 0.f, finite));      // NaN may have lost its upper half
+          for (int c = 0; c < 2; ++c) {
+            const float2 u = *reinterpret_cast<const float2*>(&sm.u[group][g + 8 * c][8 * j + 2 * t]);
+            finite = fmaf(u.x * 1.01f, 0.f, fmaf(u.y * 1.01f, 0.f, finite));
+            U[j][2 * c] = u.x; U[j][2 * c + 1] = u.y;
+            split(up, 2 * j + c, u.x, u.y);
           }
+        }
         plain = __any_sync(0xffffffffu, finite != 0.f);          // the same in the four warps
-        if (!plain && ks < 2) {
-          // o = q S + Q u: warp 0 tokens 0-7, warp 1 tokens 8-15
-          const float4 y = whole(2 + ks);
-          float O[4] = {0.f, 0.f, 0.f, 0.f}, Ol[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            if (j > ks) continue;
-            const float* base = in.mat + (8 * ks + g) * kMatRow + 2 * kCh + 8 * j + 2 * t;
-            const uint2 bh = *reinterpret_cast<const uint2*>(base), bl = *reinterpret_cast<const uint2*>(base + kCh);
-            mma_tf32(Ol, ul[j][0], ul[j][2], ul[j][1], ul[j][3], bh.x, bh.y);
-            mma_tf32(O, uh[j][0], uh[j][2], uh[j][1], uh[j][3], bh.x, bh.y);
-            mma_tf32(Ol, uh[j][0], uh[j][2], uh[j][1], uh[j][3], bl.x, bl.y);
-          }
-          const float w[4] = {y.x, y.y, y.z, y.w};
-          float* o = p.o + (static_cast<size_t>(t0 + c0 + 8 * ks + 2 * t) * H + h) * V + col0 + g;
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (8 * ks + 2 * t + (e & 1) < m && col0 + g + 8 * (e >> 1) < V) o[(e & 1) * H * V + 8 * (e >> 1)] = w[e] + (O[e] + Ol[e]);
+        if (!plain) {
+          // o = q S + Q u
+          const float4 w = whole(2 + (ks >> 1));
+          small(in.mat + kCh, U, y);
+          float* o = p.o + (static_cast<size_t>(t0 + c0 + tok) * H + h) * V + col0 + g;
+          if (tok < m && col0 + g < V) o[0] = ((ks & 1) ? w.y : w.x) + y[0];
+          if (tok < m && col0 + g + 8 < V) o[8] = ((ks & 1) ? w.w : w.z) + y[1];
         }
       }
       if (!plain) {
@@ -1156,25 +1138,21 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(co
         for (int i = 0; i < 4; ++i)
 #pragma unroll
           for (int e = 0; e < 4; ++e) d[i][e] = 0.f;
+        // rows of the tiles 2 i and 2 i + 1 side by side, of tokens 2 t, 2 t + 1 and 8 more
+        uint32_t b[4][3][2];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          // rows of the tiles 2 i and 2 i + 1 side by side, of tokens 8 j + 2 t and the next
-          uint32_t bh[4][2], bl[4][2];
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
-          for (int i = 0; i < 2; ++i)
+          for (int j = 0; j < 2; ++j) {
+            const uint8_t* at = in.g + (8 * j + 2 * t) * kStateRow + (r0 + 16 * i + 2 * g) * 4;
+            const float2 x = *reinterpret_cast<const float2*>(at), y = *reinterpret_cast<const float2*>(at + kStateRow);
+            split(b[2 * i], j, x.x, y.x);
+            split(b[2 * i + 1], j, x.y, y.y);
+          }
 #pragma unroll
-            for (int o = 0; o < 2; ++o) {
-              const float2 x = *reinterpret_cast<const float2*>(in.g + (8 * j + 2 * t + o) * kStateRow + (r0 + 16 * i + 2 * g) * 4);
-              split_tf32(x.x, bh[2 * i][o], bl[2 * i][o]);
-              split_tf32(x.y, bh[2 * i + 1][o], bl[2 * i + 1][o]);
-            }
+        for (int q = 0; q < kProducts; ++q)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) mma_tf32(d[i], ul[j][0], ul[j][2], ul[j][1], ul[j][3], bh[i][0], bh[i][1]);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) mma_tf32(d[i], uh[j][0], uh[j][2], uh[j][1], uh[j][3], bl[i][0], bl[i][1]);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) mma_tf32(d[i], uh[j][0], uh[j][2], uh[j][1], uh[j][3], bh[i][0], bh[i][1]);
-        }
+          for (int i = 0; i < 4; ++i) mma16(d[i], up[kPartA[q]], b[i][kPartB[q]]);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const float4 f = *reinterpret_cast<const float4*>(in.rec + r0 + 16 * i + 4 * t);

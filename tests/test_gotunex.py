@@ -443,6 +443,63 @@ def test_delta_rule_chunks_whatever_the_channels_reach(reach):
     assert ((state - wstate).abs() / unit).max() < 1.2e-5
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("shift", [0, -3, -6, -30])
+def test_delta_rule_chunks_are_as_exact_as_tokens(shift, monkeypatch):
+    """The fp32 outputs and states of prompts in chunks are no further from 64 bits than token by token: usual decays to none at all. The
+    root mean square over 100 thousand outputs and 64 thousand entries of states, most of which have errors of their own, varies by some
+    percent."""
+    import modular_b200.nn.delta_rule as dr
+
+    native = dr._lib()
+    H, d, dv, lens, parts = 2, 128, 128, [230, 170], {}
+
+    class Native:
+        """The kernels, which leave their fp32 outputs here; token by token if ``chunks`` is off."""
+        chunks, o = True, None
+
+        def delta_chunk_floats(self, *a):
+            return native.delta_chunk_floats(*a) if self.chunks else 0
+
+        def delta_rule(self, *a, **kw):
+            Native.o = a[12][6]
+            native.delta_rule(*a, **kw)
+
+    def change(t, H, d):
+        t["dt_bias"] += shift
+        parts.update(t)
+
+    monkeypatch.setattr(dr, "_lib", Native)
+    errs = []
+    for chunks in (True, False):
+        Native.chunks = chunks
+        (_, state), (_, wstate) = delta_step(lens, H, d, dv, 4, 1, change=change)
+        got = Native.o.view(sum(lens), H, dv).double().cpu()
+        want = torch.cat([torch.stack(o) for o in _delta_outputs(parts, lens, H, d, dv)])
+        errs.append((rel(got, want), rel(state, wstate)))
+    assert all(a <= 1.1 * b for a, b in zip(*errs)), errs
+
+
+def _delta_outputs(t, lens, H, d, dv):
+    """What the mixer of ``delta_step`` norms and gates, in 64 bits, sequence by sequence."""
+    from torch.nn import functional as F
+
+    from modular_b200.nn.delta_rule import delta_step_reference
+
+    t, t0 = {k: v.double() for k, v in t.items()}, 0
+    unit = lambda x: x / torch.sqrt((x * x).sum(-1, keepdim=True) + 1e-6)
+    C, W = 2 * H * d + H * dv, t["conv_w"].shape[1]
+    g = torch.exp(-torch.exp(t["A_log"]).view(1, H, 1) * F.softplus(t["z"] + t["dt_bias"]).view(-1, H, d))
+    for s, n in enumerate(lens):
+        slot = len(lens) - s
+        x = torch.cat([t["conv"][slot].t(), t["px"][t0: t0 + n, :C]])
+        y = F.silu(sum(x[j: j + n] * t["conv_w"][:, j] for j in range(W)))
+        q, k, v = (p.reshape(n, H, -1) for p in y.split([H * d, H * d, H * dv], 1))
+        S, beta = t["state"][slot, :, :, :d].clone(), torch.sigmoid(t["px"][t0: t0 + n, C: C + H])
+        yield [delta_step_reference(unit(q[i]) / d ** 0.5, unit(k[i]), v[i], g[t0 + i], beta[i], S) for i in range(n)]
+        t0 += n
+
+
 @pytest.mark.parametrize("device,dtype", RUNS)
 def test_delta_rule_without_a_slot(device, dtype):
     """Sequences with slot -1 start from zero and keep nothing (the dummies of a padded decode batch)."""
