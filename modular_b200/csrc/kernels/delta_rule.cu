@@ -587,6 +587,7 @@ static int scan(const MbDelta& p, int num_sms, cudaStream_t stream) {
 // and 0.93 to 1.1.
 constexpr int kCh = 16;
 constexpr int kRec = 132;          // floats of a chunk's record: b_last [128] and a flag (something in the chunk is not finite)
+constexpr int kOrder = 130;        // and in the record i of the first head the sequence that is the i-th by length
 constexpr int kRowFloats = 2 * kCh;
 constexpr int kChunkCols = 32;     // columns of a scan CTA
 
@@ -641,13 +642,22 @@ __device__ constexpr int kPartA[kProducts] = {2, 0, 1, 1, 0, 0}, kPartB[kProduct
 // Loops stay rolled up: a warp runs through every instruction once a chunk, and code that does not fit the instruction cache
 // took 67 us for a single chunk.
 template <typename T, int W>
-__global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const __grid_constant__ MbDelta p) {
+__global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const __grid_constant__ MbDelta p, unsigned unit_blocks) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const int pair = threadIdx.x >> 6, role = (threadIdx.x >> 5) & 1, lane = threadIdx.x & 31;
   ChunkPrepPair& sm = reinterpret_cast<ChunkPrepPair*>(smem_raw)[pair];
   auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory"); };
   const int H = p.heads, D = p.dim, V = p.vdim;
   constexpr int DP = 128, kBatch = 4;
+  if (blockIdx.x >= unit_blocks) {                 // the order of the sequences, longest first
+    const int i = (blockIdx.x - unit_blocks) * blockDim.x + threadIdx.x;
+    if (i >= p.B) return;
+    int ahead = 0;
+    const int mine = p.q_len[i];
+    for (int j = 0; j < p.B; ++j) ahead += p.q_len[j] > mine || (p.q_len[j] == mine && j < i);
+    p.chunk[static_cast<size_t>(ahead) * H * kRec + kOrder] = __int_as_float(i);
+    return;
+  }
   const long long unit = static_cast<long long>(blockIdx.x) * 4 + pair;
   const int id = static_cast<int>(unit / H), h = static_cast<int>(unit % H);
   int lo = 0, hi = p.B - 1;
@@ -880,7 +890,6 @@ struct ChunkScanSmem {
   float4 part[kScanWarps][4][32];                                // what a warp's rows say about keys and queries
   float u[2][16][kURow];                                         // u of a column group, a row a column
   float2 y[2][kScanWarps][2][8];                                 // delta_chunk_plain: the same for one token
-  int seq, fill[3];
 };
 static_assert(sizeof(ChunkStage) % 16 == 0 && sizeof(ChunkScanSmem) <= 112 * 1024, "two CTAs an SM");
 
@@ -963,7 +972,7 @@ template <typename T>
 __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(const __grid_constant__ MbDelta p, int col_blocks, int num_sms) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   ChunkScanSmem& sm = *reinterpret_cast<ChunkScanSmem*>(smem_raw);
-  constexpr int DP = 128, NT = kScanWarps * 32;
+  constexpr int DP = 128;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, group = warp >> 2, ks = warp & 3;
   const int H = p.heads, V = p.vdim;
   // The longest sequences first, and where some SMs get a second CTA, the longest to the SMs with one and the shortest beside the
@@ -971,16 +980,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) delta_chunk_scan_kernel(co
   const int per_seq = H * col_blocks, all = gridDim.x, place = blockIdx.x, more = all - num_sms;
   int rank = place;
   if (more > 0 && more <= num_sms) rank = place < more ? num_sms - more + place : place < num_sms ? place - more : all - 1 - (place - num_sms);
-  if (tid == 0) sm.seq = 0;
-  __syncthreads();
-  for (int i = tid; i < p.B; i += NT) {
-    int ahead = 0;
-    const int mine = p.q_len[i];
-    for (int j = 0; j < p.B; ++j) ahead += p.q_len[j] > mine || (p.q_len[j] == mine && j < i);
-    if (ahead == rank / per_seq) sm.seq = i;
-  }
-  __syncthreads();
-  const int s = sm.seq, part = rank % per_seq;
+  const int s = __float_as_int(p.chunk[static_cast<size_t>(rank / per_seq) * H * kRec + kOrder]), part = rank % per_seq;
   const int h = part / col_blocks, cbase = (part % col_blocks) * kChunkCols;
   const int t0 = p.q_start[s], n = p.q_len[s], slot = p.state_idx[s];
   const bool resume = slot >= 0 && p.kv_len[s] > n;
@@ -1206,7 +1206,8 @@ static int chunk_launch(const MbDelta& p, int num_sms, cudaStream_t stream) {
     once.done();
   }
   const long long units = (static_cast<long long>(p.T) / kCh + p.B + 1) * p.heads;
-  if (launch_plain(delta_chunk_prep_kernel<T, W>, dim3(static_cast<unsigned>((units + 3) / 4)), dim3(256), prep, stream, p) != cudaSuccess)
+  const unsigned unit_blocks = static_cast<unsigned>((units + 3) / 4);
+  if (launch_plain(delta_chunk_prep_kernel<T, W>, dim3(unit_blocks + (p.B + 255) / 256), dim3(256), prep, stream, p, unit_blocks) != cudaSuccess)
     return MB_ERR_LAUNCH;
   const int col_blocks = (p.vdim + kChunkCols - 1) / kChunkCols;
   if (launch_plain(delta_chunk_scan_kernel<T>, dim3(p.heads * col_blocks * p.B), dim3(kScanWarps * 32), scan, stream, p, col_blocks, num_sms) != cudaSuccess)
