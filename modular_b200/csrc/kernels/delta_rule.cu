@@ -1263,11 +1263,15 @@ extern "C" int mb_delta_dim_pad(int dim) {
 }
 
 // Floats of scratch for a step in chunks (records, then rows of pairs); 0 where steps run token by token: fp32 runs, decays per head, shared keys,
-// wider heads, and steps of few tokens a sequence, where most of a chunk would be padding: a layer of 16 heads of 128 x 128 takes 359 us in
-// chunks and 381 token by token for 64 sequences of 62 tokens (heads of 100 x 64: 275 and 267), 34 and 40 for one of 40; with 64 of 17 it
-// was 169 and 116 when the operands were fp16 halves.
+// wider heads, and steps of few tokens a sequence, where most of a chunk would be padding. While two CTAs an SM hold all walks, the longest chain is what
+// a step waits for, and chunks win from 40 tokens on (16 heads of 128 x 128, us in chunks and token by token: 1 sequence of 40 tokens 48 and 56, of 1000 190 and
+// 333, 4 of 40 56 and 62). Beyond, walks share the SMs, and the work counts: 16 of 1000 1327 and 1650; with a walk that took 4 % longer 64 of 40 304 and 267, of
+// 100 646 and 617, 128 of 200 2295 and 2344 (heads of 100 x 64, which chunks fill up to 128: 128 of 200 1688 and 1620, 16 of 1000 1101 and 1197). One long
+// prompt beside many rows of one token would gain there, too (2000 beside 40: 409 and 878), but the lengths are on the device.
 extern "C" long long mb_delta_chunk_floats(int T, int B, int heads, int kv_heads, int dim, int vdim, int head_decay, int dtype) {
   if (dtype != kBf16 || head_decay || heads != kv_heads || mb_delta_dim_pad(dim) != 128 || vdim % 4 || T < 40LL * B) return 0;
+  const long long walks = static_cast<long long>(heads) * ((vdim + delta::kChunkCols - 1) / delta::kChunkCols) * B;
+  if (walks > 2 * 148 && T < 256LL * B) return 0;
   return (static_cast<long long>(T) / delta::kCh + B + 1) * heads * delta::kRec + static_cast<long long>(T) * heads * delta::kRowFloats;
 }
 
