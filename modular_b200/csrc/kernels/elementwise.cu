@@ -35,6 +35,46 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
   return t;
 }
 
+// eight values of a row
+__device__ __forceinline__ uint4 add_vectors(uint4 a, uint4 b) {
+  bf162* ap = reinterpret_cast<bf162*>(&a);
+  const bf162* bp = reinterpret_cast<const bf162*>(&b);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 fa = __bfloat1622float2(ap[i]), fb = __bfloat1622float2(bp[i]);
+    ap[i] = __floats2bfloat162_rn(fa.x + fb.x, fa.y + fb.y);
+  }
+  return a;
+}
+
+__device__ __forceinline__ float add_squares(uint4 a, float ss) {
+  const bf162* ap = reinterpret_cast<const bf162*>(&a);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __bfloat1622float2(ap[i]);
+    ss += f.x * f.x + f.y * f.y;
+  }
+  return ss;
+}
+
+__device__ __forceinline__ uint4 norm_vector(uint4 a, uint4 w, float inv, float w_off, int mbc) {
+  bf162* ap = reinterpret_cast<bf162*>(&a);
+  const bf162* wp = reinterpret_cast<const bf162*>(&w);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __bfloat1622float2(ap[i]);
+    const float2 g = __bfloat1622float2(wp[i]);
+    if (mbc) {
+      ap[i] = __floats2bfloat162_rn(f.x * inv * (g.x + w_off), f.y * inv * (g.y + w_off));
+    } else {
+      const bf162 n = __floats2bfloat162_rn(f.x * inv, f.y * inv);
+      const float2 nf = __bfloat1622float2(n);
+      ap[i] = __floats2bfloat162_rn(nf.x * (g.x + w_off), nf.y * (g.y + w_off));
+    }
+  }
+  return a;
+}
+
 // out = rmsnorm(x [+ residual]) * (w + offset). When ADD, residual <- x + residual first.
 // MBC (multiply before cast): Gemma rounding order; otherwise Llama order
 // (normalise, round to bf16, then multiply by the bf16 weight).
@@ -67,21 +107,11 @@ rmsnorm_kernel(const bf16* __restrict__ x, bf16* __restrict__ residual, const bf
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     const int v = threadIdx.x + k * blockDim.x;
-    bf162* ap = reinterpret_cast<bf162*>(&a[k]);
     if (ADD && v < nvec) {
-      const bf162* bp = reinterpret_cast<const bf162*>(&b[k]);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 fa = __bfloat1622float2(ap[i]), fb = __bfloat1622float2(bp[i]);
-        ap[i] = __floats2bfloat162_rn(fa.x + fb.x, fa.y + fb.y);
-      }
+      a[k] = add_vectors(a[k], b[k]);
       *reinterpret_cast<uint4*>(rr + v * 8) = a[k];
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f = __bfloat1622float2(ap[i]);
-      ss += f.x * f.x + f.y * f.y;
-    }
+    ss = add_squares(a[k], ss);
   }
   const float tot = block_sum(ss, scratch);
   const float inv = rsqrtf(tot / static_cast<float>(cols) + eps);
@@ -89,31 +119,54 @@ rmsnorm_kernel(const bf16* __restrict__ x, bf16* __restrict__ residual, const bf
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     const int v = threadIdx.x + k * blockDim.x;
-    if (v >= nvec) continue;
-    bf162* ap = reinterpret_cast<bf162*>(&a[k]);
-    const bf162* wp = reinterpret_cast<const bf162*>(&wv[k]);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f = __bfloat1622float2(ap[i]);
-      const float2 g = __bfloat1622float2(wp[i]);
-      if (mbc) {
-        ap[i] = __floats2bfloat162_rn(f.x * inv * (g.x + w_off), f.y * inv * (g.y + w_off));
-      } else {
-        const bf162 n = __floats2bfloat162_rn(f.x * inv, f.y * inv);
-        const float2 nf = __bfloat1622float2(n);
-        ap[i] = __floats2bfloat162_rn(nf.x * (g.x + w_off), nf.y * (g.y + w_off));
-      }
-    }
-    *reinterpret_cast<uint4*>(orow + v * 8) = a[k];
+    if (v < nvec) *reinterpret_cast<uint4*>(orow + v * 8) = norm_vector(a[k], wv[k], inv, w_off, mbc);
   }
 }
 
-// The number of vectors a thread keeps depends on the width alone, so a row's sum is the same in any batch: one or two up
-// to 128 threads, four up to 256 (widths to 8192), eight beyond.
+// Wide rows: a row waits in shared memory, so that several CTAs an SM overlap one's loads with another's stores.
+template <bool ADD>
+__global__ void __launch_bounds__(256)
+rmsnorm_wide_kernel(const bf16* __restrict__ x, bf16* __restrict__ residual, const bf16* __restrict__ w,
+                    bf16* __restrict__ out, int cols, int ldx, int ldo, float eps, float w_off, int mbc) {
+  __shared__ float scratch[32];
+  extern __shared__ uint4 row_cache[];  // cols / 8 packed values (the summed row)
+  pdl_wait();
+  pdl_trigger();
+  const int row = blockIdx.x;
+  const bf16* xr = x + static_cast<size_t>(row) * ldx;
+  bf16* rr = ADD ? residual + static_cast<size_t>(row) * cols : nullptr;
+  const int nvec = cols >> 3;
+  float ss = 0.f;
+  for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
+    uint4 a = *reinterpret_cast<const uint4*>(xr + v * 8);
+    if (ADD) {
+      a = add_vectors(a, *reinterpret_cast<const uint4*>(rr + v * 8));
+      *reinterpret_cast<uint4*>(rr + v * 8) = a;
+    }
+    ss = add_squares(a, ss);
+    row_cache[v] = a;
+  }
+  const float inv = rsqrtf(block_sum(ss, scratch) / static_cast<float>(cols) + eps);
+  bf16* orow = out + static_cast<size_t>(row) * ldo;
+  for (int v = threadIdx.x; v < nvec; v += blockDim.x)
+    *reinterpret_cast<uint4*>(orow + v * 8) =
+        norm_vector(row_cache[v], *reinterpret_cast<const uint4*>(w + v * 8), inv, w_off, mbc);
+}
+
+// The form depends on the width alone, so a row's sum is the same in any batch. In registers one or two vectors a thread up to 128
+// threads, four up to 256; from 8192 columns on (8200 with a residual) in shared memory, which CTAs of so many registers
+// leave half idle: 12000 rows of 8192 73.5 us (75.8 in registers), of 16384 153 (176 with eight vectors a thread, 201 with four
+// and 512 threads), of 20480 191 (306). Rows that shared memory does not take by itself have eight vectors a thread.
+constexpr int kWideBytes = 48 * 1024 - 128;   // beside the sums
 template <bool ADD>
 static void launch_rmsnorm(const bf16* x, bf16* residual, const bf16* w, bf16* out, int rows, int cols, int ldx, int ldo,
                            float eps, float w_off, int mbc, cudaStream_t stream) {
   const int nvec = cols >> 3;
+  if (cols >= (ADD ? 8200 : 8192) && cols * 2 <= kWideBytes) {
+    launch_k(rmsnorm_wide_kernel<ADD>, dim3(rows), dim3(256), cols * 2, stream, x, residual, w, out, cols, ldx, ldo, eps,
+             w_off, mbc);
+    return;
+  }
   const int nv = nvec <= 128 ? 1 : nvec <= 256 ? 2 : nvec <= 1024 ? 4 : 8;
   const int threads = ((nvec + nv - 1) / nv + 31) / 32 * 32;
   auto kern = nv == 1 ? rmsnorm_kernel<ADD, 1> : nv == 2 ? rmsnorm_kernel<ADD, 2> : nv == 4 ? rmsnorm_kernel<ADD, 4>

@@ -1402,6 +1402,12 @@ def test_rmsnorm_widths(cols):
     assert torch.equal(res, total) and close(y, exact(total))
 
 
+@pytest.mark.parametrize("cols", [8448, 16384, 16392, 24576])
+def test_rmsnorm_wide_rows(cols):
+    """Four vectors a thread up to 512 threads, eight beyond: the same as the narrow ones."""
+    test_rmsnorm_widths(cols)
+
+
 def test_rmsnorm_of_no_columns():
     """Rows without columns are no work and no error."""
     x, w, wide = torch.empty(5, 0, device=DEV, dtype=torch.bfloat16), torch.empty(0, device=DEV, dtype=torch.bfloat16), torch.ones(5, 16, device=DEV, dtype=torch.bfloat16)
