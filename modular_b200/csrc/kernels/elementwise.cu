@@ -285,13 +285,100 @@ __global__ void gather_rows_kernel(const uint8_t* __restrict__ src, const int32_
       *reinterpret_cast<const uint4*>(src + static_cast<size_t>(idx[r]) * ld_src + c);
 }
 
+// Rope and cache store, for steps of few tokens and models of few heads.
 // One thread handles 8 consecutive dims d..d+7 of the first half of a head and the
 // matching 8 dims of the second half (rotate-half convention), or 8 consecutive dims
 // as 4 (even, odd) pairs (interleaved convention). cos_sin is [max_pos, head_dim]:
 // the first head_dim/2 entries of a row are cos, the rest sin.
-// A CTA takes one token, and a thread the same dims of every kStep-th head, kHeads of them in flight: the angles of its dims
-// are loaded once for all heads. One thread a head, with its own 16 loads of angles: 12000 tokens of 32 / 8 heads of 128
-// (46 us of bytes) 87 -> 67 us, 1000 tokens 9.4 -> 6.7 us.
+__global__ void rope_kv_store_item_kernel(bf16* __restrict__ qkv, const int32_t* __restrict__ positions,
+                                     const int64_t* __restrict__ slots,
+                                     const float* __restrict__ cos_sin, bf16* __restrict__ k_cache,
+                                     bf16* __restrict__ v_cache, int T, int n_q, int n_kv,
+                                     int head_dim, int page_size, int64_t page_stride,
+                                     int64_t head_stride, int interleaved) {
+  pdl_wait();
+  pdl_trigger();
+  const int half = head_dim >> 1;
+  const int vec_per_head = half >> 3;           // threads per (token, head) for q/k
+  const int heads_rot = n_q + n_kv;             // heads that get rotated
+  const int work_per_tok = heads_rot * vec_per_head + n_kv * (head_dim >> 3);
+  const size_t gid = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (gid >= static_cast<size_t>(T) * work_per_tok) return;
+  const int t = static_cast<int>(gid / work_per_tok);
+  int w = static_cast<int>(gid % work_per_tok);
+  const int row_elems = (n_q + 2 * n_kv) * head_dim;
+  bf16* row = qkv + static_cast<size_t>(t) * row_elems;
+  const int64_t slot = slots[t];
+  const int64_t page = slot / page_size;
+  const int off = static_cast<int>(slot % page_size);
+
+  if (w >= heads_rot * vec_per_head) {
+    // V copy: 8 dims per thread
+    w -= heads_rot * vec_per_head;
+    const int h = w / (head_dim >> 3), d = (w % (head_dim >> 3)) * 8;
+    if (slot < 0) return;
+    const uint4 v = *reinterpret_cast<const uint4*>(row + (n_q + n_kv + h) * head_dim + d);
+    *reinterpret_cast<uint4*>(v_cache + page * page_stride + h * head_stride +
+                              static_cast<int64_t>(off) * head_dim + d) = v;
+    return;
+  }
+  const int h = w / vec_per_head, d = (w % vec_per_head) * 8;
+  const float* cs = cos_sin + static_cast<size_t>(positions[t]) * head_dim;
+  bf16* hp = row + h * head_dim;
+  uint4 lo, hi;
+  if (!interleaved) {
+    lo = *reinterpret_cast<const uint4*>(hp + d);
+    hi = *reinterpret_cast<const uint4*>(hp + half + d);
+    bf16* l = reinterpret_cast<bf16*>(&lo);
+    bf16* u = reinterpret_cast<bf16*>(&hi);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float c = cs[d + i], s = cs[half + d + i];
+      const float a = __bfloat162float(l[i]), b = __bfloat162float(u[i]);
+      l[i] = __float2bfloat16(a * c - b * s);
+      u[i] = __float2bfloat16(b * c + a * s);
+    }
+  } else {
+    // dims [2d, 2d+16): pairs (2j, 2j+1) use frequency j
+    lo = *reinterpret_cast<const uint4*>(hp + 2 * d);
+    hi = *reinterpret_cast<const uint4*>(hp + 2 * d + 8);
+    bf16* l = reinterpret_cast<bf16*>(&lo);
+    bf16* u = reinterpret_cast<bf16*>(&hi);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float c = cs[d + i], s = cs[half + d + i];
+      float a = __bfloat162float(l[2 * i]), b = __bfloat162float(l[2 * i + 1]);
+      l[2 * i] = __float2bfloat16(a * c - b * s);
+      l[2 * i + 1] = __float2bfloat16(b * c + a * s);
+      c = cs[d + 4 + i]; s = cs[half + d + 4 + i];
+      a = __bfloat162float(u[2 * i]); b = __bfloat162float(u[2 * i + 1]);
+      u[2 * i] = __float2bfloat16(a * c - b * s);
+      u[2 * i + 1] = __float2bfloat16(b * c + a * s);
+    }
+  }
+  if (h < n_q) {
+    if (!interleaved) {
+      *reinterpret_cast<uint4*>(hp + d) = lo;
+      *reinterpret_cast<uint4*>(hp + half + d) = hi;
+    } else {
+      *reinterpret_cast<uint4*>(hp + 2 * d) = lo;
+      *reinterpret_cast<uint4*>(hp + 2 * d + 8) = hi;
+    }
+  } else if (slot >= 0) {
+    bf16* kc = k_cache + page * page_stride + (h - n_q) * head_stride +
+               static_cast<int64_t>(off) * head_dim;
+    if (!interleaved) {
+      *reinterpret_cast<uint4*>(kc + d) = lo;
+      *reinterpret_cast<uint4*>(kc + half + d) = hi;
+    } else {
+      *reinterpret_cast<uint4*>(kc + 2 * d) = lo;
+      *reinterpret_cast<uint4*>(kc + 2 * d + 8) = hi;
+    }
+  }
+}
+
+// The same for steps of hundreds of tokens and models of many heads. A CTA takes one token, and a thread the same dims of
+// every step-th head, kRopeHeads of them in flight: the angles of its dims are loaded once for all heads.
 constexpr int kRopeThreads = 128, kRopeHeads = 4;
 template <bool INTERLEAVED>
 __global__ void __launch_bounds__(kRopeThreads)
@@ -477,6 +564,18 @@ extern "C" int mb_rope_kv_store(void* qkv, const int32_t* positions, const int64
                                 int64_t head_stride, int interleaved, cudaStream_t stream) {
   if (T <= 0) return MB_OK;
   if (head_dim % 16) return MB_ERR_SHAPE;
+  // A CTA a token pays from 300 tokens of 256 such items on. us of a launch in a chain, an item a thread and a CTA a token: 32 / 8
+  // heads of 128 (320 items), 1 token 1.9 and 2.5, 200 2.6 and 2.9, 300 3.1 and 3.0, 1000 5.8 and 4.5, 12000 77 and 62; 24 / 8 of
+  // 128 (256), 300 3.1 and 2.8, 12000 65 and 57; 48 / 8 of 64 (224), 700 3.8 and 3.9, 12000 52 and 51; 16 / 2 of 128 (144), 12000 31 and
+  // 38; 4 / 4 of 64 (32), 12000 9 and 19.
+  const int rot = (n_q + n_kv) * (head_dim / 16);
+  if (T < 300 || rot < 256) {
+    const size_t items = static_cast<size_t>(T) * (rot + n_kv * (head_dim / 8));
+    launch_k(rope_kv_store_item_kernel, dim3(blocks_for(items, 256)), dim3(256), 0, stream, static_cast<bf16*>(qkv), positions,
+             slots, cos_sin, static_cast<bf16*>(k_cache), static_cast<bf16*>(v_cache), T, n_q, n_kv, head_dim, page_size,
+             page_stride, head_stride, interleaved);
+    return MB_LAUNCH_OK();
+  }
   launch_k(interleaved ? rope_kv_store_kernel<true> : rope_kv_store_kernel<false>, dim3(T), dim3(kRopeThreads), 0, stream,
            static_cast<bf16*>(qkv), positions, slots, cos_sin, static_cast<bf16*>(k_cache), static_cast<bf16*>(v_cache),
            n_q, n_kv, head_dim, page_size, page_stride, head_stride);

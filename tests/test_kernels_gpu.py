@@ -1417,6 +1417,29 @@ def test_rmsnorm_of_no_columns():
 
 
 @pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("T", [299, 300])
+@pytest.mark.parametrize("n_q,n_kv,hd", [(30, 2, 128), (29, 2, 128), (70, 1, 64), (1, 1, 4096), (40, 8, 128), (60, 4, 80)])
+def test_rope_on_either_side_of_the_rule(n_q, n_kv, hd, T, interleaved):
+    """From 300 tokens and 256 parts of heads on a CTA takes a token, below a thread a part of a head."""
+    torch.manual_seed(45)
+    ps = 16
+    kv = torch.zeros(20, 2, 1, n_kv, ps, hd, device=DEV, dtype=torch.bfloat16)
+    qkv = torch.randn(T, (n_q + 2 * n_kv) * hd, device=DEV).to(torch.bfloat16)
+    pos = torch.randint(0, 500, (T,), device=DEV, dtype=torch.int32)
+    slots = torch.randperm(20 * ps, device=DEV)[:T].long()
+    slots[3::50] = -1
+    ang = torch.rand(512, hd // 2, device=DEV) * 6.28
+    cos_sin = torch.cat([ang.cos(), ang.sin()], dim=1).contiguous()
+    kv_ref, qkv_ref = kv.clone(), qkv.clone()
+    ops.rope_kv_store(qkv, pos, slots, cos_sin, kv[:, 0, 0], kv[:, 1, 0], n_q, n_kv, hd, interleaved)
+    ref.rope_kv_store(qkv_ref, pos, slots, cos_sin, kv_ref[:, 0, 0], kv_ref[:, 1, 0], n_q, n_kv, hd, interleaved)
+    # one rounding to bf16 each, of sums whose fp32 terms are of order one
+    assert torch.allclose(qkv[:, : n_q * hd].float(), qkv_ref[:, : n_q * hd].float(), rtol=2 ** -7, atol=1e-5)
+    assert torch.allclose(kv.float(), kv_ref.float(), rtol=2 ** -7, atol=1e-5)
+    assert torch.equal(kv[:, 1], kv_ref[:, 1])
+
+
+@pytest.mark.parametrize("interleaved", [False, True])
 @pytest.mark.parametrize("n_q,n_kv,hd", [(1, 1, 16), (40, 8, 128), (5, 3, 80), (6, 2, 256), (70, 1, 64), (1, 1, 4096)])
 def test_rope_heads_of_a_thread(n_q, n_kv, hd, interleaved):
     """Head counts and widths that leave threads without a head, or take several rounds; a skipped row keeps its cache."""
