@@ -721,7 +721,8 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
     add_bins(want, all_in < 0, unit, 0, nclu, c, m);
   };
   // the first bin where the running sum of v reaches `target` (-1: none) and the sum before it
-  auto cross = [&](const u64 (&v)[kOwn], u64 target, int& bin, u64& above) {
+  // (`full` scales what one element of this thread's first bin weighs at most: sm->n then tells how many the bin has at least)
+  auto cross = [&](const u64 (&v)[kOwn], u64 target, int& bin, u64& above, float full = 0.f) {
     if (tid == 0) sm->bin = -1;
     u64 sum = 0, total;
 #pragma unroll
@@ -729,7 +730,11 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
     u64 run = block_before(sum, sm->red, total);
 #pragma unroll
     for (int j = 0; j < kOwn; ++j) {
-      if (run < target && run + v[j] >= target) { sm->bin = tid * kOwn + j; sm->above = run; }
+      if (run < target && run + v[j] >= target) {
+        sm->bin = tid * kOwn + j;
+        sm->above = run;
+        if (full > 0.f) sm->n = static_cast<int>(fminf(__ull2float_rz(v[j]) / (full * static_cast<float>(kStep[j])), 1e9f));
+      }
       run += v[j];
     }
     __syncthreads();
@@ -793,6 +798,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
     // 2b. bins under the maximum
     const double unit = nucleus ? edge(tid * kOwn) : 0.0;
     const bool fresh = nucleus || k > kList / 2;
+    bool fits = false;
     // (the last bin's elements have no weight)
     if (nucleus) histogram(2, -1, unit, fresh, [](float below, uint32_t) { const int b = bin_of(below); return b < kBins - 1 ? b : -1; }, c, m);
     else histogram(1, -1, unit, fresh, [](float below, uint32_t) { return bin_of(below); }, c, m);
@@ -800,7 +806,10 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
     if (nucleus) {
       block_before(m[0] + m[1], sm->red, z_all);
       ptarget = portion(tp, z_all);
-      cross(m, ptarget, last, pabove);
+      // The bin's mass says how many elements it has at least, up to 1/32 too few: more than the list holds would cost a pass for
+      // nothing (flat rows of 128256, T = 5: 74 us for one and 500 for 300, 64 and 408 without that pass).
+      cross(m, ptarget, last, pabove, static_cast<float>(unit) * 67108864.f);
+      fits = last >= 0 && last < kBins - 1 && sm->n < kBinList;
     } else {
       if (use_k) { cross(c, static_cast<u64>(k), kbin, kabove); last = kbin; }
       if (use_m) last = max(last, min_p_bin(mp));
@@ -814,7 +823,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
       if (last >= 0) n = sm->n;
     }
     uint32_t all = 0x7fffffffu;
-    if (nucleus && last >= 0 && last < kBins - 1) {
+    if (fits) {
       // One more pass takes the weight of the bins above the last one, warp by warp, and the last bin's elements, which go to
       // the first CTA: it finds the cut-off among them and draws.
       const float least = under(last);

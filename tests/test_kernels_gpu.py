@@ -604,6 +604,30 @@ def test_sampler_lists_of_single_rows(crowd):
             assert ((w * (x > mine)).sum(1) < (p + 1e-5) * w.sum(1)).all()
 
 
+@pytest.mark.parametrize("rows", [1, 40, 200])           # clusters of 8, 4 and 1
+@pytest.mark.parametrize("V", [2, 511, 512, 513, 6000])
+def test_sampler_of_few_logits_and_of_crowds(V, rows):
+    """Rows about as long as a list; min-p and nuclei that reach more elements than their lists hold."""
+    torch.manual_seed(88)
+    seeds, temp = torch.arange(rows, device=DEV, dtype=torch.int64) * 11 + 1, torch.linspace(0.5, 4.0, rows, device=DEV)
+    f32 = lambda v: torch.full((rows,), v, device=DEV)
+    k = torch.full((rows,), min(300, V - 1), device=DEV, dtype=torch.int32)
+    kws = [dict(top_p=f32(0.9)), dict(top_p=f32(0.5)), dict(min_p=f32(1e-4)), dict(min_p=f32(0.3)), dict(top_k=k), dict(top_k=k // 8 + 2, top_p=f32(0.8)),
+           dict(top_p=f32(0.7), min_p=f32(1e-3))]
+    differ = 0
+    for step in range(8):
+        lg = torch.randn(rows, V, device=DEV)
+        lg[:, step % V] = -float("inf")
+        for kw in kws:
+            a = ops.sample(lg, temperature=temp, seeds=seeds, step=step, **kw)
+            ops.set_sample_cluster(False)
+            b = ops.sample(lg, temperature=temp, seeds=seeds, step=step, **kw)
+            ops.set_sample_cluster(True)
+            assert ((a >= 0) & (a < V)).all()
+            differ += (a != b).sum().item()
+    assert differ <= max(1, 8 * len(kws) * rows // 66), differ          # as above
+
+
 def test_sampling_without_filters_is_the_same_in_any_batch():
     """Large batches take the kernel of one CTA a row, small ones clusters: a row's draw depends on neither."""
     torch.manual_seed(85)
