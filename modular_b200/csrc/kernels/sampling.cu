@@ -776,11 +776,18 @@ sample_cluster_kernel(const float* __restrict__ logits, int64_t* __restrict__ ou
     if (use_m && (last >= 0 || !use_k)) last = max(last, min_p_bin(mp));
     if (last >= 0) {
       const float least = under(last);
-      visit([&](float x, int i) {
-        if (x < least || bin_of(__fsub_rn(mx, x)) > last) return;
-        const uint32_t pos = atomicAdd(&sm->fill, 1u);
-        if (pos < kList) { sm->sx[pos] = x; sm->oi[pos] = i; }
-      });
+      // What min-p reaches may be much more than a list. Lanes that have something to list tell (n elements spread over L lanes leave e^(-n / L)
+      // of them without): from a quarter more than a list on, the pass is not begun, if lanes have eight elements or more. The sum below then
+      // says so to the whole cluster. (min_p 1e-4 on 128256 logits: 64 rows 53 us, 49 without the pass.)
+      if (use_m && seg > 128 && __syncthreads_count(lane_max >= least) > static_cast<int>(kCluThreads * (1.f - __expf(-1.25f / nclu)))) {
+        if (tid == 0) sm->fill = kList + 1;
+      } else {
+        visit([&](float x, int i) {
+          if (x < least || bin_of(__fsub_rn(mx, x)) > last) return;
+          const uint32_t pos = atomicAdd(&sm->fill, 1u);
+          if (pos < kList) { sm->sx[pos] = x; sm->oi[pos] = i; }
+        });
+      }
       cluster_sync_all();
       const uint32_t there = lane < static_cast<int>(nclu) ? ld_cluster_u32(mapa_shared(&sm->fill, lane)) : 0u;
       const uint32_t first = __reduce_add_sync(0xffffffffu, lane < static_cast<int>(rank) ? there : 0u);
