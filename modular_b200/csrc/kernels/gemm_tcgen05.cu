@@ -826,10 +826,13 @@ __device__ __forceinline__ void epilogue_rows(uint32_t tmem_acc, int quad, int l
 constexpr int kMaxRowTiles = 1024;
 // Dense products walk bands of token tiles, a band's tiles of one feature block after another: a round of 74 pairs then reads the tokens of a
 // band and a few feature blocks, which stay in L2, and the weights once a band. With all token tiles to a feature block a round reads
-// all of X (98 MB for 12001 tokens of 4096), from memory and at the price of clock, since long runs sit at the power limit. 12001 tokens
-// through 32 layers of 4096 x 14336: gate/up 2220 us a layer without bands, 1985, 1949, 1958 and 1992 with 6, 12, 16 and 24 tiles, output
-// and down projection together 1580 and 1386 with 12, the prompt 198 and 182.6 ms.
+// all of X (98 MB for 12001 tokens of 4096), from memory and at the price of clock, since long runs sit at the power limit. Half a second of
+// calls each, us without and with bands: 14336 x 2 x 4096 (SwiGLU), 24 tiles 1115 and 1101, 47 tiles 2577 and 2148; 4096 x 14336, 13 tiles 324 and
+// 322, 24 636 and 616, 47 1313 and 1172; 8192 x 28672, 13 tiles 1270 and 1253, 24 2534 and 2367, 47 5574 and 4685. Where X is small beside L2
+// (126 MB), bands only read the weights more often: SwiGLU of 13 tiles of 4096 (27 MB) 596 and 610. 12001 tokens through 32 layers of 4096 x 14336:
+// gate/up 2220 us a layer without bands, 1985, 1949, 1958 and 1992 with 6, 12, 16 and 24 tiles, the prompt 198 and 182.6 ms.
 constexpr int kBandTiles = 12;
+constexpr size_t kBandBytes = 40u << 20;   // X from which on bands are walked
 struct GroupedTail {
   int n_tiles;
   int2 tile[kMaxRowTiles];            // expert, first row
@@ -1421,7 +1424,8 @@ static int launch_pair_xw(const CUtensorMap& tw, const CUtensorMap& tx, void* Y,
   const int total = m_tiles * ((N + tile_n - 1) / tile_n);
   const int clusters = !GROUPED && total < num_sms / 2 ? total : num_sms / 2;
   // bands of equal height, at most kBandTiles
-  const int bands = (m_tiles + kBandTiles - 1) / kBandTiles, band = bands > 1 ? (m_tiles + bands - 1) / bands : (m_tiles > 0 ? m_tiles : 1);
+  const bool banded = static_cast<size_t>(M) * K * 2 > kBandBytes;
+  const int bands = banded ? (m_tiles + kBandTiles - 1) / kBandTiles : 1, band = bands > 1 ? (m_tiles + bands - 1) / bands : (m_tiles > 0 ? m_tiles : 1);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * clusters);
   cfg.blockDim = dim3(kGemmThreads);

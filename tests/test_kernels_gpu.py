@@ -111,6 +111,21 @@ def test_gemm_pair_bands_of_token_tiles(M):
     ops.check_device_error()
 
 
+@pytest.mark.parametrize("M,K", [(3329, 6304), (3329, 6296), (6401, 3280), (9300, 2264)])          # 40 MB of tokens and more, but for the second
+def test_gemm_pair_bands_of_wide_token_tiles(M, K):
+    """Bands are walked where the tokens take a good part of L2: every tile once, the same sums as the one-CTA kernel."""
+    torch.manual_seed(10)
+    N = 2312
+    x = torch.randn(M, K, device=DEV, dtype=torch.bfloat16)
+    w = (torch.randn(N, K, device=DEV) * 0.05).to(torch.bfloat16)
+    y, ys = (torch.full((M, n), float("nan"), device=DEV, dtype=torch.bfloat16) for n in (N, 1152))
+    ops.linear(x, w, out=y, impl="pair")
+    ops.linear_swiglu(x, w[:2304], out=ys, impl="pair")
+    assert torch.equal(y, ops.linear(x, w, impl="tiled"))
+    assert torch.equal(ys, ops.linear_swiglu(x, w[:2304], impl="tiled"))
+    ops.check_device_error()
+
+
 def test_gemm_pair_persistent_swiglu():
     torch.manual_seed(6)
     M, K, I = 2176, 1024, 1536                    # 17 token tiles x 6 row pairs: more tiles than pairs of SMs
