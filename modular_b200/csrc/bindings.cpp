@@ -917,7 +917,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                 "ssd_scan: x [T, H, P], dt [T, H], B/C [T, G, N] bf16, A fp32 [H]");
     const Tensor xr = packed_rows(x, 2), Br = packed_rows(B, 2), Cr = packed_rows(C, 2),
                  dtr = packed_rows(dt.dim() == 2 ? dt : dt.reshape({x.size(0), x.size(1)}), 1);
-    const int n_seqs = cu_seqlens.numel() - 1, seg = mb_ssd_segment(x.size(0), n_seqs, x.size(1), x.size(2));
+    const int n_seqs = cu_seqlens.numel() - 1, seg = mb_ssd_segment(x.size(0), n_seqs, x.size(1), x.size(2), B.size(2));
     Tensor scratch;
     if (seg > 0) scratch = at::empty({(x.size(0) / seg + n_seqs) * x.size(1) * (x.size(2) * B.size(2) + 1)}, x.options().dtype(at::kFloat));
     check_rc(mb_ssd_scan_varlen(xr.data_ptr(), dtr.data_ptr(), A.data_ptr<float>(), Br.data_ptr(), Cr.data_ptr(),

@@ -566,7 +566,7 @@ int mb_ssd_scan_varlen(const void* x, const void* dt, const float* A, const void
                        long long scratch_floats, cudaStream_t stream);
 // Tokens of the segments that long prompts are cut into (0: none). They take (tokens / segment + n_seqs) * H * (P * N + 1) floats of scratch;
 // with less, sequences are walked whole.
-int mb_ssd_segment(int tokens, int n_seqs, int H, int P);
+int mb_ssd_segment(int tokens, int n_seqs, int H, int P, int N);
 int mb_gated_rms_norm(const void* y, const void* z, const void* w, void* out, int T, int D, int ldz, float eps, cudaStream_t stream);
 int mb_apply_token_bitmask(float* logits, const int32_t* bitmask, int rows, int vocab, int ld,
                            cudaStream_t stream);

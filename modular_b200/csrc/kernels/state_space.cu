@@ -1011,10 +1011,12 @@ extern "C" int mb_selective_scan_varlen(const void* u, const void* delta, const 
 
 // Long prompts whose chains do not fill the chip are walked in segments of 512 tokens, or a sixteenth of the step if that is more (the states
 // of all segments lie in scratch): one launch makes every segment's state out of
-// nothing, another walks all segments at once from the states before them. Half of the products are done twice, so it pays where there is about
-// one CTA per SM at most, and sequences are long (80 heads x 64 x 128, us whole and in segments: 4096 tokens in one sequence 355 and 258, in two
-// 245 and 233, in four 192 and 225; 1000 tokens in two 74 and 76).
-extern "C" int mb_ssd_segment(int tokens, int n_seqs, int H, int P) {
+// nothing, another walks all segments at once from the states before them. Half of the products are done twice, so it pays where whole walks leave
+// SMs idle and sequences are long: up to two walks for three SMs, with states of up to 32 columns, whose products weigh less, up to five for four. us
+// whole and in segments, rows of 64: state 128, one sequence of 4096, 80 walks 369 and 265, 100 379 and 316, 111 381 and 334, 128 393 and 397, 160 472
+// and 474 (10000 tokens 1133 and 1232); 1536 tokens, 100 walks 147 and 146, in two sequences 110 145 and 150, four of 2048, 108 walks 180 and 194; state 64, two
+// of 2048, 100 walks 154 and 128, 160 177 and 183; state 32, two of 2048, 160 walks 148 and 134, 184 152 and 142, four of 1536, 184 114 and 115.
+extern "C" int mb_ssd_segment(int tokens, int n_seqs, int H, int P, int N) {
   static int sms = 0;
   if (sms == 0) {
     int dev = 0;
@@ -1022,7 +1024,8 @@ extern "C" int mb_ssd_segment(int tokens, int n_seqs, int H, int P) {
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
   }
   const long long chains = static_cast<long long>(n_seqs) * H * ((P + kNV - 1) / kNV);
-  if (chains * 4 > sms * 5LL || tokens < 1536LL * n_seqs) return 0;
+  if (N <= 32 ? chains * 4 > sms * 5LL : chains * 3 > sms * 2LL) return 0;
+  if (tokens < 1536LL * n_seqs) return 0;
   const int sixteenth = (tokens / 16 + kChunk - 1) / kChunk * kChunk;
   return sixteenth > 512 ? sixteenth : 512;
 }
@@ -1042,7 +1045,7 @@ extern "C" int mb_ssd_scan_varlen(const void* x, const void* dt, const float* A,
     SsdChunk p{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dt), static_cast<const __nv_bfloat16*>(B),
                static_cast<const __nv_bfloat16*>(C), A, Dskip, dt_bias, static_cast<__nv_bfloat16*>(y), ssm_state, cu_seqlens,
                state_idx, has_init, H, P, N, G, ldx, ld_dt, ldb, ldc, dt_softplus, (P + kNV - 1) / kNV, 0, n_seqs, nullptr, nullptr};
-    const int seg = mb_ssd_segment(tokens, n_seqs, H, P);
+    const int seg = mb_ssd_segment(tokens, n_seqs, H, P, N);
     const long long segments = seg > 0 ? static_cast<long long>(tokens) / seg + n_seqs : 0;
     if (seg > 0 && scratch != nullptr && scratch_floats >= segments * H * (static_cast<long long>(P) * N + 1) && segments <= 65535) {
       p.seg = seg;

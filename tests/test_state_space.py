@@ -307,6 +307,13 @@ def test_ssd_segments_continue_kept_states(lens, H, N):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("lens,H,N", [([4097], 110, 128), ([4097, 4097], 80, 24)])
+def test_ssd_segments_on_a_full_chip(lens, H, N):
+    """The most heads that one sequence, and narrow states of two, are cut into segments for: more CTAs than the chip holds at once."""
+    test_ssd_segments_continue_kept_states(lens, H, N)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("lens", [[0, 2000, 1700], [1700, 3000]])
 def test_ssd_segments_leave_rows_before_the_first_sequence(lens):
     """Sequences that begin some segments into the rows: nobody walks the rows before them, and an empty one keeps its state."""
