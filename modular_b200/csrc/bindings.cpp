@@ -902,7 +902,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                       cu_seqlens.data_ptr<int>(),
                                       state_idx.has_value() ? state_idx->data_ptr<int>() : nullptr,
                                       has_init.has_value() ? has_init->data_ptr<int>() : nullptr,
-                                      cu_seqlens.numel() - 1, u.size(1), A.size(1), u.size(1),
+                                      cu_seqlens.numel() - 1, u.size(0), u.size(1), A.size(1), u.size(1),
                                       z.has_value() ? zr.stride(0) : 0, Br.stride(0), Cr.stride(0), dt_softplus ? 1 : 0, cur_stream()),
              "selective_scan_varlen");
   });

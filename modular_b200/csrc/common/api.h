@@ -558,7 +558,7 @@ int mb_causal_conv1d_varlen(const void* x, const void* w, const void* bias, void
 int mb_selective_scan_varlen(const void* u, const void* delta, const float* A, const void* B, const void* C,
                              const float* Dskip, const void* z, const float* dt_bias, void* y, float* ssm_state,
                              const int* cu_seqlens, const int* state_idx, const int* has_init, int n_seqs,
-                             int D, int N, int ld_u, int ld_z, int ld_b, int ld_c, int dt_softplus, cudaStream_t stream);
+                             int tokens, int D, int N, int ld_u, int ld_z, int ld_b, int ld_c, int dt_softplus, cudaStream_t stream);
 int mb_ssd_scan_varlen(const void* x, const void* dt, const float* A, const void* B, const void* C,
                        const float* Dskip, const float* dt_bias, void* y, float* ssm_state,
                        const int* cu_seqlens, const int* state_idx, const int* has_init, int n_seqs, int tokens,

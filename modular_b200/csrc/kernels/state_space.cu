@@ -980,8 +980,8 @@ extern "C" int mb_causal_conv1d_varlen(const void* x, const void* w, const void*
 extern "C" int mb_selective_scan_varlen(const void* u, const void* delta, const float* A, const void* B,
                                         const void* C, const float* Dskip, const void* z, const float* dt_bias,
                                         void* y, float* ssm_state, const int* cu_seqlens, const int* state_idx,
-                                        const int* has_init, int n_seqs, int D, int N, int ld_u, int ld_z, int ld_b,
-                                        int ld_c, int dt_softplus, cudaStream_t stream) {
+                                        const int* has_init, int n_seqs, int tokens, int D, int N, int ld_u, int ld_z,
+                                        int ld_b, int ld_c, int dt_softplus, cudaStream_t stream) {
   if (n_seqs <= 0 || D <= 0) return MB_OK;
   const int vec = D % 8 == 0 && ld_u % 8 == 0 && ld_b % 8 == 0 && ld_c % 8 == 0 && aligned16(u) && aligned16(delta) &&
                   aligned16(B) && aligned16(C) && aligned16(y) && (z == nullptr || (ld_z % 8 == 0 && aligned16(z)));
@@ -989,7 +989,9 @@ extern "C" int mb_selective_scan_varlen(const void* u, const void* delta, const 
   // Four lanes a channel take 40 % fewer instructions per token than eight (wider reads of B and C, one exchange less) but give
   // half the warps; from 2048 warps on they win: 4096 channels, 4099 tokens in 3, 4 and 8 sequences 239, 187 and 145 us against 218,
   // 203 and 184; 2000 tokens in 32 72 against 86, one token of 256 each 95 against 125, 200 in two 14.1 against 13.3.
-  const bool many = static_cast<long long>(D) * n_seqs >= 16384;
+  // With 32 states a lane then has eight, whose chain is longer than the work it saves until sequences have some 32 tokens: one token of 64
+  // each 50.6 against 46.8, 16 of each level, 60 of 16 each 61 against 68 (eight lanes second).
+  const bool many = static_cast<long long>(D) * n_seqs >= 16384 && (N < 32 || tokens >= 32LL * n_seqs);
 #define MB_SCAN(Nv)                                                                                             \
   if (many) MB_SCAN_L(Nv, 4); else MB_SCAN_L(Nv, 8)
 #define MB_SCAN_L(Nv, Lv)                                                                                                \

@@ -199,6 +199,26 @@ def test_selective_scan_is_the_same_in_any_batch(N, D, lead):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("lens", [[31] * 15 + [47], [31] * 16])
+def test_selective_scan_of_32_states_is_the_same_in_any_batch(lens):
+    """Four lanes a channel from 32 tokens a sequence on, eight below and for single sequences: the same states, bit for bit."""
+    torch.manual_seed(20)
+    dev, D, N, T = "cuda", 1024, 32, sum(lens)
+    bf = lambda *s, k=1.0: (torch.randn(*s, device=dev) * k).to(torch.bfloat16)
+    u, delta, z, B, C = bf(T, D), bf(T, D, k=0.5), bf(T, D), bf(T, N), bf(T, N)
+    A, Dk, bias = -torch.rand(D, N, device=dev) * 4 - 0.1, torch.randn(D, device=dev), torch.randn(D, device=dev) * 0.1
+    idx, init = torch.arange(16, dtype=torch.int32, device=dev), torch.ones(16, dtype=torch.int32, device=dev)
+    st = torch.randn(16, D, N, device=dev)
+    one = st.clone()
+    y = ss.selective_scan_varlen(u, delta, A, B, C, Dk, z, bias, _cu(lens, dev), st, idx, init, True)
+    for i, n in enumerate(lens):
+        r = slice(sum(lens[:i]), sum(lens[:i]) + n)
+        w = ss.selective_scan_varlen(u[r], delta[r], A, B[r], C[r], Dk, z[r], bias, _cu([n], dev), one, idx[i: i + 1], init[i: i + 1], True)
+        assert _rel(y[r], w) < 2 ** -9                 # the order of a sum over 32 states, then a rounding to bf16
+    assert torch.equal(st, one)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("H,P,N,G,A0", [(4, 64, 128, 1, 1.0), (6, 32, 64, 2, 16.0), (2, 128, 16, 2, 0.1), (3, 8, 24, 1, 1.0), (2, 16, 40, 2, 4.0),
                                         (2, 4, 16, 1, 1.0), (2, 64, 136, 1, 1.0)])
 def test_ssd_chunks(H, P, N, G, A0):
