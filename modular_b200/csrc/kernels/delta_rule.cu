@@ -580,8 +580,9 @@ static int scan(const MbDelta& p, int num_sms, cudaStream_t stream) {
 // 8192 tokens in four prompts of at most 3076, 16 heads of 128 x 128, prepared, walked and gated: 792 us, token by token 1381; four prompts of 1000 388
 // and 544, one of 4000 681 and 1265. (Two tf32 numbers and three products an operand hold 23 bits and leave out 2^-22: 373 and 636 us, but outputs 1.3 to
 // 1.5 times as far from their value as token by token. Two fp16 numbers under a power of two per row hold the row's largest entries only. The small matrices
-// on the tensor cores as well: 407 and 714.) What bounds it: the walk's products (8.2 cycles a scheduler), barriers, the exchange between the four warps of
-// a column; the preparation's instructions, on the 16 warps an SM that rows in shared memory leave.
+// on the tensor cores as well: 407 and 714.) What bounds it: the walk's chain, which on the SM of the longest prompt uses 74 % of the issue slots, for
+// taking operands apart (ALU 40 % on average) more than for products (tensor pipe 34 %); the preparation's instructions, half of the issue slots of the 15
+// warps an SM that rows in shared memory leave.
 // Error against 64 bits, root mean square, in parts of that token by token: outputs 0.83 without decay, 0.77 to 0.92 with decays near one, 0.96 with usual
 // ones, 1.1 to 1.2 (1.5e-7 against 1.3e-7) where little outlasts a token, because the units cut sums off where FMAs round. States 0.64, 0.78 to 0.95, 0.94
 // and 0.93 to 1.1.
