@@ -194,6 +194,8 @@ int DecoderExecutor::forward_dec(const StepInputs& in, cudaStream_t stream) {
 
 // Steps of few tokens with bf16 weights: norms and rope ride on the split-K reductions. The bound is the rows whose
 // factors the SwiGLU kernel's epilogue holds; it also lies below the first token count of the pair kernels.
+// Decode steps at 1, 64 and 128 rows, time in parts of that without this and without attention's early start: hidden 2048, 8192 wide,
+// 32 / 8 heads of 64 0.84, 0.98, 0.99; 5120, 13824, 40 / 40 of 128 0.90, 0.98, 1.00; 8192, 3584, 8 / 1 of 128 0.76, 0.87, 0.92.
 bool DecoderExecutor::lean_usable(int T) const {
   const DecoderConfig& c = cfg;
   constexpr int kMaxRows = 128;
