@@ -500,6 +500,18 @@ def _delta_outputs(t, lens, H, d, dv):
         t0 += n
 
 
+@pytest.mark.parametrize("T,B,heads,vdim,chunks", [(40, 1, 16, 128, True), (39, 1, 16, 128, False), (160, 4, 16, 128, True), (5 * 255, 5, 16, 128, False),
+                                                   (5 * 256, 5, 16, 128, True), (37 * 40, 37, 2, 128, True), (38 * 40, 38, 2, 128, False), (74 * 40, 74, 4, 32, True)])
+def test_delta_rule_takes_chunks(T, B, heads, vdim, chunks):
+    """Scratch for chunks is asked for where steps run in them: from 40 tokens a sequence on up to 296 walks (a head, 32 columns and a sequence
+    each), beyond from 256 on. It holds a record of 132 floats a chunk and head and two rows of 16 a token."""
+    from modular_b200._native import lib
+
+    n = lib().delta_chunk_floats(T, B, heads, heads, 128, vdim, False, torch.empty(1, dtype=torch.bfloat16))
+    assert n == ((T // 16 + B + 1) * heads * 132 + T * heads * 32 if chunks else 0)
+    assert lib().delta_chunk_floats(T, B, heads, heads, 128, vdim, False, torch.empty(1)) == 0
+
+
 @pytest.mark.parametrize("device,dtype", RUNS)
 def test_delta_rule_without_a_slot(device, dtype):
     """Sequences with slot -1 start from zero and keep nothing (the dummies of a padded decode batch)."""
